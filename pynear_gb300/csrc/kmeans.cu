@@ -20,7 +20,6 @@
 // Hamming assignment, majority vote count > n_c/2, empty clusters re-seeded.
 #include <algorithm>
 #include <cstring>
-#include <limits>
 #include <random>
 #include <vector>
 
@@ -31,99 +30,180 @@
 
 namespace gn {
 
-// ── float seeding ─────────────────────────────────────────────────────────
-__global__ void kpp_update_kernel(const float *__restrict__ X, int64_t n, int d, int dp,
-                                  const float *__restrict__ c, float *__restrict__ min_sq) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float v = fdist<M_L2>(c, X + i * dp, d);
-    v = __fmul_rn(v, v);
-    if (v < min_sq[i]) min_sq[i] = v;
-}
+// ── block reductions of the seeding kernels (256 threads) ─────────────────
+constexpr int KPP_NT = 256;
 
-// Per chunk of min_sq (block b: elements [b * chunk, (b + 1) * chunk)), the sum
-// in double, in a fixed order (thread-strided, then a fixed tree).
-__global__ void __launch_bounds__(256) kpp_partial_kernel(const float *__restrict__ min_sq, int64_t n,
-                                                          int64_t chunk, double *__restrict__ part) {
-    __shared__ double red[256];
-    const int64_t b0 = (int64_t)blockIdx.x * chunk, b1 = min(n, b0 + chunk);
-    double s = 0.0;
-    for (int64_t i = b0 + threadIdx.x; i < b1; i += 256) s += (double)min_sq[i];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) part[blockIdx.x] = red[0];
-}
-
-// k-means++ draw of centroid ci (one block of 1024 threads), the reference's
-// rule (KMeans.hpp:45-70): r = u * sum(min_sq), the first point whose running
-// sum reaches r (n - 1 if none).  The reference sums in double in point order;
-// here the sums are the chunk partials, scanned, then the chosen chunk's
-// elements.  Both orders' running sums lie within 2 (n - 1) 2^-53 total of the
-// exact ones, so when r is farther than twice that from the chosen point's
-// running sums on both sides, the serial order chooses the same point; if not,
-// thread 0 repeats the reference's serial loop (rare).  The chosen row is
-// copied to C[ci].
-__global__ void __launch_bounds__(1024) kpp_pick_kernel(const float *__restrict__ min_sq, int64_t n, int64_t chunk,
-                                                        int P, const double *__restrict__ part, float u,
-                                                        const float *__restrict__ X, int dp, float *__restrict__ C,
-                                                        int64_t ci) {
-    __shared__ double pre[1024], wsum[32];
-    __shared__ int s_b, s_amb, s_found;
-    __shared__ int64_t s_chosen;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    // exclusive scan of the chunk sums (P <= 1024)
-    const double v = t < P ? part[t] : 0.0;
-    double inc = v;
+// Exclusive block-wide scan; *total = the sum of all threads' v.
+template <typename T>
+__device__ __forceinline__ T kpp_block_scan(T v, T *total) {
+    __shared__ T wsum[KPP_NT / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    T inc = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const double y = __shfl_up_sync(0xffffffffu, inc, o);
+        const T y = __shfl_up_sync(0xffffffffu, inc, o);
         if (lane >= o) inc += y;
     }
+    __syncthreads();  // wsum of an earlier call is no longer read
     if (lane == 31) wsum[warp] = inc;
+    __syncthreads();
+    T w = lane < KPP_NT / 32 ? wsum[lane] : T(0);
+#pragma unroll
+    for (int o = 1; o < KPP_NT / 32; o <<= 1) {
+        const T y = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += y;
+    }
+    *total = __shfl_sync(0xffffffffu, w, KPP_NT / 32 - 1);
+    const T before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
+    return (warp > 0 ? before : T(0)) + inc - v;
+}
+
+// True in every thread of the launch's last block to arrive (whose view then
+// holds what the others wrote before they arrived); resets the counter.
+__device__ __forceinline__ bool kpp_last_block(unsigned *done) {
+    __shared__ unsigned s_arrival;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_arrival = atomicAdd(done, 1u);
+    __syncthreads();
+    const bool last = s_arrival == gridDim.x - 1;
+    if (last) {
+        __threadfence();
+        if (threadIdx.x == 0) *done = 0;
+    }
+    return last;
+}
+
+// ── float seeding ─────────────────────────────────────────────────────────
+// One launch per k-means++ draw: every block lowers its chunk's min_sq by the
+// distances to the newest centroid (row ci - 1 of C) and sums the chunk in
+// double; the last block to finish draws centroid ci and copies its row.
+//
+// Two threads per row, each with four of the reference's eight accumulators:
+// a warp's 16-byte loads cover whole 32-byte sectors (a thread per row read
+// 16 bytes of 32 different lines at a time), and the two halves meet in the
+// fold that the reference's order has anyway (lane j + 4 onto lane j).
+//
+// The draw is the reference's rule (KMeans.hpp:45-70): r = u * sum(min_sq), the
+// first point whose running sum reaches r (n - 1 if none).  The reference sums
+// in double in point order; here the sums are the chunk sums, scanned, then
+// the chosen chunk's elements.  Both orders' running sums lie within
+// 2 (n - 1) 2^-53 total of the exact ones, so when r is farther than twice that
+// from the chosen point's running sums on both sides, the serial order chooses
+// the same point; if not, thread 0 repeats the reference's serial loop (rare).
+// What bounds it is the chain of dependent FP64 additions (the unit's latency,
+// not its rate), so every sum is a scan over lanes: 100k x 64, 255 draws:
+// 12.2 ms as three launches with serial sums over the warps' totals, 2.6 ms
+// as this one.
+__global__ void __launch_bounds__(KPP_NT) kpp_kernel(const float *__restrict__ X, int64_t n, int d, int dp,
+                                                     float *__restrict__ C, int64_t ci, float u,
+                                                     float *__restrict__ min_sq, int64_t chunk, int P,
+                                                     double *__restrict__ part, unsigned *__restrict__ done) {
+    const int t = threadIdx.x;
+    const int64_t b0 = (int64_t)blockIdx.x * chunk, b1 = min(n, b0 + chunk);
+    {
+        const int half = t & 1;
+        const int nb = d >> 3, rem = d & 7, dp4 = dp >> 2;
+        const float4 *c4 = reinterpret_cast<const float4 *>(C) + (ci - 1) * dp4;
+        const float4 *x4 = reinterpret_cast<const float4 *>(X);
+        double s = 0.0;
+        for (int64_t i0 = b0; i0 < b1; i0 += KPP_NT / 2) {
+            const int64_t i = i0 + (t >> 1);
+            const bool in = i < b1;
+            const float4 *xr = x4 + (in ? i : b0) * dp4 + half;
+            float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll 8
+            for (int c = 0; c < nb; ++c) {
+                const float4 x = xr[2 * c], q = c4[2 * c + half];
+                const float t0 = __fsub_rn(q.x, x.x), t1 = __fsub_rn(q.y, x.y);
+                const float t2 = __fsub_rn(q.z, x.z), t3 = __fsub_rn(q.w, x.w);
+                a0 = __fmaf_rn(t0, t0, a0);
+                a1 = __fmaf_rn(t1, t1, a1);
+                a2 = __fmaf_rn(t2, t2, a2);
+                a3 = __fmaf_rn(t3, t3, a3);
+            }
+            float s0 = __fadd_rn(a0, __shfl_xor_sync(0xffffffffu, a0, 1));
+            float s1 = __fadd_rn(a1, __shfl_xor_sync(0xffffffffu, a1, 1));
+            float s2 = __fadd_rn(a2, __shfl_xor_sync(0xffffffffu, a2, 1));
+            float s3 = __fadd_rn(a3, __shfl_xor_sync(0xffffffffu, a3, 1));
+            // the 4-wide step and the masked remainder (rows are zero padded past d)
+            for (int w = 0; 4 * w < rem; ++w) {
+                const float4 x = x4[(in ? i : b0) * dp4 + 2 * nb + w], q = c4[2 * nb + w];
+                const float t0 = __fsub_rn(q.x, x.x), t1 = __fsub_rn(q.y, x.y);
+                const float t2 = __fsub_rn(q.z, x.z), t3 = __fsub_rn(q.w, x.w);
+                s0 = __fmaf_rn(t0, t0, s0);
+                s1 = __fmaf_rn(t1, t1, s1);
+                s2 = __fmaf_rn(t2, t2, s2);
+                s3 = __fmaf_rn(t3, t3, s3);
+            }
+            if (in && half == 0) {
+                const float r = __fsqrt_rn(__fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3)));
+                const float v = __fmul_rn(r, r);
+                float m = ci == 1 ? 3.402823466e+38f : min_sq[i];
+                if (v < m || ci == 1) {
+                    m = v < m ? v : m;
+                    min_sq[i] = m;
+                }
+                s += (double)m;
+            }
+        }
+        double tot;
+        kpp_block_scan(s, &tot);
+        if (t == 0) part[blockIdx.x] = tot;
+    }
+    if (!kpp_last_block(done)) return;
+
+    __shared__ int s_b, s_amb, s_found;
+    __shared__ double s_base;
+    __shared__ unsigned long long s_chosen;
     if (t == 0) {
         s_b = P;
         s_amb = 0;
         s_found = 0;
-        s_chosen = n - 1;
+        s_base = 0.0;
+        s_chosen = (unsigned long long)(n - 1);
     }
-    __syncthreads();
-    double wb = 0.0;
-    for (int w = 0; w < warp; ++w) wb += wsum[w];
-    pre[t] = wb + inc - v;
-    double total = 0.0;
-    for (int w = 0; w < 32; ++w) total += wsum[w];
+    // the chunk that holds the point: every thread walks a contiguous span of chunk sums
+    const int span = (P + KPP_NT - 1) / KPP_NT;
+    const int p0 = min(P, t * span), p1 = min(P, p0 + span);
+    double own = 0.0;
+    for (int p = p0; p < p1; ++p) own += __ldcg(part + p);
+    double total;
+    const double pre = kpp_block_scan(own, &total);
     const double r = (double)u * total;
     const double band = 4.0 * (double)n * 1.1102230246251565e-16 * total;  // 2 x 2 (n - 1) 2^-53 total, rounded up
-    __syncthreads();
-    if (t < P && pre[t] + v >= r) atomicMin(&s_b, t);
+    int mine = P;
+    double mbase = 0.0;
+    {
+        double cum = pre;
+        for (int p = p0; p < p1; ++p) {
+            const double nx = cum + __ldcg(part + p);
+            if (nx >= r) {
+                mine = p;
+                mbase = cum;
+                break;
+            }
+            cum = nx;
+        }
+    }
+    if (mine < P) atomicMin(&s_b, mine);
     __syncthreads();
     const int b = s_b;
+    if (b < P && mine == b) s_base = mbase;
+    __syncthreads();
     if (b < P) {
         // running sums inside chunk b: each thread takes a contiguous piece
         const int64_t c0 = (int64_t)b * chunk, c1 = min(n, c0 + chunk);
-        const int64_t per = (c1 - c0 + 1023) / 1024;
-        const int64_t p0 = min(c1, c0 + t * per), p1 = min(c1, p0 + per);
+        const int64_t per = (c1 - c0 + KPP_NT - 1) / KPP_NT;
+        const int64_t e0 = min(c1, c0 + t * per), e1 = min(c1, e0 + per);
         double ls = 0.0;
-        for (int64_t i = p0; i < p1; ++i) ls += (double)min_sq[i];
-        double li = ls;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, li, o);
-            if (lane >= o) li += y;
-        }
-        if (lane == 31) wsum[warp] = li;
-        __syncthreads();
-        double base = pre[b];
-        for (int w = 0; w < warp; ++w) base += wsum[w];
-        double cum = base + li - ls;  // running sum before this thread's piece
+        for (int64_t i = e0; i < e1; ++i) ls += (double)__ldcg(min_sq + i);
+        double lt;
+        double cum = s_base + kpp_block_scan(ls, &lt);  // running sum before this thread's piece
         int64_t found = -1;
         double before = 0.0, at = 0.0;
-        for (int64_t i = p0; i < p1; ++i) {
-            const double nx = cum + (double)min_sq[i];
+        for (int64_t i = e0; i < e1; ++i) {
+            const double nx = cum + (double)__ldcg(min_sq + i);
             if (nx >= r) {
                 found = i;
                 before = cum;
@@ -134,11 +214,11 @@ __global__ void __launch_bounds__(1024) kpp_pick_kernel(const float *__restrict_
         }
         // the first piece holding the point: pieces are ordered, so the lowest index wins
         if (found >= 0) {
-            atomicMin(reinterpret_cast<unsigned long long *>(&s_chosen), (unsigned long long)found);
+            atomicMin(&s_chosen, (unsigned long long)found);
             s_found = 1;
         }
         __syncthreads();
-        if (found >= 0 && found == s_chosen && !(at - r > band && r - before > band)) s_amb = 1;
+        if (found >= 0 && (unsigned long long)found == s_chosen && !(at - r > band && r - before > band)) s_amb = 1;
         // the chunk's elements summed in this order fell short of r: the serial rule decides
         if (t == 0 && !s_found) s_amb = 1;
     } else if (t == 0) {
@@ -147,27 +227,22 @@ __global__ void __launch_bounds__(1024) kpp_pick_kernel(const float *__restrict_
     __syncthreads();
     if (s_amb && t == 0) {
         double tot = 0.0;
-        for (int64_t i = 0; i < n; ++i) tot += (double)min_sq[i];
+        for (int64_t i = 0; i < n; ++i) tot += (double)__ldcg(min_sq + i);
         const double rr = (double)u * tot;
         double c = 0.0;
         int64_t ch = n - 1;
         for (int64_t i = 0; i < n; ++i) {
-            c += (double)min_sq[i];
+            c += (double)__ldcg(min_sq + i);
             if (c >= rr) {
                 ch = i;
                 break;
             }
         }
-        s_chosen = ch;
+        s_chosen = (unsigned long long)ch;
     }
     __syncthreads();
-    const int64_t ch = s_chosen;
-    for (int j = t; j < dp; j += 1024) C[ci * dp + j] = X[ch * dp + j];
-}
-
-__global__ void fill_float_kernel(float *p, int64_t n, float v) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
+    const int64_t ch = (int64_t)s_chosen;
+    for (int j = t; j < dp; j += KPP_NT) C[ci * dp + j] = X[ch * dp + j];
 }
 
 // ── row norms ─────────────────────────────────────────────────────────────
@@ -242,9 +317,13 @@ __global__ void __launch_bounds__(GT_THREADS) kmeans_assign_kernel(const float *
 }
 
 // ── float update: FP64 sums ───────────────────────────────────────────────
+// (this kernel and the next do nothing when no label changed, so that the host
+// can launch a whole iteration before it reads the change count)
 __global__ void kmeans_accumulate_kernel(const float *__restrict__ X, int64_t n, int d, int dp,
-                                         const int32_t *__restrict__ labels, double *__restrict__ sums,
+                                         const int32_t *__restrict__ labels,
+                                         const unsigned long long *__restrict__ n_changed, double *__restrict__ sums,
                                          int64_t *__restrict__ counts) {
+    if (*n_changed == 0) return;
     const int64_t p = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (p >= n) return;
@@ -254,7 +333,9 @@ __global__ void kmeans_accumulate_kernel(const float *__restrict__ X, int64_t n,
 }
 
 __global__ void kmeans_finalize_kernel(const double *__restrict__ sums, const int64_t *__restrict__ counts, int k,
-                                       int d, int dp, float *__restrict__ C) {
+                                       int d, int dp, const unsigned long long *__restrict__ n_changed,
+                                       float *__restrict__ C) {
+    if (*n_changed == 0) return;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= (int64_t)k * dp) return;
     const int c = (int)(t / dp), j = (int)(t % dp);
@@ -272,52 +353,46 @@ int kmeans_l2_device(const float *X, int64_t n, int d, int dp, int64_t k, int64_
     // k-means++ seeding, all on the device: the reference's draws (the first
     // point, then one uniform per further centroid) do not depend on the data,
     // so they are taken from the mt19937 stream up front in the reference's
-    // order; each further centroid is then picked by kpp_pick_kernel
+    // order; each further centroid is one kpp_kernel launch
     GN_CUDA_TRY(cudaMemcpyAsync(C, X + pick_point(rng) * dp, row_bytes, cudaMemcpyDeviceToDevice, st));
-    std::vector<float> draws((size_t)std::max<int64_t>(k, 1));
-    for (int64_t ci = 1; ci < k; ++ci) draws[(size_t)ci] = unif01(rng);
-    DBuf dmin, dpart;
+    DBuf dmin, dpart, ddone;
     GN_TRY(dmin.ensure((size_t)n * sizeof(float)));
-    const int64_t chunk = std::max<int64_t>(256, ceil_div(n, 1024));
-    const int P = (int)ceil_div(n, chunk);  // <= 1024 chunk sums
+    // a block of 256 threads takes 128 rows a step; at most 1024 chunk sums
+    const int64_t chunk = std::max<int64_t>(KPP_NT / 2, round_up(ceil_div(n, 1024), KPP_NT / 2));
+    const int P = (int)ceil_div(n, chunk);
     GN_TRY(dpart.ensure((size_t)P * sizeof(double)));
-    const unsigned nb = (unsigned)ceil_div(n, 256);
-    fill_float_kernel<<<nb, 256, 0, st>>>(dmin.as<float>(), n, std::numeric_limits<float>::max());
-    for (int64_t ci = 1; ci < k; ++ci) {
-        kpp_update_kernel<<<nb, 256, 0, st>>>(X, n, d, dp, C + (ci - 1) * dp, dmin.as<float>());
-        kpp_partial_kernel<<<(unsigned)P, 256, 0, st>>>(dmin.as<float>(), n, chunk, dpart.as<double>());
-        kpp_pick_kernel<<<1, 1024, 0, st>>>(dmin.as<float>(), n, chunk, P, dpart.as<double>(), draws[(size_t)ci], X,
-                                            dp, C, ci);
-    }
+    GN_TRY(ddone.ensure(sizeof(unsigned)));
+    GN_CUDA_TRY(cudaMemsetAsync(ddone.p, 0, sizeof(unsigned), st));
+    for (int64_t ci = 1; ci < k; ++ci)
+        kpp_kernel<<<(unsigned)P, KPP_NT, 0, st>>>(X, n, d, dp, C, ci, unif01(rng), dmin.as<float>(), chunk, P,
+                                                   dpart.as<double>(), ddone.as<unsigned>());
     GN_CUDA_TRY(cudaGetLastError());
 
-    // Lloyd iterations
-    DBuf dsum, dcnt, dchg;
+    // Lloyd iterations; one host synchronisation each (the change count and the
+    // cluster sizes together)
+    DBuf dsum, dstat;
     GN_TRY(dsum.ensure((size_t)k * dp * sizeof(double)));
-    GN_TRY(dcnt.ensure((size_t)k * sizeof(int64_t)));
-    GN_TRY(dchg.ensure(sizeof(unsigned long long)));
+    GN_TRY(dstat.ensure((size_t)(k + 1) * sizeof(int64_t)));  // change count, then rows per cluster
+    unsigned long long *dchg = dstat.as<unsigned long long>();
+    int64_t *dcnt = dstat.as<int64_t>() + 1;
     GN_CUDA_TRY(cudaMemsetAsync(labels, 0, (size_t)n * sizeof(int32_t), st));
-    std::vector<int64_t> hcnt((size_t)k);
+    std::vector<int64_t> hstat((size_t)k + 1);
     int64_t it = 0;
     for (; it < max_iter; ++it) {
         row_norms_kernel<<<(unsigned)ceil_div(k, 8), 256, 0, st>>>(C, k, dp, cnorm);
-        GN_CUDA_TRY(cudaMemsetAsync(dchg.p, 0, sizeof(unsigned long long), st));
-        kmeans_assign_kernel<<<(unsigned)ceil_div(n, GT_BM), GT_THREADS, 0, st>>>(
-            X, n, dp, C, cnorm, (int)k, labels, dchg.as<unsigned long long>());
-        unsigned long long changed = 0;
-        GN_CUDA_TRY(cudaMemcpyAsync(&changed, dchg.p, sizeof(changed), cudaMemcpyDeviceToHost, st));
-        GN_CUDA_TRY(cudaStreamSynchronize(st));
-        if (changed == 0) break;
+        GN_CUDA_TRY(cudaMemsetAsync(dstat.p, 0, hstat.size() * sizeof(int64_t), st));
         GN_CUDA_TRY(cudaMemsetAsync(dsum.p, 0, (size_t)k * dp * sizeof(double), st));
-        GN_CUDA_TRY(cudaMemsetAsync(dcnt.p, 0, (size_t)k * sizeof(int64_t), st));
-        kmeans_accumulate_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, st>>>(X, n, d, dp, labels, dsum.as<double>(),
-                                                                          dcnt.as<int64_t>());
-        kmeans_finalize_kernel<<<(unsigned)ceil_div(k * dp, 256), 256, 0, st>>>(dsum.as<double>(),
-                                                                              dcnt.as<int64_t>(), (int)k, d, dp, C);
-        GN_CUDA_TRY(cudaMemcpyAsync(hcnt.data(), dcnt.p, (size_t)k * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+        kmeans_assign_kernel<<<(unsigned)ceil_div(n, GT_BM), GT_THREADS, 0, st>>>(X, n, dp, C, cnorm, (int)k, labels,
+                                                                                  dchg);
+        kmeans_accumulate_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, st>>>(X, n, d, dp, labels, dchg,
+                                                                          dsum.as<double>(), dcnt);
+        kmeans_finalize_kernel<<<(unsigned)ceil_div(k * dp, 256), 256, 0, st>>>(dsum.as<double>(), dcnt, (int)k, d, dp,
+                                                                              dchg, C);
+        GN_CUDA_TRY(cudaMemcpyAsync(hstat.data(), dstat.p, hstat.size() * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
         GN_CUDA_TRY(cudaStreamSynchronize(st));
+        if (hstat[0] == 0) break;
         for (int64_t c = 0; c < k; ++c)
-            if (hcnt[(size_t)c] == 0)
+            if (hstat[(size_t)c + 1] == 0)
                 GN_CUDA_TRY(cudaMemcpyAsync(C + c * dp, X + pick_point(rng) * dp, row_bytes,
                                             cudaMemcpyDeviceToDevice, st));
     }
@@ -332,61 +407,133 @@ void row_norms(const float *X, int64_t n, int dp, float *out, cudaStream_t st) {
 }
 
 // ── binary k-means ────────────────────────────────────────────────────────
-__global__ void bin_kpp_update_kernel(const uint4 *__restrict__ X, int64_t n, int w4, const uint4 *__restrict__ c,
-                                      int64_t *__restrict__ min_d) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int64_t v = hdist(c, X + i * w4, w4);
-    if (v < min_d[i]) min_d[i] = v;
-}
-
-__global__ void fill_i64_kernel(int64_t *p, int64_t n, int64_t v) {
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
-}
-
-constexpr int SCAN_CHUNK = 4096;
-
-// per-chunk sums of min_d (exact int64)
-__global__ void chunk_sum_kernel(const int64_t *__restrict__ v, int64_t n, int64_t *__restrict__ sums) {
-    __shared__ int64_t red[32];
-    const int64_t base = (int64_t)blockIdx.x * SCAN_CHUNK;
-    int64_t s = 0;
-    for (int i = threadIdx.x; i < SCAN_CHUNK; i += blockDim.x)
-        if (base + i < n) s += v[base + i];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+// The point of the running sums: the first index i with min_d[0] + .. +
+// min_d[i] > r (0 <= r < total), exact in int64, by one block: sums holds the
+// sums of P chunks of `chunk` rows, pre this thread's running sum before its
+// span of them.  Writes row i of X to C[ci].
+__device__ __forceinline__ void bin_pick(const uint4 *__restrict__ X, int64_t n, int w4, uint4 *C, int64_t ci,
+                                         const int32_t *min_d, int64_t chunk, int P, const int64_t *sums, int64_t r,
+                                         int64_t pre) {
+    __shared__ int s_chunk;
+    __shared__ int64_t s_before, s_row;
+    const int t = threadIdx.x;
+    const int span = (P + KPP_NT - 1) / KPP_NT;
+    const int p0 = min(P, t * span), p1 = min(P, p0 + span);
+    if (t == 0) {  // in range whatever r is
+        s_chunk = 0;
+        s_before = 0;
+        s_row = 0;
+    }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-        sums[blockIdx.x] = t;
+    int64_t cum = pre;
+    for (int p = p0; p < p1; ++p) {  // sums are not negative: exactly one chunk takes the running sum past r
+        const int64_t v = __ldcg(sums + p);
+        if (cum <= r && cum + v > r) {
+            s_chunk = p;
+            s_before = cum;
+        }
+        cum += v;
+    }
+    __syncthreads();
+    const int64_t c0 = (int64_t)s_chunk * chunk, c1 = min(n, c0 + chunk);
+    const int64_t per = (c1 - c0 + KPP_NT - 1) / KPP_NT;
+    const int64_t e0 = min(c1, c0 + t * per), e1 = min(c1, e0 + per);
+    int64_t ls = 0, lt;
+    for (int64_t i = e0; i < e1; ++i) ls += __ldcg(min_d + i);
+    cum = s_before + kpp_block_scan(ls, &lt);
+    for (int64_t i = e0; i < e1; ++i) {
+        const int64_t v = __ldcg(min_d + i);
+        if (cum <= r && cum + v > r) s_row = i;
+        cum += v;
+    }
+    __syncthreads();
+    const int64_t row = s_row;
+    for (int j = t; j < w4; j += KPP_NT) C[ci * w4 + j] = X[row * w4 + j];
+}
+
+// std::uniform_int_distribution's value in [0, range) from a stream of 32-bit
+// generator outputs: Lemire's multiply-and-reject method (ACM TOMACS 29(1),
+// 2019), which libstdc++ uses for ranges that fit 32 bits.  Takes outputs from
+// raw at *cur; a stream that runs out leaves *cur past nraw.
+__device__ __forceinline__ uint32_t bin_draw(const uint32_t *__restrict__ raw, int nraw, int *cur, uint32_t range) {
+    uint64_t prod = (uint64_t)(*cur < nraw ? raw[*cur] : 0u) * range;
+    ++*cur;
+    if ((uint32_t)prod < range) {
+        const uint32_t floor = (0u - range) % range;
+        while ((uint32_t)prod < floor && *cur < nraw) {
+            prod = (uint64_t)raw[*cur] * range;
+            ++*cur;
+        }
+    }
+    return (uint32_t)(prod >> 32);
+}
+
+// One launch per draw of the binary k-means++ (BinaryIVF.hpp:140-170): every
+// block lowers its chunk's distances by the newest centroid (row ci - 1) and
+// sums the chunk; the last block to finish draws centroid ci as the reference
+// does: pick(rng), then, when the total is positive, r = wsel(rng) in
+// [0, total) and the first row whose running sum passes r.  The generator's
+// outputs come from raw at *cursor (the host moves its generator on by what
+// was used).  raw == NULL: the last block only writes the total, and the host
+// draws (bin_pick_kernel follows).
+// 200k x 32 bytes, 255 draws: 58.6 ms with one thread walking the sums and two
+// host round trips per draw, 1.3 ms as one launch each.
+__global__ void __launch_bounds__(KPP_NT) bin_kpp_kernel(const uint4 *__restrict__ X, int64_t n, int w4, uint4 *C,
+                                                         int64_t ci, int32_t *min_d, int64_t chunk, int P,
+                                                         int64_t *sums, unsigned *done,
+                                                         const uint32_t *__restrict__ raw, int nraw, int *cursor,
+                                                         int64_t *total_out) {
+    const int t = threadIdx.x;
+    const int64_t b0 = (int64_t)blockIdx.x * chunk, b1 = min(n, b0 + chunk);
+    const uint4 *c = C + (ci - 1) * w4;
+    int64_t s = 0, tot;
+    for (int64_t i = b0 + t; i < b1; i += KPP_NT) {
+        const int32_t v = (int32_t)hdist(c, X + i * w4, w4);
+        int32_t m = v;
+        if (ci > 1) m = min(v, min_d[i]);
+        min_d[i] = m;
+        s += m;
+    }
+    kpp_block_scan(s, &tot);
+    if (t == 0) sums[blockIdx.x] = tot;
+    if (!kpp_last_block(done)) return;
+
+    const int span = (P + KPP_NT - 1) / KPP_NT;
+    const int p0 = min(P, t * span), p1 = min(P, p0 + span);
+    int64_t own = 0, total;
+    for (int p = p0; p < p1; ++p) own += __ldcg(sums + p);
+    const int64_t pre = kpp_block_scan(own, &total);
+    if (!raw) {
+        if (t == 0) *total_out = total;
+        return;
+    }
+    __shared__ int64_t s_r, s_first;
+    if (t == 0) {
+        int cur = *cursor;
+        s_first = bin_draw(raw, nraw, &cur, (uint32_t)n);
+        s_r = -1;
+        if (total > 0) s_r = (int64_t)bin_draw(raw, nraw, &cur, (uint32_t)total);
+        *cursor = cur;
+    }
+    __syncthreads();
+    if (s_r >= 0) {
+        bin_pick(X, n, w4, C, ci, min_d, chunk, P, sums, s_r, pre);
+    } else {  // every row equals a centroid: the first draw stands
+        for (int j = t; j < w4; j += KPP_NT) C[ci * w4 + j] = X[s_first * w4 + j];
     }
 }
 
-// first index i with prefix_sum(v)[0..i] > r (exact int64), one block
-__global__ void find_weighted_kernel(const int64_t *__restrict__ v, int64_t n, const int64_t *__restrict__ sums,
-                                     int64_t nchunks, int64_t r, int64_t *__restrict__ out) {
-    __shared__ int64_t s_chunk, s_before;
-    if (threadIdx.x == 0) {
-        int64_t cum = 0, c = 0;
-        for (; c < nchunks; ++c) {
-            if (cum + sums[c] > r) break;
-            cum += sums[c];
-        }
-        s_chunk = c;
-        s_before = cum;
-        int64_t res = -1;
-        if (c < nchunks) {
-            const int64_t base = c * SCAN_CHUNK;
-            for (int64_t i = base; i < min(n, base + SCAN_CHUNK); ++i) {
-                cum += v[i];
-                if (cum > r) { res = i; break; }
-            }
-        }
-        *out = res;
-    }
+// The pick for an r that the host drew.
+__global__ void __launch_bounds__(KPP_NT) bin_pick_kernel(const uint4 *__restrict__ X, int64_t n, int w4, uint4 *C,
+                                                          int64_t ci, const int32_t *min_d, int64_t chunk, int P,
+                                                          const int64_t *sums, int64_t r) {
+    const int t = threadIdx.x;
+    const int span = (P + KPP_NT - 1) / KPP_NT;
+    const int p0 = min(P, t * span), p1 = min(P, p0 + span);
+    int64_t own = 0, total;
+    for (int p = p0; p < p1; ++p) own += __ldcg(sums + p);
+    const int64_t pre = kpp_block_scan(own, &total);
+    bin_pick(X, n, w4, C, ci, min_d, chunk, P, sums, r, pre);
 }
 
 // assignment to the first nearest centroid; centroids staged in shared memory
@@ -420,39 +567,55 @@ __global__ void bin_assign_kernel(const uint4 *__restrict__ X, int64_t n, int w4
     if ((threadIdx.x & 31) == 0 && m) atomicAdd(n_changed, (unsigned long long)__popc(m));
 }
 
-// bit counts per cluster: one thread per (point, 32-bit word)
-__global__ void bin_bitcount_kernel(const uint32_t *__restrict__ X, int64_t n, int w32, int nbits,
-                                    const int32_t *__restrict__ labels, int32_t *__restrict__ counts,
-                                    int32_t *__restrict__ cc) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n * w32) return;
-    const int64_t p = t / w32;
-    const int w = (int)(t % w32);
-    const int32_t c = labels[p];
-    if (w == 0) atomicAdd(cc + c, 1);
-    uint32_t bits = X[p * w32 + w];
-    while (bits) {
-        const int b = __ffs(bits) - 1;
-        bits &= bits - 1;
-        const int bit = w * 32 + b;
-        if (bit < nbits) atomicAdd(counts + (int64_t)c * nbits + bit, 1);
+// Bit counts per cluster.  Block (x, y, z): a chunk of rows, 32-bit word y of
+// each, clusters [z * BC_SLAB, ..).  A row adds its word to its cluster's 32
+// shared counters as 16 atomic additions of two 16-bit counters each (bits b
+// and b + 16; a chunk has at most BC_ROWS < 65536 rows), and the block adds
+// its totals to the global counts once: 200k x 256 bits, 256 clusters: one
+// global atomic per set bit took 208 us, this 12 us.
+constexpr int BC_SLAB = 1024, BC_ROWS = 8192, BC_NT = 512;
+__global__ void __launch_bounds__(BC_NT) bin_bitcount_kernel(const uint32_t *__restrict__ X, int64_t n, int w32,
+                                                             int rows, const int32_t *__restrict__ labels, int k,
+                                                             const unsigned long long *__restrict__ n_changed,
+                                                             int32_t *__restrict__ counts, int32_t *__restrict__ cc) {
+    extern __shared__ uint32_t bc[];  // [16][slab]: cluster c's pair j at bc[j * slab + c]; then, word 0, [slab] rows
+    if (*n_changed == 0) return;
+    const int slab0 = blockIdx.z * BC_SLAB, slab = min(BC_SLAB, k - slab0);
+    const int w = blockIdx.y;
+    const int words = slab * (w == 0 ? 17 : 16);
+    for (int i = threadIdx.x; i < words; i += BC_NT) bc[i] = 0;
+    __syncthreads();
+    const int64_t r0 = (int64_t)blockIdx.x * rows, r1 = min(n, r0 + rows);
+    for (int64_t p = r0 + threadIdx.x; p < r1; p += BC_NT) {
+        const int c = labels[p] - slab0;
+        if (c < 0 || c >= slab) continue;
+        const uint32_t bits = X[p * w32 + w];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) atomicAdd(bc + j * slab + c, (bits >> j) & 0x00010001u);
+        if (w == 0) atomicAdd(bc + 16 * slab + c, 1u);
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < slab * 32; i += BC_NT) {
+        const int c = i >> 5, b = i & 31;
+        const uint32_t v = (bc[(b & 15) * slab + c] >> (b & 16)) & 0xffffu;
+        if (v) atomicAdd(counts + ((int64_t)(slab0 + c) * w32 + w) * 32 + b, (int32_t)v);
+    }
+    if (w == 0)
+        for (int c = threadIdx.x; c < slab; c += BC_NT)
+            if (const uint32_t v = bc[16 * slab + c]) atomicAdd(cc + slab0 + c, (int32_t)v);
 }
 
-// majority vote (count > n_c / 2); clusters with no point are left for the host
-__global__ void bin_majority_kernel(const int32_t *__restrict__ counts, const int32_t *__restrict__ cc, int k,
-                                    int nbits, int w32, uint32_t *__restrict__ C) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (int64_t)k * w32) return;
-    const int c = (int)(t / w32), w = (int)(t % w32);
-    if (cc[c] == 0) return;
-    const int32_t half = cc[c] / 2;
-    uint32_t word = 0;
-    for (int b = 0; b < 32; ++b) {
-        const int bit = w * 32 + b;
-        if (bit < nbits && counts[(int64_t)c * nbits + bit] > half) word |= 1u << b;
-    }
-    C[t] = word;
+// majority vote (count > n_c / 2), a warp per word of a centroid; clusters with
+// no point are left for the host, and so is everything when no label changed
+__global__ void bin_majority_kernel(const int32_t *__restrict__ counts, const int32_t *__restrict__ cc, int64_t words,
+                                    int w32, const unsigned long long *__restrict__ n_changed,
+                                    uint32_t *__restrict__ C) {
+    const int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (t >= words || *n_changed == 0) return;
+    const int32_t m = cc[t / w32];
+    if (m == 0) return;
+    const uint32_t word = __ballot_sync(0xffffffffu, counts[t * 32 + (threadIdx.x & 31)] > m / 2);
+    if ((threadIdx.x & 31) == 0) C[t] = word;
 }
 
 int kmeans_bin_device(const uint8_t *X, int64_t n, int nbytes, int w4, int32_t k, int32_t max_iter, uint32_t seed,
@@ -462,67 +625,98 @@ int kmeans_bin_device(const uint8_t *X, int64_t n, int nbytes, int w4, int32_t k
     const size_t row = (size_t)w4 * 16;
     const uint4 *X4 = reinterpret_cast<const uint4 *>(X);
     GN_CUDA_TRY(cudaMemcpyAsync(C, X + pick(rng) * row, row, cudaMemcpyDeviceToDevice, st));
-    DBuf dmin, dsums, dout;
-    const int64_t nchunks = ceil_div(n, SCAN_CHUNK);
-    GN_TRY(dmin.ensure((size_t)n * 8));
-    GN_TRY(dsums.ensure((size_t)nchunks * 8));
-    GN_TRY(dout.ensure(8));
-    const unsigned nb = (unsigned)ceil_div(n, 256);
-    fill_i64_kernel<<<nb, 256, 0, st>>>(dmin.as<int64_t>(), n, std::numeric_limits<int64_t>::max());
-    std::vector<int64_t> hs((size_t)nchunks);
-    for (int32_t ci = 1; ci < k; ++ci) {
-        bin_kpp_update_kernel<<<nb, 256, 0, st>>>(X4, n, w4, reinterpret_cast<const uint4 *>(C + (size_t)(ci - 1) * row),
-                                                  dmin.as<int64_t>());
-        chunk_sum_kernel<<<(unsigned)nchunks, 256, 0, st>>>(dmin.as<int64_t>(), n, dsums.as<int64_t>());
-        GN_CUDA_TRY(cudaMemcpyAsync(hs.data(), dsums.p, (size_t)nchunks * 8, cudaMemcpyDeviceToHost, st));
+    DBuf dmin, dsums, daux, draw;
+    // chunk sums: blocks of 256 rows a step, about four blocks per SM slot at most
+    const int64_t chunk = std::max<int64_t>(KPP_NT, round_up(ceil_div(n, 2048), KPP_NT));
+    const int P = (int)ceil_div(n, chunk);
+    GN_TRY(dmin.ensure((size_t)n * 4));
+    GN_TRY(dsums.ensure((size_t)P * 8));
+    GN_TRY(daux.ensure(24));  // [0] total (int64), [2] arrival counter, [3] stream cursor
+    GN_CUDA_TRY(cudaMemsetAsync(daux.p, 0, 24, st));
+    int64_t *dtotal = daux.as<int64_t>();
+    unsigned *ddone = daux.as<unsigned>() + 2;
+    int *dcur = daux.as<int>() + 3;
+    uint4 *C4 = reinterpret_cast<uint4 *>(C);
+    // Every range below 2^32 (the rows, and the distances' total, at most n
+    // rows x nbytes * 8 bits): the draws run on the device from the generator's
+    // next outputs.  A draw takes two outputs and, rarely, more (each is
+    // rejected with a probability below 1/2); 8 per centroid are on hand, and if
+    // they should not do, the host draws instead, as for larger ranges.
+#if defined(_GLIBCXX_RELEASE) && _GLIBCXX_RELEASE >= 11
+    bool on_device = (uint64_t)n * (uint64_t)nbytes * 8 < (1ull << 32);
+#else
+    bool on_device = false;  // another library's distribution may draw differently
+#endif
+    if (on_device && k > 1) {
+        std::vector<uint32_t> raw((size_t)k * 8 + 256);
+        std::mt19937 ahead = rng;
+        for (uint32_t &v : raw) v = (uint32_t)ahead();
+        GN_TRY(draw.ensure(raw.size() * 4));
+        GN_CUDA_TRY(cudaMemcpyAsync(draw.p, raw.data(), raw.size() * 4, cudaMemcpyHostToDevice, st));
+        for (int32_t ci = 1; ci < k; ++ci)
+            bin_kpp_kernel<<<(unsigned)P, KPP_NT, 0, st>>>(X4, n, w4, C4, ci, dmin.as<int32_t>(), chunk, P,
+                                                           dsums.as<int64_t>(), ddone, draw.as<uint32_t>(),
+                                                           (int)raw.size(), dcur, dtotal);
+        int used = 0;
+        GN_CUDA_TRY(cudaMemcpyAsync(&used, dcur, 4, cudaMemcpyDeviceToHost, st));
         GN_CUDA_TRY(cudaStreamSynchronize(st));
-        int64_t total = 0;
-        for (int64_t v : hs) total += v;
-        size_t chosen = pick(rng);
-        if (total > 0) {
-            std::uniform_int_distribution<int64_t> wsel(0, total - 1);
-            const int64_t r = wsel(rng);
-            find_weighted_kernel<<<1, 32, 0, st>>>(dmin.as<int64_t>(), n, dsums.as<int64_t>(), nchunks, r,
-                                                   dout.as<int64_t>());
-            int64_t res = -1;
-            GN_CUDA_TRY(cudaMemcpyAsync(&res, dout.p, 8, cudaMemcpyDeviceToHost, st));
-            GN_CUDA_TRY(cudaStreamSynchronize(st));
-            if (res >= 0) chosen = (size_t)res;
-        }
-        GN_CUDA_TRY(cudaMemcpyAsync(C + (size_t)ci * row, X + chosen * row, row, cudaMemcpyDeviceToDevice, st));
+        on_device = used <= (int)raw.size() - 1;
+        if (on_device) rng.discard((unsigned long long)used);
     }
+    if (!on_device)
+        for (int32_t ci = 1; ci < k; ++ci) {
+            bin_kpp_kernel<<<(unsigned)P, KPP_NT, 0, st>>>(X4, n, w4, C4, ci, dmin.as<int32_t>(), chunk, P,
+                                                           dsums.as<int64_t>(), ddone, nullptr, 0, dcur, dtotal);
+            int64_t total = 0;
+            GN_CUDA_TRY(cudaMemcpyAsync(&total, dtotal, 8, cudaMemcpyDeviceToHost, st));
+            GN_CUDA_TRY(cudaStreamSynchronize(st));
+            const size_t chosen = pick(rng);
+            if (total > 0) {
+                std::uniform_int_distribution<int64_t> wsel(0, total - 1);
+                bin_pick_kernel<<<1, KPP_NT, 0, st>>>(X4, n, w4, C4, ci, dmin.as<int32_t>(), chunk, P,
+                                                      dsums.as<int64_t>(), wsel(rng));
+            } else {
+                GN_CUDA_TRY(cudaMemcpyAsync(C + (size_t)ci * row, X + chosen * row, row, cudaMemcpyDeviceToDevice, st));
+            }
+        }
 
-    const int nbits = nbytes * 8;
+    // Lloyd iterations; one host synchronisation each (the change count and the
+    // cluster sizes together): the update's kernels do nothing when no label changed
     const int w32 = w4 * 4;
-    DBuf dcounts, dcc, dchg;
-    GN_TRY(dcounts.ensure((size_t)k * nbits * 4));
-    GN_TRY(dcc.ensure((size_t)k * 4));
-    GN_TRY(dchg.ensure(8));
+    DBuf dcounts, dstat;
+    GN_TRY(dcounts.ensure((size_t)k * w32 * 32 * 4));
+    GN_TRY(dstat.ensure(8 + (size_t)k * 4));  // change count, then rows per cluster
+    unsigned long long *dchg = dstat.as<unsigned long long>();
+    int32_t *dcc = dstat.as<int32_t>() + 2;
     GN_CUDA_TRY(cudaMemsetAsync(labels, 0, (size_t)n * 4, st));
     const size_t smem = (size_t)k * row;
     if (smem > (size_t)dev_info().max_smem_optin)
         return fail(GN_ERR_UNSUPPORTED, "binary k-means: nlist * row bytes exceeds shared memory");
     if (smem > 48 * 1024)
         GN_CUDA_TRY(cudaFuncSetAttribute(bin_assign_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    std::vector<int32_t> hcc((size_t)k);
+    const size_t bc_smem = (size_t)std::min(k, BC_SLAB) * 17 * 4;
+    if (bc_smem > 48 * 1024)
+        GN_CUDA_TRY(cudaFuncSetAttribute(bin_bitcount_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)bc_smem));
+    const int slabs = (int)ceil_div(k, BC_SLAB);
+    // rows per counting block: about two blocks per SM over the words and slabs
+    const int64_t row_blocks = std::max<int64_t>(1, 2LL * dev_info().num_sms / ((int64_t)w32 * slabs));
+    const int bc_rows = (int)std::min<int64_t>(BC_ROWS, std::max<int64_t>(BC_NT, ceil_div(n, row_blocks)));
+    const dim3 bc_grid((unsigned)ceil_div(n, bc_rows), (unsigned)w32, (unsigned)slabs);
+    std::vector<int32_t> hstat((size_t)k + 2);
     for (int32_t it = 0; it < max_iter; ++it) {
-        GN_CUDA_TRY(cudaMemsetAsync(dchg.p, 0, 8, st));
-        bin_assign_kernel<<<nb, 256, smem, st>>>(X4, n, w4, reinterpret_cast<const uint4 *>(C), k, labels,
-                                                 dchg.as<unsigned long long>());
-        unsigned long long changed = 0;
-        GN_CUDA_TRY(cudaMemcpyAsync(&changed, dchg.p, 8, cudaMemcpyDeviceToHost, st));
+        GN_CUDA_TRY(cudaMemsetAsync(dstat.p, 0, 8 + (size_t)k * 4, st));
+        GN_CUDA_TRY(cudaMemsetAsync(dcounts.p, 0, (size_t)k * w32 * 32 * 4, st));
+        bin_assign_kernel<<<(unsigned)ceil_div(n, 256), 256, smem, st>>>(X4, n, w4, C4, k, labels, dchg);
+        bin_bitcount_kernel<<<bc_grid, BC_NT, bc_smem, st>>>(reinterpret_cast<const uint32_t *>(X), n, w32, bc_rows,
+                                                             labels, k, dchg, dcounts.as<int32_t>(), dcc);
+        bin_majority_kernel<<<(unsigned)ceil_div((int64_t)k * w32, 8), 256, 0, st>>>(
+            dcounts.as<int32_t>(), dcc, (int64_t)k * w32, w32, dchg, reinterpret_cast<uint32_t *>(C));
+        GN_CUDA_TRY(cudaMemcpyAsync(hstat.data(), dstat.p, hstat.size() * 4, cudaMemcpyDeviceToHost, st));
         GN_CUDA_TRY(cudaStreamSynchronize(st));
-        if (changed == 0) break;
-        GN_CUDA_TRY(cudaMemsetAsync(dcounts.p, 0, (size_t)k * nbits * 4, st));
-        GN_CUDA_TRY(cudaMemsetAsync(dcc.p, 0, (size_t)k * 4, st));
-        bin_bitcount_kernel<<<(unsigned)ceil_div(n * w32, 256), 256, 0, st>>>(
-            reinterpret_cast<const uint32_t *>(X), n, w32, nbits, labels, dcounts.as<int32_t>(), dcc.as<int32_t>());
-        bin_majority_kernel<<<(unsigned)ceil_div((int64_t)k * w32, 256), 256, 0, st>>>(
-            dcounts.as<int32_t>(), dcc.as<int32_t>(), k, nbits, w32, reinterpret_cast<uint32_t *>(C));
-        GN_CUDA_TRY(cudaMemcpyAsync(hcc.data(), dcc.p, (size_t)k * 4, cudaMemcpyDeviceToHost, st));
-        GN_CUDA_TRY(cudaStreamSynchronize(st));
+        if (hstat[0] == 0 && hstat[1] == 0) break;
         for (int32_t c = 0; c < k; ++c)
-            if (hcc[(size_t)c] == 0)
+            if (hstat[(size_t)c + 2] == 0)
                 GN_CUDA_TRY(cudaMemcpyAsync(C + (size_t)c * row, X + pick(rng) * row, row, cudaMemcpyDeviceToDevice, st));
     }
     GN_CUDA_TRY(cudaGetLastError());

@@ -7,65 +7,185 @@
 // search1NN of all pixels against the seeds (demo/voronoi.py:93-110).  Here the
 // grid is never materialised: the kernel reads the two coordinate vectors.
 //
-// Layout: one block per (row, 1024-column strip); 256 threads, 4 pixels per
-// thread at stride 256 so every store is coalesced.  Seeds stream through
-// shared memory in tiles of 2048 as (sx, dy²), dy² = (py − sy)² computed once
-// per row, so a pixel–seed pair costs one subtract, one multiply, one add and
-// (seeds taken four at a time) three quarters of a minimum and a quarter of a
-// compare.  The distance is the flat L2 kernel's arithmetic for d = 2,
-// sqrt(rn(rn(dx²) + rn(dy²))) with dx = px − sx, dy = py − sy; the argmin is
-// over that sqrt value with ties to the lower seed index, the same answer the
-// exact flat search1NN gives.  The squared sum prefilters: sqrt is monotone,
-// so a pair can only win if its squared sum is below the current best one,
-// and the sqrt is taken only then (about ln(ns) times per pixel).  Seeds go
-// four at a time: one compare of the four squared sums' minimum against the
-// best decides (almost always) that none of them can win, and only otherwise
-// are the four offered one by one in seed order, so the branch is taken
-// rarely and costs a quarter of a compare per pair.
+// Answer per pixel: the lexicographic minimum of (sqrt(rn(rn(dx²) + rn(dy²))),
+// seed index), dx = px − sx, dy = py − sy, the flat L2 kernel's arithmetic for
+// d = 2.  Seeds are offered in index order; a squared sum below the best one
+// is needed to win (sqrt is monotone), so the sqrt is rarely taken.
+//
+// Seeds that cannot win are left out by tiles of pixels, in two levels: a
+// block's tile (128 x 64 pixels, 32 x 32 where that leaves SMs idle), then a
+// warp's 16 x 8.  For a tile with coordinates in [x0, x1] x [y0, y1], a seed's
+// |dx| lies between the rounded distances from sx to the interval's nearest and
+// farthest end, because rounding is monotone, and so are the rounded square,
+// sum and root: with lb / ub the same arithmetic on those ends,
+//     lb(seed) <= its squared sum at every pixel of the tile <= ub(seed)
+// holds exactly, without a margin.  A seed with sqrt(lb) > sqrt(min ub) is
+// strictly farther than another one everywhere in the tile; equal roots are
+// kept, so ties still go to the lower index.  NaN pixels keep id 0 and +inf
+// whatever is left out, NaN seeds never win, and an infinite pixel coordinate
+// makes min ub infinite, which keeps every seed.
+//
+// Block list: up to VR_CAP surviving seeds in shared memory; where more
+// survive (seeds crowded together), the warps read all seeds instead.  A warp
+// collects its own survivors VR_WCAP at a time and evaluates four seeds for
+// its four neighbouring pixels per thread in packed FP32 (two results an
+// instruction: the loop is bound by issue slots).  3840 x 2160, 4,096 seeds:
+// 5.12 ms evaluating every pair, 0.068 ms with the tiles (66 MB of ids and
+// colours out: 0.010 ms of HBM time; what is left is the two levels of bounds).
 #include <cmath>
 
+#include "f32x2.cuh"
 #include "index.cuh"
 
 namespace gn {
 
 constexpr int VR_NT = 256;    // threads per block
-constexpr int VR_PX = 4;      // pixels per thread
-constexpr int VR_TILE = 2048; // seeds per shared-memory tile (16 KB)
-constexpr int VR_STRIP = VR_NT * VR_PX;
+constexpr int VR_WARPS = VR_NT / 32;
+constexpr int VR_CAP = 1024;  // seeds in a block's list
+constexpr int VR_WCAP = 64;   // seeds a warp collects before it evaluates them (a multiple of 32)
+constexpr int VR_SW = 16, VR_SH = 8;  // a warp's pixels: four neighbours per thread
 
+// Smallest and largest squared sum of a seed over [x0, x1] x [y0, y1].
+__device__ __forceinline__ void vr_bounds(float2 s, float x0, float x1, float y0, float y1, float &lb, float &ub) {
+    const float ax = __fsub_rn(x0, s.x), bx = __fsub_rn(x1, s.x), ay = __fsub_rn(y0, s.y), by = __fsub_rn(y1, s.y);
+    const float fx = fmaxf(fabsf(ax), fabsf(bx)), fy = fmaxf(fabsf(ay), fabsf(by));
+    const float nx = fmaxf(fmaxf(ax, -bx), 0.f), ny = fmaxf(fmaxf(ay, -by), 0.f);
+    lb = __fadd_rn(__fmul_rn(nx, nx), __fmul_rn(ny, ny));
+    ub = __fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy));
+}
+
+// Block tile: TX x TY warp tiles.
+template <int TX, int TY>
 __global__ void __launch_bounds__(VR_NT) voronoi_kernel(const float2 *__restrict__ seeds, int ns,
                                                         const float *__restrict__ xs, const float *__restrict__ ys,
-                                                        int w, int h, int32_t *__restrict__ ids,
+                                                        int w, int h, int tiles_y, int32_t *__restrict__ ids,
                                                         float *__restrict__ dist,
                                                         const uchar4 *__restrict__ palette, int npal,
                                                         uchar4 *__restrict__ rgba) {
-    __shared__ __align__(16) float2 sm[VR_TILE];
-    const int cbase = blockIdx.x * VR_STRIP + threadIdx.x;
-    float px[VR_PX];
-#pragma unroll
-    for (int p = 0; p < VR_PX; ++p) {
-        const int c = cbase + p * VR_NT;
-        px[p] = c < w ? xs[c] : 0.f;
-    }
-    for (int row = blockIdx.y; row < h; row += gridDim.y) {
-        const float py = ys[row];
-        float bs[VR_PX], br[VR_PX];
-        int bi[VR_PX];
-#pragma unroll
-        for (int p = 0; p < VR_PX; ++p) {
-            bs[p] = INFINITY;
-            br[p] = INFINITY;
-            bi[p] = 0;
+    __shared__ float2 bxy[VR_CAP];
+    __shared__ int bid[VR_CAP];
+    __shared__ float2 wxy[VR_WARPS][VR_WCAP + 32];
+    __shared__ int wid[VR_WARPS][VR_WCAP + 32];
+    __shared__ float red[5][VR_WARPS];
+    __shared__ int wcount[VR_WARPS];
+    constexpr float INF = INFINITY;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    for (int ty = blockIdx.y; ty < tiles_y; ty += gridDim.y) {
+        const int c0 = blockIdx.x * TX * VR_SW, r0 = ty * TY * VR_SH;
+        const int nc = min(TX * VR_SW, w - c0), nr = min(TY * VR_SH, h - r0);
+        // the tile's coordinate ranges (NaN coordinates drop out of the minima)
+        float x0 = INF, x1 = -INF, y0 = INF, y1 = -INF;
+        for (int i = t; i < nc; i += VR_NT) {
+            x0 = fminf(x0, xs[c0 + i]);
+            x1 = fmaxf(x1, xs[c0 + i]);
         }
-        for (int t0 = 0; t0 < ns; t0 += VR_TILE) {
-            const int tn = min(VR_TILE, ns - t0);
-            __syncthreads();  // the previous tile (or row) is no longer read
-            for (int j = threadIdx.x; j < tn; j += VR_NT) {
-                const float2 s = seeds[t0 + j];
-                const float dy = __fsub_rn(py, s.y);
-                sm[j] = make_float2(s.x, __fmul_rn(dy, dy));
+        for (int i = t; i < nr; i += VR_NT) {
+            y0 = fminf(y0, ys[r0 + i]);
+            y1 = fmaxf(y1, ys[r0 + i]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            x0 = fminf(x0, __shfl_xor_sync(0xffffffffu, x0, o));
+            x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, o));
+            y0 = fminf(y0, __shfl_xor_sync(0xffffffffu, y0, o));
+            y1 = fmaxf(y1, __shfl_xor_sync(0xffffffffu, y1, o));
+        }
+        __syncthreads();  // the previous tile is done with the lists
+        if (lane == 0) {
+            red[0][warp] = x0;
+            red[1][warp] = x1;
+            red[2][warp] = y0;
+            red[3][warp] = y1;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < VR_WARPS; ++i) {
+            x0 = fminf(x0, red[0][i]);
+            x1 = fmaxf(x1, red[1][i]);
+            y0 = fminf(y0, red[2][i]);
+            y1 = fmaxf(y1, red[3][i]);
+        }
+        // some seed is within `u` of every pixel
+        float u = INF, lb, ub;
+        for (int j = t; j < ns; j += VR_NT) {
+            vr_bounds(seeds[j], x0, x1, y0, y1, lb, ub);
+            u = fminf(u, ub);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) u = fminf(u, __shfl_xor_sync(0xffffffffu, u, o));
+        if (lane == 0) red[4][warp] = u;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < VR_WARPS; ++i) u = fminf(u, red[4][i]);
+        u = __fsqrt_rn(u);
+        // the block's list, in index order
+        int m = 0;
+        for (int j0 = 0; j0 < ns && m <= VR_CAP; j0 += VR_NT) {
+            const int j = j0 + t;
+            float2 s = make_float2(0.f, 0.f);
+            bool keep = false;
+            if (j < ns) {
+                s = seeds[j];
+                vr_bounds(s, x0, x1, y0, y1, lb, ub);
+                keep = __fsqrt_rn(lb) <= u;
             }
+            const unsigned mask = __ballot_sync(0xffffffffu, keep);
+            if (lane == 0) wcount[warp] = __popc(mask);
             __syncthreads();
+            int before = m, all = 0;
+#pragma unroll
+            for (int i = 0; i < VR_WARPS; ++i) {
+                const int cnt = wcount[i];
+                if (i < warp) before += cnt;
+                all += cnt;
+            }
+            const int at = before + __popc(mask & ((1u << lane) - 1));
+            if (keep && at < VR_CAP) {
+                bxy[at] = s;
+                bid[at] = j;
+            }
+            m += all;
+            __syncthreads();
+        }
+        const bool listed = m <= VR_CAP;  // else: too many, read the seeds themselves
+        const int nsrc = listed ? m : ns;
+
+        for (int wt = warp; wt < TX * TY; wt += VR_WARPS) {
+            const int wc = c0 + (wt % TX) * VR_SW, wr = r0 + (wt / TX) * VR_SH;
+            if (wc >= w || wr >= h) continue;
+            const int pc = wc + (lane & 3) * 4, pr = wr + (lane >> 2);
+            const float py = ys[min(pr, h - 1)];
+            float px[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) px[p] = xs[min(pc + p, w - 1)];
+            float a0 = fminf(fminf(px[0], px[1]), fminf(px[2], px[3])), b0 = py;
+            float a1 = fmaxf(fmaxf(px[0], px[1]), fmaxf(px[2], px[3])), b1 = py;
+#pragma unroll
+            for (int o = 1; o < 4; o <<= 1) {
+                a0 = fminf(a0, __shfl_xor_sync(0xffffffffu, a0, o));
+                a1 = fmaxf(a1, __shfl_xor_sync(0xffffffffu, a1, o));
+            }
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                b0 = fminf(b0, __shfl_xor_sync(0xffffffffu, b0, o));
+                b1 = fmaxf(b1, __shfl_xor_sync(0xffffffffu, b1, o));
+            }
+            float wu = INF;
+            for (int j = lane; j < nsrc; j += 32) {
+                vr_bounds(listed ? bxy[j] : seeds[j], a0, a1, b0, b1, lb, ub);
+                wu = fminf(wu, ub);
+            }
+            wu = __fsqrt_rn(__uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(wu))));
+
+            float bs[4], br[4];
+            int bi[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+                bs[p] = INF;
+                br[p] = INF;
+                bi[p] = 0;
+            }
+            const f32x2 px01 = pack2(px[0], px[1]), px23 = pack2(px[2], px[3]);
             // offer seed `idx` with squared sum s to pixel p (seed order is kept)
             auto offer = [&](int p, float s, int idx) {
                 if (s < bs[p]) {
@@ -77,44 +197,113 @@ __global__ void __launch_bounds__(VR_NT) voronoi_kernel(const float2 *__restrict
                     }
                 }
             };
-            int j = 0;
-#pragma unroll 2
-            for (; j + 4 <= tn; j += 4) {
-                const float4 e01 = *reinterpret_cast<const float4 *>(sm + j);      // (x, dy²) of seeds j, j + 1
-                const float4 e23 = *reinterpret_cast<const float4 *>(sm + j + 2);  // seeds j + 2, j + 3
+            auto sums = [&](float2 s, float (&o)[4]) {  // the four pixels' squared sums
+                const float dy = __fsub_rn(py, s.y);
+                const f32x2 dy2 = dup2(__fmul_rn(dy, dy)), nx = dup2(-s.x);
+                const f32x2 d01 = add2(px01, nx), d23 = add2(px23, nx);
+                float d0, d1, d2, d3;
+                unpack2(d01, d0, d1);
+                unpack2(d23, d2, d3);
+                // scalar products: a packed product and sum came out fused (one rounding
+                // instead of the two of the reference's arithmetic)
+                unpack2(add2(pack2(__fmul_rn(d0, d0), __fmul_rn(d1, d1)), dy2), o[0], o[1]);
+                unpack2(add2(pack2(__fmul_rn(d2, d2), __fmul_rn(d3, d3)), dy2), o[2], o[3]);
+            };
+            float2 *lxy = wxy[warp];
+            int *lid = wid[warp];
+            auto evaluate = [&](int cnt) {
+                int j = 0;
+                for (; j + 4 <= cnt; j += 4) {
+                    float s0[4], s1[4], s2[4], s3[4];
+                    sums(lxy[j], s0);
+                    sums(lxy[j + 1], s1);
+                    sums(lxy[j + 2], s2);
+                    sums(lxy[j + 3], s3);
 #pragma unroll
-                for (int p = 0; p < VR_PX; ++p) {
-                    const float d0 = __fsub_rn(px[p], e01.x), d1 = __fsub_rn(px[p], e01.z);
-                    const float d2 = __fsub_rn(px[p], e23.x), d3 = __fsub_rn(px[p], e23.z);
-                    const float s0 = __fadd_rn(__fmul_rn(d0, d0), e01.y);
-                    const float s1 = __fadd_rn(__fmul_rn(d1, d1), e01.w);
-                    const float s2 = __fadd_rn(__fmul_rn(d2, d2), e23.y);
-                    const float s3 = __fadd_rn(__fmul_rn(d3, d3), e23.w);
-                    if (fminf(fminf(s0, s1), fminf(s2, s3)) < bs[p]) {
-                        offer(p, s0, t0 + j);
-                        offer(p, s1, t0 + j + 1);
-                        offer(p, s2, t0 + j + 2);
-                        offer(p, s3, t0 + j + 3);
-                    }
+                    for (int p = 0; p < 4; ++p)
+                        if (fminf(fminf(s0[p], s1[p]), fminf(s2[p], s3[p])) < bs[p]) {
+                            offer(p, s0[p], lid[j]);
+                            offer(p, s1[p], lid[j + 1]);
+                            offer(p, s2[p], lid[j + 2]);
+                            offer(p, s3[p], lid[j + 3]);
+                        }
+                }
+                for (; j < cnt; ++j) {
+                    float s0[4];
+                    sums(lxy[j], s0);
+#pragma unroll
+                    for (int p = 0; p < 4; ++p) offer(p, s0[p], lid[j]);
+                }
+            };
+            int cnt = 0;
+            for (int j0 = 0; j0 < nsrc; j0 += 32) {
+                const int j = j0 + lane;
+                float2 s = make_float2(0.f, 0.f);
+                bool keep = false;
+                if (j < nsrc) {
+                    s = listed ? bxy[j] : seeds[j];
+                    vr_bounds(s, a0, a1, b0, b1, lb, ub);
+                    keep = __fsqrt_rn(lb) <= wu;
+                }
+                const unsigned mask = __ballot_sync(0xffffffffu, keep);
+                if (keep) {
+                    const int at = cnt + __popc(mask & ((1u << lane) - 1));
+                    lxy[at] = s;
+                    lid[at] = listed ? bid[j] : j;
+                }
+                cnt += __popc(mask);
+                if (cnt >= VR_WCAP) {
+                    __syncwarp();
+                    evaluate(cnt);
+                    __syncwarp();
+                    cnt = 0;
                 }
             }
-            for (; j < tn; ++j) {
-                const float2 e = sm[j];
+            __syncwarp();
+            evaluate(cnt);
+            __syncwarp();
+
+            if (pr >= h) continue;
+            const int64_t off = (int64_t)pr * w + pc;
+            uchar4 col[4];
+            if (rgba) {
 #pragma unroll
-                for (int p = 0; p < VR_PX; ++p) {
-                    const float dx = __fsub_rn(px[p], e.x);
-                    offer(p, __fadd_rn(__fmul_rn(dx, dx), e.y), t0 + j);
+                for (int p = 0; p < 4; ++p) col[p] = palette[bi[p] < npal ? bi[p] : bi[p] % npal];
+            }
+            // whole 16-byte stores where the row starts allow them
+            const bool vec = pc + 4 <= w && (w & 3) == 0;
+            if (ids) {
+                if (vec && ((uintptr_t)ids & 15) == 0) {
+                    *reinterpret_cast<int4 *>(ids + off) = make_int4(bi[0], bi[1], bi[2], bi[3]);
+                } else {
+#pragma unroll
+                    for (int p = 0; p < 4; ++p)
+                        if (pc + p < w) ids[off + p] = bi[p];
                 }
             }
-        }
-        const int64_t rowoff = (int64_t)row * w;
+            if (dist) {
+                if (vec && ((uintptr_t)dist & 15) == 0) {
+                    *reinterpret_cast<float4 *>(dist + off) = make_float4(br[0], br[1], br[2], br[3]);
+                } else {
 #pragma unroll
-        for (int p = 0; p < VR_PX; ++p) {
-            const int c = cbase + p * VR_NT;
-            if (c >= w) continue;
-            if (ids) ids[rowoff + c] = bi[p];
-            if (dist) dist[rowoff + c] = br[p];
-            if (rgba) rgba[rowoff + c] = palette[bi[p] % npal];
+                    for (int p = 0; p < 4; ++p)
+                        if (pc + p < w) dist[off + p] = br[p];
+                }
+            }
+            if (rgba) {
+                if (vec && ((uintptr_t)rgba & 15) == 0) {
+                    uint4 v;
+                    v.x = *reinterpret_cast<unsigned *>(&col[0]);
+                    v.y = *reinterpret_cast<unsigned *>(&col[1]);
+                    v.z = *reinterpret_cast<unsigned *>(&col[2]);
+                    v.w = *reinterpret_cast<unsigned *>(&col[3]);
+                    *reinterpret_cast<uint4 *>(rgba + off) = v;
+                } else {
+#pragma unroll
+                    for (int p = 0; p < 4; ++p)
+                        if (pc + p < w) rgba[off + p] = col[p];
+                }
+            }
         }
     }
 }
@@ -138,10 +327,19 @@ static int voronoi_launch(const float *seeds, int64_t ns, const float *xs, const
     if ((reinterpret_cast<uintptr_t>(seeds) & 7) || (reinterpret_cast<uintptr_t>(palette) & 3) ||
         (reinterpret_cast<uintptr_t>(rgba) & 3))
         return fail(GN_ERR_INVALID, "seeds must be 8-byte aligned, palette and RGBA output 4-byte aligned");
-    dim3 grid((unsigned)ceil_div(w, VR_STRIP), (unsigned)std::min<int64_t>(h, 65535));
-    voronoi_kernel<<<grid, VR_NT, 0, st>>>(reinterpret_cast<const float2 *>(seeds), (int)ns, xs, ys, (int)w, (int)h,
-                                           ids, dist, reinterpret_cast<const uchar4 *>(palette), (int)npal,
-                                           reinterpret_cast<uchar4 *>(rgba));
+    auto launch = [&](auto kern, int tw, int th) {
+        const int64_t tiles_y = ceil_div(h, th);
+        dim3 grid((unsigned)ceil_div(w, tw), (unsigned)std::min<int64_t>(tiles_y, 65535));
+        kern<<<grid, VR_NT, 0, st>>>(reinterpret_cast<const float2 *>(seeds), (int)ns, xs, ys, (int)w, (int)h,
+                                     (int)tiles_y, ids, dist, reinterpret_cast<const uchar4 *>(palette), (int)npal,
+                                     reinterpret_cast<uchar4 *>(rgba));
+    };
+    // large tiles share one pass over the seeds among 64 warp tiles; small ones
+    // where large ones would not give every SM two blocks
+    if (ceil_div(w, 8 * VR_SW) * ceil_div(h, 8 * VR_SH) >= 2 * dev_info().num_sms)
+        launch(voronoi_kernel<8, 8>, 8 * VR_SW, 8 * VR_SH);
+    else
+        launch(voronoi_kernel<2, 4>, 2 * VR_SW, 4 * VR_SH);
     GN_CUDA_TRY(cudaGetLastError());
     return GN_OK;
 }

@@ -125,3 +125,36 @@ def test_lattice_seeds_many_ties_against_oracle(gn, oracle):
     o_ids, o_dist = oracle.voronoi_raster(seeds, xs, ys)
     assert np.array_equal(r.ids, o_ids)
     assert np.array_equal(r.dist.view(np.uint32), o_dist.view(np.uint32))
+
+
+@pytest.mark.parametrize("w,h", [(2500, 1001), (131, 70)])
+def test_crowded_seeds_and_both_tile_sizes(gn, oracle, w, h):
+    """More seeds than a block's list can hold survive in the tiles around a
+    crowd; large and small rasters (the two tile sizes), ragged edges."""
+    rng = np.random.default_rng(w)
+    seeds = np.concatenate([0.4 + 1e-3 * rng.random((3000, 2)), rng.random((77, 2))]).astype(np.float32)
+    xs, ys = gn.voronoi.grid_axes(w, h)
+    r = gn.voronoi_raster(seeds, xs=xs, ys=ys, with_distance=True)
+    rows = np.unique(np.r_[0:h:97, int(0.4 * h):int(0.4 * h) + 9, h - 1])
+    o_ids, o_dist = oracle.voronoi_raster(seeds, xs, ys[rows])
+    assert np.array_equal(r.ids[rows], o_ids)
+    assert np.array_equal(r.dist[rows].view(np.uint32), o_dist.view(np.uint32))
+
+
+def test_non_finite_coordinates(gn):
+    """NaN pixels and pixels at infinity have no nearest seed (id 0, +inf), NaN
+    seeds never win, and neither changes the other pixels of their tile."""
+    rng = np.random.default_rng(9)
+    seeds = rng.random((500, 2), dtype=np.float32)
+    seeds[7] = np.nan
+    xs, ys = gn.voronoi.grid_axes(150, 70)
+    want = gn.voronoi_raster(np.delete(seeds, 7, 0), xs=xs, ys=ys, with_distance=True)
+    xb, yb = xs.copy(), ys.copy()
+    xb[[3, 40, 149]] = np.nan
+    xb[90] = np.inf
+    yb[33] = np.nan
+    r = gn.voronoi_raster(seeds, xs=xb, ys=yb, with_distance=True)
+    ok = np.isfinite(yb)[:, None] & np.isfinite(xb)[None, :]
+    assert np.array_equal(np.where(r.ids > 7, r.ids - 1, r.ids)[ok], want.ids[ok])
+    assert np.array_equal(r.dist[ok].view(np.uint32), want.dist[ok].view(np.uint32))
+    assert (r.ids[~ok] == 0).all() and np.isposinf(r.dist[~ok]).all()

@@ -32,30 +32,40 @@ namespace gn {
 
 // ── block reductions of the seeding kernels (256 threads) ─────────────────
 constexpr int KPP_NT = 256;
+constexpr int KPP_ROWS = KPP_NT / 2;  // rows a block of the float seeding takes at a time
+constexpr int KPP_SPAN = 4;           // chunk sums per thread of the pick: at most KPP_NT * KPP_SPAN chunks
 
-// Exclusive block-wide scan; *total = the sum of all threads' v.
+// Exclusive block-wide scan; *total = the sum of all threads' v.  Threads from
+// `active` on hold zero: their warps add nothing (FP64 runs at two lanes per
+// clock and SM, so additions of zeros would cost as much as the others).
 template <typename T>
-__device__ __forceinline__ T kpp_block_scan(T v, T *total) {
-    __shared__ T wsum[KPP_NT / 32];
+__device__ __forceinline__ T kpp_block_scan(T v, T *total, int active = KPP_NT) {
+    __shared__ T wsum[KPP_NT / 32 + 1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     T inc = v;
+    if (warp * 32 < active) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const T y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
+        for (int o = 1; o < 32; o <<= 1) {
+            const T y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
     }
     __syncthreads();  // wsum of an earlier call is no longer read
-    if (lane == 31) wsum[warp] = inc;
+    if (lane == 31) wsum[warp + 1] = inc;
     __syncthreads();
-    T w = lane < KPP_NT / 32 ? wsum[lane] : T(0);
+    if (warp == 0) {
+        T w = lane < KPP_NT / 32 ? wsum[lane + 1] : T(0);
 #pragma unroll
-    for (int o = 1; o < KPP_NT / 32; o <<= 1) {
-        const T y = __shfl_up_sync(0xffffffffu, w, o);
-        if (lane >= o) w += y;
+        for (int o = 1; o < KPP_NT / 32; o <<= 1) {
+            const T y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        if (lane < KPP_NT / 32) wsum[lane + 1] = w;
+        if (lane == 0) wsum[0] = T(0);
     }
-    *total = __shfl_sync(0xffffffffu, w, KPP_NT / 32 - 1);
-    const T before = __shfl_sync(0xffffffffu, w, warp > 0 ? warp - 1 : 0);
-    return (warp > 0 ? before : T(0)) + inc - v;
+    __syncthreads();
+    *total = wsum[KPP_NT / 32];
+    return warp * 32 < active ? wsum[warp] + (inc - v) : wsum[KPP_NT / 32];
 }
 
 // True in every thread of the launch's last block to arrive (whose view then
@@ -93,7 +103,7 @@ __device__ __forceinline__ bool kpp_last_block(unsigned *done) {
 // the same point; if not, thread 0 repeats the reference's serial loop (rare).
 // What bounds it is the chain of dependent FP64 additions (the unit's latency,
 // not its rate), so every sum is a scan over lanes: 100k x 64, 255 draws:
-// 12.2 ms as three launches with serial sums over the warps' totals, 2.6 ms
+// 12.2 ms as three launches with serial sums over the warps' totals, 3.8 ms
 // as this one.
 __global__ void __launch_bounds__(KPP_NT) kpp_kernel(const float *__restrict__ X, int64_t n, int d, int dp,
                                                      float *__restrict__ C, int64_t ci, float u,
@@ -101,13 +111,14 @@ __global__ void __launch_bounds__(KPP_NT) kpp_kernel(const float *__restrict__ X
                                                      double *__restrict__ part, unsigned *__restrict__ done) {
     const int t = threadIdx.x;
     const int64_t b0 = (int64_t)blockIdx.x * chunk, b1 = min(n, b0 + chunk);
+    __shared__ float s_m[KPP_ROWS];
     {
         const int half = t & 1;
         const int nb = d >> 3, rem = d & 7, dp4 = dp >> 2;
         const float4 *c4 = reinterpret_cast<const float4 *>(C) + (ci - 1) * dp4;
         const float4 *x4 = reinterpret_cast<const float4 *>(X);
-        double s = 0.0;
-        for (int64_t i0 = b0; i0 < b1; i0 += KPP_NT / 2) {
+        double s = 0.0;  // warp 0: this lane's share of the chunk's sum
+        for (int64_t i0 = b0; i0 < b1; i0 += KPP_ROWS) {
             const int64_t i = i0 + (t >> 1);
             const bool in = i < b1;
             const float4 *xr = x4 + (in ? i : b0) * dp4 + half;
@@ -136,20 +147,32 @@ __global__ void __launch_bounds__(KPP_NT) kpp_kernel(const float *__restrict__ X
                 s2 = __fmaf_rn(t2, t2, s2);
                 s3 = __fmaf_rn(t3, t3, s3);
             }
-            if (in && half == 0) {
-                const float r = __fsqrt_rn(__fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3)));
-                const float v = __fmul_rn(r, r);
-                float m = ci == 1 ? 3.402823466e+38f : min_sq[i];
-                if (v < m || ci == 1) {
-                    m = v < m ? v : m;
-                    min_sq[i] = m;
+            if (half == 0) {
+                float m = 0.f;
+                if (in) {
+                    const float r = __fsqrt_rn(__fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3)));
+                    const float v = __fmul_rn(r, r);
+                    m = ci == 1 ? 3.402823466e+38f : min_sq[i];
+                    if (v < m || ci == 1) {
+                        m = v < m ? v : m;
+                        min_sq[i] = m;
+                    }
                 }
-                s += (double)m;
+                s_m[t >> 1] = m;
             }
+            // the step's 128 values in double by one warp (see kpp_block_scan on FP64's rate)
+            __syncthreads();
+            if (t < 32) {
+                s += ((double)s_m[t] + (double)s_m[t + 32]) + ((double)s_m[t + 64] + (double)s_m[t + 96]);
+                __syncwarp();
+            }
+            if (i0 + KPP_ROWS < b1) __syncthreads();
         }
-        double tot;
-        kpp_block_scan(s, &tot);
-        if (t == 0) part[blockIdx.x] = tot;
+        if (t < 32) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (t == 0) part[blockIdx.x] = s;
+        }
     }
     if (!kpp_last_block(done)) return;
 
@@ -163,25 +186,30 @@ __global__ void __launch_bounds__(KPP_NT) kpp_kernel(const float *__restrict__ X
         s_base = 0.0;
         s_chosen = (unsigned long long)(n - 1);
     }
-    // the chunk that holds the point: every thread walks a contiguous span of chunk sums
-    const int span = (P + KPP_NT - 1) / KPP_NT;
-    const int p0 = min(P, t * span), p1 = min(P, p0 + span);
+    // the chunk that holds the point: every thread has KPP_SPAN neighbouring chunk sums
+    double ps[KPP_SPAN];
+#pragma unroll
+    for (int i = 0; i < KPP_SPAN; ++i) {
+        const int p = t * KPP_SPAN + i;
+        ps[i] = p < P ? __ldcg(part + p) : 0.0;
+    }
+    const int pick_threads = (P + KPP_SPAN - 1) / KPP_SPAN;
     double own = 0.0;
-    for (int p = p0; p < p1; ++p) own += __ldcg(part + p);
+    if ((t & ~31) < pick_threads) own = (ps[0] + ps[1]) + (ps[2] + ps[3]);
     double total;
-    const double pre = kpp_block_scan(own, &total);
+    const double pre = kpp_block_scan(own, &total, pick_threads);
     const double r = (double)u * total;
     const double band = 4.0 * (double)n * 1.1102230246251565e-16 * total;  // 2 x 2 (n - 1) 2^-53 total, rounded up
     int mine = P;
     double mbase = 0.0;
-    {
+    if ((t & ~31) < pick_threads) {
         double cum = pre;
-        for (int p = p0; p < p1; ++p) {
-            const double nx = cum + __ldcg(part + p);
-            if (nx >= r) {
-                mine = p;
+#pragma unroll
+        for (int i = 0; i < KPP_SPAN; ++i) {
+            const double nx = cum + ps[i];
+            if (mine == P && nx >= r && t * KPP_SPAN + i < P) {
+                mine = t * KPP_SPAN + i;
                 mbase = cum;
-                break;
             }
             cum = nx;
         }
@@ -196,14 +224,15 @@ __global__ void __launch_bounds__(KPP_NT) kpp_kernel(const float *__restrict__ X
         const int64_t c0 = (int64_t)b * chunk, c1 = min(n, c0 + chunk);
         const int64_t per = (c1 - c0 + KPP_NT - 1) / KPP_NT;
         const int64_t e0 = min(c1, c0 + t * per), e1 = min(c1, e0 + per);
+        const int chunk_threads = (int)((c1 - c0 + per - 1) / per);
         double ls = 0.0;
         for (int64_t i = e0; i < e1; ++i) ls += (double)__ldcg(min_sq + i);
         double lt;
-        double cum = s_base + kpp_block_scan(ls, &lt);  // running sum before this thread's piece
+        double cum = s_base + kpp_block_scan(ls, &lt, chunk_threads);  // running sum before this thread's piece
         int64_t found = -1;
         double before = 0.0, at = 0.0;
         for (int64_t i = e0; i < e1; ++i) {
-            const double nx = cum + (double)__ldcg(min_sq + i);
+            const double nx = per == 1 ? cum + ls : cum + (double)__ldcg(min_sq + i);
             if (nx >= r) {
                 found = i;
                 before = cum;
@@ -357,8 +386,7 @@ int kmeans_l2_device(const float *X, int64_t n, int d, int dp, int64_t k, int64_
     GN_CUDA_TRY(cudaMemcpyAsync(C, X + pick_point(rng) * dp, row_bytes, cudaMemcpyDeviceToDevice, st));
     DBuf dmin, dpart, ddone;
     GN_TRY(dmin.ensure((size_t)n * sizeof(float)));
-    // a block of 256 threads takes 128 rows a step; at most 1024 chunk sums
-    const int64_t chunk = std::max<int64_t>(KPP_NT / 2, round_up(ceil_div(n, 1024), KPP_NT / 2));
+    const int64_t chunk = round_up(ceil_div(n, KPP_NT * KPP_SPAN), KPP_ROWS);
     const int P = (int)ceil_div(n, chunk);
     GN_TRY(dpart.ensure((size_t)P * sizeof(double)));
     GN_TRY(ddone.ensure(sizeof(unsigned)));
@@ -407,18 +435,26 @@ void row_norms(const float *X, int64_t n, int dp, float *out, cudaStream_t st) {
 }
 
 // ── binary k-means ────────────────────────────────────────────────────────
+// This thread's KPP_SPAN neighbouring sums of the P chunks, and their total.
+__device__ __forceinline__ int64_t bin_span(const int64_t *sums, int P, int64_t (&ps)[KPP_SPAN]) {
+#pragma unroll
+    for (int i = 0; i < KPP_SPAN; ++i) {
+        const int p = threadIdx.x * KPP_SPAN + i;
+        ps[i] = p < P ? __ldcg(sums + p) : 0;
+    }
+    return (ps[0] + ps[1]) + (ps[2] + ps[3]);
+}
+
 // The point of the running sums: the first index i with min_d[0] + .. +
 // min_d[i] > r (0 <= r < total), exact in int64, by one block: sums holds the
 // sums of P chunks of `chunk` rows, pre this thread's running sum before its
-// span of them.  Writes row i of X to C[ci].
+// KPP_SPAN sums ps.  Writes row i of X to C[ci].
 __device__ __forceinline__ void bin_pick(const uint4 *__restrict__ X, int64_t n, int w4, uint4 *C, int64_t ci,
-                                         const int32_t *min_d, int64_t chunk, int P, const int64_t *sums, int64_t r,
-                                         int64_t pre) {
+                                         const int32_t *min_d, int64_t chunk, const int64_t (&ps)[KPP_SPAN],
+                                         int64_t r, int64_t pre) {
     __shared__ int s_chunk;
     __shared__ int64_t s_before, s_row;
     const int t = threadIdx.x;
-    const int span = (P + KPP_NT - 1) / KPP_NT;
-    const int p0 = min(P, t * span), p1 = min(P, p0 + span);
     if (t == 0) {  // in range whatever r is
         s_chunk = 0;
         s_before = 0;
@@ -426,13 +462,13 @@ __device__ __forceinline__ void bin_pick(const uint4 *__restrict__ X, int64_t n,
     }
     __syncthreads();
     int64_t cum = pre;
-    for (int p = p0; p < p1; ++p) {  // sums are not negative: exactly one chunk takes the running sum past r
-        const int64_t v = __ldcg(sums + p);
-        if (cum <= r && cum + v > r) {
-            s_chunk = p;
+#pragma unroll
+    for (int i = 0; i < KPP_SPAN; ++i) {  // sums are not negative: exactly one chunk takes the running sum past r
+        if (cum <= r && cum + ps[i] > r) {
+            s_chunk = t * KPP_SPAN + i;
             s_before = cum;
         }
-        cum += v;
+        cum += ps[i];
     }
     __syncthreads();
     const int64_t c0 = (int64_t)s_chunk * chunk, c1 = min(n, c0 + chunk);
@@ -442,7 +478,7 @@ __device__ __forceinline__ void bin_pick(const uint4 *__restrict__ X, int64_t n,
     for (int64_t i = e0; i < e1; ++i) ls += __ldcg(min_d + i);
     cum = s_before + kpp_block_scan(ls, &lt);
     for (int64_t i = e0; i < e1; ++i) {
-        const int64_t v = __ldcg(min_d + i);
+        const int64_t v = per == 1 ? ls : __ldcg(min_d + i);
         if (cum <= r && cum + v > r) s_row = i;
         cum += v;
     }
@@ -477,7 +513,7 @@ __device__ __forceinline__ uint32_t bin_draw(const uint32_t *__restrict__ raw, i
 // was used).  raw == NULL: the last block only writes the total, and the host
 // draws (bin_pick_kernel follows).
 // 200k x 32 bytes, 255 draws: 58.6 ms with one thread walking the sums and two
-// host round trips per draw, 1.3 ms as one launch each.
+// host round trips per draw, 2.4 ms as one launch each.
 __global__ void __launch_bounds__(KPP_NT) bin_kpp_kernel(const uint4 *__restrict__ X, int64_t n, int w4, uint4 *C,
                                                          int64_t ci, int32_t *min_d, int64_t chunk, int P,
                                                          int64_t *sums, unsigned *done,
@@ -498,11 +534,8 @@ __global__ void __launch_bounds__(KPP_NT) bin_kpp_kernel(const uint4 *__restrict
     if (t == 0) sums[blockIdx.x] = tot;
     if (!kpp_last_block(done)) return;
 
-    const int span = (P + KPP_NT - 1) / KPP_NT;
-    const int p0 = min(P, t * span), p1 = min(P, p0 + span);
-    int64_t own = 0, total;
-    for (int p = p0; p < p1; ++p) own += __ldcg(sums + p);
-    const int64_t pre = kpp_block_scan(own, &total);
+    int64_t ps[KPP_SPAN], total;
+    const int64_t pre = kpp_block_scan(bin_span(sums, P, ps), &total);
     if (!raw) {
         if (t == 0) *total_out = total;
         return;
@@ -517,7 +550,7 @@ __global__ void __launch_bounds__(KPP_NT) bin_kpp_kernel(const uint4 *__restrict
     }
     __syncthreads();
     if (s_r >= 0) {
-        bin_pick(X, n, w4, C, ci, min_d, chunk, P, sums, s_r, pre);
+        bin_pick(X, n, w4, C, ci, min_d, chunk, ps, s_r, pre);
     } else {  // every row equals a centroid: the first draw stands
         for (int j = t; j < w4; j += KPP_NT) C[ci * w4 + j] = X[s_first * w4 + j];
     }
@@ -527,13 +560,9 @@ __global__ void __launch_bounds__(KPP_NT) bin_kpp_kernel(const uint4 *__restrict
 __global__ void __launch_bounds__(KPP_NT) bin_pick_kernel(const uint4 *__restrict__ X, int64_t n, int w4, uint4 *C,
                                                           int64_t ci, const int32_t *min_d, int64_t chunk, int P,
                                                           const int64_t *sums, int64_t r) {
-    const int t = threadIdx.x;
-    const int span = (P + KPP_NT - 1) / KPP_NT;
-    const int p0 = min(P, t * span), p1 = min(P, p0 + span);
-    int64_t own = 0, total;
-    for (int p = p0; p < p1; ++p) own += __ldcg(sums + p);
-    const int64_t pre = kpp_block_scan(own, &total);
-    bin_pick(X, n, w4, C, ci, min_d, chunk, P, sums, r, pre);
+    int64_t ps[KPP_SPAN], total;
+    const int64_t pre = kpp_block_scan(bin_span(sums, P, ps), &total);
+    bin_pick(X, n, w4, C, ci, min_d, chunk, ps, r, pre);
 }
 
 // assignment to the first nearest centroid; centroids staged in shared memory
@@ -572,7 +601,7 @@ __global__ void bin_assign_kernel(const uint4 *__restrict__ X, int64_t n, int w4
 // shared counters as 16 atomic additions of two 16-bit counters each (bits b
 // and b + 16; a chunk has at most BC_ROWS < 65536 rows), and the block adds
 // its totals to the global counts once: 200k x 256 bits, 256 clusters: one
-// global atomic per set bit took 208 us, this 12 us.
+// global atomic per set bit took 208 us, this 18 us.
 constexpr int BC_SLAB = 1024, BC_ROWS = 8192, BC_NT = 512;
 __global__ void __launch_bounds__(BC_NT) bin_bitcount_kernel(const uint32_t *__restrict__ X, int64_t n, int w32,
                                                              int rows, const int32_t *__restrict__ labels, int k,
@@ -626,8 +655,7 @@ int kmeans_bin_device(const uint8_t *X, int64_t n, int nbytes, int w4, int32_t k
     const uint4 *X4 = reinterpret_cast<const uint4 *>(X);
     GN_CUDA_TRY(cudaMemcpyAsync(C, X + pick(rng) * row, row, cudaMemcpyDeviceToDevice, st));
     DBuf dmin, dsums, daux, draw;
-    // chunk sums: blocks of 256 rows a step, about four blocks per SM slot at most
-    const int64_t chunk = std::max<int64_t>(KPP_NT, round_up(ceil_div(n, 2048), KPP_NT));
+    const int64_t chunk = round_up(ceil_div(n, KPP_NT * KPP_SPAN), KPP_NT);
     const int P = (int)ceil_div(n, chunk);
     GN_TRY(dmin.ensure((size_t)n * 4));
     GN_TRY(dsums.ensure((size_t)P * 8));

@@ -1,32 +1,48 @@
-// tc_scan.cu — tensor-core L2 candidate stage: BF16 GEMM on tcgen05 with a
-// fused per-query top-S epilogue, and the exact FP32 re-rank that follows it.
+// tc_scan.cu — tensor-core candidate scans: a tcgen05 GEMM with a fused
+// per-query top-S epilogue, and the exact FP32 re-rank that follows it.
 //
-// One persistent CTA per SM walks a list of work units.  A unit is a tile of up
-// to 128 "A" rows (queries) against a range [r0, r1) of "B" rows (database
-// rows), both K-major, in one of two precisions:
-//   BF16       K padded to a multiple of 64 elements;
-//   FP8 E4M3   with one FP32 scale per row (row = scale x E4M3 values, the
-//              row's largest magnitude mapped to 448), K padded to 128;
-// either way a pipeline stage holds 128 bytes of K per row.
-//   warp 0     TMA producer: 128-byte K slices of A (128 rows) and B (256 rows)
-//              into a 2- or 3-stage shared-memory ring (128-byte swizzle);
+// Used by the flat L2 shortlist (BF16, or FP8 E4M3 with one FP32 scale per
+// row; rows scored as |x|^2 - 2 q.x) and by large batches of the exact Hamming
+// scan (bits as E4M3 +1 / -1: the inner product of two rows is nbits - 2 h,
+// exact in FP32, so the "shortlist" is the answer).
+//
+// One persistent CTA per SM walks work units.  A unit is one or two M = 128 tiles
+// of queries ("A" rows) against a chunk of the database ("B" rows, taken 256 at
+// a time), all K-major; a pipeline stage holds 128 bytes of K per row.
+//   warp 0     TMA producer: the unit's queries once (where their K fits shared
+//              memory: "resident"), then 256-row, 128-byte K slices of the
+//              database into a ring (otherwise a query slice rides along), and
+//              the rows' norms into a ring of their own;
 //   warp 1     allocates 512 TMEM columns, one thread issues tcgen05.mma
-//              (M=128, N=256, K=16 BF16 or K=32 FP8) into one of two
-//              256-column accumulators;
-//   warps 2-9  epilogue: tcgen05.ld of the accumulator rows of their TMEM lane
-//              quadrant, half of the columns each; score = |x|^2 - 2 q.x
-//              (exact FP32 |x|^2; FP8: q.x = scale_q scale_x acc); each thread
-//              owns one query row and keeps the S best (score, row) keys of its
-//              columns in a shared-memory max-heap.  A block of 32 scores is
-//              first reduced to its minimum, which is compared with the
-//              threshold (the heap's root, and the other half's root): most
-//              blocks end there, the rest are filtered score by score.
-// At the end of a unit each query's S keys go to its partial slot.  A full
-// list's S-th best score is published as the query's bound (atomicMin) every
-// tile, and every tile reads it back, so the units of a query that run at the
-// same time (its other database chunks) and later ones filter below it; the re-rank kernel
-// merges a query's slots, keeps the S best by BF16 score, recomputes their
-// distances exactly in FP32 and returns the k nearest.
+//              (M=128, N=256) into one of two 256-column accumulators, query
+//              tile by query tile for each database tile;
+//   warps 2-17 epilogue: TMEM lane quadrant x column quarter; thread = query.
+//              tcgen05.ld of 32 columns at a time; a block's smallest score
+//              against the query's threshold ends most blocks.
+//              Passing (score, row) pairs are appended to the query's buffer
+//              in global memory (a plain store, no list is kept in order);
+//              only a buffer that fills is sorted, by its warp, down to the S
+//              best, whose last is the new threshold.
+// At the end of a unit each thread appends its buffer (at most the S best of it)
+// to the query's candidate list, whose length the re-rank reads.
+//
+// What makes passing scores rare is the bound that every unit starts from.
+// With a warp's 32 lanes being 32 queries, a block of 32 x 32 scores is only
+// cheap when none of 1,024 passes.  So a pilot launch of the same pipeline first
+// scores every 8th tile or so and keeps, per query, only the minima of groups
+// of rows (32 per unit, one per column of a block: no insertion, no branch).
+// The S-th smallest minimum over at least S groups is a score that at least S
+// rows reach, hence an upper bound of the query's S-th best score, and close
+// to the sample's own S-th best (1/8 of the rows: about 320 rows of the
+// database pass instead of 1,600 per unit from empty lists).  Rows at the bound pass,
+// so the S best (score, row) keys are the same as without it.
+//
+// Two query tiles per unit (where a whole database tile fits the ring, K of at
+// most 256 bytes) because one, with its queries streamed next to each database
+// slice, read 30 GB through L2 for 1M x 128 and 10k queries and kept to 1.0 of
+// 1.93 PFLOP/s without any epilogue work; resident queries used twice read 10 GB.
+// N = 256 rather than 128 because the issuing thread's waits and commits, about
+// 300 cycles each, stand beside every 128 bytes of K.
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
 
@@ -35,6 +51,7 @@
 #include <vector>
 
 #include "distance.cuh"
+#include "f32x2.cuh"
 #include "gemm_topk.cuh"
 #include "index.cuh"
 #include "kmeans.cuh"
@@ -46,90 +63,149 @@
 
 namespace gn {
 
-constexpr int TC_M = 128, TC_N = 256, TC_BK = 64;  // TC_BK: BF16 elements per 128-byte K slice
-constexpr int TC_BK8 = 128;                          // FP8 elements per 128-byte K slice
-constexpr int TC_A_BYTES = TC_M * TC_BK * 2;   // 16 KB
-constexpr int TC_B_BYTES = TC_N * TC_BK * 2;   // 32 KB
-constexpr int TC_STAGE_BYTES = TC_A_BYTES + TC_B_BYTES;
-// Epilogue warps: 8, two per TMEM lane quadrant, each covering half of the
-// accumulator's columns (top-S mode: each thread keeps a query row's list for
-// its half; the halves merge at the end of a unit).
-__host__ __device__ constexpr int tc_nepi(int S) { return 8; }
-__host__ __device__ constexpr int tc_threads(int S) { return 64 + 32 * tc_nepi(S); }
-// pipeline depth: three stages, two where the lists need the room (S above
-// 40; S = 40 with FP8's column scales)
-__host__ __device__ constexpr int tc_stages(int S, bool f8 = false) { return S > 40 || (S > 32 && f8) ? 2 : 3; }
+constexpr int TC_M = 128, TC_N = 256;   // queries per MMA tile, database rows per tile
+constexpr int TC_BK = 64;               // BF16 elements per 128-byte K slice
+constexpr int TC_BK8 = 128;             // FP8 elements per 128-byte K slice
+constexpr int TC_ASLICE = TC_M * 128;   // bytes of a K slice of a query tile
+constexpr int TC_BSLICE = TC_N * 128;   // ... of a database tile
+constexpr int TC_NEPI = 16;             // epilogue warps: TMEM lane quadrant x column quarter (eight warps of
+                                        // two quarters each were bound by their own latency: 440 cycles a block)
+constexpr int TC_COLS = TC_N / (TC_NEPI / 4);  // columns of a tile per epilogue warp
+constexpr int TC_THREADS = 64 + 32 * TC_NEPI;
+constexpr int TC_MAX_STAGES = 6;
+constexpr int TC_NR = 4;                // tiles of row norms (and scales) in flight
+constexpr int TC_CAP = 128;             // entries of a buffer (S <= 64, and a block adds up to 32)
 
-__host__ __device__ constexpr size_t tc_smem_bytes(int S, bool f8 = false) {
-    // S == 0 is the store mode: a 32x33 transpose tile per epilogue warp;
-    // top-S mode: two lists (one per column half) of S keys per query row;
-    // per epilogue warp 32 column norms (and, FP8, 32 column scales)
-    return 1024 /*alignment slack*/ + (size_t)tc_stages(S, f8) * TC_STAGE_BYTES +
-           (S ? (size_t)2 * TC_M * S * 8 : (size_t)tc_nepi(S) * 32 * 33 * 4) +
-           (size_t)tc_nepi(S) * 32 * 4 * (f8 ? 2 : 1) + 256;
+// Shared memory: [queries, resident: qt x nk slices][ring][norms, scales of TC_NR tiles][barriers].
+struct TcGeom {
+    int nk, qt, resident, stages;
+    size_t stage_bytes, smem;
+};
+static TcGeom tc_geom(int nk, bool pilot) {
+    constexpr size_t fixed = 1024 + (size_t)TC_NR * TC_N * 4 * 2 + 256;  // alignment, norms and scales, barriers
+    constexpr size_t room = 227 * 1024 - fixed;
+    TcGeom g;
+    g.nk = nk;
+    g.qt = nk <= 2 && !pilot ? 2 : 1;  // the pilot keeps its minima in registers: one query tile
+    g.resident = nk <= 6;
+    g.stage_bytes = g.resident ? TC_BSLICE : TC_BSLICE + TC_ASLICE;
+    const size_t a = g.resident ? (size_t)nk * g.qt * TC_ASLICE : 0;
+    g.stages = (int)std::min<size_t>(TC_MAX_STAGES, (room - a) / g.stage_bytes);
+    g.smem = fixed + a + (size_t)g.stages * g.stage_bytes;
+    return g;
 }
 
-// Max-heap of S keys in a thread's strided shared-memory list (element i at
-// L[i * TC_M]): replace the root (the largest) by a smaller key and sift down.
-__device__ __noinline__ void tc_heap_replace_top(uint64_t *L, int S, uint64_t key) {
-    int i = 0;
-    while (true) {
-        const int c = 2 * i + 1;
-        if (c >= S) break;
-        uint64_t cv = L[c * TC_M];
-        int cm = c;
-        if (c + 1 < S) {
-            const uint64_t c2 = L[(c + 1) * TC_M];
-            if (c2 > cv) {
-                cv = c2;
-                cm = c + 1;
+// Ascending bitonic sort of 32 R keys, element r * 32 + lane in v[r].
+template <int R>
+__device__ __forceinline__ void warp_sort(uint64_t (&v)[R]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int size = 2; size <= 32 * R; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            if (stride >= 32) {
+                const int rs = stride / 32;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (r & rs) continue;
+                    const bool up = ((r * 32) & size) == 0;  // size > stride >= 32: the lane has no say
+                    const uint64_t a = v[r], b = v[r | rs];
+                    const bool swap = (a > b) == up;
+                    v[r] = swap ? b : a;
+                    v[r | rs] = swap ? a : b;
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const uint64_t o = __shfl_xor_sync(0xffffffffu, v[r], stride);
+                    const bool up = ((r * 32 + lane) & size) == 0;
+                    const bool low = (lane & stride) == 0;
+                    const bool keep_min = up == low;
+                    v[r] = keep_min == (o < v[r]) ? o : v[r];
+                }
             }
         }
-        if (cv <= key) break;
-        L[i * TC_M] = cv;
-        i = cm;
     }
-    L[i * TC_M] = key;
 }
 
-template <int S, bool F8>
-__global__ void __launch_bounds__(tc_threads(S), 1)
-    tc_topk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                   const TcUnit *__restrict__ units, const int64_t *__restrict__ n_units_ptr,
-                   const int64_t *__restrict__ cta_off, int K, int kblk,
-                   const float *__restrict__ bnorm, const float *__restrict__ ascale,
-                   const float *__restrict__ bscale, const int64_t *__restrict__ arow_slot,
-                   uint64_t *__restrict__ part, float *__restrict__ scores, uint32_t *__restrict__ qbound,
-                   int *__restrict__ err) {
-    constexpr bool STORE = (S == 0);
-    static_assert(!(STORE && F8), "the store mode is BF16 only");
-    constexpr int SL = STORE ? 1 : 2 * S;  // list keys per query row (two column halves)
-    constexpr int NEPI = tc_nepi(S);
-    constexpr int TC_STAGES = tc_stages(S, F8);
+// A buffer entry is (score bits, row); keys order by (score, row).  (Signs: the
+// score is -(inner product) = 2 h - nbits, and the candidate list gets (h, row).)
+__device__ __forceinline__ uint64_t tc_entry_key(const uint2 *buf, int i, int cnt) {
+    if (i >= cnt) return KEY_EMPTY;
+    const uint2 e = buf[i];
+    return make_key(f2ord(__uint_as_float(e.x)), e.y);
+}
+
+// The warp sorts the first cnt entries of buf (cnt <= 32 R), writes the S best
+// back, and returns the S-th key (KEY_EMPTY if there are fewer).
+template <int R>
+__device__ __forceinline__ uint64_t tc_compact(uint2 *buf, int cnt, int S) {
+    const int lane = threadIdx.x & 31;
+    uint64_t v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = tc_entry_key(buf, r * 32 + lane, cnt);
+    warp_sort<R>(v);
+    __syncwarp();
+    uint64_t last = KEY_EMPTY;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int p = r * 32 + lane;
+        if (p < S && v[r] != KEY_EMPTY) buf[p] = make_uint2(__float_as_uint(ord2f(key_dist(v[r]))), key_idx(v[r]));
+        if (r == (S - 1) / 32) last = __shfl_sync(0xffffffffu, v[r], (S - 1) & 31);
+    }
+    __syncwarp();
+    return last;
+}
+
+__device__ __forceinline__ float min3(float a, float b, float c) {
+    float r;
+    asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
+// MODE: operand form.  PILOT: group minima of the sampled tiles instead of lists.
+// QT: query tiles per unit.  Tile i of the launch is database tile i * tstride;
+// unit u is (chunk u / nqp of the tiles, queries 128 QT (u % nqp) ..): chunk-major,
+// so that the CTAs running together scan the same chunk and L2 serves it.
+template <int MODE, bool PILOT, int QT>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+    tc_topk_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, TcScanArgs a) {
+    static_assert(!PILOT || QT == 1, "the pilot's minima are one query tile's");
+    constexpr int UQ = TC_M * QT;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint8_t *stage_base = smem;
-    uint64_t *lists = reinterpret_cast<uint64_t *>(smem + TC_STAGES * TC_STAGE_BYTES);  // [2][S][TC_M]
-    float *xpose = reinterpret_cast<float *>(smem + TC_STAGES * TC_STAGE_BYTES);  // store mode: [NEPI][32][33]
-    float *snorm = STORE ? xpose + NEPI * 32 * 33 : reinterpret_cast<float *>(lists + TC_M * SL);
-    float *sscale = snorm + NEPI * 32;  // FP8: per-warp column scales
-    uint64_t *bars = reinterpret_cast<uint64_t *>(snorm + NEPI * 32 * (F8 ? 2 : 1));
-    uint64_t *full = bars, *empty = bars + TC_STAGES, *accfull = bars + 2 * TC_STAGES,
-             *accempty = bars + 2 * TC_STAGES + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * TC_STAGES + 4);
+    const int nk = a.nk, ST = a.stages;
+    const bool res = QT == 2 || a.resident != 0;
+    const uint32_t stage_bytes = res ? TC_BSLICE : TC_BSLICE + TC_ASLICE;
+    uint8_t *sA = smem;  // resident queries: slice (qt, kb) at (qt * nk + kb) * TC_ASLICE
+    uint8_t *ring = smem + (res ? (size_t)nk * QT * TC_ASLICE : 0);  // stage: database slice [, query slice]
+    float *snorm = reinterpret_cast<float *>(ring + (size_t)ST * stage_bytes);  // [TC_NR][TC_N] norms, then scales
+    float *sscale = snorm + TC_NR * TC_N;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sscale + TC_NR * TC_N);
+    uint64_t *full = bars, *empty = bars + TC_MAX_STAGES, *nfull = bars + 2 * TC_MAX_STAGES, *nempty = nfull + TC_NR,
+             *accfull = nempty + TC_NR, *accempty = accfull + 2, *afull = accfull + 4, *aempty = accfull + 5,
+             *drain = accfull + 6;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(accfull + 7);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    volatile int *verr = err;
+    volatile int *verr = a.err;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < TC_STAGES; ++s) {
+        for (int s = 0; s < ST; ++s) {
             mbar_init(full + s, 1);
             mbar_init(empty + s, 1);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(accfull + b, 1);
-            mbar_init(accempty + b, NEPI);
+            mbar_init(accempty + b, TC_NEPI);
         }
+        for (int b = 0; b < TC_NR; ++b) {
+            mbar_init(nfull + b, 1);
+            mbar_init(nempty + b, TC_NEPI);
+        }
+        mbar_init(afull, 1);
+        mbar_init(aempty, 1);
+        mbar_init(drain, 1);
         mbar_fence_init();
     }
     if (warp == 1) tmem_alloc(tmem_slot, 512);
@@ -138,289 +214,321 @@ __global__ void __launch_bounds__(tc_threads(S), 1)
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // this CTA's units: [u_begin, u_end) with stride u_step
-    const int64_t n_units = *n_units_ptr;
-    int64_t u_begin = blockIdx.x, u_end = n_units, u_step = gridDim.x;
-    if (cta_off) {
-        u_begin = cta_off[blockIdx.x];
-        u_end = cta_off[blockIdx.x + 1];
-        u_step = 1;
-    }
-    const int nk = K / kblk;
+    const int64_t nqp = (a.nq + UQ - 1) / UQ;
+    const int64_t n_units = nqp * a.nchunks;
+    auto unit = [&](int64_t u, int64_t &q0, int &na, int64_t &t0, int64_t &t1) {
+        const int64_t c = u / nqp;
+        q0 = (u % nqp) * UQ;
+        na = (int)min((int64_t)UQ, a.nq - q0);
+        t0 = a.ntiles * c / a.nchunks;
+        t1 = a.ntiles * (c + 1) / a.nchunks;
+        return c;
+    };
 
     if (warp == 0) {
         // ── TMA producer ──
         if (lane == 0) {
-            uint32_t it = 0;
+            uint32_t it = 0, un = 0, tile_it = 0;
+            int sl = 0;
+            uint32_t ph = 1;  // parity of the ring pass before this one: slots start free
             bool ok = true;
-            for (int64_t u = u_begin; u < u_end && ok; u += u_step) {
-                const TcUnit un = units[u];
-                const int ntile = (int)((un.r1 - un.r0 + TC_N - 1) / TC_N);
-                for (int t = 0; t < ntile && ok; ++t)
-                    for (int kb = 0; kb < nk && ok; ++kb, ++it) {
-                        const int s = it % TC_STAGES;
-                        const uint32_t ph = (it / TC_STAGES) & 1;
-                        if (!mbar_wait(empty + s, ph ^ 1, verr)) { ok = false; break; }
-                        uint8_t *sa = stage_base + s * TC_STAGE_BYTES;
-                        mbar_expect_tx(full + s, TC_STAGE_BYTES);
-                        tma_load_2d(sa, &tmA, kb * kblk, (int)un.a0, full + s);
-                        tma_load_2d(sa + TC_A_BYTES, &tmB, kb * kblk, (int)(un.r0 + (int64_t)t * TC_N), full + s);
+            for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++un) {
+                int64_t q0, t0, t1;
+                int na;
+                unit(u, q0, na, t0, t1);
+                const int nqt = QT == 2 && na > TC_M ? 2 : 1;
+                if (res) {  // the unit's queries, once the previous unit's MMAs have read theirs
+                    if (!mbar_wait(aempty, (un & 1) ^ 1, verr)) { ok = false; break; }
+                    mbar_expect_tx(afull, (uint32_t)(nqt * nk) * TC_ASLICE);
+                    for (int qt = 0; qt < nqt; ++qt)
+                        for (int kb = 0; kb < nk; ++kb)
+                            tma_load_2d(sA + (size_t)(qt * nk + kb) * TC_ASLICE, &tmA, kb * a.kblk,
+                                        (int)(q0 + qt * TC_M), afull);
+                }
+                for (int64_t t = t0; t < t1 && ok; ++t, ++tile_it) {
+                    const int n0 = (int)(t * a.tstride * TC_N);
+                    for (int kb = 0; kb < nk; ++kb, ++it) {
+                        if (!mbar_wait(empty + sl, ph, verr)) { ok = false; break; }
+                        uint8_t *sb = ring + (size_t)sl * stage_bytes;
+                        mbar_expect_tx(full + sl, stage_bytes);
+                        tma_load_2d(sb, &tmB, kb * a.kblk, n0, full + sl);
+                        if (!res) tma_load_2d(sb + TC_BSLICE, &tmA, kb * a.kblk, (int)q0, full + sl);
+                        if (++sl == ST) {
+                            sl = 0;
+                            ph ^= 1;
+                        }
                     }
+                    if (MODE != TC_SIGN && ok) {
+                        const int ns = tile_it % TC_NR;
+                        if (!mbar_wait(nempty + ns, ((tile_it / TC_NR) & 1) ^ 1, verr)) { ok = false; break; }
+                        mbar_expect_tx(nfull + ns, TC_N * 4 * (MODE == TC_FP8 ? 2 : 1));
+                        bulk_load(snorm + ns * TC_N, a.bnorm + n0, TC_N * 4, nfull + ns);
+                        if (MODE == TC_FP8) bulk_load(sscale + ns * TC_N, a.bscale + n0, TC_N * 4, nfull + ns);
+                    }
+                }
+            }
+            if (!ok) {  // let the copies in flight land (bounded) before the CTA ends
+                auto settle = [&](uint64_t *bar, uint32_t parity) {
+                    const long long c0 = clock64();
+                    while (!mbar_try_wait(bar, parity) && clock64() - c0 < 400000) {
+                    }
+                };
+                for (uint32_t x = it > (uint32_t)ST ? it - ST : 0; x < it; ++x) settle(full + x % ST, (x / ST) & 1);
+                if (MODE != TC_SIGN)
+                    for (uint32_t x = tile_it > TC_NR ? tile_it - TC_NR : 0; x < tile_it; ++x)
+                        settle(nfull + x % TC_NR, (x / TC_NR) & 1);
+                if (res) settle(afull, un & 1);
             }
         }
     } else if (warp == 1) {
         // ── MMA issuer ──
         if (lane == 0) {
-            const uint32_t idesc = F8 ? idesc_e4m3_f32(TC_M, TC_N) : idesc_bf16_f32(TC_M, TC_N);
-            uint32_t it = 0, tile_it = 0;
+            constexpr uint32_t idesc = MODE == TC_BF16 ? idesc_bf16_f32(TC_M, TC_N) : idesc_e4m3_f32(TC_M, TC_N);
+            const uint64_t ring_desc = sdesc_sw128(smem_u32(ring)), a_desc = sdesc_sw128(smem_u32(sA));
+            const uint32_t stage16 = stage_bytes >> 4;  // descriptor addresses count 16-byte units
+            uint32_t vt = 0, un = 0, ph = 0, sl = 0;    // vt: accumulators filled so far
             bool ok = true;
-            for (int64_t u = u_begin; u < u_end && ok; u += u_step) {
-                const TcUnit un = units[u];
-                const int ntile = (int)((un.r1 - un.r0 + TC_N - 1) / TC_N);
-                for (int t = 0; t < ntile && ok; ++t, ++tile_it) {
-                    const int b = tile_it & 1;
-                    const uint32_t tph = (tile_it >> 1) & 1;
-                    if (!mbar_wait(accempty + b, tph ^ 1, verr)) { ok = false; break; }
-                    tc_fence_after();
-                    const uint32_t dt = tmem + (uint32_t)(b * TC_N);
-                    for (int kb = 0; kb < nk; ++kb, ++it) {
-                        const int s = it % TC_STAGES;
-                        const uint32_t ph = (it / TC_STAGES) & 1;
-                        if (!mbar_wait(full + s, ph, verr)) { ok = false; break; }
+            for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++un) {
+                int64_t q0, t0, t1;
+                int na;
+                unit(u, q0, na, t0, t1);
+                const int nqt = QT == 2 && na > TC_M ? 2 : 1;
+                if (res && !mbar_wait(afull, un & 1, verr)) { ok = false; break; }
+                const int tiles = (int)(t1 - t0);
+                for (int t = 0; t < tiles && ok; ++t) {
+                    for (int qt = 0; qt < nqt && ok; ++qt, ++vt) {
+                        const uint32_t b = vt & 1;
+                        if (!mbar_wait(accempty + b, ((vt >> 1) & 1) ^ 1, verr)) { ok = false; break; }
                         tc_fence_after();
-                        const uint32_t sa = smem_u32(stage_base + s * TC_STAGE_BYTES);
-                        const uint64_t da = sdesc_sw128(sa), db = sdesc_sw128(sa + TC_A_BYTES);
-                        // four MMAs of 32 bytes of K each (16 BF16 or 32 FP8 elements):
-                        // the descriptors advance by 32 bytes (2 in 16-byte units)
+                        const uint32_t dt = tmem + b * TC_N;
+                        uint32_t s = sl, sph = ph;  // each query tile takes the tile's slices anew
+                        for (int kb = 0; kb < nk; ++kb) {
+                            if (qt == 0) {
+                                if (!mbar_wait(full + s, sph, verr)) { ok = false; break; }
+                                tc_fence_after();
+                            }
+                            const uint64_t db = ring_desc + s * stage16;
+                            const uint64_t da = res ? a_desc + (uint32_t)(qt * nk + kb) * (TC_ASLICE >> 4)
+                                                    : db + (TC_BSLICE >> 4);
+                            // four MMAs of 32 bytes of K each (16 BF16 or 32 FP8 elements):
+                            // the descriptors advance by 32 bytes (2 in 16-byte units)
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {
-                            if constexpr (F8) umma_f8(dt, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
-                            else umma_bf16(dt, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+                            for (int kk = 0; kk < 4; ++kk) {
+                                if constexpr (MODE == TC_BF16)
+                                    umma_bf16(dt, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+                                else
+                                    umma_f8(dt, da + 2 * kk, db + 2 * kk, idesc, (kb | kk) ? 1u : 0u);
+                            }
+                            if (qt == nqt - 1) umma_commit(empty + s);
+                            if (++s == (uint32_t)ST) {
+                                s = 0;
+                                sph ^= 1;
+                            }
                         }
-                        umma_commit(empty + s);
+                        if (ok) umma_commit(accfull + b);
+                        if (qt == nqt - 1) {
+                            sl = s;
+                            ph = sph;
+                        }
                     }
-                    if (ok) umma_commit(accfull + b);
                 }
+                if (ok && res) umma_commit(aempty);
             }
-        }
-    } else if constexpr (STORE) {
-        // ── epilogue (store mode): scores of a 32x32 block go through a padded
-        // shared tile so that each store instruction writes 32 consecutive
-        // floats of one query's segment ──
-        const int quad = warp & 3;
-        const int grp = (warp - 2) >> 2;  // which half of the 256 columns
-        constexpr int CPG = (TC_N / 32) / (NEPI / 4);
-        float *xp = xpose + (warp - 2) * 32 * 33;
-        float *sn = snorm + (warp - 2) * 32;
-        uint32_t tile_it = 0;
-        bool ok = true;
-        for (int64_t u = u_begin; u < u_end && ok; u += u_step) {
-            const TcUnit un = units[u];
-            const int ntile = (int)((un.r1 - un.r0 + TC_N - 1) / TC_N);
-            // segment base of each of this warp's 32 query rows (lane r holds row r's)
-            const int qrow = quad * 32 + lane;
-            const int64_t myseg = (qrow < un.na) ? arow_slot[un.a0 + qrow] - un.rbase : INT64_MIN;
-            for (int t = 0; t < ntile; ++t, ++tile_it) {
-                const int b = tile_it & 1;
-                const uint32_t tph = (tile_it >> 1) & 1;
-                const int64_t n0 = un.r0 + (int64_t)t * TC_N;
-                float nrm[CPG];
-#pragma unroll
-                for (int cc = 0; cc < CPG; ++cc) {
-                    const int64_t col = n0 + (grp * CPG + cc) * 32 + lane;
-                    nrm[cc] = col < un.r1 ? __ldg(bnorm + col) : 0.f;
+            if (!ok) {  // the MMAs issued so far end (bounded) before the CTA does
+                umma_commit(drain);
+                const long long c0 = clock64();
+                while (!mbar_try_wait(drain, 0) && clock64() - c0 < 400000) {
                 }
-                if (!mbar_wait(accfull + b, tph, verr)) { ok = false; break; }
-                tc_fence_after();
-#pragma unroll 1
-                for (int cc = 0; cc < CPG; ++cc) {
-                    const int c = grp * CPG + cc;
-                    const int64_t col0 = n0 + c * 32;
-                    __syncwarp();
-                    sn[lane] = nrm[cc];
-                    __syncwarp();
-                    float acc[32];
-                    tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * TC_N + c * 32), acc);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) xp[lane * 33 + j] = fmaf(-2.f, acc[j], sn[j]);
-                    __syncwarp();
-                    const bool colok = col0 + lane < un.r1;
-#pragma unroll 4
-                    for (int r = 0; r < 32; ++r) {
-                        const int64_t seg = __shfl_sync(0xffffffffu, myseg, r);
-                        if (seg != INT64_MIN && colok) scores[seg + col0 + lane] = xp[r * 33 + lane];
-                    }
-                }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(accempty + b);
             }
         }
     } else {
-        // ── epilogue: warps 2..9, TMEM lane quadrant = warp % 4, column half =
-        // (warp - 2) / 4; each thread keeps the S best keys of one query row
-        // over its half of the columns at lists[(half * S + i) * TC_M + row]
-        // (bank-conflict free) as a max-heap: a new key replaces the root (the
-        // S-th best) and sifts down.  At the end of a unit the two halves of a
-        // row are merged.
-        const int quad = warp & 3, half = (warp - 2) >> 2;
-        const int row = quad * 32 + lane;
-        __shared__ volatile int pair_ok[8];
-        uint64_t *L = lists + (size_t)half * S * TC_M + row;
-        // the other half's heap root (its current S-th best key of this row):
-        // only ever holds final root values, so it can be read at any time
-        const volatile uint64_t *other_root = lists + (size_t)(half ^ 1) * S * TC_M + row;
-        float *sn = snorm + (warp - 2) * 32;
-        float *sc = sscale + (warp - 2) * 32;
-        uint32_t tile_it = 0;
+        // ── epilogue ──
+        const int quad = warp & 3, ew = warp - 2, quarter = ew >> 2;
+        uint2 *const ebuf = a.cand + ((size_t)blockIdx.x * TC_NEPI + ew) * QT * 32 * TC_CAP;  // the warp's buffers
+        const float inf = __int_as_float(0x7f800000);
+        uint32_t tile_it = 0, vt = 0;
         bool ok = true;
-        for (int64_t u = u_begin; u < u_end && ok; u += u_step) {
-            const TcUnit un = units[u];
-            const int ntile = (int)((un.r1 - un.r0 + TC_N - 1) / TC_N);
-#pragma unroll 4
-            for (int i = 0; i < S; ++i) L[i * TC_M] = KEY_EMPTY;
-            uint64_t thr = KEY_EMPTY;  // the heap's root: the S-th best key so far
-            // the query's bound from units already finished: the S-th best score of
-            // some unit's S rows, so no key above it can reach the query's S best;
-            // it caps the filter threshold for the whole unit (the list's own root
-            // only takes over once it is lower)
-            float gbound = __int_as_float(0x7f800000);  // +inf
-            if (qbound && row < un.na) {
-                const uint32_t g = *reinterpret_cast<volatile uint32_t *>(qbound + un.a0 + row);
-                if (g != 0xffffffffu) gbound = ord2f(g);
-            }
-            float thr_f = gbound;
-            // score = |x|^2 + qc * (column factor) * acc: qc = -2 (BF16) or
-            // -2 scale_q (FP8, column factor scale_x)
-            const float qc = F8 ? (row < un.na ? -2.f * __ldg(ascale + un.a0 + row) : 0.f) : -2.f;
-            asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");  // both halves reset before either reads
-            for (int t = 0; t < ntile; ++t, ++tile_it) {
-                const int b = tile_it & 1;
-                const uint32_t tph = (tile_it >> 1) & 1;
-                const int64_t n0 = un.r0 + (int64_t)t * TC_N;
-                // the query's bound as the units running beside this one (its other
-                // database chunks) have lowered it so far, read before the wait
-                uint32_t gnow = 0xffffffffu;
-                if (qbound && row < un.na) gnow = *reinterpret_cast<volatile uint32_t *>(qbound + un.a0 + row);
-                // row norms of this warp's 128 columns, fetched before the wait
-                float nrm[TC_N / 64], csc[TC_N / 64];
+        for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            int64_t q0, t0, t1;
+            int na;
+            const int64_t chunk = unit(u, q0, na, t0, t1);
+            const int nqt = QT == 2 && na > TC_M ? 2 : 1;
+            // per query tile: scores at or below thr pass; cnt of them are in the buffer.
+            // The current tile's state is thr[0], cnt[0] (the tiles take turns)
+            float thr[QT], qc[QT];
+            int cnt[QT];
 #pragma unroll
-                for (int c = 0; c < TC_N / 64; ++c) {
-                    const int64_t col = n0 + (half * (TC_N / 64) + c) * 32 + lane;
-                    nrm[c] = col < un.r1 ? __ldg(bnorm + col) : 0.f;
-                    if constexpr (F8) csc[c] = col < un.r1 ? __ldg(bscale + col) : 0.f;
+            for (int i = 0; i < QT; ++i) {
+                const int row = i * TC_M + quad * 32 + lane;  // query within the unit
+                const bool live = row < na;
+                thr[i] = live ? inf : __int_as_float(0x7fc00000);  // NaN: nothing passes
+                cnt[i] = 0;
+                if (!PILOT && live) {
+                    const uint32_t g = *reinterpret_cast<volatile uint32_t *>(a.qbound + q0 + row);
+                    if (g != 0xffffffffu) thr[i] = ord2f(g);
                 }
-                if (!mbar_wait(accfull + b, tph, verr)) { ok = false; break; }
-                tc_fence_after();
-                if (gnow != 0xffffffffu) {
-                    gbound = fminf(gbound, ord2f(gnow));
-                    thr_f = fminf(thr_f, gbound);
-                }
-                // the other half's S-th best also bounds this row: a key not below
-                // it has S better keys in the other half
-                {
-                    const uint64_t o = *other_root;
-                    if (o != KEY_EMPTY) thr_f = fminf(thr_f, ord2f(key_dist(o)));
-                }
-                // publish this half's S-th best (once its list is full) for the
-                // query's other units
-                if (qbound && thr != KEY_EMPTY && row < un.na && key_dist(thr) < gnow)
-                    atomicMin(qbound + un.a0 + row, key_dist(thr));
+                // score = |x|^2 + qc * (column factor) * acc: qc = -2 (BF16) or
+                // -2 scale_q (FP8, column factor scale_x); signs: -acc
+                qc[i] = -2.f;
+                if (MODE == TC_FP8) qc[i] = live ? -2.f * __ldg(a.ascale + q0 + row) : 0.f;
+            }
+            float g[PILOT ? 32 : 1];
+#pragma unroll
+            for (int j = 0; j < (PILOT ? 32 : 1); ++j) g[j] = inf;
+
+            for (int64_t t = t0; t < t1 && ok; ++t, ++tile_it) {
+                const int64_t n0 = t * a.tstride * TC_N + quarter * TC_COLS;
+                const bool tail = MODE == TC_SIGN && n0 + TC_COLS > a.n;
+                const int ns = tile_it % TC_NR;
+                // the tile's row norms (NaN past the last row: such scores never pass)
+                const float *sn = snorm + ns * TC_N + quarter * TC_COLS, *sc = sn + TC_NR * TC_N;
 #pragma unroll 1
-                for (int cc = 0; cc < TC_N / 64; ++cc) {
-                    const int c = half * (TC_N / 64) + cc;
-                    const int64_t col0 = n0 + c * 32;
-                    // columns past the unit's last row (the tail of its last tile,
-                    // TMA zero fill) are never offered; col0 is warp-uniform
-                    if (col0 >= un.r1) break;
-                    __syncwarp();
-                    sn[lane] = nrm[cc];
-                    if constexpr (F8) sc[lane] = csc[cc];
-                    __syncwarp();
+                for (int qt = 0; qt < nqt; ++qt, ++vt) {
+                    const int b = vt & 1;
+                    if (!mbar_wait(accfull + b, (vt >> 1) & 1, verr)) { ok = false; break; }
+                    tc_fence_after();
+                    if (MODE != TC_SIGN && qt == 0 && !mbar_wait(nfull + ns, (tile_it / TC_NR) & 1, verr)) {
+                        ok = false;
+                        break;
+                    }
+                    uint2 *const wbuf = ebuf + (size_t)qt * 32 * TC_CAP;
+                    uint2 *const buf = wbuf + (size_t)lane * TC_CAP;
+                    const f32x2 qc2 = dup2(qc[0]);
+                    const uint32_t tacc =
+                        tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * TC_N + quarter * TC_COLS);
+                    // v: accumulators of the warp's columns [32 c, 32 c + 32), then their scores
+                    auto block = [&](float (&v)[32], int c) {
+                        if (MODE == TC_SIGN) {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) v[j] = -v[j];
+                            if (tail) {
+#pragma unroll
+                                for (int j = 0; j < 32; ++j)
+                                    if (n0 + c * 32 + j >= a.n) v[j] = __int_as_float(0x7fc00000);
+                            }
+                        } else {
+                            const float4 *sn4 = reinterpret_cast<const float4 *>(sn + c * 32);
+                            const float4 *sc4 = reinterpret_cast<const float4 *>(sc + c * 32);
+#pragma unroll
+                            for (int j4 = 0; j4 < 8; ++j4) {
+                                const float4 nv = sn4[j4];
+                                f32x2 f01 = qc2, f23 = qc2;
+                                if (MODE == TC_FP8) {
+                                    const float4 sv = sc4[j4];
+                                    f01 = pack2(__fmul_rn(qc[0], sv.x), __fmul_rn(qc[0], sv.y));
+                                    f23 = pack2(__fmul_rn(qc[0], sv.z), __fmul_rn(qc[0], sv.w));
+                                }
+                                float *x = v + 4 * j4;
+                                unpack2(fma2(f01, pack2(x[0], x[1]), pack2(nv.x, nv.y)), x[0], x[1]);
+                                unpack2(fma2(f23, pack2(x[2], x[3]), pack2(nv.z, nv.w)), x[2], x[3]);
+                            }
+                        }
+                        if (PILOT) {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j) g[PILOT ? j : 0] = fminf(g[PILOT ? j : 0], v[j]);
+                            return;
+                        }
+                        float m[4];  // minima of eight columns each
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            const float *x = v + 8 * e;
+                            m[e] = min3(min3(x[0], x[1], x[2]), min3(x[3], x[4], x[5]), fminf(x[6], x[7]));
+                        }
+                        if (!__any_sync(0xffffffffu, fminf(fminf(m[0], m[1]), fminf(m[2], m[3])) <= thr[0])) return;
+                        const uint32_t col = (uint32_t)(n0 + c * 32);
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            if (!__any_sync(0xffffffffu, m[e] <= thr[0])) continue;
+#pragma unroll
+                            for (int j = 8 * e; j < 8 * e + 8; ++j)
+                                if (v[j] <= thr[0]) {
+                                    buf[cnt[0]] = make_uint2(__float_as_uint(v[j]), col + j);
+                                    ++cnt[0];
+                                }
+                        }
+                        unsigned fullm = __ballot_sync(0xffffffffu, cnt[0] > TC_CAP - 32);
+                        while (fullm) {  // the warp sorts a lane's buffer down to its S best
+                            const int l = __ffs(fullm) - 1;
+                            fullm &= fullm - 1;
+                            __syncwarp();
+                            const uint64_t last = tc_compact<TC_CAP / 32>(
+                                wbuf + (size_t)l * TC_CAP, __shfl_sync(0xffffffffu, cnt[0], l), a.S);
+                            if (lane == l) {
+                                cnt[0] = a.S;
+                                // later rows of the unit have higher indices: only lower scores displace the S-th
+                                thr[0] = fminf(thr[0], ord2f(key_dist(last) - 1));
+                            }
+                        }
+                    };
+                    static_assert(TC_COLS == 64, "two blocks per warp and tile");
                     float acc[32];
-                    tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(b * TC_N + c * 32), acc);
-                    // scores and their minimum (four independent chains)
-                    const float4 *sn4 = reinterpret_cast<const float4 *>(sn);
-                    const float4 *sc4 = reinterpret_cast<const float4 *>(sc);
-                    const float inf = __int_as_float(0x7f800000);
-                    float mn4[4] = {inf, inf, inf, inf};
-#pragma unroll
-                    for (int j4 = 0; j4 < 8; ++j4) {
-                        const float4 nv = sn4[j4];
-                        float4 cf = make_float4(qc, qc, qc, qc);
-                        if constexpr (F8) {
-                            const float4 sv = sc4[j4];
-                            cf = make_float4(qc * sv.x, qc * sv.y, qc * sv.z, qc * sv.w);
-                        }
-                        acc[4 * j4 + 0] = fmaf(cf.x, acc[4 * j4 + 0], nv.x);
-                        acc[4 * j4 + 1] = fmaf(cf.y, acc[4 * j4 + 1], nv.y);
-                        acc[4 * j4 + 2] = fmaf(cf.z, acc[4 * j4 + 2], nv.z);
-                        acc[4 * j4 + 3] = fmaf(cf.w, acc[4 * j4 + 3], nv.w);
-                        mn4[0] = fminf(mn4[0], acc[4 * j4 + 0]);
-                        mn4[1] = fminf(mn4[1], acc[4 * j4 + 1]);
-                        mn4[2] = fminf(mn4[2], acc[4 * j4 + 2]);
-                        mn4[3] = fminf(mn4[3], acc[4 * j4 + 3]);
+                    tmem_ld32(tacc, acc);
+                    block(acc, 0);
+                    tmem_ld32(tacc + 32, acc);
+                    // every column is in registers: a later tile may overwrite the accumulator
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(accempty + b);
+                    block(acc, 1);
+                    if (MODE != TC_SIGN && qt == nqt - 1) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(nempty + ns);
                     }
-                    if (!(fminf(fminf(mn4[0], mn4[1]), fminf(mn4[2], mn4[3])) <= thr_f)) continue;
-                    const int nvalid = (int)min((int64_t)32, un.r1 - col0);  // 1..32
-                    // filter: a pass mask from independent compares (four partial
-                    // masks, no serial chain); the rare passing scores are offered
-                    uint32_t pm4[4] = {0u, 0u, 0u, 0u};
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) pm4[j & 3] |= (acc[j] <= thr_f ? 1u : 0u) << j;
-                    uint32_t pm = (pm4[0] | pm4[1]) | (pm4[2] | pm4[3]);
-                    if (nvalid < 32) pm &= (1u << nvalid) - 1u;
-                    while (pm) {
-                        const int j = __ffs(pm) - 1;
-                        pm &= pm - 1;
-                        float v = acc[0];
-#pragma unroll
-                        for (int jj = 1; jj < 32; ++jj) v = jj == j ? acc[jj] : v;
-                        const uint64_t key = make_key(f2ord(v), (uint32_t)(col0 + j));
-                        if (key < thr) {
-                            tc_heap_replace_top(L, S, key);
-                            thr = L[0];
-                            thr_f = (thr == KEY_EMPTY) ? gbound : fminf(gbound, ord2f(key_dist(thr)));
-                        }
+                    if (QT == 2 && nqt == 2) {  // the other query tile's turn
+                        const float tf = thr[0], tq = qc[0];
+                        const int ti = cnt[0];
+                        thr[0] = thr[QT - 1];
+                        qc[0] = qc[QT - 1];
+                        cnt[0] = cnt[QT - 1];
+                        thr[QT - 1] = tf;
+                        qc[QT - 1] = tq;
+                        cnt[QT - 1] = ti;
                     }
                 }
-                tc_fence_before();
+            }
+            if (!ok) break;
+            if (PILOT) {
+                if (quad * 32 + lane < na) {
+                    float4 *dst = reinterpret_cast<float4 *>(
+                        a.gmin + (((q0 + quad * 32 + lane) * a.nchunks + chunk) * (TC_NEPI / 4) + quarter) * 32);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        dst[j] = make_float4(g[PILOT ? 4 * j : 0], g[PILOT ? 4 * j + 1 : 0], g[PILOT ? 4 * j + 2 : 0],
+                                             g[PILOT ? 4 * j + 3 : 0]);
+                }
+            } else {
                 __syncwarp();
-                if (lane == 0) mbar_arrive(accempty + b);
-            }
-            // merge the two halves of each row (the two warps of a quadrant meet
-            // at a named barrier and agree on whether to go on), then the
-            // first half sorts and writes
-            if (lane == 0) pair_ok[quad * 2 + half] = ok ? 1 : 0;
-            asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");
-            ok = pair_ok[quad * 2] && pair_ok[quad * 2 + 1];
-            if (half == 0 && ok) {
-                const uint64_t *L2 = L + (size_t)S * TC_M;
-                for (int i = 0; i < S; ++i) {
-                    const uint64_t key = L2[i * TC_M];
-                    if (key < thr) {
-                        tc_heap_replace_top(L, S, key);
-                        thr = L[0];
-                    }
-                }
-                if (row < un.na) {
-                    for (int i = 1; i < S; ++i) {  // ascending, for the re-rank's merge
-                        const uint64_t key = L[i * TC_M];
-                        int p = i;
-                        while (p > 0 && L[(p - 1) * TC_M] > key) {
-                            L[p * TC_M] = L[(p - 1) * TC_M];
-                            --p;
+#pragma unroll 1
+                for (int i = 0; i < nqt; ++i) {
+                    const int row = i * TC_M + quad * 32 + lane;
+                    int n = i == 0 ? cnt[0] : cnt[QT - 1];
+                    uint2 *const wbuf = ebuf + (size_t)i * 32 * TC_CAP;
+                    unsigned longm = __ballot_sync(0xffffffffu, n > a.S);
+                    while (longm) {  // only a buffer's S best can be among the query's
+                        const int l = __ffs(longm) - 1;
+                        longm &= longm - 1;
+                        const uint64_t last = tc_compact<TC_CAP / 32>(wbuf + (size_t)l * TC_CAP,
+                                                                      __shfl_sync(0xffffffffu, n, l), a.S);
+                        if (lane == l) {
+                            n = a.S;
+                            // a full list bounds the query's S-th best score for later units
+                            atomicMin(a.qbound + q0 + row, key_dist(last));
                         }
-                        L[p * TC_M] = key;
                     }
-                    uint64_t *dst = part + (arow_slot[un.a0 + row] + un.rch) * S;
+                    if (row < na && n > 0) {
+                        const int64_t q = q0 + row;
+                        uint64_t *dst = a.part + q * a.slot_keys + atomicAdd(a.qcount + q, n);
+                        const uint2 *src = wbuf + (size_t)lane * TC_CAP;
 #pragma unroll 4
-                    for (int i = 0; i < S; ++i) dst[i] = L[i * TC_M];
-                    // a full list bounds the query's S-th best score for later units
-                    if (qbound && thr != KEY_EMPTY) atomicMin(qbound + un.a0 + row, key_dist(thr));
+                        for (int e = 0; e < n; ++e) {
+                            const uint2 x = src[e];
+                            const float sc = __uint_as_float(x.x);
+                            dst[e] = make_key(MODE == TC_SIGN ? (uint32_t)((a.nbits + (int)sc) >> 1) : f2ord(sc), x.y);
+                        }
+                    }
                 }
+                __syncwarp();
             }
-            asm volatile("bar.sync %0, 64;" ::"r"(1 + quad) : "memory");
         }
     }
     tc_fence_before();
@@ -429,7 +537,34 @@ __global__ void __launch_bounds__(tc_threads(S), 1)
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-// ── host: tensor maps and launch ──────────────────────────────────────────
+// A query's bound from the pilot's minima (m groups of 32, warp per query): the
+// S-th smallest of up to 128 groups' minima (groups joined four ways beyond
+// that) is reached by at least S rows.  Fewer than S groups: no bound.
+__global__ void tc_bound_kernel(const float *__restrict__ gmin, int m, int64_t nq, int S,
+                                uint32_t *__restrict__ qbound) {
+    const int lane = threadIdx.x & 31;
+    const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (q >= nq) return;
+    const float *p = gmin + q * m * 32;
+    const float inf = __int_as_float(0x7f800000);
+    float g[4] = {inf, inf, inf, inf};
+    for (int i = 0; i < m; i += 4) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+            if (i + r < m) g[r] = fminf(g[r], p[(i + r) * 32 + lane]);
+    }
+    uint64_t v[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) v[r] = r < m ? make_key(f2ord(g[r]), (uint32_t)(r * 32 + lane)) : KEY_EMPTY;
+    warp_sort<4>(v);
+    uint64_t key = KEY_EMPTY;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+        if (r == (S - 1) / 32) key = __shfl_sync(0xffffffffu, v[r], (S - 1) & 31);
+    if (lane == 0) qbound[q] = key == KEY_EMPTY ? 0xffffffffu : key_dist(key);
+}
+
+// ── host: tensor maps, plan and launch ────────────────────────────────────
 // K-major operand rows of K elements (BF16, or FP8 stored as bytes), boxes of
 // 128 bytes of K by box_rows rows, 128-byte swizzle.
 static int make_tmap_rows(CUtensorMap *map, const void *base, int64_t rows, int64_t K, int box_rows, bool f8) {
@@ -438,49 +573,112 @@ static int make_tmap_rows(CUtensorMap *map, const void *base, int64_t rows, int6
                           (uint32_t)box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
-int tc_topk_launch(const TcLaunch &a, cudaStream_t st) {
-    const int kblk = a.fp8 ? TC_BK8 : TC_BK;
-    if (a.K % kblk)
-        return fail(GN_ERR_INVALID, a.fp8 ? "tensor-core scan: FP8 K must be a multiple of 128"
-                                          : "tensor-core scan: K must be a multiple of 64");
-    if (a.fp8 && (a.S == 0 || a.S > 56 || !a.ascale || !a.bscale))
-        return fail(GN_ERR_UNSUPPORTED, "FP8 shortlist: S must be 16, 32, 40, 48 or 56, with row scales");
+// Chunks of the nt tiles: the smallest count whose units fill whole waves of
+// CTAs best, at least `lo`, chunks of at least `tiles` tiles.
+static int64_t tc_chunks(int64_t nqp, int64_t nt, int64_t lo, int64_t hi, int64_t tiles) {
+    const int sms = dev_info().num_sms;
+    hi = std::max<int64_t>(1, std::min(hi, nt / std::max<int64_t>(1, tiles)));
+    lo = std::min(lo, hi);
+    int64_t best = lo;
+    double eff_best = -1.0;
+    for (int64_t c = lo; c <= hi; ++c) {
+        const int64_t units = nqp * c;
+        const double eff = (double)units / (double)(ceil_div(units, sms) * sms);
+        if (eff > eff_best + 0.01) {
+            eff_best = eff;
+            best = c;
+        }
+    }
+    return best;
+}
+
+static int tc_slices(int mode, int K) { return K / (mode == TC_BF16 ? TC_BK : TC_BK8); }
+
+TcPlan tc_plan(int mode, int K, int64_t nq, int64_t n, int S) {
+    TcPlan p;
+    const int nk = tc_slices(mode, K);
+    const int64_t sms = dev_info().num_sms, nt = ceil_div(n, TC_N);
+    const int64_t nqp = ceil_div(nq, TC_M * tc_geom(nk, false).qt), nqp1 = ceil_div(nq, TC_M);
+    // about five units per SM at most: shorter ones sort more lists at their ends
+    // than they save in the last wave
+    p.nchunks = (int)tc_chunks(nqp, nt, 1, std::min<int64_t>(64, std::max<int64_t>(1, ceil_div(5 * sms, nqp))), 2);
+    // pilot: every 8th tile (more where that would be under 16k rows), full tiles
+    // only; below 32k rows the lists' own first fill costs less than the launches
+    const int64_t full = n / TC_N;
+    if (n >= 32768) {
+        p.pilot_stride = (int)std::max<int64_t>(1, std::min<int64_t>(8, full / 64));
+        p.pilot_tiles = full / p.pilot_stride;
+        // 128 groups of minima per chunk
+        p.pilot_chunks = (int)tc_chunks(nqp1, p.pilot_tiles, 1, std::max<int64_t>(1, ceil_div(4 * sms, nqp1)), 2);
+    }
+    p.slot_keys = (int64_t)p.nchunks * (TC_NEPI / 4) * S;
+    return p;
+}
+
+int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream_t st) {
+    const bool f8 = a.mode != TC_BF16;
+    const int kblk = f8 ? TC_BK8 : TC_BK;
+    if (a.K <= 0 || a.K % kblk) return fail(GN_ERR_INVALID, "tensor-core scan: K must be whole 128-byte slices");
+    if (a.S < 1 || a.S > 64) return fail(GN_ERR_UNSUPPORTED, "tensor-core scan: 1 to 64 results per query");
+    if (a.mode == TC_FP8 && (!a.ascale || !a.bscale)) return fail(GN_ERR_INVALID, "FP8 shortlist: no row scales");
     CUtensorMap ma, mb;
-    GN_TRY(make_tmap_rows(&ma, a.A, std::max<int64_t>(a.a_rows, 1), a.K, TC_M, a.fp8));
-    GN_TRY(make_tmap_rows(&mb, a.B, std::max<int64_t>(a.b_rows, 1), a.K, TC_N, a.fp8));
-    auto launch = [&](auto SC, auto FC) -> int {
-        constexpr int Sv = decltype(SC)::value;
-        constexpr bool Fv = decltype(FC)::value;
-        // 227 KB of shared memory per block, less the kernel's static 32 bytes
-        static_assert(tc_smem_bytes(Sv, Fv) + 32 <= 227 * 1024, "shortlist stages and lists exceed shared memory");
-        const size_t smem = tc_smem_bytes(Sv, Fv);
-        GN_CUDA_TRY(cudaFuncSetAttribute(tc_topk_kernel<Sv, Fv>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem));
-        tc_topk_kernel<Sv, Fv><<<a.grid, tc_threads(Sv), smem, st>>>(ma, mb, a.units, a.n_units, a.cta_off, a.K,
-                                                                     kblk, a.bnorm, a.ascale, a.bscale, a.arow_slot,
-                                                                     a.part, a.scores, a.qbound, a.err);
+    GN_TRY(make_tmap_rows(&ma, a.A, a.a_rows, a.K, TC_M, f8));
+    GN_TRY(make_tmap_rows(&mb, a.B, a.b_rows, a.K, TC_N, f8));
+    const int sms = dev_info().num_sms;
+    GN_TRY(sc.qbound.ensure((size_t)a.nq * 4));
+    GN_TRY(sc.cand.ensure((size_t)sms * TC_NEPI * 2 * 32 * TC_CAP * sizeof(uint2)));
+    TcScanArgs s;
+    s.nq = a.nq;
+    s.n = a.n;
+    s.kblk = kblk;
+    s.S = a.S;
+    s.nbits = a.nbits;
+    s.bnorm = a.bnorm;
+    s.ascale = a.ascale;
+    s.bscale = a.bscale;
+    s.part = a.part;
+    s.qcount = a.qcount;
+    s.slot_keys = p.slot_keys;
+    s.qbound = sc.qbound.as<uint32_t>();
+    s.cand = sc.cand.as<uint2>();
+    s.gmin = nullptr;
+    s.err = a.err;
+    auto run = [&](auto kern, const TcGeom &g) -> int {
+        s.nk = g.nk;
+        s.stages = g.stages;
+        s.resident = g.resident;
+        GN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+        const int64_t units = ceil_div(a.nq, TC_M * g.qt) * s.nchunks;
+        kern<<<(unsigned)std::min<int64_t>(sms, units), TC_THREADS, g.smem, st>>>(ma, mb, s);
         return GN_OK;
     };
-    using F0 = std::false_type;
-    using F1 = std::true_type;
-    if (a.fp8) switch (a.S) {
-        case 16: return launch(std::integral_constant<int, 16>(), F1());
-        case 32: return launch(std::integral_constant<int, 32>(), F1());
-        case 40: return launch(std::integral_constant<int, 40>(), F1());
-        case 48: return launch(std::integral_constant<int, 48>(), F1());
-        case 56: return launch(std::integral_constant<int, 56>(), F1());
-        default: break;
-        }
-    switch (a.S) {
-    case 0: return launch(std::integral_constant<int, 0>(), F0());
-    case 16: return launch(std::integral_constant<int, 16>(), F0());
-    case 32: return launch(std::integral_constant<int, 32>(), F0());
-    case 40: return launch(std::integral_constant<int, 40>(), F0());
-    case 48: return launch(std::integral_constant<int, 48>(), F0());
-    case 56: return launch(std::integral_constant<int, 56>(), F0());
-    case 64: return launch(std::integral_constant<int, 64>(), F0());
-    default: return fail(GN_ERR_UNSUPPORTED, "shortlist size must be 16, 32, 40, 48, 56 or 64");
+    const TcGeom g = tc_geom(a.K / kblk, false);
+    GN_CUDA_TRY(cudaMemsetAsync(a.qcount, 0, (size_t)a.nq * 4, st));
+    if (p.pilot_chunks) {
+        const TcGeom gp = tc_geom(a.K / kblk, true);
+        GN_TRY(sc.gmin.ensure((size_t)a.nq * p.pilot_chunks * TC_N / 2 * 4));
+        s.gmin = sc.gmin.as<float>();
+        s.nchunks = p.pilot_chunks;
+        s.ntiles = p.pilot_tiles;
+        s.tstride = p.pilot_stride;
+        GN_TRY(a.mode == TC_BF16  ? run(tc_topk_kernel<TC_BF16, true, 1>, gp)
+               : a.mode == TC_FP8 ? run(tc_topk_kernel<TC_FP8, true, 1>, gp)
+                                  : run(tc_topk_kernel<TC_SIGN, true, 1>, gp));
+        tc_bound_kernel<<<(unsigned)ceil_div(a.nq, 8), 256, 0, st>>>(s.gmin, (TC_NEPI / 4) * p.pilot_chunks, a.nq,
+                                                                    a.S, s.qbound);
+    } else {
+        GN_CUDA_TRY(cudaMemsetAsync(s.qbound, 0xff, (size_t)a.nq * 4, st));
     }
+    s.nchunks = p.nchunks;
+    s.ntiles = ceil_div(a.n, TC_N);
+    s.tstride = 1;
+    if (g.qt == 2)
+        return a.mode == TC_BF16  ? run(tc_topk_kernel<TC_BF16, false, 2>, g)
+               : a.mode == TC_FP8 ? run(tc_topk_kernel<TC_FP8, false, 2>, g)
+                                  : run(tc_topk_kernel<TC_SIGN, false, 2>, g);
+    return a.mode == TC_BF16  ? run(tc_topk_kernel<TC_BF16, false, 1>, g)
+           : a.mode == TC_FP8 ? run(tc_topk_kernel<TC_FP8, false, 1>, g)
+                              : run(tc_topk_kernel<TC_SIGN, false, 1>, g);
 }
 
 // ── conversion and norms ──────────────────────────────────────────────────
@@ -527,45 +725,130 @@ void to_e4m3_rows(const float *X, int64_t n, int d, int ldx, void *out, float *s
 }
 
 // ── exact re-rank ─────────────────────────────────────────────────────────
-// One warp per query: merge its nslot partial lists (S keys each, by BF16
-// score), keep the S best, recompute their L2 distance in the reference's FP32
-// order (bit-identical to the exact flat scan), return the k nearest.
-template <int RS>
-__global__ void tc_rerank_kernel(const uint64_t *__restrict__ part, int nslot, int S, const float *__restrict__ Q,
-                                 const float *__restrict__ X, int d, int dp, const int32_t *__restrict__ ids,
-                                 int64_t nq, int k, int sqrt_out, int64_t *__restrict__ out_idx,
-                                 float *__restrict__ out_dist) {
-    const int lane = threadIdx.x & 31;
-    const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (q >= nq) return;
-    WarpTopK<RS> L;
-    L.init();
-    uint64_t thr = KEY_EMPTY;
-    const uint64_t *p = part + q * (int64_t)nslot * S;
-    for (int sl = 0; sl < nslot; ++sl)
-        for (int j0 = 0; j0 < S; j0 += 32) {
-            const int j = j0 + lane;
-            const uint64_t key = (j < S) ? p[(int64_t)sl * S + j] : KEY_EMPTY;
-            if (__all_sync(0xffffffffu, key >= thr)) break;
-            L.offer(key, thr, S);
+// The S smallest of a warp's m keys (all distinct) without order: thr gets a
+// bound such that exactly min(S, m) keys are at or below it.  The keys are lane-
+// strided in registers (key i * 32 + lane in v[i], KEY_EMPTY past m), and the
+// bound is built bit by bit from the count of keys below each trial value: 32
+// steps for the scores, and only where several keys share the S-th score 32 more
+// for the rows.  (Inserting ~400 keys into an ordered register list took about
+// 130 insertions of 40 instructions.)
+template <int R>
+__device__ __forceinline__ uint64_t warp_select(const uint64_t (&v)[R], int m, int S) {
+    if (m <= S) return KEY_EMPTY - 1;
+    uint32_t score = 0;
+    int below = 0;  // keys with a score below `score`
+    for (int bit = 31; bit >= 0; --bit) {
+        const uint32_t trial = score | (1u << bit);
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) c += key_dist(v[i]) < trial;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c < S) {
+            score = trial;
+            below = c;
         }
-    // exact distances of the shortlist, then top-k by (distance, id)
+    }
+    int at = 0;
+#pragma unroll
+    for (int i = 0; i < R; ++i) at += key_dist(v[i]) == score && v[i] != KEY_EMPTY;
+    at = __reduce_add_sync(0xffffffffu, at);
+    if (below + at <= S) return make_key(score, 0xffffffffu);
+    const int want = S - below;  // of the keys with this score, the lowest rows
+    uint32_t row = 0;
+    for (int bit = 31; bit >= 0; --bit) {
+        const uint32_t trial = row | (1u << bit);
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) c += key_dist(v[i]) == score && key_idx(v[i]) < trial;
+        if (__reduce_add_sync(0xffffffffu, c) < want) row = trial;
+    }
+    return make_key(score, row);
+}
+
+// The S best of a query's m candidate keys into sel[0 .. min(S, m)), any order,
+// by one warp; returns their number.
+constexpr int SEL_R = 16;  // keys per lane held in registers at a time
+__device__ __forceinline__ int warp_best(const uint64_t *__restrict__ p, int m, int S, uint64_t *sel) {
+    const int lane = threadIdx.x & 31;
+    int kept = 0;
+    for (int i0 = 0; i0 < m;) {
+        // earlier rounds' best join each round's keys
+        const int take = min(m - i0, SEL_R * 32 - kept);
+        uint64_t v[SEL_R];
+#pragma unroll
+        for (int i = 0; i < SEL_R; ++i) {
+            const int x = i * 32 + lane;
+            v[i] = x < kept ? sel[x] : x - kept < take ? p[i0 + x - kept] : KEY_EMPTY;
+        }
+        i0 += take;
+        const uint64_t thr = warp_select<SEL_R>(v, kept + take, S);
+        __syncwarp();
+        kept = 0;
+#pragma unroll
+        for (int i = 0; i < SEL_R; ++i) {
+            const bool in = v[i] <= thr && v[i] != KEY_EMPTY;
+            const unsigned b = __ballot_sync(0xffffffffu, in);
+            if (in) sel[kept + __popc(b & ((1u << lane) - 1))] = v[i];
+            kept += __popc(b);
+        }
+        __syncwarp();
+    }
+    return kept;
+}
+
+// One warp per query: the S best candidates by score, their L2 distances in the
+// reference's FP32 order (bit-identical to the exact flat scan), the k nearest.
+// Two lanes per candidate row, each with four of the reference's eight
+// accumulators, so a warp's loads take whole 32-byte sectors of 16 rows.
+constexpr int RR_WARPS = 4;
+__global__ void __launch_bounds__(RR_WARPS * 32)
+    tc_rerank_kernel(const uint64_t *__restrict__ part, const int *__restrict__ qcount, int64_t slot_keys, int S,
+                     const float *__restrict__ Q, const float *__restrict__ X, int d, int dp, int64_t nq, int k,
+                     int64_t *__restrict__ out_idx, float *__restrict__ out_dist) {
+    __shared__ uint64_t s_sel[RR_WARPS][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t q = (int64_t)blockIdx.x * RR_WARPS + warp;
+    if (q >= nq) return;
+    uint64_t *sel = s_sel[warp];
+    const int m = warp_best(part + q * slot_keys, qcount[q], S, sel);
+    const float4 *q4 = reinterpret_cast<const float4 *>(Q + q * dp);
+    const int half = lane & 1;
+    const int nb = d >> 3, rem = d & 7;
     WarpTopK<1> F;
     F.init();
     uint64_t fthr = KEY_EMPTY;
-#pragma unroll
-    for (int r = 0; r < RS; ++r) {
-        const int pos = r * 32 + lane;
-        const uint64_t key = L.v[r];
-        uint64_t fk = KEY_EMPTY;
-        if (pos < S && key != KEY_EMPTY) {
-            const int64_t row = key_idx(key);
-            float dd = fdist<M_L2>(Q + q * dp, X + row * dp, d);
-            if (!sqrt_out) dd = __fmul_rn(dd, dd);
-            const uint32_t oid = ids ? (uint32_t)ids[row] : (uint32_t)row;
-            fk = make_key(__float_as_uint(dd), oid);
+    for (int c0 = 0; c0 < m; c0 += 16) {
+        const int c = c0 + (lane >> 1);
+        const bool in = c < m;
+        const uint32_t row = in ? key_idx(sel[c]) : key_idx(sel[0]);
+        const float4 *x4 = reinterpret_cast<const float4 *>(X + (int64_t)row * dp);
+        float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll 8
+        for (int b = 0; b < nb; ++b) {
+            const float4 x = x4[2 * b + half], y = q4[2 * b + half];
+            const float t0 = __fsub_rn(y.x, x.x), t1 = __fsub_rn(y.y, x.y);
+            const float t2 = __fsub_rn(y.z, x.z), t3 = __fsub_rn(y.w, x.w);
+            a0 = __fmaf_rn(t0, t0, a0);
+            a1 = __fmaf_rn(t1, t1, a1);
+            a2 = __fmaf_rn(t2, t2, a2);
+            a3 = __fmaf_rn(t3, t3, a3);
         }
-        F.offer(fk, fthr, k);
+        float s0 = __fadd_rn(a0, __shfl_xor_sync(0xffffffffu, a0, 1));
+        float s1 = __fadd_rn(a1, __shfl_xor_sync(0xffffffffu, a1, 1));
+        float s2 = __fadd_rn(a2, __shfl_xor_sync(0xffffffffu, a2, 1));
+        float s3 = __fadd_rn(a3, __shfl_xor_sync(0xffffffffu, a3, 1));
+        // the 4-wide step and the masked remainder (rows are zero padded past d)
+        for (int w = 0; 4 * w < rem; ++w) {
+            const float4 x = x4[2 * nb + w], y = q4[2 * nb + w];
+            const float t0 = __fsub_rn(y.x, x.x), t1 = __fsub_rn(y.y, x.y);
+            const float t2 = __fsub_rn(y.z, x.z), t3 = __fsub_rn(y.w, x.w);
+            s0 = __fmaf_rn(t0, t0, s0);
+            s1 = __fmaf_rn(t1, t1, s1);
+            s2 = __fmaf_rn(t2, t2, s2);
+            s3 = __fmaf_rn(t3, t3, s3);
+        }
+        const float dd = __fsqrt_rn(__fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3)));
+        F.offer(in && half == 0 ? make_key(__float_as_uint(dd), row) : KEY_EMPTY, fthr, k);
     }
     if (lane < k) {
         const uint64_t key = F.v[0];
@@ -575,16 +858,6 @@ __global__ void tc_rerank_kernel(const uint64_t *__restrict__ part, int nslot, i
     }
 }
 
-int tc_rerank_launch(const uint64_t *part, int nslot, int S, const float *Q, const float *X, int d, int dp,
-                     const int32_t *ids, int64_t nq, int k, int sqrt_out, int64_t *out_idx, float *out_dist,
-                     cudaStream_t st) {
-    if (k > 32) return fail(GN_ERR_UNSUPPORTED, "tensor-core path supports k <= 32");
-    const unsigned blocks = (unsigned)ceil_div(nq, 4);
-    if (S <= 32) tc_rerank_kernel<1><<<blocks, 128, 0, st>>>(part, nslot, S, Q, X, d, dp, ids, nq, k, sqrt_out, out_idx, out_dist);
-    else tc_rerank_kernel<2><<<blocks, 128, 0, st>>>(part, nslot, S, Q, X, d, dp, ids, nq, k, sqrt_out, out_idx, out_dist);
-    return GN_OK;
-}
-
 // ── flat tensor-core index (exact L2 via shortlist + re-rank) ─────────────
 struct TcFlatState {
     int d = 0, dp = 0, K = 0;
@@ -592,9 +865,8 @@ struct TcFlatState {
     int fp8 = 0;  // 0: BF16 operands; 1: FP8 E4M3 with per-row scales
     int64_t n = 0;
     DBuf x32, x16, xnorm, xscale;  // fp32 rows (dp), low-precision rows (K), |x|^2, FP8 row scales
-    DBuf q32, q16, qscale, units, nunits, aslot, part, qbound, err, out_idx, out_dist;
-    int64_t planned_nq = -1;
-    int nchunks = 1, grid = 0;
+    DBuf q32, q16, qscale, part, qcount, err, out_idx, out_dist;
+    TcScratch scr;
 };
 
 // The database's low-precision copy in the index's precision, from its FP32
@@ -605,73 +877,13 @@ static int tcflat_lowp(TcFlatState &S, cudaStream_t st) {
     GN_TRY(S.x16.ensure(bytes));
     GN_CUDA_TRY(cudaMemsetAsync(S.x16.p, 0, bytes, st));
     if (S.fp8) {
-        GN_TRY(S.xscale.ensure((size_t)S.n * 4));
+        GN_TRY(S.xscale.ensure((size_t)round_up(S.n, TC_N) * 4));  // whole tiles are read
         to_e4m3_rows(S.x32.as<float>(), S.n, S.d, S.dp, S.x16.p, S.xscale.as<float>(), S.K, st);
     } else {
         S.xscale.release();
         to_bf16_rows(S.x32.as<float>(), S.n, S.d, S.dp, S.x16.p, S.K, st);
     }
     GN_CUDA_TRY(cudaGetLastError());
-    return GN_OK;
-}
-
-// Work units: (query tile, database chunk), chunk-major: the database is cut
-// into C chunks and every query tile's unit for chunk c comes before any unit
-// of chunk c + 1, the CTAs taking units in turn (unit u: CTA u mod grid).  So
-// the CTAs running at any moment scan the same one or two chunks: each chunk
-// comes from DRAM about once and is served to the other query tiles from L2.
-// A unit starts its lists empty, but below the query's bound published by the
-// units that finished before it (tc_topk_kernel), so later chunks insert few
-// keys.  C is chosen so that the units fill whole waves of CTAs (chunks of at
-// least 32 tiles, and of about 100k rows or more once there are enough units
-// for every SM).
-static int tcflat_plan(TcFlatState &S, int64_t nq, cudaStream_t st) {
-    const int sms = dev_info().num_sms;
-    const int64_t qt = ceil_div(nq, TC_M);
-    const int64_t nt = ceil_div(S.n, TC_N);
-    int64_t C = 1;
-    double best = -1.0;
-    // chunks of at least ~100k rows once the units fill the SMs: a unit's
-    // lists start empty, so the longer its chunk the tighter its threshold
-    // over most of it (1M x 128, 10k queries: 6.93 ms at 8 chunks, 7.35 ms at
-    // 19, 9.93 ms at 48)
-    const int64_t cmax = std::min<int64_t>(std::min<int64_t>(std::max<int64_t>(1, nt / 32), 64),
-                                           std::max<int64_t>(ceil_div(sms, qt), S.n / 100000));
-    for (int64_t c = 1; c <= cmax; ++c) {
-        const int64_t units = qt * c;
-        const double eff = (double)units / (double)(ceil_div(units, sms) * sms);
-        if (eff > best + 0.02) {  // more chunks only for a clearly fuller last wave
-            best = eff;
-            C = c;
-        }
-    }
-    std::vector<TcUnit> units;
-    units.reserve((size_t)(qt * C));
-    for (int64_t c = 0; c < C; ++c) {
-        const int64_t t0 = nt * c / C, t1 = nt * (c + 1) / C;
-        for (int64_t t = 0; t < qt; ++t) {
-            TcUnit u{};
-            u.a0 = t * TC_M;
-            u.na = (int32_t)std::min<int64_t>(TC_M, nq - u.a0);
-            u.r0 = t0 * TC_N;
-            u.r1 = std::min<int64_t>(S.n, t1 * TC_N);
-            u.rch = (int32_t)c;
-            units.push_back(u);
-        }
-    }
-    S.nchunks = (int)C;
-    std::vector<int64_t> aslot((size_t)nq);
-    for (int64_t q = 0; q < nq; ++q) aslot[(size_t)q] = q * C;
-    const int64_t nu = (int64_t)units.size();
-    GN_TRY(S.units.ensure(units.size() * sizeof(TcUnit)));
-    GN_TRY(S.nunits.ensure(8));
-    GN_TRY(S.aslot.ensure((size_t)nq * 8));
-    GN_CUDA_TRY(cudaMemcpyAsync(S.units.p, units.data(), units.size() * sizeof(TcUnit), cudaMemcpyHostToDevice, st));
-    GN_CUDA_TRY(cudaMemcpyAsync(S.nunits.p, &nu, 8, cudaMemcpyHostToDevice, st));
-    GN_CUDA_TRY(cudaMemcpyAsync(S.aslot.p, aslot.data(), (size_t)nq * 8, cudaMemcpyHostToDevice, st));
-    GN_CUDA_TRY(cudaStreamSynchronize(st));
-    S.grid = (int)std::max<int64_t>(1, std::min<int64_t>(sms, nu));
-    S.planned_nq = nq;
     return GN_OK;
 }
 
@@ -711,14 +923,16 @@ int gn_tcflat_set(gn_index *ix, const float *data, int64_t n, int64_t d) {
     S.d = (int)d;
     S.dp = (int)round_up(d, 4);
     GN_TRY(upload_rows(S.x32, data, n, d * 4, S.dp / 4, st));
-    GN_TRY(S.xnorm.ensure((size_t)n * 4));
-    row_norms(S.x32.as<float>(), n, S.dp, S.xnorm.as<float>(), st);  // |x|^2 in FP32
+    // |x|^2 in FP32, up to whole tiles: NaN past the last row
+    const size_t np = (size_t)round_up(n, TC_N);
+    GN_TRY(S.xnorm.ensure(np * 4));
+    GN_CUDA_TRY(cudaMemsetAsync(S.xnorm.as<float>() + n, 0xff, (np - (size_t)n) * 4, st));
+    row_norms(S.x32.as<float>(), n, S.dp, S.xnorm.as<float>(), st);
     GN_TRY(tcflat_lowp(S, st));
     GN_TRY(S.err.ensure(4));
     GN_CUDA_TRY(cudaMemsetAsync(S.err.p, 0, 4, st));
     GN_CUDA_TRY(cudaStreamSynchronize(st));
     GN_CUDA_TRY(cudaGetLastError());
-    S.planned_nq = -1;
     ix->n = n;
     ix->dim = d;
     return GN_OK;
@@ -737,42 +951,38 @@ static int tcflat_check(gn_index *ix, int64_t k) {
 static int tcflat_search_locked(gn_index *ix, const float *d_queries, int64_t nq, int64_t k, int64_t *d_idx,
                                 float *d_dist, cudaStream_t st) {
     TcFlatState &S = *tcs(ix);
-    if (S.planned_nq != nq) GN_TRY(tcflat_plan(S, nq, st));
+    const TcPlan plan = tc_plan(S.fp8 ? TC_FP8 : TC_BF16, S.K, nq, S.n, S.S);
     GN_TRY(S.q16.ensure((size_t)std::max<int64_t>(nq, TC_M) * S.K * (S.fp8 ? 1 : 2)));  // >= one 128-row TMA box
-    GN_TRY(S.part.ensure((size_t)nq * S.nchunks * S.S * 8));
+    GN_TRY(S.part.ensure((size_t)nq * plan.slot_keys * 8));
+    GN_TRY(S.qcount.ensure((size_t)nq * 4));
     if (S.fp8) {
         GN_TRY(S.qscale.ensure((size_t)nq * 4));
         to_e4m3_rows(d_queries, nq, S.d, S.dp, S.q16.p, S.qscale.as<float>(), S.K, st);
     } else {
         to_bf16_rows(d_queries, nq, S.d, S.dp, S.q16.p, S.K, st);
     }
-    // no bounds yet (every unit of this search publishes into them)
-    GN_TRY(S.qbound.ensure((size_t)nq * 4));
-    GN_CUDA_TRY(cudaMemsetAsync(S.qbound.p, 0xff, (size_t)nq * 4, st));
     TcLaunch a;
+    a.mode = S.fp8 ? TC_FP8 : TC_BF16;
     a.A = S.q16.p;
+    a.nq = nq;
     a.a_rows = std::max<int64_t>(nq, TC_M);
     a.B = S.x16.p;
+    a.n = S.n;
     a.b_rows = std::max<int64_t>(S.n, TC_N);
     a.K = S.K;
-    a.units = S.units.as<TcUnit>();
-    a.n_units = S.nunits.as<int64_t>();
-    a.cta_off = nullptr;  // unit u on CTA u mod grid (chunk-major order)
-    a.qbound = S.qbound.as<uint32_t>();
     a.bnorm = S.xnorm.as<float>();
-    a.arow_slot = S.aslot.as<int64_t>();
     a.part = S.part.as<uint64_t>();
+    a.qcount = S.qcount.as<int>();
     a.err = S.err.as<int>();
     a.S = S.S;
-    a.grid = S.grid;
-    a.fp8 = S.fp8;
     a.ascale = S.fp8 ? S.qscale.as<float>() : nullptr;
     a.bscale = S.fp8 ? S.xscale.as<float>() : nullptr;
     timing_begin(st, "tc_topk_kernel");
-    GN_TRY(tc_topk_launch(a, st));
+    GN_TRY(tc_topk_launch(a, plan, S.scr, st));
     timing_end(st);
-    GN_TRY(tc_rerank_launch(S.part.as<uint64_t>(), S.nchunks, S.S, d_queries, S.x32.as<float>(), S.d, S.dp,
-                            nullptr, nq, (int)k, 1, d_idx, d_dist, st));
+    tc_rerank_kernel<<<(unsigned)ceil_div(nq, RR_WARPS), RR_WARPS * 32, 0, st>>>(
+        S.part.as<uint64_t>(), S.qcount.as<int>(), plan.slot_keys, S.S, d_queries, S.x32.as<float>(), S.d, S.dp, nq,
+        (int)k, d_idx, d_dist);
     GN_CUDA_TRY(cudaGetLastError());
     return GN_OK;
 }

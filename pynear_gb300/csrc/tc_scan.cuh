@@ -1,7 +1,7 @@
 // tc_scan.cuh — launcher interface of the tensor-core candidate stage.
 #pragma once
 
-#include "common.cuh"
+#include "index.cuh"
 
 namespace gn {
 
@@ -17,37 +17,56 @@ struct TcUnit {
     int32_t rch;
 };
 
+// Operand form of a scan: BF16 rows, FP8 E4M3 rows with one FP32 scale each, or
+// bits as E4M3 +1 / -1 (exact Hamming).
+enum TcMode : int { TC_BF16 = 0, TC_FP8 = 1, TC_SIGN = 2 };
+
 struct TcLaunch {
-    const void *A = nullptr;  // BF16 (or FP8) [a_rows x K], K-major
-    int64_t a_rows = 0;
-    const void *B = nullptr;  // BF16 (or FP8) [b_rows x K], K-major
-    int64_t b_rows = 0;
-    int K = 0;                // elements: multiple of 64 (BF16) or 128 (FP8)
-    const TcUnit *units = nullptr;
-    const int64_t *n_units = nullptr;  // device scalar
-    const int64_t *cta_off = nullptr;  // optional [grid+1] unit range per CTA (else strided)
-    const float *bnorm = nullptr;      // |B row|^2, FP32
-    const int64_t *arow_slot = nullptr;
-    uint64_t *part = nullptr;          // slots x S keys
-    uint32_t *qbound = nullptr;        // optional, per A row: bound of its S-th best score (ordered key;
-                                       // all ones = none), read at each unit's start, lowered at its end
-    int *err = nullptr;                // device error word (0 = ok)
-    int S = 40;
-    int grid = 0;
-    // store mode (S == 0): write every score instead of keeping the top S;
-    // query row a0 + i stores column c at scores[arow_slot[a0 + i] + c - rbase]
-    float *scores = nullptr;
-    // FP8 E4M3 operands (K a multiple of 128) with one FP32 scale per row
-    int fp8 = 0;
-    const float *ascale = nullptr;
-    const float *bscale = nullptr;
+    int mode = TC_BF16;
+    const void *A = nullptr;       // nq query rows of K elements, K-major (a_rows of them allocated, >= 128)
+    int64_t nq = 0, a_rows = 0;
+    const void *B = nullptr;       // n database rows (b_rows allocated, >= 256)
+    int64_t n = 0, b_rows = 0;
+    int K = 0;                     // elements: multiple of 64 (BF16) or 128 (FP8)
+    int nbits = 0;                 // TC_SIGN: bits per row
+    const float *bnorm = nullptr;  // |B row|^2, FP32, whole 256-row tiles, NaN past n (not TC_SIGN)
+    const float *ascale = nullptr, *bscale = nullptr;  // TC_FP8 (bscale: whole tiles)
+    uint64_t *part = nullptr;      // per query slot_keys keys: its candidate list ...
+    int *qcount = nullptr;         // ... and its length (the S best keys are among them)
+    int *err = nullptr;            // device error word (0 = ok)
+    int S = 40;                    // best keys wanted per query, <= 64
 };
 
-int tc_topk_launch(const TcLaunch &a, cudaStream_t st);
+// Launch shape for nq queries over n rows.
+struct TcPlan {
+    int nchunks = 1;                                       // database chunks
+    int64_t slot_keys = 0;                                 // room of a query's candidate list
+    int pilot_chunks = 0, pilot_stride = 1;                // 0: no pilot
+    int64_t pilot_tiles = 0;
+};
+
+// Device scratch of a scan, kept by the index.
+struct TcScratch {
+    DBuf qbound, cand, gmin;
+};
+
+// Kernel arguments.
+struct TcScanArgs {
+    int64_t nq, n, ntiles;
+    int nk, kblk, stages, resident, nchunks, tstride, S, nbits;
+    const float *bnorm, *ascale, *bscale;
+    int64_t slot_keys;
+    uint64_t *part;
+    int *qcount;
+    uint32_t *qbound;
+    uint2 *cand;
+    float *gmin;
+    int *err;
+};
+
+TcPlan tc_plan(int mode, int K, int64_t nq, int64_t n, int S);
+int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream_t st);
 void to_bf16_rows(const float *X, int64_t n, int d, int ldx, void *out, int K, cudaStream_t st);
 void to_e4m3_rows(const float *X, int64_t n, int d, int ldx, void *out, float *scale, int K, cudaStream_t st);
-int tc_rerank_launch(const uint64_t *part, int nslot, int S, const float *Q, const float *X, int d, int dp,
-                     const int32_t *ids, int64_t nq, int k, int sqrt_out, int64_t *out_idx, float *out_dist,
-                     cudaStream_t st);
 
 }  // namespace gn

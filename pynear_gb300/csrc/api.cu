@@ -6,6 +6,7 @@
 
 #include "flat_scan.cuh"
 #include "index.cuh"
+#include "tc_scan.cuh"
 
 namespace gn {
 
@@ -267,6 +268,7 @@ int gn_flat_set(gn_index *ix, const void *data, int64_t n, int64_t dim) {
     GN_TRY(make_stream(ix));
     ix->n = 0;
     ix->dim = 0;
+    ham_tc_reset(ix);
     if (n == 0) return GN_OK;  // an empty index: searches raise GN_ERR_EMPTY
     const int s4 = row_stride4(ix->metric, dim);
     const int64_t row_bytes = (ix->metric == GN_METRIC_HAMMING) ? dim : dim * 4;
@@ -293,17 +295,24 @@ static int flat_search_dev(gn_index *ix, const void *d_q, int64_t nq, int64_t k,
     a.out_idx = d_idx;
     a.out_dist = d_dist;
     if (nq == 0) return GN_OK;
+    auto error_word = [&]() -> int {
+        if (!ix->err.p) {
+            GN_TRY(ix->err.ensure(4));
+            GN_CUDA_TRY(cudaMemsetAsync(ix->err.p, 0, 4, st));
+        }
+        a.err = ix->err.as<int>();
+        return GN_OK;
+    };
+    if (ix->metric == M_HAMMING && ham_tc_wanted(ix, nq, k)) {
+        GN_TRY(error_word());
+        const int rc = ham_tc_search(ix, d_q, nq, (int)k, d_idx, reinterpret_cast<int64_t *>(d_dist), a.err, st);
+        if (rc != GN_ERR_UNSUPPORTED) return rc;
+    }
     if (k <= FLAT_MAX_K_WARP) {
         flat_plan(a);
         if (!flat_smem_ok(a)) return fail(GN_ERR_UNSUPPORTED, "dimension too large for the exact flat scan");
         GN_TRY(ix->part.ensure(flat_part_bytes(a)));
-        if (a.metric != M_HAMMING) {
-            if (!ix->err.p) {
-                GN_TRY(ix->err.ensure(4));
-                GN_CUDA_TRY(cudaMemsetAsync(ix->err.p, 0, 4, st));
-            }
-            a.err = ix->err.as<int>();
-        }
+        if (a.metric != M_HAMMING) GN_TRY(error_word());
         GN_TRY(flat_launch(a, ix->part.as<uint64_t>(), st));
     } else {
         // materialise keys for chunks of queries (<= 512 MB of keys per chunk)

@@ -66,6 +66,13 @@ struct TcScanArgs {
 
 TcPlan tc_plan(int mode, int K, int64_t nq, int64_t n, int S);
 int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream_t st);
+// Exact Hamming k-NN of a flat Hamming index on the tensor cores: whether a
+// search should take it, the search on device buffers (err: device error word),
+// and the end of what it keeps of the rows.
+bool ham_tc_wanted(const gn_index *ix, int64_t nq, int64_t k);
+int ham_tc_search(gn_index *ix, const void *d_q, int64_t nq, int k, int64_t *d_idx, int64_t *d_dist, int *err,
+                  cudaStream_t st);
+void ham_tc_reset(gn_index *ix);
 void to_bf16_rows(const float *X, int64_t n, int d, int ldx, void *out, int K, cudaStream_t st);
 void to_e4m3_rows(const float *X, int64_t n, int d, int ldx, void *out, float *scale, int K, cudaStream_t st);
 

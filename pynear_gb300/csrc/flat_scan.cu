@@ -1,19 +1,25 @@
 // flat_scan.cu — exact exhaustive k-NN scans (Hamming and float metrics).
 //
-// Work decomposition: the query set is cut into groups of WARPS*QW queries and
-// the database into n_slices row slices; one CTA handles one (slice, group)
-// unit.  Units are numbered slice-major so that the CTAs resident at the same
-// time read the same slice and share it through L2.  Each warp owns QW queries;
-// lane l scores row base+l against all of them (the row stays in registers,
-// query words come from shared memory as broadcasts), then offers the keys to
-// the warp's register top-k lists.  Each (query, slice) writes its sorted k
-// keys to a partial buffer; flat_merge_kernel (flat_merge_split_kernel for
-// small batches) reduces the slices.
+// Work decomposition: the query set is cut into groups and the database into
+// n_slices row slices; one CTA handles one (slice, group) unit.  Units are
+// numbered slice-major so that the CTAs resident at the same time read the same
+// slice and share it through L2.
+//
+// Hamming: each warp owns QW queries; lane l scores row base+l against all of
+// them (query words come from shared memory as broadcasts), then offers the
+// keys to the warp's register top-k lists.  Each (query, slice) writes its sorted
+// k keys to a partial buffer; flat_merge_kernel (flat_merge_split_kernel for
+// small batches) reduces the slices.  Large batches go to the tensor cores
+// instead (tc_scan.cu).  Float: see float_scan_kernel.
 //
 // Reference semantics (pynear/include/VPTree.hpp:143-191): exact k nearest rows
 // per query; here ties go to the lower row index.
+#include <algorithm>
+
 #include "distance.cuh"
+#include "f32x2.cuh"
 #include "flat_scan.cuh"
+#include "select.cuh"
 #include "tc_sm100.cuh"
 #include "timing.cuh"
 #include "tmap.cuh"
@@ -79,193 +85,512 @@ __global__ void __launch_bounds__(128) hamming_scan_kernel(const uint4 *__restri
 // ── float scan (L2 / L1 / Linf in the reference's arithmetic order) ───────
 // db: n rows of dp floats (dp % 4 == 0, zero padded past d).
 //
-// Lane l of every warp scores row base + l, the whole row in one thread (the
-// reference's eight-accumulator order needs it).  The rows reach shared memory
-// by TMA (cp.async.bulk.tensor) in boxes of 32 floats (128 bytes) x the
-// stage's rows with the 128-byte swizzle, so the 16-byte chunk c of row r sits
-// at chunk c ^ (r & 7) of the row's 128 bytes and the eight lanes of each
-// quarter-warp phase of a 16-byte shared load (eight consecutive rows, same
-// logical chunk) hit eight different bank groups.  Thread 0 keeps FS_STAGES - 1
-// stages in flight ahead of the one consumed (one mbarrier per stage, bounded
-// waits); the warps (16 queries) share each staged row block.
-constexpr int FS_ROWS = 128;  // slices are whole multiples of the short-row stage
-constexpr int FS_BOX = 32;    // floats per box row (128 bytes)
+// A unit is (row slice, query group).  Four warps: WQ across the group's
+// queries (QW each), WR = 4 / WQ across a stage's rows; a lane scores RPT rows
+// against the warp's QW queries at a time, each (row, query) pair whole in one
+// thread (the reference's eight-accumulator order needs it), so a row's 16-byte
+// shared load serves QW queries and a query's broadcast RPT rows.  Arithmetic is
+// packed FP32 (f32x2.cuh) on row + (-query): the squares and magnitudes are those
+// of query - row bit for bit.
+//
+// Rows reach shared memory by TMA (cp.async.bulk.tensor) in boxes of 32 floats
+// (128 bytes) x the stage's rows with the 128-byte swizzle, so the 16-byte chunk
+// c of row r sits at chunk c ^ (r & 7) of the row's 128 bytes and the eight lanes
+// of each quarter-warp phase of a 16-byte shared load (eight consecutive rows,
+// same logical chunk) hit eight different bank groups.  Thread 0 keeps
+// FS_STAGES - 1 stages in flight ahead of the one consumed (one mbarrier per
+// stage in each direction, bounded waits; the warps may be a stage apart).
+//
+// Selection: a pair that can still be among its list's k nearest is appended to
+// the list's buffer of `cap` keys without order (one ballot); a full buffer is
+// cut down to its k best by counting (select.cuh), which also lowers the list's
+// threshold.  An ordered register list took ~300 cycles per insertion and, for
+// k = 100 over 11 slices, 95 % of the scan.  At the end of its slice a list adds
+// its k best to the query's candidates, from which flat_finish_kernel takes the
+// answer.
+//
+// Measured, scan alone (before: one row per lane and four queries per warp in
+// scalar arithmetic, ordered lists): 100k x 32, 1,000 queries, k 5: 519 -> 416 us
+// (FP32 pipe 41 % busy; floor 159 us); L1 over 30,011 x 97, 513 queries, k 100:
+// 1611 -> 284 us (floor 74 us); 1M x 128, 8 queries: 180 -> 166 us (512 MB, 76 us
+// of HBM time); 20k x 64, 1 query: 14.9 -> 7.7 us.
+constexpr int FS_BOX = 32;      // floats per box row (128 bytes)
 constexpr int FS_STAGES = 3;
+constexpr int FS_STAGE = 16384; // bytes of a stage at most
+constexpr int FS_THREADS = 128, FS_WARPS = 4;
+constexpr int FS_CAP_S = 128, FS_CAP_L = 512;  // buffer keys for k <= 64 (shared memory) and k <= 256 (global)
 
-// Stage shape: rows of at most 64 floats go 128 rows at a time (four 32-row
-// blocks, the whole row in one stage); longer rows 32 rows at a time, up to
-// 256 floats (8 boxes) per stage and in column chunks beyond that, so that a
-// thread's accumulators (its one row) carry across the chunks of its row.
-// Rows narrower than 32 floats are one box exactly the row's width, without
-// swizzle (16-byte chunk c of row r at r * dp * 4 + 16 c).
+// Launch shape (FlatScanArgs::fs).
 struct FsGeom {
-    int nbx;     // boxes of 32 floats per row
-    int rows;    // rows per stage (128 or 32)
-    int cb;      // boxes per stage
-    int nchunk;  // column chunks per row
-    int bw;      // floats per box row: 32 (swizzled) or the row width (narrow rows)
+    int qw, rpt, wq, wr;  // queries per warp, rows per lane, warps across queries and rows
+    int nbx, bw;          // boxes per row, floats per box row: 32 (swizzled) or the row width (narrow rows)
+    int rows, cb, nchunk; // rows and boxes per stage, column chunks per row
+    int cap, most;        // keys of a list's buffer, and how many it may hold before it is cut
+    size_t smem;
 };
-__host__ __device__ inline FsGeom fs_geom(int dp4) {
+
+static FsGeom fs_geom(int64_t nq, int k, int dp4) {
     FsGeom g;
+    g.cap = k <= 64 ? FS_CAP_S : FS_CAP_L;
+    // a late cut leaves the threshold loose, an early one is paid more often
+    g.most = k <= 64 ? std::min(g.cap - 32, 2 * k + 24) : g.cap - 32;
+    // small batches: one or two queries per warp, every warp on its own rows; from
+    // five queries on a row's load serves four of them
+    g.qw = nq <= 1 ? 1 : nq <= 2 ? 2 : 4;
+    g.wq = nq <= 4 ? 1 : nq <= 8 ? 2 : 4;
+    // the queries must fit beside the ring and the buffers
+    auto qbytes = [&]() { return (size_t)g.wq * g.qw * dp4 * 16; };
+    while (qbytes() > 100 * 1024 && g.wq > 1) g.wq >>= 1;
+    while (qbytes() > 130 * 1024 && g.qw > 1) g.qw >>= 1;
+    g.rpt = g.wq > 1 ? 2 : 1;  // (several warps across the queries: four queries each)
+    g.wr = FS_WARPS / g.wq;
+    const int unit = 32 * g.rpt * g.wr;  // rows the four warps take at a time
     g.nbx = (dp4 * 4 + FS_BOX - 1) / FS_BOX;
     g.bw = dp4 * 4 < FS_BOX ? dp4 * 4 : FS_BOX;
-    if (g.nbx <= 2) {
-        g.rows = 128;
-        g.cb = g.nbx;
-    } else {
-        g.rows = 32;
-        g.cb = g.nbx < 8 ? g.nbx : 8;
-    }
+    g.cb = std::min(g.nbx, std::max(1, FS_STAGE / (unit * 128)));
     g.nchunk = (g.nbx + g.cb - 1) / g.cb;
+    g.rows = unit;
+    if (g.nchunk == 1)  // short rows: more of them per stage (a TMA box has at most 256 rows)
+        while (g.rows * 2 <= 256 && (size_t)g.rows * 2 * g.cb * g.bw * 4 <= FS_STAGE) g.rows *= 2;
+    g.smem = qbytes() + 1024 + (size_t)FS_STAGES * g.cb * g.rows * g.bw * 4 + FS_STAGES * 16 +
+             (g.cap == FS_CAP_S ? (size_t)FS_WARPS * g.qw * FS_CAP_S * 8 : 0);
     return g;
 }
-inline size_t fs_stage_bytes(int dp4) {
-    const FsGeom g = fs_geom(dp4);
-    return (size_t)g.cb * g.rows * g.bw * 4;
-}
-// queries, then 1024-byte aligned stages, then the stage barriers
-inline size_t fs_smem_bytes(int warps, int qw, int dp4) {
-    return (size_t)warps * qw * dp4 * 16 + 1024 + FS_STAGES * fs_stage_bytes(dp4) + FS_STAGES * 8;
-}
 
-// DW: the row width when known at compile time (32, 64 or 128 floats, no
-// padding): every shared-memory address and loop bound becomes a constant, so
-// the inner loop is the arithmetic and the loads alone; 0 = any width.
-template <int METRIC, int QW, int R, int DW = 0>
-__global__ void __launch_bounds__(128) float_scan_kernel(const __grid_constant__ CUtensorMap tm, int64_t n,
-                                                         int d_arg, int dp, const float *__restrict__ q, int64_t nq,
-                                                         int k, int n_slices, int64_t slice_rows, int n_groups,
-                                                         uint64_t *__restrict__ part, int *__restrict__ err) {
-    const int d = DW ? DW : d_arg;
-    extern __shared__ float4 sqf[];  // [WARPS*QW][dp/4] queries, then the stage ring
-    const int warps = blockDim.x >> 5;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int unit = blockIdx.x;
-    const int slice = unit / n_groups, group = unit % n_groups;
-    const int64_t q0 = (int64_t)group * warps * QW;
-    const int dp4 = DW ? DW / 4 : dp >> 2;
-    const FsGeom g = fs_geom(dp4);
-    const uint32_t box_bytes = (uint32_t)g.rows * g.bw * 4;
-    const uint32_t stage_bytes = (uint32_t)g.cb * box_bytes;
-    uint8_t *ring = reinterpret_cast<uint8_t *>(
-        (reinterpret_cast<uintptr_t>(sqf + warps * QW * dp4) + 1023) & ~(uintptr_t)1023);
-    uint64_t *full = reinterpret_cast<uint64_t *>(ring + FS_STAGES * stage_bytes);
-    volatile int *verr = err;
+struct FsArgs {
+    int64_t n, nq, slice_rows, list_keys;
+    int d, dp4, k, n_slices, n_groups;
+    int wq, wr, nbx, bw, rows, cb, nchunk, cap, most;
+    const float *q;
+    uint64_t *gbuf;  // buffers of k > 64: per CTA, warp and query, cap keys
+    uint64_t *cand;  // per query list_keys candidate keys ...
+    int *qcount;     // ... and how many there are
+    int *err;
+};
 
-    const float4 *q4 = reinterpret_cast<const float4 *>(q);
-    for (int i = threadIdx.x; i < warps * QW * dp4; i += blockDim.x) {
-        int64_t qi = q0 + i / dp4;
-        sqf[i] = (qi < nq) ? q4[qi * dp4 + (i % dp4)] : make_float4(0.f, 0.f, 0.f, 0.f);
+// One (row, query) pair's accumulators: the packed form of distance.cuh's FAcc.
+template <int METRIC>
+struct FPair {
+    f32x2 p[4];  // L2: lanes (0, 1) (2, 3) (4, 5) (6, 7); else unused
+    float a[8];  // L1, Linf
+    __device__ __forceinline__ void zero() {
+        if (METRIC == M_L2) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) p[i] = 0ull;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) a[i] = 0.f;
+        }
     }
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < FS_STAGES; ++s) mbar_init(full + s, 1);
-        mbar_fence_init();
-    }
-
-    const int64_t r0 = (int64_t)slice * slice_rows;
-    const int64_t r1 = min(n, r0 + slice_rows);
-    const float4 *myq = sqf + warp * QW * dp4;
-    const int nb = d >> 3, rem = d & 7;
-    const int tail4 = 2 * nb;  // float4 index of the remainder pair (when rem > 0)
-    const int64_t nrb = (r1 - r0 + g.rows - 1) / g.rows;
-    const int64_t nstage = nrb * g.nchunk;
-
-    // stage si = (row group si / nchunk, column chunk si % nchunk) into ring slot si % FS_STAGES
-    auto issue = [&](int64_t si) {
-        const int slot = (int)(si % FS_STAGES);
-        const int y = (int)(r0 + (si / g.nchunk) * g.rows);
-        const int b0 = (int)(si % g.nchunk) * g.cb;
-        const int nbox = min(g.cb, g.nbx - b0);
-        uint8_t *dst = ring + (size_t)slot * stage_bytes;
-        mbar_expect_tx(full + slot, (uint32_t)nbox * box_bytes);
-        for (int bi = 0; bi < nbox; ++bi) tma_load_2d(dst + bi * box_bytes, &tm, (b0 + bi) * g.bw, y, full + slot);
-    };
-
-    WarpTopK<R> lists[QW];
-    uint64_t thr[QW];
+    // eight coordinates: x the row's, m the query's negated
+    __device__ __forceinline__ void block8(const f32x2 (&x)[4], const f32x2 (&m)[4]) {
 #pragma unroll
-    for (int j = 0; j < QW; ++j) { lists[j].init(); thr[j] = KEY_EMPTY; }
-
-    __syncthreads();  // queries and barriers ready
-    if (threadIdx.x == 0)
-        for (int64_t si = 0; si < min((int64_t)FS_STAGES - 1, nstage); ++si) issue(si);
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    FAcc<METRIC> acc[QW];
-    float4 x0t = zero4, x1t = zero4;  // the row's remainder pair
-    bool ok = true;
-    int64_t si = 0;
-    for (; si < nstage; ++si) {
-        // keep FS_STAGES - 1 stages in flight: slot (si - 1) % FS_STAGES was
-        // released by every thread at the end of the previous iteration
-        if (threadIdx.x == 0 && si + FS_STAGES - 1 < nstage) issue(si + FS_STAGES - 1);
-        const int slot = (int)(si % FS_STAGES);
-        if (!mbar_wait(full + slot, (uint32_t)((si / FS_STAGES) & 1), verr)) ok = false;
-        if (__syncthreads_or(!ok)) break;  // a wait ran out: every thread leaves together
-        const int kc = (int)(si % g.nchunk);
-        const int c0 = kc * g.cb * 8;                      // first float4 of this column chunk
-        const int c1 = min(dp4, c0 + g.cb * 8);
-        const int cb0 = c0 >> 1, cb1 = min(nb, c1 >> 1);  // full blocks of eight in this chunk
-        const uint8_t *st = ring + (size_t)slot * stage_bytes;
-        for (int rb = 0; rb < g.rows / 32; ++rb) {
-            const int rl = rb * 32 + lane;  // row within the stage
-            const int sw = rl & 7;
-            // float4 c of this lane's row (c in [c0, c1)): box (c - c0) / 8, swizzled chunk
-            auto rowf4 = [&](int c) -> float4 {
-                const int cc = c - c0;
-                if (g.bw < FS_BOX) return *reinterpret_cast<const float4 *>(st + rl * (g.bw * 4) + cc * 16);
-                return *reinterpret_cast<const float4 *>(st + (cc >> 3) * box_bytes + rl * 128 +
-                                                         (((cc & 7) ^ sw) << 4));
-            };
-            if (kc == 0) {
-#pragma unroll
-                for (int j = 0; j < QW; ++j) acc[j].zero();
-            }
-#pragma unroll 2
-            for (int c = cb0; c < cb1; ++c) {
-                const float4 x0 = rowf4(2 * c), x1 = rowf4(2 * c + 1);
-#pragma unroll
-                for (int j = 0; j < QW; ++j) acc[j].block8(myq[j * dp4 + 2 * c], myq[j * dp4 + 2 * c + 1], x0, x1);
-            }
-            if (rem > 0 && tail4 >= c0 && tail4 < c1) {
-                x0t = rowf4(tail4);
-                if (rem > 4) x1t = rowf4(tail4 + 1);
-            }
-            if (kc == g.nchunk - 1) {
-                const int64_t row = r0 + (si / g.nchunk) * g.rows + rl;
-                const bool valid = row < r1;
-#pragma unroll
-                for (int j = 0; j < QW; ++j) {
-                    float4 qa = zero4, qb = zero4;
-                    if (rem > 0) qa = myq[j * dp4 + tail4];
-                    if (rem > 4) qb = myq[j * dp4 + tail4 + 1];
-                    float dist = acc[j].finish(rem, qa, qb, x0t, x1t);
-                    uint64_t key = valid ? make_key(__float_as_uint(dist), (uint32_t)row) : KEY_EMPTY;
-                    lists[j].offer(key, thr[j], k);
+        for (int i = 0; i < 4; ++i) {
+            const f32x2 t = add2(x[i], m[i]);
+            if (METRIC == M_L2) {
+                p[i] = fma2(t, t, p[i]);
+            } else {
+                float lo, hi;
+                unpack2(t, lo, hi);
+                if (METRIC == M_L1) {
+                    a[2 * i] = __fadd_rn(a[2 * i], fabsf(lo));
+                    a[2 * i + 1] = __fadd_rn(a[2 * i + 1], fabsf(hi));
+                } else {
+                    a[2 * i] = fmaxf(a[2 * i], fabsf(lo));
+                    a[2 * i + 1] = fmaxf(a[2 * i + 1], fabsf(hi));
                 }
             }
         }
-        __syncthreads();  // slot si % FS_STAGES is free for the next issue
+    }
+    // After the blocks of eight, in FAcc::finish's order: fold, then for d % 8 = rem
+    // coordinates left (q0, q1 and x0, x1, the query's negated, zero past d) tail,
+    // then value: what orders rows as the distance does, for L2 the squared sum
+    // under the root, else the distance.
+    __device__ __forceinline__ void fold() {
+        if (METRIC == M_L2) {
+            p[0] = add2(p[2], p[0]);
+            p[1] = add2(p[3], p[1]);
+        } else {
+#pragma unroll
+            for (int i = 1; i < 8; ++i) a[0] = METRIC == M_L1 ? __fadd_rn(a[0], a[i]) : fmaxf(a[0], a[i]);
+        }
+    }
+    __device__ __forceinline__ void tail(int rem, const float4 &q0, const float4 &q1, const float4 &x0,
+                                         const float4 &x1) {
+        const float t[8] = {__fadd_rn(x0.x, q0.x), __fadd_rn(x0.y, q0.y), __fadd_rn(x0.z, q0.z),
+                            __fadd_rn(x0.w, q0.w), __fadd_rn(x1.x, q1.x), __fadd_rn(x1.y, q1.y),
+                            __fadd_rn(x1.z, q1.z), __fadd_rn(x1.w, q1.w)};
+        if (METRIC == M_L2) {
+            const f32x2 t01 = pack2(t[0], t[1]), t23 = pack2(t[2], t[3]);
+            p[0] = fma2(t01, t01, p[0]);
+            p[1] = fma2(t23, t23, p[1]);
+            if (rem > 4) {
+                const f32x2 t45 = pack2(t[4], t[5]), t67 = pack2(t[6], t[7]);
+                p[0] = fma2(t45, t45, p[0]);
+                p[1] = fma2(t67, t67, p[1]);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 7; ++i)
+                if (i < rem) a[0] = METRIC == M_L1 ? __fadd_rn(a[0], fabsf(t[i])) : fmaxf(a[0], fabsf(t[i]));
+        }
+    }
+    __device__ __forceinline__ float value() const {
+        if (METRIC != M_L2) return a[0];
+        float s0, s1, s2, s3;
+        unpack2(p[0], s0, s1);
+        unpack2(p[1], s2, s3);
+        return __fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3));
+    }
+};
+
+// The largest finish() value (as bits) of a distance below thr: L2, a squared sum
+// above thr * thr (rounded up) has a root of at least thr, so the root itself is
+// taken only for rows that may enter.
+template <int METRIC>
+__device__ __forceinline__ uint32_t fs_limit(uint32_t thr) {
+    if (METRIC != M_L2 || thr >= 0x7f800000u) return thr;  // no bound yet, or one that is not finite
+    const float t = __uint_as_float(thr);
+    return __float_as_uint(__fmul_ru(t, t));
+}
+
+// Cut a buffer of m keys (k < m <= 32 R) down to its k best, in place; returns
+// the k-th best key's distance bits.  (A call, not inlined: it runs a few times
+// per list and would crowd the scan's registers and instruction cache.)
+template <int R>
+__device__ __noinline__ uint32_t fs_cut(uint64_t *buf, int m, int k) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    uint64_t v[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) v[i] = i * 32 + lane < m ? buf[i * 32 + lane] : KEY_EMPTY;
+    const uint64_t thr = warp_select<R>(v, m, k);
+    __syncwarp();
+    int kept = 0;
+    uint32_t far = 0u;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const bool in = v[i] <= thr && v[i] != KEY_EMPTY;
+        const unsigned b = __ballot_sync(0xffffffffu, in);
+        if (in) {
+            buf[kept + __popc(b & ((1u << lane) - 1))] = v[i];
+            far = max(far, key_dist(v[i]));
+        }
+        kept += __popc(b);
+    }
+    __syncwarp();
+    return __reduce_max_sync(0xffffffffu, far);
+}
+
+// Add the lanes' rows whose distance stays below thr to a list's buffer of cnt
+// keys, cutting it once it holds more than `most`; v: finish() bits, in: the lane's
+// row may enter.  Returns (count, threshold).  (A call: see fs_cut.)
+template <int METRIC>
+__device__ __noinline__ uint2 fs_add(uint64_t *buf, uint2 state, uint32_t v, bool in, uint32_t row, int k, int most) {
+    if (METRIC == M_L2) v = __float_as_uint(__fsqrt_rn(__uint_as_float(v)));
+    in = in && v < state.y;
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    const int lane = threadIdx.x & 31;
+    if (in) buf[state.x + __popc(m & ((1u << lane) - 1))] = make_key(v, row);
+    state.x += __popc(m);
+    if ((int)state.x > most) {
+        state.y = k <= 64 ? fs_cut<FS_CAP_S / 32>(buf, state.x, k) : fs_cut<FS_CAP_L / 32>(buf, state.x, k);
+        state.x = k;
+    }
+    return state;
+}
+
+// ONE: a stage holds whole rows (the accumulators then never outlive a group).
+template <int METRIC, int QW, int RPT, bool ONE>
+__global__ void __launch_bounds__(FS_THREADS, 3)
+    float_scan_kernel(const __grid_constant__ CUtensorMap tm, const FsArgs a) {
+    extern __shared__ float4 sqf[];  // [WQ * QW][dp4] negated queries, buffers (k <= 64), the stage ring, barriers
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int slice = blockIdx.x / a.n_groups, group = blockIdx.x % a.n_groups;
+    const int wqi = warp % a.wq, wri = warp / a.wq;
+    const int64_t q0 = (int64_t)group * a.wq * QW;
+    const int dp4 = a.dp4, k = a.k;
+    uint64_t *sbuf = reinterpret_cast<uint64_t *>(sqf + a.wq * QW * dp4);
+    const int cap = a.cap;
+    // (an offset from the shared array, not a rounded pointer: the loads stay shared-memory loads)
+    const uint32_t ring_at = (uint32_t)(a.wq * QW * dp4) * 16 + (cap == FS_CAP_S ? FS_WARPS * QW * FS_CAP_S * 8 : 0);
+    const uint32_t smem0 = smem_u32(sqf);
+    uint8_t *ring = reinterpret_cast<uint8_t *>(sqf) + (((smem0 + ring_at + 1023) & ~1023u) - smem0);
+    const uint32_t pitch = (uint32_t)a.bw * 4, box_bytes = (uint32_t)a.rows * pitch;
+    const uint32_t stage_bytes = (uint32_t)a.cb * box_bytes;
+    uint64_t *full = reinterpret_cast<uint64_t *>(ring + FS_STAGES * stage_bytes);
+    volatile int *verr = a.err;
+
+    const float4 *q4 = reinterpret_cast<const float4 *>(a.q);
+    for (int i = threadIdx.x; i < a.wq * QW * dp4; i += FS_THREADS) {
+        const int64_t qi = q0 + i / dp4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (qi < a.nq) v = q4[qi * dp4 + (i % dp4)];
+        sqf[i] = make_float4(-v.x, -v.y, -v.z, -v.w);
+    }
+    uint64_t *empty = full + FS_STAGES;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < FS_STAGES; ++s) {
+            mbar_init(full + s, 1);
+            mbar_init(empty + s, FS_WARPS);
+        }
+        mbar_fence_init();
+    }
+
+    const int64_t r0 = (int64_t)slice * a.slice_rows;
+    const int64_t r1 = min(a.n, r0 + a.slice_rows);
+    const float4 *myq = sqf + wqi * QW * dp4;
+    const int nb = a.d >> 3, rem = a.d & 7;
+    const int nstage = (int)((r1 - r0 + a.rows - 1) / a.rows) * a.nchunk;
+
+    // stages in order (row group, then its column chunks) into ring slots in turn; the
+    // issuing thread's place in that order
+    int iss = 0, iss_slot = 0, iss_y = (int)r0, iss_b0 = 0;
+    uint32_t iss_ph = 0;  // parity of the release that frees the slot: its use before
+    auto issue = [&]() {
+        const int nbox = min(a.cb, a.nbx - iss_b0);
+        uint8_t *dst = ring + (uint32_t)iss_slot * stage_bytes;
+        mbar_expect_tx(full + iss_slot, (uint32_t)nbox * box_bytes);
+        for (int bi = 0; bi < nbox; ++bi)
+            tma_load_2d(dst + bi * box_bytes, &tm, (iss_b0 + bi) * a.bw, iss_y, full + iss_slot);
+        ++iss;
+        iss_b0 += a.cb;
+        if (ONE || iss_b0 >= a.nbx) {
+            iss_b0 = 0;
+            iss_y += a.rows;
+        }
+        if (++iss_slot == FS_STAGES) {
+            iss_slot = 0;
+            iss_ph ^= 1;
+        }
+    };
+
+    // a list: its buffer, the keys in it, and the distance bits that a new key must
+    // stay below (rows come in ascending order, so an equal distance loses the tie)
+    uint64_t *buf0 = cap == FS_CAP_S ? sbuf + warp * QW * FS_CAP_S
+                                     : a.gbuf + ((size_t)blockIdx.x * FS_WARPS + warp) * QW * cap;
+    int cnt[QW];
+    uint32_t thr[QW], lim[QW];  // lim: fs_limit(thr)
+#pragma unroll
+    for (int j = 0; j < QW; ++j) {
+        cnt[j] = 0;
+        thr[j] = lim[j] = q0 + wqi * QW + j < a.nq ? 0xffffffffu : 0u;
+    }
+    __syncthreads();  // queries and barriers ready
+    if (threadIdx.x == 0)
+        while (iss < min(FS_STAGES - 1, nstage)) issue();
+    const uint32_t sw = a.bw < FS_BOX ? 0u : (uint32_t)(lane & 7);  // a lane's rows are lane modulo 32
+    uint32_t off[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) off[c] = ((uint32_t)c ^ sw) << 4;
+    const int wrows = 32 * RPT;  // rows a warp takes at a time
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    FPair<METRIC> acc[RPT][QW];
+    bool ok = true;
+    int slot = 0, kc = 0;
+    uint32_t ph = 0;
+    int si = 0;
+    int64_t y0 = r0;
+    for (; si < nstage; ++si) {
+        // keep FS_STAGES - 1 stages in flight: the next goes to the slot of stage si - 1,
+        // once every warp has left that (the warps may be a stage apart)
+        if (threadIdx.x == 0 && iss < nstage) {
+            if (iss >= FS_STAGES && !mbar_wait(empty + iss_slot, iss_ph ^ 1, verr)) ok = false;
+            else issue();
+        }
+        if (!__all_sync(0xffffffffu, ok && mbar_wait(full + slot, ph, verr))) {
+            ok = false;
+            break;
+        }
+        const uint8_t *st = ring + (size_t)slot * stage_bytes;
+        const int b0 = kc * a.cb, nbox = min(a.cb, a.nbx - b0);
+        const bool last = ONE || kc == a.nchunk - 1;
+        for (int g = wri * wrows; g < a.rows; g += a.wr * wrows) {
+            if (y0 + g >= r1) break;
+            const uint8_t *rp[RPT];
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) rp[r] = st + (uint32_t)(g + r * 32 + lane) * pitch;
+            if (ONE || kc == 0) {
+#pragma unroll
+                for (int r = 0; r < RPT; ++r)
+#pragma unroll
+                    for (int j = 0; j < QW; ++j) acc[r][j].zero();
+            }
+            // coordinates 8 e .. of the box at boff; o0, o1: its two chunks' offsets in a row
+            auto eight = [&](uint32_t boff, const float4 *qb, uint32_t o0, uint32_t o1, int e) {
+                f32x2 x[RPT][4];
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) {
+                    const ulonglong2 lo = *reinterpret_cast<const ulonglong2 *>(rp[r] + boff + o0);
+                    const ulonglong2 hi = *reinterpret_cast<const ulonglong2 *>(rp[r] + boff + o1);
+                    x[r][0] = lo.x;
+                    x[r][1] = lo.y;
+                    x[r][2] = hi.x;
+                    x[r][3] = hi.y;
+                }
+#pragma unroll
+                for (int j = 0; j < QW; ++j) {
+                    const ulonglong2 lo = *reinterpret_cast<const ulonglong2 *>(qb + j * dp4 + 2 * e);
+                    const ulonglong2 hi = *reinterpret_cast<const ulonglong2 *>(qb + j * dp4 + 2 * e + 1);
+                    const f32x2 m[4] = {lo.x, lo.y, hi.x, hi.y};
+#pragma unroll
+                    for (int r = 0; r < RPT; ++r) acc[r][j].block8(x[r], m);
+                }
+            };
+            // whole boxes, then the blocks of eight of a partial one
+            const int blocks = min(nb - b0 * 4, nbox * 4), whole = blocks >> 2;
+            for (int bi = 0; bi < whole; ++bi) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    eight((uint32_t)bi * box_bytes, myq + (b0 + bi) * 8, off[2 * e], off[2 * e + 1], e);
+            }
+#pragma unroll 1
+            for (int e = 0; e < blocks - whole * 4; ++e)
+                eight((uint32_t)whole * box_bytes, myq + (b0 + whole) * 8, ((uint32_t)(2 * e) ^ sw) << 4,
+                      ((uint32_t)(2 * e + 1) ^ sw) << 4, e);
+            if (!last) continue;
+            const int left = (int)min((int64_t)a.rows, r1 - y0) - g;  // rows from this group on
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) {
+#pragma unroll
+                for (int j = 0; j < QW; ++j) acc[r][j].fold();
+            }
+            if (rem > 0) {  // the remainder's coordinates sit in the last box
+                const int tail4 = 2 * nb;
+                const uint32_t tb = (uint32_t)((tail4 >> 3) - b0) * box_bytes;
+                const uint32_t o0 = ((uint32_t)(tail4 & 7) ^ sw) << 4, o1 = ((uint32_t)((tail4 & 7) + 1) ^ sw) << 4;
+                const float4 *tq = myq + tail4;
+#pragma unroll
+                for (int r = 0; r < RPT; ++r) {
+                    const float4 x0 = *reinterpret_cast<const float4 *>(rp[r] + tb + o0);
+                    const float4 x1 = rem > 4 ? *reinterpret_cast<const float4 *>(rp[r] + tb + o1) : zero4;
+#pragma unroll
+                    for (int j = 0; j < QW; ++j)
+                        acc[r][j].tail(rem, tq[j * dp4], rem > 4 ? tq[j * dp4 + 1] : zero4, x0, x1);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < RPT; ++r) {
+                uint32_t bits[QW];
+                bool any = false;
+#pragma unroll
+                for (int j = 0; j < QW; ++j) {
+                    bits[j] = __float_as_uint(acc[r][j].value());
+                    any = any || bits[j] <= lim[j];
+                }
+                if (!__any_sync(0xffffffffu, any)) continue;
+                const uint32_t row = (uint32_t)(y0 + g) + r * 32 + lane;
+#pragma unroll
+                for (int j = 0; j < QW; ++j) {
+                    const bool in = bits[j] <= lim[j] && r * 32 + lane < left;
+                    if (!__any_sync(0xffffffffu, in)) continue;
+                    const uint2 ns = fs_add<METRIC>(buf0 + j * cap, make_uint2(cnt[j], thr[j]), bits[j], in, row, k,
+                                                    a.most);
+                    cnt[j] = (int)ns.x;
+                    if (ns.y != thr[j]) {
+                        thr[j] = ns.y;
+                        lim[j] = fs_limit<METRIC>(ns.y);
+                    }
+                }
+            }
+        }
+        if (ONE || ++kc == a.nchunk) {
+            kc = 0;
+            y0 += a.rows;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty + slot);
+        if (++slot == FS_STAGES) {
+            slot = 0;
+            ph ^= 1;
+        }
     }
     if (!ok) {
-        // a wait ran out in stage si: let the copies issued for stages si ..
-        // si + FS_STAGES - 1 land (each wait bounded) before the CTA leaves
+        // a wait ran out in stage si (the other warps find the error word set, or run
+        // out themselves): let the copies issued from stage si on land (each wait bounded)
+        // before the issuing thread leaves
         if (threadIdx.x == 0)
-            for (int64_t x = si; x < min(nstage, si + FS_STAGES); ++x) {
-                const int slot = (int)(x % FS_STAGES);
+            for (int x = si; x < iss; ++x) {
                 const long long t0 = clock64();
-                while (!mbar_try_wait(full + slot, (uint32_t)((x / FS_STAGES) & 1)) && clock64() - t0 < 400000) {
+                while (!mbar_try_wait(full + x % FS_STAGES, (uint32_t)((x / FS_STAGES) & 1)) &&
+                       clock64() - t0 < 400000) {
                 }
             }
         return;
     }
 #pragma unroll
     for (int j = 0; j < QW; ++j) {
-        int64_t qi = q0 + warp * QW + j;
-        if (qi < nq) lists[j].store(part + ((size_t)qi * n_slices + slice) * k, k);
+        const int64_t qi = q0 + wqi * QW + j;
+        if (qi >= a.nq) continue;
+        uint64_t *b = buf0 + j * cap;
+        int c = cnt[j];
+        if (c > k) {
+            if (cap == FS_CAP_S) fs_cut<FS_CAP_S / 32>(b, c, k);
+            else fs_cut<FS_CAP_L / 32>(b, c, k);
+            c = k;
+        }
+        __syncwarp();
+        int at = 0;
+        if (lane == 0) at = atomicAdd(a.qcount + qi, c);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        uint64_t *dst = a.cand + qi * a.list_keys + at;
+        for (int i = lane; i < c; i += 32) dst[i] = b[i];
     }
 }
 
-// ── merge of per-slice partial lists → final output ───────────────────────
+// The answer from a query's candidates: each of the block's W warps takes the k
+// best of its share, the first warp the k best of theirs, sorted.  One warp per
+// query where the batch alone fills the GPU, 8 or 24 for smaller batches, whose
+// queries have hundreds of lists each.
+template <int W, int R>
+__global__ void __launch_bounds__(W * 32)
+    flat_finish_kernel(const uint64_t *__restrict__ cand, const int *__restrict__ qcount, int64_t list_keys, int k,
+                       int64_t *__restrict__ out_idx, float *__restrict__ out_dist) {
+    __shared__ uint64_t s_sel[(W + 1) * R * 32];
+    __shared__ int s_n[W];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t q = blockIdx.x;
+    const uint64_t *p = cand + q * list_keys;
+    const int total = qcount[q];
+    const int share = (total + W - 1) / W;
+    const int b = min(total, warp * share), e = min(total, b + share);
+    const int mine = warp_best(p + b, e - b, k, s_sel + warp * R * 32);
+    uint64_t *res = s_sel;
+    int m = mine;
+    if (W > 1) {
+        if (lane == 0) s_n[warp] = mine;
+        __syncthreads();
+        if (warp != 0) return;
+        // the warps' keys, moved together (each group moves down, in order)
+        m = mine;
+        for (int w = 1; w < W; ++w) {
+            const int nw = s_n[w];
+            for (int i = 0; i < nw; i += 32) {
+                const uint64_t key = i + lane < nw ? s_sel[w * R * 32 + i + lane] : 0ull;
+                __syncwarp();
+                if (i + lane < nw) s_sel[m + i + lane] = key;
+                __syncwarp();
+            }
+            m += nw;
+        }
+        res = s_sel + W * R * 32;
+        m = warp_best(s_sel, m, k, res);
+    }
+    uint64_t v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = r * 32 + lane < m ? res[r * 32 + lane] : KEY_EMPTY;
+    warp_sort<R>(v);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int pos = r * 32 + lane;
+        if (pos >= k) continue;
+        const bool empty = v[r] == KEY_EMPTY;
+        out_idx[q * k + pos] = empty ? -1 : (int64_t)key_idx(v[r]);
+        out_dist[q * k + pos] = empty ? 0.f : __uint_as_float(key_dist(v[r]));
+    }
+}
+
+// ── Hamming scan: merge of per-slice partial lists → final output ─────────
 // Offer a query's sorted per-slice lists s_begin, s_begin + s_step, ... (k <=
 // 32: one 32-key chunk per slice) to a warp's list: the chunks of MERGE_AHEAD
 // slices are loaded together, so that a small batch's hundreds of slices cost
@@ -287,11 +612,10 @@ __device__ __forceinline__ void merge_slices_ahead(const uint64_t *__restrict__ 
     }
 }
 
-// Write a query's k nearest: idx (int64, -1 for empty), dist as float32
-// (float metrics) or int64 (Hamming).
+// Write a query's k nearest: idx (-1 for empty) and distance.
 template <int R>
-__device__ __forceinline__ void merge_store(const WarpTopK<R> &L, int64_t qi, int k, int is_hamming, int lane,
-                                            int64_t *__restrict__ out_idx, void *__restrict__ out_dist) {
+__device__ __forceinline__ void merge_store(const WarpTopK<R> &L, int64_t qi, int k, int lane,
+                                            int64_t *__restrict__ out_idx, int64_t *__restrict__ out_dist) {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         int pos = r * 32 + lane;
@@ -299,16 +623,15 @@ __device__ __forceinline__ void merge_store(const WarpTopK<R> &L, int64_t qi, in
             uint64_t key = L.v[r];
             bool e = key == KEY_EMPTY;
             out_idx[qi * k + pos] = e ? -1 : (int64_t)key_idx(key);
-            if (is_hamming) reinterpret_cast<int64_t *>(out_dist)[qi * k + pos] = e ? 0 : (int64_t)key_dist(key);
-            else reinterpret_cast<float *>(out_dist)[qi * k + pos] = e ? 0.f : __uint_as_float(key_dist(key));
+            out_dist[qi * k + pos] = e ? 0 : (int64_t)key_dist(key);
         }
     }
 }
 
 // One warp per query.
 template <int R>
-__global__ void flat_merge_kernel(const uint64_t *__restrict__ part, int n_slices, int k, int64_t nq, int is_hamming,
-                                  int64_t *__restrict__ out_idx, void *__restrict__ out_dist) {
+__global__ void flat_merge_kernel(const uint64_t *__restrict__ part, int n_slices, int k, int64_t nq,
+                                  int64_t *__restrict__ out_idx, int64_t *__restrict__ out_dist) {
     const int lane = threadIdx.x & 31;
     const int64_t qi = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (qi >= nq) return;
@@ -327,7 +650,7 @@ __global__ void flat_merge_kernel(const uint64_t *__restrict__ part, int n_slice
             L.offer(key, thr, k);
         }
     }
-    merge_store(L, qi, k, is_hamming, lane, out_idx, out_dist);
+    merge_store(L, qi, k, lane, out_idx, out_dist);
 }
 
 // Small batches (k <= 32): one block of MERGE_WARPS warps per query, so that
@@ -337,8 +660,8 @@ __global__ void flat_merge_kernel(const uint64_t *__restrict__ part, int n_slice
 // list.  The k nearest are the same keys in the same order as flat_merge_kernel's.
 constexpr int MERGE_WARPS = 8;
 __global__ void __launch_bounds__(MERGE_WARPS * 32)
-    flat_merge_split_kernel(const uint64_t *__restrict__ part, int n_slices, int k, int is_hamming,
-                            int64_t *__restrict__ out_idx, void *__restrict__ out_dist) {
+    flat_merge_split_kernel(const uint64_t *__restrict__ part, int n_slices, int k, int64_t *__restrict__ out_idx,
+                            int64_t *__restrict__ out_dist) {
     __shared__ uint64_t wl[MERGE_WARPS][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t qi = blockIdx.x;
@@ -354,7 +677,7 @@ __global__ void __launch_bounds__(MERGE_WARPS * 32)
         const uint64_t key = wl[w][lane];
         if (!__all_sync(0xffffffffu, key >= thr)) L.offer(key, thr, k);
     }
-    merge_store(L, qi, k, is_hamming, lane, out_idx, out_dist);
+    merge_store(L, qi, k, lane, out_idx, out_dist);
 }
 
 // ── large-k path: materialised keys + radix select + bitonic sort ────────
@@ -450,163 +773,176 @@ __global__ void keys_to_output_kernel(const uint64_t *__restrict__ sorted, int64
 }
 
 // ── host-side launchers ───────────────────────────────────────────────────
-template <int R>
-static int launch_scan(const FlatScanArgs &a, int n_groups, int threads, size_t smem, uint64_t *part,
-                       cudaStream_t st) {
-    const int units = n_groups * a.n_slices;
+// CTAs of the float scan per SM: three by registers, fewer by shared memory.
+static int fs_occupancy(const FsGeom &g) { return (int)std::min<size_t>(3, (size_t)227 * 1024 / (g.smem + 1024)); }
+
+void flat_plan(FlatScanArgs &a) {
+    const DevInfo &di = dev_info();
     if (a.metric == M_HAMMING) {
+        const size_t per_warp = (size_t)8 * a.stride4 * 16;
+        int warps = 4;
+        while (warps > 1 && per_warp * warps > 200 * 1024) warps >>= 1;
+        a.warps = warps;
+        const int64_t n_groups = ceil_div(a.nq, (int64_t)warps * 8);
+        // slices of at least 128 rows, about 16 CTAs per SM over the launch
+        const int64_t max_slices = std::max<int64_t>(1, a.n / 128);
+        const int64_t slices = std::min<int64_t>(std::max<int64_t>(1, ceil_div(16LL * di.num_sms, n_groups)), max_slices);
+        a.slice_rows = round_up(ceil_div(a.n, slices), 32);
+        a.n_slices = (int)ceil_div(a.n, a.slice_rows);
+        a.n_groups = (int)n_groups;
+        return;
+    }
+    const FsGeom g = fs_geom(a.nq, a.k, a.stride4);
+    const int64_t n_groups = ceil_div(a.nq, (int64_t)g.wq * g.qw);
+    // units of equal cost: the slice count (up to about two waves of resident
+    // CTAs) whose last wave is fullest, the fewest slices on a tie: every slice
+    // starts its lists empty
+    const int64_t slots = (int64_t)std::max(1, fs_occupancy(g)) * di.num_sms;
+    const int64_t max_slices = std::max<int64_t>(1, ceil_div(a.n, g.rows));
+    const int64_t hi = std::min<int64_t>(max_slices, std::max<int64_t>(1, ceil_div(2 * slots, n_groups)));
+    int64_t slices = 1;
+    double best = -1.0;
+    for (int64_t s = 1; s <= hi; ++s) {
+        const int64_t units = n_groups * s;
+        const double eff = (double)units / (double)(ceil_div(units, slots) * slots);
+        if (eff > best + 0.02) {
+            best = eff;
+            slices = s;
+        }
+    }
+    if (n_groups * max_slices <= slots) slices = max_slices;  // one stage each
+    a.slice_rows = round_up(ceil_div(a.n, slices), g.rows);
+    a.n_slices = (int)ceil_div(a.n, a.slice_rows);
+    a.n_groups = (int)n_groups;
+    a.list_keys = (int64_t)a.n_slices * g.wr * a.k;
+    a.units = (int64_t)a.n_slices * n_groups;
+    a.gbuf_keys = g.cap == FS_CAP_L ? a.units * FS_WARPS * g.qw * FS_CAP_L : 0;
+}
+
+// Scratch: Hamming, the slices' partial lists; float, the queries' counters
+// (first), candidates and, for k > 64, the scan's buffers.
+size_t flat_part_bytes(const FlatScanArgs &a) {
+    if (a.metric == M_HAMMING) return (size_t)a.nq * a.n_slices * a.k * sizeof(uint64_t);
+    return (size_t)round_up(a.nq * 4, 256) + (size_t)(a.nq * a.list_keys + a.gbuf_keys) * sizeof(uint64_t);
+}
+
+// Rows whose queries fit the scan.  (Float: the widths accepted are those of a
+// stage ring of 32-row stages of up to 256 floats beside 1, 2 or 4 queries per
+// warp; what the scan itself needs is less.)
+int flat_smem_ok(const FlatScanArgs &a) {
+    if (a.metric == M_HAMMING) return (size_t)a.warps * 8 * a.stride4 * 16 <= (size_t)dev_info().max_smem_optin;
+    const int qw = (a.k <= 32 && a.nq <= 4) ? 1 : (a.k <= 32 && a.nq <= 8) ? 2 : 4;
+    const size_t per_warp = (size_t)qw * a.stride4 * 16;
+    int warps = (int)std::min<int64_t>(4, std::max<int64_t>(1, ceil_div(a.nq, (int64_t)qw)));
+    while (warps > 1 && per_warp * warps > 200 * 1024) warps >>= 1;
+    const int nbx = (a.stride4 * 4 + FS_BOX - 1) / FS_BOX;
+    const size_t stage = nbx <= 2 ? (size_t)nbx * 128 * std::min(a.stride4 * 4, FS_BOX) * 4
+                                  : (size_t)std::min(nbx, 8) * 32 * FS_BOX * 4;
+    return per_warp * warps + 1024 + 3 * stage + 24 <= (size_t)dev_info().max_smem_optin &&
+           fs_geom(a.nq, a.k, a.stride4).smem <= (size_t)dev_info().max_smem_optin;
+}
+
+static int hamming_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) {
+    const int units = a.n_groups * a.n_slices, threads = a.warps * 32;
+    const size_t smem = (size_t)a.warps * 8 * a.stride4 * 16;
+    auto go = [&](auto RC) {
+        constexpr int R = decltype(RC)::value;
         timing_begin(st, "hamming_scan_kernel");
         auto kern = hamming_scan_kernel<8, R>;
         if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         kern<<<units, threads, smem, st>>>(reinterpret_cast<const uint4 *>(a.db), a.n, a.stride4,
                                            reinterpret_cast<const uint4 *>(a.q), a.nq, a.k, a.n_slices, a.slice_rows,
-                                           n_groups, part);
+                                           a.n_groups, part);
         timing_end(st);
-    } else {
-        if (!a.err) return fail(GN_ERR_INVALID, "float scan: no error word");
-        // the rows as a TMA tensor: n rows x dp floats, boxes of 32 floats x the stage's rows, 128-byte swizzle
-        CUtensorMap tm;
-        const FsGeom fg = fs_geom(a.stride4);
-        GN_TRY(tmap_encode_2d(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.db, (uint64_t)a.stride4 * 4, (uint64_t)a.n,
-                              (uint64_t)a.stride4 * 16, (uint32_t)fg.bw, (uint32_t)fg.rows,
-                              fg.bw == FS_BOX ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE));
-        timing_begin(st, "float_scan_kernel");
-        // rows of exactly 32, 64 or 128 floats with k <= 32: the width as a compile-time constant
-        const int dw = (R == 1 && a.d == a.stride4 * 4 && (a.d == 32 || a.d == 64 || a.d == 128)) ? a.d : 0;
-        auto go = [&](auto MC, auto QC) {
-            constexpr int Mv = decltype(MC)::value, Qv = decltype(QC)::value;
-            auto launch = [&](auto kern) {
-                if (smem > 48 * 1024)
-                    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                kern<<<units, threads, smem, st>>>(tm, a.n, a.d, a.stride4 * 4, reinterpret_cast<const float *>(a.q),
-                                                   a.nq, a.k, a.n_slices, a.slice_rows, n_groups, part, a.err);
-            };
-            if (R == 1 && dw == 32) launch(float_scan_kernel<Mv, Qv, 1, 32>);
-            else if (R == 1 && dw == 64) launch(float_scan_kernel<Mv, Qv, 1, 64>);
-            else if (R == 1 && dw == 128) launch(float_scan_kernel<Mv, Qv, 1, 128>);
-            else launch(float_scan_kernel<Mv, Qv, (Qv == 4 ? R : 1)>);
-        };
-        auto by_qw = [&](auto MC) {
-            // fewer queries per warp only for small batches with k <= 32 (R == 1)
-            if (a.qw == 1 && R == 1) go(MC, std::integral_constant<int, 1>());
-            else if (a.qw == 2 && R == 1) go(MC, std::integral_constant<int, 2>());
-            else go(MC, std::integral_constant<int, 4>());
-        };
-        if (a.metric == M_L2) by_qw(std::integral_constant<int, M_L2>());
-        else if (a.metric == M_L1) by_qw(std::integral_constant<int, M_L1>());
-        else by_qw(std::integral_constant<int, M_LINF>());
-        timing_end(st);
-    }
-    // a batch of up to two queries per SM over many slices: a block per query
-    if (R == 1 && a.nq > 0 && a.nq <= 2 * dev_info().num_sms && a.n_slices >= 2 * MERGE_WARPS) {
-        flat_merge_split_kernel<<<(unsigned)a.nq, MERGE_WARPS * 32, 0, st>>>(
-            part, a.n_slices, a.k, a.metric == M_HAMMING, a.out_idx, a.out_dist);
-        return GN_OK;
-    }
-    const int qpb = 4;  // queries (warps) per merge block
-    flat_merge_kernel<R><<<(unsigned)ceil_div(a.nq, qpb), qpb * 32, 0, st>>>(
-        part, a.n_slices, a.k, a.nq, a.metric == M_HAMMING, a.out_idx, a.out_dist);
+        // a batch of up to two queries per SM over many slices: a block per query
+        if (R == 1 && a.nq > 0 && a.nq <= 2 * dev_info().num_sms && a.n_slices >= 2 * MERGE_WARPS) {
+            flat_merge_split_kernel<<<(unsigned)a.nq, MERGE_WARPS * 32, 0, st>>>(
+                part, a.n_slices, a.k, a.out_idx, reinterpret_cast<int64_t *>(a.out_dist));
+            return;
+        }
+        const int qpb = 4;  // queries (warps) per merge block
+        flat_merge_kernel<R><<<(unsigned)ceil_div(a.nq, qpb), qpb * 32, 0, st>>>(
+            part, a.n_slices, a.k, a.nq, a.out_idx, reinterpret_cast<int64_t *>(a.out_dist));
+    };
+    if (a.k <= 32) go(std::integral_constant<int, 1>());
+    else if (a.k <= 64) go(std::integral_constant<int, 2>());
+    else if (a.k <= 128) go(std::integral_constant<int, 4>());
+    else go(std::integral_constant<int, 8>());
     return GN_OK;
 }
 
-// CTAs of the float scan resident per SM for this metric and list size.
-template <int M, int R, int QW = 4>
-static int float_scan_occupancy1(int threads, size_t smem) {
-    int nb = 0;
-    auto kern = float_scan_kernel<M, QW, R>;
-    cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, threads, smem);
-    if (e != cudaSuccess) {  // a refused query reads as 0
-        cudaGetLastError();
-        nb = 0;
-    }
-    return nb;
-}
-template <int R>
-static int float_scan_occupancy(int metric, int qw, int threads, size_t smem) {
-    if (R == 1 && qw == 1)
-        return metric == M_L2 ? float_scan_occupancy1<M_L2, 1, 1>(threads, smem)
-               : metric == M_L1 ? float_scan_occupancy1<M_L1, 1, 1>(threads, smem)
-                                : float_scan_occupancy1<M_LINF, 1, 1>(threads, smem);
-    if (R == 1 && qw == 2)
-        return metric == M_L2 ? float_scan_occupancy1<M_L2, 1, 2>(threads, smem)
-               : metric == M_L1 ? float_scan_occupancy1<M_L1, 1, 2>(threads, smem)
-                                : float_scan_occupancy1<M_LINF, 1, 2>(threads, smem);
-    if (metric == M_L2) return float_scan_occupancy1<M_L2, R>(threads, smem);
-    if (metric == M_L1) return float_scan_occupancy1<M_L1, R>(threads, smem);
-    return float_scan_occupancy1<M_LINF, R>(threads, smem);
-}
-
-void flat_plan(FlatScanArgs &a) {
-    const DevInfo &di = dev_info();
-    // float metrics: four queries per warp, fewer for a small batch with
-    // k <= 32 so that every warp scores real queries; and no more warps than
-    // the batch fills (every warp of a CTA reads each staged row block from
-    // shared memory, so a warp of padding queries takes shared-memory
-    // bandwidth from the scan: one query over 1M x 128 rows 0.131 -> 0.092 ms).
-    // More warps with fewer queries each beat fewer warps with more (4 queries:
-    // 4 warps of one 0.133 ms, 1 warp of four 0.167 ms).
-    const int qw = (a.metric == M_HAMMING) ? 8 : (a.k <= 32 && a.nq <= 4) ? 1 : (a.k <= 32 && a.nq <= 8) ? 2 : 4;
-    const size_t per_warp = (size_t)qw * a.stride4 * 16;
-    int warps = a.metric == M_HAMMING ? 4 : (int)std::min<int64_t>(4, std::max<int64_t>(1, ceil_div(a.nq, (int64_t)qw)));
-    while (warps > 1 && per_warp * warps > 200 * 1024) warps >>= 1;
-    a.warps = warps;
-    a.qw = qw;
-    const int64_t n_groups = ceil_div(a.nq, (int64_t)warps * qw);
-    // slices of at least 128 rows (one float stage): a small database spreads
-    // over more SMs instead of running a few CTAs through many stages
-    const int64_t max_slices = std::max<int64_t>(1, a.n / 128);
-    int64_t slices;
-    if (a.metric == M_HAMMING) {
-        // aim for ~16 CTAs per SM over the launch
-        slices = std::min<int64_t>(std::max<int64_t>(1, ceil_div(16LL * di.num_sms, n_groups)), max_slices);
-    } else {
-        // units of equal cost: pick the slice count (up to about four waves of
-        // resident CTAs) whose last wave is fullest, the fewest slices on a tie
-        const int threads = warps * 32;
-        const size_t smem = fs_smem_bytes(warps, qw, a.stride4);
-        int occ = a.k <= 32 ? float_scan_occupancy<1>(a.metric, qw, threads, smem)
-                  : a.k <= 64 ? float_scan_occupancy<2>(a.metric, qw, threads, smem)
-                  : a.k <= 128 ? float_scan_occupancy<4>(a.metric, qw, threads, smem)
-                               : float_scan_occupancy<8>(a.metric, qw, threads, smem);
-        const int64_t slots = (int64_t)std::max(occ, 1) * di.num_sms;
-        const int64_t hi = std::min<int64_t>(max_slices, std::max<int64_t>(1, ceil_div(4 * slots, n_groups)));
-        slices = 1;
-        double best = -1.0;
-        for (int64_t s = 1; s <= hi; ++s) {
-            const int64_t units = n_groups * s;
-            const double eff = (double)units / (double)(ceil_div(units, slots) * slots);
-            if (eff > best + 1e-9) {
-                best = eff;
-                slices = s;
-            }
-        }
-    }
-    // float scans stage up to 128 rows at a time: whole stages per slice
-    a.slice_rows = round_up(ceil_div(a.n, slices), a.metric == M_HAMMING ? 32 : FS_ROWS);
-    a.n_slices = (int)ceil_div(a.n, a.slice_rows);
-    a.n_groups = (int)n_groups;
+static int float_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) {
+    if (!a.err) return fail(GN_ERR_INVALID, "float scan: no error word");
+    const FsGeom g = fs_geom(a.nq, a.k, a.stride4);
+    // the rows as a TMA tensor: n rows x dp floats, boxes of 32 floats x the stage's rows, 128-byte swizzle
+    CUtensorMap tm;
+    GN_TRY(tmap_encode_2d(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.db, (uint64_t)a.stride4 * 4, (uint64_t)a.n,
+                          (uint64_t)a.stride4 * 16, (uint32_t)g.bw, (uint32_t)g.rows,
+                          g.bw == FS_BOX ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE));
+    FsArgs f;
+    f.n = a.n;
+    f.nq = a.nq;
+    f.slice_rows = a.slice_rows;
+    f.list_keys = a.list_keys;
+    f.d = a.d;
+    f.dp4 = a.stride4;
+    f.k = a.k;
+    f.n_slices = a.n_slices;
+    f.n_groups = a.n_groups;
+    f.wq = g.wq;
+    f.wr = g.wr;
+    f.nbx = g.nbx;
+    f.bw = g.bw;
+    f.rows = g.rows;
+    f.cb = g.cb;
+    f.nchunk = g.nchunk;
+    f.cap = g.cap;
+    f.most = g.most;
+    f.q = reinterpret_cast<const float *>(a.q);
+    f.qcount = reinterpret_cast<int *>(part);
+    f.cand = part + round_up(a.nq * 4, 256) / 8;
+    f.gbuf = f.cand + a.nq * a.list_keys;
+    f.err = a.err;
+    GN_CUDA_TRY(cudaMemsetAsync(f.qcount, 0, (size_t)a.nq * 4, st));
+    timing_begin(st, "float_scan_kernel");
+    auto go = [&](auto MC) -> int {
+        constexpr int M = decltype(MC)::value;
+        auto launch = [&](auto kern) -> int {
+            if (g.smem > 48 * 1024)
+                GN_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem));
+            kern<<<(unsigned)a.units, FS_THREADS, g.smem, st>>>(tm, f);
+            return GN_OK;
+        };
+        const bool one = g.nchunk == 1;
+        if (g.rpt == 2) return one ? launch(float_scan_kernel<M, 4, 2, true>) : launch(float_scan_kernel<M, 4, 2, false>);
+        if (g.qw == 4) return one ? launch(float_scan_kernel<M, 4, 1, true>) : launch(float_scan_kernel<M, 4, 1, false>);
+        if (g.qw == 2) return one ? launch(float_scan_kernel<M, 2, 1, true>) : launch(float_scan_kernel<M, 2, 1, false>);
+        return one ? launch(float_scan_kernel<M, 1, 1, true>) : launch(float_scan_kernel<M, 1, 1, false>);
+    };
+    GN_TRY(a.metric == M_L2   ? go(std::integral_constant<int, M_L2>())
+           : a.metric == M_L1 ? go(std::integral_constant<int, M_L1>())
+                              : go(std::integral_constant<int, M_LINF>()));
+    timing_end(st);
+    auto finish = [&](auto RC) {
+        constexpr int R = decltype(RC)::value;
+        float *od = reinterpret_cast<float *>(a.out_dist);
+        if (a.nq <= dev_info().num_sms && R <= 2)
+            flat_finish_kernel<24, R><<<(unsigned)a.nq, 768, 0, st>>>(f.cand, f.qcount, a.list_keys, a.k, a.out_idx, od);
+        else if (a.nq <= 4 * dev_info().num_sms)
+            flat_finish_kernel<8, R><<<(unsigned)a.nq, 256, 0, st>>>(f.cand, f.qcount, a.list_keys, a.k, a.out_idx, od);
+        else
+            flat_finish_kernel<1, R><<<(unsigned)a.nq, 32, 0, st>>>(f.cand, f.qcount, a.list_keys, a.k, a.out_idx, od);
+    };
+    if (a.k <= 32) finish(std::integral_constant<int, 1>());
+    else if (a.k <= 64) finish(std::integral_constant<int, 2>());
+    else if (a.k <= 128) finish(std::integral_constant<int, 4>());
+    else finish(std::integral_constant<int, 8>());
+    return GN_OK;
 }
 
-size_t flat_part_bytes(const FlatScanArgs &a) { return (size_t)a.nq * a.n_slices * a.k * sizeof(uint64_t); }
-
-static size_t flat_smem_bytes(const FlatScanArgs &a) {
-    return a.metric == M_HAMMING ? (size_t)a.warps * a.qw * a.stride4 * 16 : fs_smem_bytes(a.warps, a.qw, a.stride4);
-}
-
-int flat_smem_ok(const FlatScanArgs &a) {
-    return flat_smem_bytes(a) <= (size_t)dev_info().max_smem_optin;
-}
-
-// Launch the warp-select path (k <= 256).  part: flat_part_bytes(a) scratch.
+// Launch the k <= 256 path.  part: flat_part_bytes(a) scratch.
 int flat_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) {
-    const int threads = a.warps * 32;
-    const size_t smem = flat_smem_bytes(a);
-    if (a.k <= 32) return launch_scan<1>(a, a.n_groups, threads, smem, part, st);
-    if (a.k <= 64) return launch_scan<2>(a, a.n_groups, threads, smem, part, st);
-    if (a.k <= 128) return launch_scan<4>(a, a.n_groups, threads, smem, part, st);
-    return launch_scan<8>(a, a.n_groups, threads, smem, part, st);
+    return a.metric == M_HAMMING ? hamming_launch(a, part, st) : float_launch(a, part, st);
 }
 
 int64_t next_pow2(int64_t v) {

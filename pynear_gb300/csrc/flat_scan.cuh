@@ -18,8 +18,9 @@ struct FlatScanArgs {
     void *out_dist = nullptr;    // nq*k float32 or int64
     int *err = nullptr;          // float metrics: device error word of the scan's bounded waits
     // filled by flat_plan
-    int warps = 4, qw = 8, n_slices = 1, n_groups = 1;
+    int warps = 4, n_slices = 1, n_groups = 1;
     int64_t slice_rows = 0;
+    int64_t units = 0, list_keys = 0, gbuf_keys = 0;  // float scan: CTAs, candidates per query, buffer keys
 };
 
 constexpr int FLAT_MAX_K_WARP = 256;

@@ -47,14 +47,13 @@
 #include <cuda_fp8.h>
 
 #include <algorithm>
-#include <cstring>
-#include <vector>
 
 #include "distance.cuh"
 #include "f32x2.cuh"
 #include "gemm_topk.cuh"
 #include "index.cuh"
 #include "kmeans.cuh"
+#include "select.cuh"
 #include "tc_scan.cuh"
 #include "tc_sm100.cuh"
 #include "tmap.cuh"
@@ -94,39 +93,6 @@ static TcGeom tc_geom(int nk, bool pilot) {
     g.stages = (int)std::min<size_t>(TC_MAX_STAGES, (room - a) / g.stage_bytes);
     g.smem = fixed + a + (size_t)g.stages * g.stage_bytes;
     return g;
-}
-
-// Ascending bitonic sort of 32 R keys, element r * 32 + lane in v[r].
-template <int R>
-__device__ __forceinline__ void warp_sort(uint64_t (&v)[R]) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int size = 2; size <= 32 * R; size <<= 1) {
-#pragma unroll
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            if (stride >= 32) {
-                const int rs = stride / 32;
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    if (r & rs) continue;
-                    const bool up = ((r * 32) & size) == 0;  // size > stride >= 32: the lane has no say
-                    const uint64_t a = v[r], b = v[r | rs];
-                    const bool swap = (a > b) == up;
-                    v[r] = swap ? b : a;
-                    v[r | rs] = swap ? a : b;
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                    const uint64_t o = __shfl_xor_sync(0xffffffffu, v[r], stride);
-                    const bool up = ((r * 32 + lane) & size) == 0;
-                    const bool low = (lane & stride) == 0;
-                    const bool keep_min = up == low;
-                    v[r] = keep_min == (o < v[r]) ? o : v[r];
-                }
-            }
-        }
-    }
 }
 
 // A buffer entry is (score bits, row); keys order by (score, row).  (Signs: the
@@ -726,77 +692,6 @@ void to_e4m3_rows(const float *X, int64_t n, int d, int ldx, void *out, float *s
 }
 
 // ── exact re-rank ─────────────────────────────────────────────────────────
-// The S smallest of a warp's m keys (all distinct) without order: thr gets a
-// bound such that exactly min(S, m) keys are at or below it.  The keys are lane-
-// strided in registers (key i * 32 + lane in v[i], KEY_EMPTY past m), and the
-// bound is built bit by bit from the count of keys below each trial value: 32
-// steps for the scores, and only where several keys share the S-th score 32 more
-// for the rows.  (Inserting ~400 keys into an ordered register list took about
-// 130 insertions of 40 instructions.)
-template <int R>
-__device__ __forceinline__ uint64_t warp_select(const uint64_t (&v)[R], int m, int S) {
-    if (m <= S) return KEY_EMPTY - 1;
-    uint32_t score = 0;
-    int below = 0;  // keys with a score below `score`
-    for (int bit = 31; bit >= 0; --bit) {
-        const uint32_t trial = score | (1u << bit);
-        int c = 0;
-#pragma unroll
-        for (int i = 0; i < R; ++i) c += key_dist(v[i]) < trial;
-        c = __reduce_add_sync(0xffffffffu, c);
-        if (c < S) {
-            score = trial;
-            below = c;
-        }
-    }
-    int at = 0;
-#pragma unroll
-    for (int i = 0; i < R; ++i) at += key_dist(v[i]) == score && v[i] != KEY_EMPTY;
-    at = __reduce_add_sync(0xffffffffu, at);
-    if (below + at <= S) return make_key(score, 0xffffffffu);
-    const int want = S - below;  // of the keys with this score, the lowest rows
-    uint32_t row = 0;
-    for (int bit = 31; bit >= 0; --bit) {
-        const uint32_t trial = row | (1u << bit);
-        int c = 0;
-#pragma unroll
-        for (int i = 0; i < R; ++i) c += key_dist(v[i]) == score && key_idx(v[i]) < trial;
-        if (__reduce_add_sync(0xffffffffu, c) < want) row = trial;
-    }
-    return make_key(score, row);
-}
-
-// The S best of a query's m candidate keys into sel[0 .. min(S, m)), any order,
-// by one warp; returns their number.
-constexpr int SEL_R = 16;  // keys per lane held in registers at a time
-__device__ __forceinline__ int warp_best(const uint64_t *__restrict__ p, int m, int S, uint64_t *sel) {
-    const int lane = threadIdx.x & 31;
-    int kept = 0;
-    for (int i0 = 0; i0 < m;) {
-        // earlier rounds' best join each round's keys
-        const int take = min(m - i0, SEL_R * 32 - kept);
-        uint64_t v[SEL_R];
-#pragma unroll
-        for (int i = 0; i < SEL_R; ++i) {
-            const int x = i * 32 + lane;
-            v[i] = x < kept ? sel[x] : x - kept < take ? p[i0 + x - kept] : KEY_EMPTY;
-        }
-        i0 += take;
-        const uint64_t thr = warp_select<SEL_R>(v, kept + take, S);
-        __syncwarp();
-        kept = 0;
-#pragma unroll
-        for (int i = 0; i < SEL_R; ++i) {
-            const bool in = v[i] <= thr && v[i] != KEY_EMPTY;
-            const unsigned b = __ballot_sync(0xffffffffu, in);
-            if (in) sel[kept + __popc(b & ((1u << lane) - 1))] = v[i];
-            kept += __popc(b);
-        }
-        __syncwarp();
-    }
-    return kept;
-}
-
 // One warp per query: the S best candidates by score, their L2 distances in the
 // reference's FP32 order (bit-identical to the exact flat scan), the k nearest.
 // Two lanes per candidate row, each with four of the reference's eight

@@ -118,7 +118,6 @@ constexpr int FS_BOX = 32;      // floats per box row (128 bytes)
 constexpr int FS_STAGES = 3;
 constexpr int FS_STAGE = 16384; // bytes of a stage at most
 constexpr int FS_THREADS = 128, FS_WARPS = 4;
-constexpr int FS_CAP_S = 128, FS_CAP_L = 512;  // buffer keys for k <= 64 (shared memory) and k <= 256 (global)
 
 // Launch shape (FlatScanArgs::fs).
 struct FsGeom {
@@ -131,9 +130,8 @@ struct FsGeom {
 
 static FsGeom fs_geom(int64_t nq, int k, int dp4) {
     FsGeom g;
-    g.cap = k <= 64 ? FS_CAP_S : FS_CAP_L;
-    // a late cut leaves the threshold loose, an early one is paid more often
-    g.most = k <= 64 ? std::min(g.cap - 32, 2 * k + 24) : g.cap - 32;
+    g.cap = list_cap(k);  // k <= 64: in shared memory, else in global
+    g.most = list_most(k);
     // small batches: one or two queries per warp, every warp on its own rows; from
     // five queries on a row's load serves four of them
     g.qw = nq <= 1 ? 1 : nq <= 2 ? 2 : 4;
@@ -153,7 +151,7 @@ static FsGeom fs_geom(int64_t nq, int k, int dp4) {
     if (g.nchunk == 1)  // short rows: more of them per stage (a TMA box has at most 256 rows)
         while (g.rows * 2 <= 256 && (size_t)g.rows * 2 * g.cb * g.bw * 4 <= FS_STAGE) g.rows *= 2;
     g.smem = qbytes() + 1024 + (size_t)FS_STAGES * g.cb * g.rows * g.bw * 4 + FS_STAGES * 16 +
-             (g.cap == FS_CAP_S ? (size_t)FS_WARPS * g.qw * FS_CAP_S * 8 : 0);
+             (g.cap == LIST_CAP_S ? (size_t)FS_WARPS * g.qw * LIST_CAP_S * 8 : 0);
     return g;
 }
 
@@ -254,50 +252,11 @@ __device__ __forceinline__ uint32_t fs_limit(uint32_t thr) {
     return __float_as_uint(__fmul_ru(t, t));
 }
 
-// Cut a buffer of m keys (k < m <= 32 R) down to its k best, in place; returns
-// the k-th best key's distance bits.  (A call, not inlined: it runs a few times
-// per list and would crowd the scan's registers and instruction cache.)
-template <int R>
-__device__ __noinline__ uint32_t fs_cut(uint64_t *buf, int m, int k) {
-    const int lane = threadIdx.x & 31;
-    __syncwarp();
-    uint64_t v[R];
-#pragma unroll
-    for (int i = 0; i < R; ++i) v[i] = i * 32 + lane < m ? buf[i * 32 + lane] : KEY_EMPTY;
-    const uint64_t thr = warp_select<R>(v, m, k);
-    __syncwarp();
-    int kept = 0;
-    uint32_t far = 0u;
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const bool in = v[i] <= thr && v[i] != KEY_EMPTY;
-        const unsigned b = __ballot_sync(0xffffffffu, in);
-        if (in) {
-            buf[kept + __popc(b & ((1u << lane) - 1))] = v[i];
-            far = max(far, key_dist(v[i]));
-        }
-        kept += __popc(b);
-    }
-    __syncwarp();
-    return __reduce_max_sync(0xffffffffu, far);
-}
-
-// Add the lanes' rows whose distance stays below thr to a list's buffer of cnt
-// keys, cutting it once it holds more than `most`; v: finish() bits, in: the lane's
-// row may enter.  Returns (count, threshold).  (A call: see fs_cut.)
+// list_add for finish() bits v, as a call (see list_cut): L2 takes the root here.
 template <int METRIC>
 __device__ __noinline__ uint2 fs_add(uint64_t *buf, uint2 state, uint32_t v, bool in, uint32_t row, int k, int most) {
     if (METRIC == M_L2) v = __float_as_uint(__fsqrt_rn(__uint_as_float(v)));
-    in = in && v < state.y;
-    const unsigned m = __ballot_sync(0xffffffffu, in);
-    const int lane = threadIdx.x & 31;
-    if (in) buf[state.x + __popc(m & ((1u << lane) - 1))] = make_key(v, row);
-    state.x += __popc(m);
-    if ((int)state.x > most) {
-        state.y = k <= 64 ? fs_cut<FS_CAP_S / 32>(buf, state.x, k) : fs_cut<FS_CAP_L / 32>(buf, state.x, k);
-        state.x = k;
-    }
-    return state;
+    return list_add<true>(buf, state, v, in, row, k, most);
 }
 
 // ONE: a stage holds whole rows (the accumulators then never outlive a group).
@@ -313,7 +272,7 @@ __global__ void __launch_bounds__(FS_THREADS, 3)
     uint64_t *sbuf = reinterpret_cast<uint64_t *>(sqf + a.wq * QW * dp4);
     const int cap = a.cap;
     // (an offset from the shared array, not a rounded pointer: the loads stay shared-memory loads)
-    const uint32_t ring_at = (uint32_t)(a.wq * QW * dp4) * 16 + (cap == FS_CAP_S ? FS_WARPS * QW * FS_CAP_S * 8 : 0);
+    const uint32_t ring_at = (uint32_t)(a.wq * QW * dp4) * 16 + (cap == LIST_CAP_S ? FS_WARPS * QW * LIST_CAP_S * 8 : 0);
     const uint32_t smem0 = smem_u32(sqf);
     uint8_t *ring = reinterpret_cast<uint8_t *>(sqf) + (((smem0 + ring_at + 1023) & ~1023u) - smem0);
     const uint32_t pitch = (uint32_t)a.bw * 4, box_bytes = (uint32_t)a.rows * pitch;
@@ -367,7 +326,7 @@ __global__ void __launch_bounds__(FS_THREADS, 3)
 
     // a list: its buffer, the keys in it, and the distance bits that a new key must
     // stay below (rows come in ascending order, so an equal distance loses the tie)
-    uint64_t *buf0 = cap == FS_CAP_S ? sbuf + warp * QW * FS_CAP_S
+    uint64_t *buf0 = cap == LIST_CAP_S ? sbuf + warp * QW * LIST_CAP_S
                                      : a.gbuf + ((size_t)blockIdx.x * FS_WARPS + warp) * QW * cap;
     int cnt[QW];
     uint32_t thr[QW], lim[QW];  // lim: fs_limit(thr)
@@ -525,8 +484,7 @@ __global__ void __launch_bounds__(FS_THREADS, 3)
         uint64_t *b = buf0 + j * cap;
         int c = cnt[j];
         if (c > k) {
-            if (cap == FS_CAP_S) fs_cut<FS_CAP_S / 32>(b, c, k);
-            else fs_cut<FS_CAP_L / 32>(b, c, k);
+            list_cut_k(b, c, k);
             c = k;
         }
         __syncwarp();
@@ -545,7 +503,7 @@ __global__ void __launch_bounds__(FS_THREADS, 3)
 template <int W, int R>
 __global__ void __launch_bounds__(W * 32)
     flat_finish_kernel(const uint64_t *__restrict__ cand, const int *__restrict__ qcount, int64_t list_keys, int k,
-                       int64_t *__restrict__ out_idx, float *__restrict__ out_dist) {
+                       int64_t *__restrict__ out_idx, float *__restrict__ out_dist, int64_t *__restrict__ out_cnt) {
     __shared__ uint64_t s_sel[(W + 1) * R * 32];
     __shared__ int s_n[W];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -576,6 +534,7 @@ __global__ void __launch_bounds__(W * 32)
         res = s_sel + W * R * 32;
         m = warp_best(s_sel, m, k, res);
     }
+    if (out_cnt && lane == 0) out_cnt[q] = m;
     uint64_t v[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = r * 32 + lane < m ? res[r * 32 + lane] : KEY_EMPTY;
@@ -816,7 +775,7 @@ void flat_plan(FlatScanArgs &a) {
     a.n_groups = (int)n_groups;
     a.list_keys = (int64_t)a.n_slices * g.wr * a.k;
     a.units = (int64_t)a.n_slices * n_groups;
-    a.gbuf_keys = g.cap == FS_CAP_L ? a.units * FS_WARPS * g.qw * FS_CAP_L : 0;
+    a.gbuf_keys = g.cap == LIST_CAP_L ? a.units * FS_WARPS * g.qw * LIST_CAP_L : 0;
 }
 
 // Scratch: Hamming, the slices' partial lists; float, the queries' counters
@@ -868,6 +827,24 @@ static int hamming_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st
     else if (a.k <= 64) go(std::integral_constant<int, 2>());
     else if (a.k <= 128) go(std::integral_constant<int, 4>());
     else go(std::integral_constant<int, 8>());
+    return GN_OK;
+}
+
+int candidates_finish(const uint64_t *cand, const int *qcount, int64_t list_keys, int64_t nq, int k, int64_t *out_idx,
+                      float *out_dist, int64_t *out_cnt, cudaStream_t st) {
+    auto finish = [&](auto RC) {
+        constexpr int R = decltype(RC)::value;
+        if (nq <= dev_info().num_sms && R <= 2)
+            flat_finish_kernel<24, R><<<(unsigned)nq, 768, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist, out_cnt);
+        else if (nq <= 4 * dev_info().num_sms)
+            flat_finish_kernel<8, R><<<(unsigned)nq, 256, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist, out_cnt);
+        else
+            flat_finish_kernel<1, R><<<(unsigned)nq, 32, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist, out_cnt);
+    };
+    if (k <= 32) finish(std::integral_constant<int, 1>());
+    else if (k <= 64) finish(std::integral_constant<int, 2>());
+    else if (k <= 128) finish(std::integral_constant<int, 4>());
+    else finish(std::integral_constant<int, 8>());
     return GN_OK;
 }
 
@@ -923,21 +900,8 @@ static int float_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) 
            : a.metric == M_L1 ? go(std::integral_constant<int, M_L1>())
                               : go(std::integral_constant<int, M_LINF>()));
     timing_end(st);
-    auto finish = [&](auto RC) {
-        constexpr int R = decltype(RC)::value;
-        float *od = reinterpret_cast<float *>(a.out_dist);
-        if (a.nq <= dev_info().num_sms && R <= 2)
-            flat_finish_kernel<24, R><<<(unsigned)a.nq, 768, 0, st>>>(f.cand, f.qcount, a.list_keys, a.k, a.out_idx, od);
-        else if (a.nq <= 4 * dev_info().num_sms)
-            flat_finish_kernel<8, R><<<(unsigned)a.nq, 256, 0, st>>>(f.cand, f.qcount, a.list_keys, a.k, a.out_idx, od);
-        else
-            flat_finish_kernel<1, R><<<(unsigned)a.nq, 32, 0, st>>>(f.cand, f.qcount, a.list_keys, a.k, a.out_idx, od);
-    };
-    if (a.k <= 32) finish(std::integral_constant<int, 1>());
-    else if (a.k <= 64) finish(std::integral_constant<int, 2>());
-    else if (a.k <= 128) finish(std::integral_constant<int, 4>());
-    else finish(std::integral_constant<int, 8>());
-    return GN_OK;
+    return candidates_finish(f.cand, f.qcount, a.list_keys, a.nq, a.k, a.out_idx, reinterpret_cast<float *>(a.out_dist),
+                             nullptr, st);
 }
 
 // Launch the k <= 256 path.  part: flat_part_bytes(a) scratch.

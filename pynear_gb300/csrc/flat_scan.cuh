@@ -29,6 +29,10 @@ void flat_plan(FlatScanArgs &a);
 size_t flat_part_bytes(const FlatScanArgs &a);
 int flat_smem_ok(const FlatScanArgs &a);
 int flat_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st);
+// The k nearest (k <= 256) of each query's qcount[q] candidate (distance, index)
+// keys at cand + q * list_keys, nearest first, with their number where out_cnt is given.
+int candidates_finish(const uint64_t *cand, const int *qcount, int64_t list_keys, int64_t nq, int k, int64_t *out_idx,
+                      float *out_dist, int64_t *out_cnt, cudaStream_t st);
 int flat_preload_hamming();
 int64_t next_pow2(int64_t v);
 void flat_large_k_launch(const FlatScanArgs &a, int64_t q_begin, int64_t qc, uint64_t *keys, uint64_t *sorted,

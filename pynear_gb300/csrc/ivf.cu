@@ -2,15 +2,16 @@
 //
 // Search of a query batch runs entirely on the device, with no host round
 // trip between its kernels:
-//   1. coarse   the nprobe nearest centroids of every query (fused GEMM +
-//               warp top-k for L2; the exact Hamming flat scan for binary);
+//   1. coarse   the nprobe nearest centroids of every query (GEMM, then a
+//               selection, for L2; the exact Hamming flat scan for binary);
 //   2. buckets  (query, probe) pairs grouped by list: counts, offsets, fill;
 //   3. plan     work items = (list, chunk of queries probing it, chunk of list
-//               rows); every (query, probe, row chunk) owns one partial slot;
-//   4. scan     a persistent kernel pulls items from an atomic counter, scores
-//               the chunk (FP32 tile GEMM for L2, popcount for Hamming) and
+//               rows); binary: every (query, probe, row chunk) owns one partial slot;
+//   4. scan     a persistent kernel pulls items from an atomic counter and scores
+//               the chunk (FP32 tile GEMM for L2, popcount for Hamming); L2 appends
+//               what can be among the query's k nearest to its candidates, binary
 //               writes each query's partial top-k to its slot;
-//   5. merge    one warp per query reduces its slots to the final top-k.
+//   5. finish   the final top-k of the candidates, or of the slots.
 // Lists are stored as a CSR (offsets, rows in list order, original ids).  The
 // float index orders its lists by descending size so the persistent scan
 // starts with the longest items.
@@ -30,6 +31,7 @@
 #include "ivf.cuh"
 #include "kmeans.cuh"
 #include "prober.cuh"
+#include "select.cuh"
 #include "timing.cuh"
 #include "topk.cuh"
 
@@ -38,91 +40,100 @@ namespace gn {
 constexpr int IVF_QCHUNK_L2 = GT_BM;  // queries per float work item
 constexpr int IVF_QCHUNK_BIN = 32;    // queries per binary work item (4 warps x 8)
 
-// ── coarse probing (float): GEMM + per-query top-nprobe ───────────────────
-// blockIdx.y selects a slice of cps centroids (one slice when the batch alone
-// fills the GPU); with several slices each writes its sorted partial top-np
-// keys to part[(q * gridDim.y + slice) * np ...] for coarse_merge_kernel.
-template <int R>
-__global__ void __launch_bounds__(GT_THREADS) ivf_coarse_kernel(const float *__restrict__ Q,
-                                                                const float *__restrict__ qn, int64_t nq, int dp,
-                                                                const float *__restrict__ C,
-                                                                const float *__restrict__ cn, int nc, int np,
-                                                                int cps, int32_t *__restrict__ probes,
-                                                                uint64_t *__restrict__ part) {
-    __shared__ GemmTileSmem s;
+// ── coarse probing (float): GEMM, then per-query top-nprobe ───────────────
+// Squared distances of a tile of 64 queries to a tile of 128 centroids, written
+// out: with the selection in the same kernel (ordered register lists, 8 queries
+// per warp) 1,000 queries against 512 centroids took 52 + 6 us, the two kernels
+// 15 + 6.
+__global__ void __launch_bounds__(GT_THREADS, 2) ivf_coarse_kernel(const float *__restrict__ Q,
+                                                                   const float *__restrict__ qn, int64_t nq, int dp,
+                                                                   const float *__restrict__ C,
+                                                                   const float *__restrict__ cn, int nc, int ldd,
+                                                                   float *__restrict__ D) {
+    extern __shared__ __align__(16) uint8_t gt_raw[];
+    GemmTileSmem<1> &s = *reinterpret_cast<GemmTileSmem<1> *>(gt_raw);
     __shared__ int64_t arow[GT_BM];
     const int64_t q0 = (int64_t)blockIdx.x * GT_BM;
-    const int cb = blockIdx.y * cps, ce = min(nc, cb + cps);
+    const int c0 = blockIdx.y * GT_BN;
     if (threadIdx.x < GT_BM) arow[threadIdx.x] = (q0 + threadIdx.x < nq) ? q0 + threadIdx.x : -1;
     __syncthreads();
-    const int tm = threadIdx.x >> 5, tn = threadIdx.x & 31;
-    WarpTopK<R> L[8];
-    uint64_t thr[8];
+    f32x2 acc[8][2];
+    gt_tile<1>(s, acc, Q, arow, dp, C, c0, nc, dp, dp);
+    const int c = c0 + gt_col(0);
+    float cv[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { L[i].init(); thr[i] = KEY_EMPTY; }
-    float acc[8][4];
-    for (int c0 = cb; c0 < ce; c0 += GT_BN) {
-        gt_tile(s, acc, Q, arow, dp, C, c0, ce, dp, dp);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int64_t q = arow[tm * 8 + i];
-            const float qv = q >= 0 ? qn[q] : 0.f;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int c = c0 + tn * 4 + j;
-                uint64_t key = KEY_EMPTY;
-                if (c < ce && q >= 0) {
-                    const float v = fmaxf(0.f, fmaf(-2.f, acc[i][j], qv + cn[c]));
-                    key = make_key(__float_as_uint(v), (uint32_t)c);
-                }
-                L[i].offer(key, thr[i], np);
-            }
-        }
-    }
-    const int lane = threadIdx.x & 31;
+    for (int j = 0; j < 4; ++j) cv[j] = c + j < nc ? cn[c + j] : 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int64_t q = arow[tm * 8 + i];
-        if (q < 0) continue;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-            const int p = r * 32 + lane;
-            if (p >= np) continue;
-            if (part) part[((size_t)q * gridDim.y + blockIdx.y) * np + p] = L[i].v[r];
-            else probes[q * np + p] = (L[i].v[r] == KEY_EMPTY) ? -1 : (int32_t)key_idx(L[i].v[r]);
-        }
+        const int64_t q = arow[(threadIdx.x >> 5) * 8 + i];
+        if (q < 0 || c >= nc) continue;
+        const float qv = qn[q];
+        float a[4];
+        unpack2(acc[i][0], a[0], a[1]);
+        unpack2(acc[i][1], a[2], a[3]);
+        float4 v;  // columns past nc land in the row's padding
+        v.x = fmaxf(0.f, fmaf(-2.f, a[0], qv + cv[0]));
+        v.y = fmaxf(0.f, fmaf(-2.f, a[1], qv + cv[1]));
+        v.z = fmaxf(0.f, fmaf(-2.f, a[2], qv + cv[2]));
+        v.w = fmaxf(0.f, fmaf(-2.f, a[3], qv + cv[3]));
+        *reinterpret_cast<float4 *>(D + q * ldd + c) = v;
     }
 }
 
+// The np nearest centroids of each query, nearest first (ties to the lower), by
+// one warp: as list ids (probes) or as (distance, list) keys.
+constexpr int CS_WARPS = 4;
 template <int R>
-__global__ void coarse_merge_kernel(const uint64_t *__restrict__ part, int nsplit, int np, int64_t nq,
-                                    int32_t *__restrict__ probes, uint64_t *__restrict__ keys_out) {
-    const int lane = threadIdx.x & 31;
-    const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+__global__ void __launch_bounds__(CS_WARPS * 32)
+    coarse_select_kernel(const float *__restrict__ D, int ldd, int nc, int np, int64_t nq,
+                         int32_t *__restrict__ probes, uint64_t *__restrict__ keys_out) {
+    __shared__ uint64_t s_sel[CS_WARPS][R * 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t q = (int64_t)blockIdx.x * CS_WARPS + warp;
     if (q >= nq) return;
-    WarpTopK<R> L;
-    L.init();
-    uint64_t thr = KEY_EMPTY;
-    for (int sp = 0; sp < nsplit; ++sp)
-        for (int j0 = 0; j0 < np; j0 += 32) {
-            const int j = j0 + lane;
-            L.offer(j < np ? part[((size_t)q * nsplit + sp) * np + j] : KEY_EMPTY, thr, np);
-        }
+    const float *d = D + q * ldd;
+    const int m = warp_best_of([&](int c) { return make_key(__float_as_uint(d[c]), (uint32_t)c); }, nc, np,
+                               s_sel[warp]);
+    uint64_t v[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = r * 32 + lane < m ? s_sel[warp][r * 32 + lane] : KEY_EMPTY;
+    warp_sort<R>(v);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         const int p = r * 32 + lane;
         if (p >= np) continue;
-        if (keys_out) keys_out[q * np + p] = L.v[r];
-        else probes[q * np + p] = (L.v[r] == KEY_EMPTY) ? -1 : (int32_t)key_idx(L.v[r]);
+        if (keys_out) keys_out[q * np + p] = v[r];
+        else probes[q * np + p] = v[r] == KEY_EMPTY ? -1 : (int32_t)key_idx(v[r]);
     }
 }
 
 // ── bucketing and planning ────────────────────────────────────────────────
-__global__ void ivf_bucket_count_kernel(const int32_t *__restrict__ probes, int64_t npairs, int32_t *__restrict__ bcnt) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= npairs) return;
-    const int32_t l = probes[t];
-    if (l >= 0) atomicAdd(bcnt + l, 1);
+// A block takes BK_PAIRS pairs and counts them by list in shared memory, so that
+// a list that many queries probe gets one global atomic per block instead of one
+// per pair (115k pairs over 1,024 lists of Zipf sizes: counting 31 us and filling
+// 33 us with an atomic per pair, 5 and 8 us so).
+constexpr int BK_NT = 1024, BK_PAIRS = 4 * BK_NT;
+__global__ void __launch_bounds__(BK_NT) ivf_bucket_count_kernel(const int32_t *__restrict__ probes, int64_t npairs,
+                                                                int nc, bool shared, int32_t *__restrict__ bcnt) {
+    extern __shared__ int32_t bk_cnt[];  // [nc]
+    if (!shared) {  // more lists than shared memory counts
+        for (int64_t t = (int64_t)blockIdx.x * BK_PAIRS + threadIdx.x, e = min(npairs, t - threadIdx.x + BK_PAIRS); t < e;
+             t += BK_NT)
+            if (const int32_t l = probes[t]; l >= 0) atomicAdd(bcnt + l, 1);
+        return;
+    }
+    for (int l = threadIdx.x; l < nc; l += BK_NT) bk_cnt[l] = 0;
+    __syncthreads();
+    const int64_t b0 = (int64_t)blockIdx.x * BK_PAIRS;
+#pragma unroll
+    for (int i = 0; i < BK_PAIRS / BK_NT; ++i) {
+        const int64_t t = b0 + i * BK_NT + threadIdx.x;
+        const int32_t l = t < npairs ? probes[t] : -1;
+        if (l >= 0) atomicAdd(bk_cnt + l, 1);
+    }
+    __syncthreads();
+    for (int l = threadIdx.x; l < nc; l += BK_NT)
+        if (const int32_t c = bk_cnt[l]) atomicAdd(bcnt + l, c);
 }
 
 // Exclusive block-wide scan of per-thread totals (one block of 1024 threads).
@@ -183,13 +194,35 @@ __global__ void __launch_bounds__(1024) ivf_plan_kernel(const int32_t *__restric
     }
 }
 
-__global__ void ivf_bucket_fill_kernel(const int32_t *__restrict__ probes, int64_t npairs,
-                                       const int64_t *__restrict__ boff, int32_t *__restrict__ fill,
-                                       int64_t *__restrict__ bucket) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= npairs) return;
-    const int32_t l = probes[t];
-    if (l >= 0) bucket[boff[l] + atomicAdd(fill + l, 1)] = t;
+__global__ void __launch_bounds__(BK_NT) ivf_bucket_fill_kernel(const int32_t *__restrict__ probes, int64_t npairs,
+                                                               int nc, bool shared, const int64_t *__restrict__ boff,
+                                                               int32_t *__restrict__ fill,
+                                                               int64_t *__restrict__ bucket) {
+    extern __shared__ int32_t bk_cnt[];  // [nc] counts, then the block's first place in each list's bucket
+    if (!shared) {
+        for (int64_t t = (int64_t)blockIdx.x * BK_PAIRS + threadIdx.x, e = min(npairs, t - threadIdx.x + BK_PAIRS); t < e;
+             t += BK_NT)
+            if (const int32_t l = probes[t]; l >= 0) bucket[boff[l] + atomicAdd(fill + l, 1)] = t;
+        return;
+    }
+    for (int l = threadIdx.x; l < nc; l += BK_NT) bk_cnt[l] = 0;
+    __syncthreads();
+    const int64_t b0 = (int64_t)blockIdx.x * BK_PAIRS;
+    int32_t list[BK_PAIRS / BK_NT], rank[BK_PAIRS / BK_NT];
+#pragma unroll
+    for (int i = 0; i < BK_PAIRS / BK_NT; ++i) {
+        const int64_t t = b0 + i * BK_NT + threadIdx.x;
+        list[i] = t < npairs ? probes[t] : -1;
+        rank[i] = list[i] >= 0 ? atomicAdd(bk_cnt + list[i], 1) : 0;
+    }
+    __syncthreads();
+    for (int l = threadIdx.x; l < nc; l += BK_NT)
+        if (const int32_t c = bk_cnt[l]) bk_cnt[l] = atomicAdd(fill + l, c);
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < BK_PAIRS / BK_NT; ++i)
+        if (list[i] >= 0)
+            bucket[boff[list[i]] + bk_cnt[list[i]] + rank[i]] = b0 + i * BK_NT + threadIdx.x;
 }
 
 // per query (one warp): slot offset of each probe (relative, exclusive scan
@@ -245,8 +278,8 @@ __global__ void __launch_bounds__(1024) ivf_plan_small_kernel(
     int qchunk, int slot_rc, int32_t *__restrict__ bcnt, int64_t *__restrict__ boff, int64_t *__restrict__ item_off,
     int64_t *__restrict__ bucket, int64_t *__restrict__ slot_rel, int64_t *__restrict__ qcount,
     int64_t *__restrict__ qslot, int64_t *__restrict__ counter) {
-    extern __shared__ int32_t plan_sm[];  // [nc] counts, [nc] fill cursors
-    int32_t *s_cnt = plan_sm, *s_fill = plan_sm + nc;
+    extern __shared__ int32_t plan_sm[];  // [nc] counts, [nc] fill cursors, [nc] slots of a list
+    int32_t *s_cnt = plan_sm, *s_fill = plan_sm + nc, *s_slots = plan_sm + 2 * nc;
     const int t = threadIdx.x, nt = blockDim.x;
     const int64_t npairs = nq * np;
     for (int l = t; l < nc; l += nt) s_cnt[l] = s_fill[l] = 0;
@@ -272,6 +305,7 @@ __global__ void __launch_bounds__(1024) ivf_plan_small_kernel(
         for (int l = b; l < e; ++l) {
             const int64_t cnt = s_cnt[l], len = list_off[l + 1] - list_off[l];
             bcnt[l] = (int32_t)cnt;
+            if (slot_rc > 0) s_slots[l] = (int32_t)((len + slot_rc - 1) / slot_rc);
             boff[l] = xb;
             item_off[l] = xi;
             xb += cnt;
@@ -287,27 +321,40 @@ __global__ void __launch_bounds__(1024) ivf_plan_small_kernel(
         const int32_t l = probes[i];
         if (l >= 0) bucket[boff[l] + atomicAdd(&s_fill[l], 1)] = i;
     }
-    // slots: warp per query
-    const int lane = t & 31;
-    for (int64_t q = t >> 5; q < nq; q += nt >> 5) {
-        int64_t s = 0;
-        for (int p0 = 0; p0 < np; p0 += 32) {
-            const int p = p0 + lane;
-            int64_t c = 0;
-            if (p < np) {
+    if (slot_rc <= 0) return;  // no partial slots
+    if (nq > nt / 32) {  // slots: thread per query
+        for (int64_t q = t; q < nq; q += nt) {
+            int64_t s = 0;
+#pragma unroll 4
+            for (int p = 0; p < np; ++p) {
                 const int32_t l = probes[q * np + p];
-                if (l >= 0) c = (list_off[l + 1] - list_off[l] + slot_rc - 1) / slot_rc;
+                slot_rel[q * np + p] = s;
+                s += l >= 0 ? s_slots[l] : 0;
             }
-            int64_t inc = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int64_t v = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += v;
-            }
-            if (p < np) slot_rel[q * np + p] = s + inc - c;
-            s += __shfl_sync(0xffffffffu, inc, 31);
+            qcount[q] = s;
         }
-        if (lane == 0) qcount[q] = s;
+    } else {  // few queries: warp per query
+        const int lane = t & 31;
+        for (int64_t q = t >> 5; q < nq; q += nt >> 5) {
+            int64_t s = 0;
+            for (int p0 = 0; p0 < np; p0 += 32) {
+                const int p = p0 + lane;
+                int64_t c = 0;
+                if (p < np) {
+                    const int32_t l = probes[q * np + p];
+                    if (l >= 0) c = s_slots[l];
+                }
+                int64_t inc = c;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int64_t v = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= o) inc += v;
+                }
+                if (p < np) slot_rel[q * np + p] = s + inc - c;
+                s += __shfl_sync(0xffffffffu, inc, 31);
+            }
+            if (lane == 0) qcount[q] = s;
+        }
     }
     __syncthreads();
     {
@@ -336,19 +383,102 @@ __device__ __forceinline__ int find_list(const int64_t *item_off, int nc, int64_
 }
 
 // ── float list scan (persistent) ──────────────────────────────────────────
-template <int R>
-__global__ void __launch_bounds__(GT_THREADS) ivf_scan_kernel(
+// Bound of each query's k-th smallest distance from up to IB_ROWS rows of its
+// first probed lists (evenly spaced in the list that fills the rest; the lists
+// are in order of distance), in the scan's own arithmetic: qbound = a distance
+// (bits) that k rows stay below.  Warp per query, four rows per lane.
+constexpr int IB_ROWS = 128, IB_WARPS = 4;
+__global__ void __launch_bounds__(IB_WARPS * 32)
+    ivf_bound_kernel(const float *__restrict__ Q, const float *__restrict__ qn, int np, int dp,
+                     const float *__restrict__ V, const float *__restrict__ vn, const int64_t *__restrict__ list_off,
+                     const int32_t *__restrict__ probes, int64_t nq, int k, uint32_t *__restrict__ qbound) {
+    const int lane = threadIdx.x & 31;
+    const int64_t q = (int64_t)blockIdx.x * IB_WARPS + (threadIdx.x >> 5);
+    if (q >= nq) return;
+    int64_t row[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) row[i] = -1;
+    int have = 0;
+    for (int p = 0; p < np && have < IB_ROWS; ++p) {
+        const int32_t l = probes[q * np + p];
+        if (l < 0) continue;
+        const int64_t lb = list_off[l], len = list_off[l + 1] - lb;
+        const int take = (int)min(len, (int64_t)(IB_ROWS - have));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int x = i * 32 + lane - have;
+            if (x >= 0 && x < take) row[i] = lb + x * len / take;
+        }
+        have += take;
+    }
+    uint32_t bound = 0xffffffffu;
+    if (have >= k) {
+        const float4 *q4 = reinterpret_cast<const float4 *>(Q + q * dp);
+        const float4 *x4[4];
+        float acc[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            x4[i] = reinterpret_cast<const float4 *>(V + max(row[i], (int64_t)0) * dp);
+            acc[i] = 0.f;
+        }
+#pragma unroll 4
+        for (int j = 0; j < dp / 4; ++j) {
+            const float4 a = q4[j];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 x = x4[i][j];
+                acc[i] = fmaf(a.x, x.x, acc[i]);
+                acc[i] = fmaf(a.y, x.y, acc[i]);
+                acc[i] = fmaf(a.z, x.z, acc[i]);
+                acc[i] = fmaf(a.w, x.w, acc[i]);
+            }
+        }
+        const float qv = qn[q];
+        uint64_t v[4];
+        uint32_t far = 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[i] = KEY_EMPTY;
+            if (row[i] < 0) continue;
+            const uint32_t bits = __float_as_uint(fmaxf(0.f, fmaf(-2.f, acc[i], qv + vn[row[i]])));
+            v[i] = make_key(bits, (uint32_t)(i * 32 + lane));
+            far = max(far, bits);
+        }
+        bound = (have == k ? __reduce_max_sync(0xffffffffu, far) : key_dist(warp_select<4>(v, have, k))) + 1u;
+    }
+    if (lane == 0) qbound[q] = bound;
+}
+
+// list_add as a call (see list_cut); a lane holds four neighbouring rows, so ids do
+// not come in order.
+__device__ __noinline__ uint2 ivf_add(uint64_t *buf, uint2 state, uint32_t bits, bool in, uint32_t id, int k, int most) {
+    return list_add<false>(buf, state, bits, in, id, k, most);
+}
+
+// Items (list, 64 of its queries, rc of its rows) from a counter.  A row's
+// distance to a query is a candidate while it is below the query's bound (from
+// ivf_bound_kernel, lowered by items that filled a buffer); an item's k best
+// candidates of a query join the query's list, from which candidates_finish
+// answers.  200k x 128 over 512 lists of Zipf sizes, 1,000 queries, 10 probes, k
+// 10: 698 us with an ordered list per (query, item) and items of up to 4,096 rows
+// (one of 64 queries kept a CTA busy for the whole scan), 261 us so, and 27 us for
+// the bounds.
+template <int H>
+__global__ void __launch_bounds__(GT_THREADS, 2) ivf_scan_kernel(
     const float *__restrict__ Q, const float *__restrict__ qn, int np, int dp, const float *__restrict__ V,
     const float *__restrict__ vn, const int32_t *__restrict__ ids, const int64_t *__restrict__ list_off, int nc,
     const int64_t *__restrict__ boff, const int64_t *__restrict__ bucket, const int64_t *__restrict__ item_off,
-    int rc, const int64_t *__restrict__ qslot, const int64_t *__restrict__ slot_rel, int k,
-    int *__restrict__ counter, uint64_t *__restrict__ part) {
-    __shared__ GemmTileSmem s;
-    __shared__ int64_t arow[GT_BM], apair[GT_BM];
+    int rc, int k, int *__restrict__ counter, uint32_t *qbound, uint64_t *__restrict__ bufs,
+    uint64_t *__restrict__ cand, int *__restrict__ qcount, int64_t list_keys) {
+    extern __shared__ __align__(16) uint8_t gt_raw[];
+    GemmTileSmem<H> &s = *reinterpret_cast<GemmTileSmem<H> *>(gt_raw);
+    __shared__ int64_t arow[GT_BM];
     __shared__ int64_t s_item;
     __shared__ int s_list;
     const int64_t total = item_off[nc];
-    const int tm = threadIdx.x >> 5, tn = threadIdx.x & 31;
+    const int tm = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int cap = list_cap(k), most = list_most(k);
+    uint64_t *const buf = bufs + ((size_t)blockIdx.x * GT_BM + tm * 8) * cap;
     for (;;) {
         if (threadIdx.x == 0) {
             s_item = atomicAdd(counter, 1);
@@ -363,56 +493,74 @@ __global__ void __launch_bounds__(GT_THREADS) ivf_scan_kernel(
         const int64_t local = item - item_off[l];
         const int64_t qc = local / nrc, rch = local % nrc;
         const int64_t b0 = boff[l] + qc * GT_BM, b1 = min(boff[l + 1], b0 + GT_BM);
-        if (threadIdx.x < GT_BM) {
-            const int64_t pr = (b0 + threadIdx.x < b1) ? bucket[b0 + threadIdx.x] : -1;
-            apair[threadIdx.x] = pr;
-            arow[threadIdx.x] = pr >= 0 ? pr / np : -1;
-        }
+        if (threadIdx.x < GT_BM) arow[threadIdx.x] = b0 + threadIdx.x < b1 ? bucket[b0 + threadIdx.x] / np : -1;
         __syncthreads();
         const int64_t r0 = lb + rch * rc, r1 = min(le, r0 + rc);
-        WarpTopK<R> L[8];
-        uint64_t thr[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) { L[i].init(); thr[i] = KEY_EMPTY; }
         float qv[8];
+        int cnt[8];
+        uint32_t thr[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int64_t q = arow[tm * 8 + i];
             qv[i] = q >= 0 ? qn[q] : 0.f;
+            thr[i] = q >= 0 ? *reinterpret_cast<volatile uint32_t *>(qbound + q) : 0u;
+            cnt[i] = 0;
         }
-        float acc[8][4];
-        for (int64_t rb = r0; rb < r1; rb += GT_BN) {
-            gt_tile(s, acc, Q, arow, dp, V, rb, r1, dp, dp);
-            float xn[4];
-            uint32_t xid[4];
+        f32x2 acc[8][2 * H];
+        for (int64_t rb = r0; rb < r1; rb += GT_BN * H) {
+            gt_tile<H>(s, acc, Q, arow, dp, V, rb, r1, dp, dp);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int64_t row = rb + tn * 4 + j;
-                xn[j] = row < r1 ? vn[row] : 0.f;
-                xid[j] = row < r1 ? (uint32_t)ids[row] : 0u;
-            }
+            for (int h = 0; h < H; ++h) {
+                const int64_t row = rb + gt_col(2 * h);
+                float xn[4];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const bool qok = arow[tm * 8 + i] >= 0;
+                for (int j = 0; j < 4; ++j) xn[j] = row + j < r1 ? vn[row + j] : 0.f;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int64_t row = rb + tn * 4 + j;
-                    uint64_t key = KEY_EMPTY;
-                    if (qok && row < r1) {
-                        const float v = fmaxf(0.f, fmaf(-2.f, acc[i][j], qv[i] + xn[j]));
-                        key = make_key(__float_as_uint(v), xid[j]);
+                for (int i = 0; i < 8; ++i) {
+                    float a[4];
+                    unpack2(acc[i][2 * h], a[0], a[1]);
+                    unpack2(acc[i][2 * h + 1], a[2], a[3]);
+                    uint32_t bits[4];
+                    bool any = false;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        bits[j] = __float_as_uint(fmaxf(0.f, fmaf(-2.f, a[j], qv[i] + xn[j])));
+                        any = any || bits[j] < thr[i];
                     }
-                    L[i].offer(key, thr[i], k);
+                    if (!__any_sync(0xffffffffu, any && row < r1)) continue;
+                    uint2 st = make_uint2(cnt[i], thr[i]);
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const bool in = bits[j] < thr[i] && row + j < r1;
+                        if (__any_sync(0xffffffffu, in))
+                            st = ivf_add(buf + i * cap, st, bits[j], in, in ? (uint32_t)ids[row + j] : 0u, k, most);
+                    }
+                    cnt[i] = (int)st.x;
+                    thr[i] = st.y;
                 }
             }
         }
+        // each list's k best to its query's candidates, places taken by eight lanes at once
+        int n = 0;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int64_t pr = apair[tm * 8 + i];
-            if (pr >= 0) {
-                const int64_t slot = qslot[pr / np] + slot_rel[pr] + rch;
-                L[i].store(part + slot * k, k);
+            int c = cnt[i];
+            if (c > k) {
+                const uint32_t far = list_cut_k(buf + i * cap, c, k);
+                if (lane == 0) atomicMin(qbound + arow[tm * 8 + i], far + 1u);
+                c = k;
             }
+            if (lane == i) n = c;
+        }
+        __syncwarp();
+        int at = 0;
+        if (n > 0) at = atomicAdd(qcount + arow[tm * 8 + (lane & 7)], n);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int c = __shfl_sync(0xffffffffu, n, i), p = __shfl_sync(0xffffffffu, at, i);
+            if (c == 0) continue;
+            uint64_t *dst = cand + arow[tm * 8 + i] * list_keys + p;
+            for (int e = lane; e < c; e += 32) dst[e] = buf[i * cap + e];
         }
         __syncthreads();
     }
@@ -489,10 +637,10 @@ __global__ void __launch_bounds__(128) ivfbin_scan_kernel(
     }
 }
 
-// ── merge of a query's slots ──────────────────────────────────────────────
+// ── merge of a query's slots (binary) ──────────────────────────────────────────────
 template <int R>
 __global__ void ivf_merge_kernel(const uint64_t *__restrict__ part, const int64_t *__restrict__ qslot, int64_t nq,
-                                 int k, int is_hamming, int64_t *__restrict__ out_idx, void *__restrict__ out_dist,
+                                 int k, int64_t *__restrict__ out_idx, int64_t *__restrict__ out_dist,
                                  int64_t *__restrict__ out_cnt) {
     const int lane = threadIdx.x & 31;
     const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -517,8 +665,7 @@ __global__ void ivf_merge_kernel(const uint64_t *__restrict__ part, const int64_
         cnt += __popc(__ballot_sync(0xffffffffu, pos < k && !e));
         if (pos < k) {
             out_idx[q * k + pos] = e ? -1 : (int64_t)key_idx(L.v[r]);
-            if (is_hamming) reinterpret_cast<int64_t *>(out_dist)[q * k + pos] = e ? 0 : (int64_t)key_dist(L.v[r]);
-            else reinterpret_cast<float *>(out_dist)[q * k + pos] = e ? 0.f : __uint_as_float(key_dist(L.v[r]));
+            out_dist[q * k + pos] = e ? 0 : (int64_t)key_dist(L.v[r]);
         }
     }
     if (lane == 0 && out_cnt) out_cnt[q] = cnt;
@@ -548,7 +695,7 @@ __global__ void i64_to_i32_kernel(const int64_t *__restrict__ a, int64_t n, int3
 }
 
 // ── shared host helpers ───────────────────────────────────────────────────
-static int g_scan_blocks_l2 = 0, g_scan_blocks_bin = 0;
+static int g_scan_blocks_bin = 0;
 
 template <typename F>
 static int dispatch_r(int k, F &&f) {
@@ -594,11 +741,12 @@ constexpr int64_t PLAN_SMALL_PAIRS = 16384;  // batches planned by one block
 constexpr int PLAN_SMALL_LISTS = 8192;
 
 // Bucket the (query, probe) pairs by list and plan the work items; probes
-// (int32, nq*np) must be filled.  Produces boff, bucket, item_off, slot_rel,
-// qslot in S.  All on the device, no host synchronisation.
+// (int32, nq*np) must be filled.  Produces boff, bucket, item_off and, unless
+// slot_rc is negative, slot_rel, qslot in S.  All on the device, no host
+// synchronisation.
 int ivf_plan(IvfScratch &S, int64_t nq, int np, int nc, const int64_t *d_list_off, int rc, int qchunk,
              cudaStream_t st, int slot_rc) {
-    if (slot_rc <= 0) slot_rc = rc;
+    if (slot_rc == 0) slot_rc = rc;
     const int64_t npairs = nq * np;
     GN_TRY(S.bcnt.ensure((size_t)nc * 4));
     GN_TRY(S.fill.ensure((size_t)nc * 4));
@@ -610,11 +758,11 @@ int ivf_plan(IvfScratch &S, int64_t nq, int np, int nc, const int64_t *d_list_of
     GN_TRY(S.qslot.ensure((size_t)(nq + 1) * 8));
     GN_TRY(S.counter.ensure(8));
     if (npairs <= PLAN_SMALL_PAIRS && nc <= PLAN_SMALL_LISTS) {  // one block does it all
-        const size_t smem = (size_t)nc * 2 * sizeof(int32_t);
+        const size_t smem = (size_t)nc * 3 * sizeof(int32_t);
         static bool attr = false;
         if (!attr) {
             GN_CUDA_TRY(cudaFuncSetAttribute(ivf_plan_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)(PLAN_SMALL_LISTS * 2 * sizeof(int32_t))));
+                                             (int)(PLAN_SMALL_LISTS * 3 * sizeof(int32_t))));
             attr = true;
         }
         ivf_plan_small_kernel<<<1, 1024, smem, st>>>(S.probes.as<int32_t>(), nq, np, nc, d_list_off, rc, qchunk,
@@ -628,33 +776,40 @@ int ivf_plan(IvfScratch &S, int64_t nq, int np, int nc, const int64_t *d_list_of
     GN_CUDA_TRY(cudaMemsetAsync(S.bcnt.p, 0, (size_t)nc * 4, st));
     GN_CUDA_TRY(cudaMemsetAsync(S.fill.p, 0, (size_t)nc * 4, st));
     GN_CUDA_TRY(cudaMemsetAsync(S.counter.p, 0, 8, st));
-    const unsigned pb = (unsigned)ceil_div(npairs, 256);
-    ivf_bucket_count_kernel<<<pb, 256, 0, st>>>(S.probes.as<int32_t>(), npairs, S.bcnt.as<int32_t>());
+    const bool shared = (size_t)nc * sizeof(int32_t) <= (size_t)dev_info().max_smem_optin;
+    const size_t bsm = shared ? (size_t)nc * sizeof(int32_t) : 0;
+    if (bsm > 48 * 1024) {
+        GN_CUDA_TRY(cudaFuncSetAttribute(ivf_bucket_count_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm));
+        GN_CUDA_TRY(cudaFuncSetAttribute(ivf_bucket_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bsm));
+    }
+    const unsigned pb = (unsigned)ceil_div(npairs, BK_PAIRS);
+    ivf_bucket_count_kernel<<<pb, BK_NT, bsm, st>>>(S.probes.as<int32_t>(), npairs, nc, shared, S.bcnt.as<int32_t>());
     ivf_plan_kernel<<<1, 1024, 0, st>>>(S.bcnt.as<int32_t>(), d_list_off, nc, rc, qchunk, S.boff.as<int64_t>(),
                                         S.item_off.as<int64_t>());
-    ivf_bucket_fill_kernel<<<pb, 256, 0, st>>>(S.probes.as<int32_t>(), npairs, S.boff.as<int64_t>(),
-                                               S.fill.as<int32_t>(), S.bucket.as<int64_t>());
-    ivf_slots_kernel<<<(unsigned)ceil_div(nq, 4), 128, 0, st>>>(S.probes.as<int32_t>(), nq, np, d_list_off,
-                                                                  slot_rc, S.slot_rel.as<int64_t>(),
-                                                                  S.qcount.as<int64_t>());
-    ivf_qscan_kernel<<<1, 1024, 0, st>>>(S.qcount.as<int64_t>(), nq, S.qslot.as<int64_t>());
+    ivf_bucket_fill_kernel<<<pb, BK_NT, bsm, st>>>(S.probes.as<int32_t>(), npairs, nc, shared, S.boff.as<int64_t>(),
+                                                   S.fill.as<int32_t>(), S.bucket.as<int64_t>());
+    if (slot_rc > 0) {
+        ivf_slots_kernel<<<(unsigned)ceil_div(nq, 4), 128, 0, st>>>(S.probes.as<int32_t>(), nq, np, d_list_off, slot_rc,
+                                                                    S.slot_rel.as<int64_t>(), S.qcount.as<int64_t>());
+        ivf_qscan_kernel<<<1, 1024, 0, st>>>(S.qcount.as<int64_t>(), nq, S.qslot.as<int64_t>());
+    }
     GN_CUDA_TRY(cudaGetLastError());
     return GN_OK;
 }
 
-// Plan, run the metric's scan kernel (scan_launch(grid)), merge the slots.
+// Binary: plan, run the scan kernel (scan_launch(grid)), merge the slots.
 template <typename ScanLaunch>
 static int ivf_run_lists(IvfScratch &S, int64_t nq, int np, int nc, const int64_t *d_list_off, int rc, int qchunk,
-                         int k, int is_hamming, int64_t *d_idx, void *d_dist, int64_t *d_cnt, int grid,
-                         ScanLaunch &&scan_launch, cudaStream_t st) {
+                         int k, int64_t *d_idx, int64_t *d_dist, int64_t *d_cnt, int grid, ScanLaunch &&scan_launch,
+                         cudaStream_t st) {
     GN_TRY(ivf_plan(S, nq, np, nc, d_list_off, rc, qchunk, st));
-    timing_begin(st, is_hamming ? "ivfbin_scan_kernel" : "ivf_scan_kernel");
+    timing_begin(st, "ivfbin_scan_kernel");
     GN_TRY(scan_launch(grid));
     timing_end(st);
     return dispatch_r(k, [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         ivf_merge_kernel<R><<<(unsigned)ceil_div(nq, 4), 128, 0, st>>>(S.part.as<uint64_t>(), S.qslot.as<int64_t>(),
-                                                                       nq, k, is_hamming, d_idx, d_dist, d_cnt);
+                                                                       nq, k, d_idx, d_dist, d_cnt);
         return GN_OK;
     });
 }
@@ -710,51 +865,42 @@ static int ivfl2_build_from_labels(gn_index *ix, const float *dX, int64_t n, int
 }
 
 // Coarse probing of a float IVF: qn = |q|^2 and the np nearest lists of each
-// query.  Small batches split the centroids over more CTAs.  With keep_keys
-// the sorted partial key lists stay in T.cpart (nsplit of them per query) and
-// probes are not written; otherwise probes get the merged list ids.
-int ivfl2_coarse_run(gn_index *ix, const float *dQ, int64_t nq, int np, bool keep_keys, int *nsplit_out,
-                     cudaStream_t st) {
+// query, nearest first, as list ids in T.probes, or (keys given) as sorted
+// (squared distance, list) keys.  The distances of up to CS_BYTES of queries are
+// written out at a time.
+constexpr int64_t CS_BYTES = 256ll << 20;
+static int ivfl2_coarse_run(gn_index *ix, const float *dQ, int64_t nq, int np, uint64_t *keys, cudaStream_t st) {
     IvfL2State &S = *ix->ivfl2;
     IvfScratch &T = S.s;
     GN_TRY(T.qn.ensure((size_t)nq * 4));
     GN_TRY(T.probes.ensure((size_t)nq * np * 4));
     row_norms(dQ, nq, S.dp, T.qn.as<float>(), st);
-    const int64_t qblocks = ceil_div(nq, GT_BM);
-    int nsplit = 1;
-    while (qblocks * nsplit * 2 <= dev_info().num_sms && (int64_t)GT_BN * nsplit * 2 <= S.nc) nsplit *= 2;
-    const int cps = (int)round_up(ceil_div(S.nc, nsplit), GT_BN);
-    nsplit = (int)ceil_div(S.nc, cps);
-    const bool use_part = keep_keys || nsplit > 1;
-    if (use_part) GN_TRY(T.cpart.ensure((size_t)nq * nsplit * np * 8));
-    if (nsplit_out) *nsplit_out = nsplit;
-    return dispatch_r(np, [&](auto RC) {
-        constexpr int R = decltype(RC)::value;
-        ivf_coarse_kernel<R><<<dim3((unsigned)qblocks, (unsigned)nsplit), GT_THREADS, 0, st>>>(
-            dQ, T.qn.as<float>(), nq, S.dp, S.cent.as<float>(), S.cnorm.as<float>(), S.nc, np, cps,
-            T.probes.as<int32_t>(), use_part ? T.cpart.as<uint64_t>() : nullptr);
-        if (use_part && !keep_keys)
-            coarse_merge_kernel<R><<<(unsigned)ceil_div(nq, 4), 128, 0, st>>>(T.cpart.as<uint64_t>(), nsplit, np, nq,
-                                                                              T.probes.as<int32_t>(), nullptr);
-        return GN_OK;
-    });
+    const int ldd = (int)round_up(S.nc, 4);
+    const int64_t step = std::min<int64_t>(nq, round_up(std::max<int64_t>(1, CS_BYTES / (4 * ldd)), GT_BM));
+    GN_TRY(T.cpart.ensure((size_t)step * ldd * 4));
+    float *D = T.cpart.as<float>();
+    for (int64_t q0 = 0; q0 < nq; q0 += step) {
+        const int64_t m = std::min(step, nq - q0);
+        ivf_coarse_kernel<<<dim3((unsigned)ceil_div(m, GT_BM), (unsigned)ceil_div(S.nc, GT_BN)), GT_THREADS,
+                            sizeof(GemmTileSmem<1>), st>>>(dQ + q0 * S.dp, T.qn.as<float>() + q0, m, S.dp,
+                                                           S.cent.as<float>(), S.cnorm.as<float>(), S.nc, ldd, D);
+        GN_TRY(dispatch_r(np, [&](auto RC) {
+            constexpr int R = decltype(RC)::value;
+            coarse_select_kernel<R><<<(unsigned)ceil_div(m, CS_WARPS), CS_WARPS * 32, 0, st>>>(
+                D, ldd, S.nc, np, m, T.probes.as<int32_t>() + q0 * np, keys ? keys + q0 * np : nullptr);
+            return GN_OK;
+        }));
+    }
+    return GN_OK;
 }
 
 int ivfl2_coarse(gn_index *ix, const float *dQ, int64_t nq, int np, cudaStream_t st) {
-    return ivfl2_coarse_run(ix, dQ, nq, np, false, nullptr, st);
+    return ivfl2_coarse_run(ix, dQ, nq, np, nullptr, st);
 }
 
 // The np nearest lists of each query as sorted keys (squared distance, list).
 int ivfl2_coarse_sorted_keys(gn_index *ix, const float *dQ, int64_t nq, int np, uint64_t *keys, cudaStream_t st) {
-    int nsplit = 1;
-    GN_TRY(ivfl2_coarse_run(ix, dQ, nq, np, true, &nsplit, st));
-    IvfScratch &T = ix->ivfl2->s;
-    return dispatch_r(np, [&](auto RC) {
-        constexpr int R = decltype(RC)::value;
-        coarse_merge_kernel<R><<<(unsigned)ceil_div(nq, 4), 128, 0, st>>>(T.cpart.as<uint64_t>(), nsplit, np, nq,
-                                                                          nullptr, keys);
-        return GN_OK;
-    });
+    return ivfl2_coarse_run(ix, dQ, nq, np, keys, st);
 }
 
 // Probes of a batch: the learned prober when one is attached (up to 64 lists,
@@ -796,28 +942,45 @@ static int ivfl2_scan_fp32(gn_index *ix, const float *dQ, int64_t nq, int np, in
                            int64_t *d_cnt, cudaStream_t st) {
     IvfL2State &S = *ix->ivfl2;
     IvfScratch &T = S.s;
-    const int64_t slots = nq * max_slots_per_query(S.top_rows, np, S.rc);
-    GN_TRY(T.part.ensure((size_t)slots * k * 8));
-    if (!g_scan_blocks_l2) {
-        int per = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, ivf_scan_kernel<1>, GT_THREADS, 0);
-        g_scan_blocks_l2 = std::max(1, per) * dev_info().num_sms;
-    }
-    return ivf_run_lists(
-        T, nq, np, S.nc, S.list_off.as<int64_t>(), S.rc, IVF_QCHUNK_L2, k, 0, d_idx, d_dist, d_cnt,
-        g_scan_blocks_l2,
-        [&](int grid) {
-            return dispatch_r(k, [&](auto RC) {
-                constexpr int R = decltype(RC)::value;
-                ivf_scan_kernel<R><<<grid, GT_THREADS, 0, st>>>(
-                    dQ, T.qn.as<float>(), np, S.dp, S.vecs.as<float>(), S.vnorm.as<float>(), S.ids.as<int32_t>(),
-                    S.list_off.as<int64_t>(), S.nc, T.boff.as<int64_t>(), T.bucket.as<int64_t>(),
-                    T.item_off.as<int64_t>(), S.rc, T.qslot.as<int64_t>(), T.slot_rel.as<int64_t>(), k,
-                    T.counter.as<int>(), T.part.as<uint64_t>());
-                return GN_OK;
-            });
-        },
-        st);
+    if (k > 256) return fail(GN_ERR_UNSUPPORTED, "IVF search supports k <= 256");
+    // rows per item: about 40 us of one CTA's arithmetic for 64 queries, so that a
+    // batch's items spread over the SMs; longer (up to the index's own chunk) only
+    // where the candidate lists, k per query and item, would pass 512 MB
+    int rc = (int)std::max<int64_t>(GT_BN, std::min<int64_t>(2048, round_up(32768 / S.dp, GT_BN)));
+    constexpr int64_t room = 512ll << 20;
+    const int rc0 = rc;
+    while (rc < S.rc && nq * max_slots_per_query(S.top_rows, np, rc) * k * 8 > room) rc *= 2;
+    const int64_t list_keys = max_slots_per_query(S.top_rows, np, rc) * k;
+    const int grid = 2 * dev_info().num_sms;
+    // (with longer items, room for a smaller batch's shorter ones too)
+    GN_TRY(T.part.ensure((size_t)std::max<int64_t>(nq * list_keys * 8, rc > rc0 ? room : 0)));
+    GN_TRY(T.ccount.ensure((size_t)nq * 4));
+    GN_TRY(T.qbound.ensure((size_t)nq * 4));
+    GN_TRY(T.lbuf.ensure((size_t)grid * GT_BM * list_cap(k) * 8));
+    GN_TRY(ivf_plan(T, nq, np, S.nc, S.list_off.as<int64_t>(), rc, IVF_QCHUNK_L2, st, -1));
+    GN_CUDA_TRY(cudaMemsetAsync(T.ccount.p, 0, (size_t)nq * 4, st));
+    if (k <= IB_ROWS)
+        ivf_bound_kernel<<<(unsigned)ceil_div(nq, IB_WARPS), IB_WARPS * 32, 0, st>>>(
+            dQ, T.qn.as<float>(), np, S.dp, S.vecs.as<float>(), S.vnorm.as<float>(), S.list_off.as<int64_t>(),
+            T.probes.as<int32_t>(), nq, k, T.qbound.as<uint32_t>());
+    else
+        GN_CUDA_TRY(cudaMemsetAsync(T.qbound.p, 0xff, (size_t)nq * 4, st));
+    timing_begin(st, "ivf_scan_kernel");
+    auto scan = [&](auto HC) -> int {
+        constexpr int H = decltype(HC)::value;
+        GN_CUDA_TRY(cudaFuncSetAttribute(ivf_scan_kernel<H>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(GemmTileSmem<H>)));
+        ivf_scan_kernel<H><<<grid, GT_THREADS, sizeof(GemmTileSmem<H>), st>>>(
+            dQ, T.qn.as<float>(), np, S.dp, S.vecs.as<float>(), S.vnorm.as<float>(), S.ids.as<int32_t>(),
+            S.list_off.as<int64_t>(), S.nc, T.boff.as<int64_t>(), T.bucket.as<int64_t>(), T.item_off.as<int64_t>(), rc, k,
+            T.counter.as<int>(), T.qbound.as<uint32_t>(), T.lbuf.as<uint64_t>(), T.part.as<uint64_t>(),
+            T.ccount.as<int>(), list_keys);
+        return GN_OK;
+    };
+    if (rc > GT_BN) GN_TRY(scan(std::integral_constant<int, 2>()));
+    else GN_TRY(scan(std::integral_constant<int, 1>()));
+    timing_end(st);
+    return candidates_finish(T.part.as<uint64_t>(), T.ccount.as<int>(), list_keys, nq, k, d_idx, d_dist, d_cnt, st);
 }
 
 // ── binary IVF ────────────────────────────────────────────────────────────
@@ -863,7 +1026,7 @@ static int ivfbin_search_dev(gn_index *ix, const uint8_t *dQ, int64_t nq, int k,
         g_scan_blocks_bin = std::max(1, per) * dev_info().num_sms;
     }
     return ivf_run_lists(
-        T, nq, np, S.kc, S.list_off.as<int64_t>(), S.rc, IVF_QCHUNK_BIN, k, 1, d_idx, d_dist, d_cnt,
+        T, nq, np, S.kc, S.list_off.as<int64_t>(), S.rc, IVF_QCHUNK_BIN, k, d_idx, d_dist, d_cnt,
         g_scan_blocks_bin,
         [&](int grid) {
             return dispatch_r(k, [&](auto RC) {

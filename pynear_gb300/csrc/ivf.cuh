@@ -13,6 +13,8 @@ constexpr int IVF_RHO = 64;  // per list: radii of its rows nearest the centroid
 struct IvfScratch {
     DBuf q, qn, probes, probes64, pdist, bcnt, boff, bucket, fill, slot_rel, qcount, qslot, item_off, counter, part,
         cpart, nprobed, qbound,  // qbound: per query, the ordered score bound of the tensor-core list scan
+        ckeys,                   // learned probing on the FP32 engine: nearest lists as keys
+        ccount, lbuf,            // FP32 scan: candidates per query (part holds them), the CTAs' list buffers
         mh1, mcand, mcb, mqn;    // batched prober MLP: first-layer outputs, candidates, their bounds, |q|^2
 };
 
@@ -98,14 +100,11 @@ struct IvfBinState {
     IvfScratch s;
 };
 
-// slot_rc: rows per partial slot (defaults to rc); 1 makes every (query, probe)
-// own a segment of one entry per list row (the tensor-core store mode).
+// slot_rc: rows per partial slot (0: rc, negative: no slots).
 int ivf_plan(IvfScratch &S, int64_t nq, int np, int nc, const int64_t *d_list_off, int rc, int qchunk,
              cudaStream_t st, int slot_rc = 0);
 int64_t ivf_max_slots_per_query(const std::vector<int64_t> &top, int np, int rc);
 int ivfl2_coarse(gn_index *ix, const float *dQ, int64_t nq, int np, cudaStream_t st);
-int ivfl2_coarse_run(gn_index *ix, const float *dQ, int64_t nq, int np, bool keep_keys, int *nsplit_out,
-                     cudaStream_t st);
 int ivfl2_coarse_sorted_keys(gn_index *ix, const float *dQ, int64_t nq, int np, uint64_t *keys, cudaStream_t st);
 int ivfl2_probes(gn_index *ix, const float *dQ, int64_t nq, int *np_out, cudaStream_t st);
 int ivfl2_search_core(gn_index *ix, const float *dQ, int64_t nq, int k, int64_t *d_idx, float *d_dist, int64_t *d_cnt,

@@ -290,12 +290,14 @@ __global__ void row_norms_kernel(const float *__restrict__ X, int64_t n, int dp,
 }
 
 // ── float assignment: tile GEMM + argmin ──────────────────────────────────
-__global__ void __launch_bounds__(GT_THREADS) kmeans_assign_kernel(const float *__restrict__ X, int64_t n, int dp,
-                                                                   const float *__restrict__ C,
-                                                                   const float *__restrict__ cnorm, int k,
-                                                                   int32_t *__restrict__ labels,
-                                                                   unsigned long long *__restrict__ n_changed) {
-    __shared__ GemmTileSmem s;
+template <int H>
+__global__ void __launch_bounds__(GT_THREADS, 2) kmeans_assign_kernel(const float *__restrict__ X, int64_t n, int dp,
+                                                                      const float *__restrict__ C,
+                                                                      const float *__restrict__ cnorm, int k,
+                                                                      int32_t *__restrict__ labels,
+                                                                      unsigned long long *__restrict__ n_changed) {
+    extern __shared__ __align__(16) uint8_t gt_raw[];
+    GemmTileSmem<H> &s = *reinterpret_cast<GemmTileSmem<H> *>(gt_raw);
     __shared__ int64_t arow[GT_BM];
     const int64_t p0 = (int64_t)blockIdx.x * GT_BM;
     if (threadIdx.x < GT_BM) arow[threadIdx.x] = (p0 + threadIdx.x < n) ? p0 + threadIdx.x : -1;
@@ -304,18 +306,22 @@ __global__ void __launch_bounds__(GT_THREADS) kmeans_assign_kernel(const float *
     uint64_t best[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) best[i] = KEY_EMPTY;
-    float acc[8][4];
-    for (int c0 = 0; c0 < k; c0 += GT_BN) {
-        gt_tile(s, acc, X, arow, dp, C, c0, k, dp, dp);
+    f32x2 acc[8][2 * H];
+    for (int c0 = 0; c0 < k; c0 += GT_BN * H) {
+        gt_tile<H>(s, acc, X, arow, dp, C, c0, k, dp, dp);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int c = c0 + tn * 4 + j;
-            if (c < k) {
-                const float cn = cnorm[c];
+        for (int p = 0; p < 2 * H; ++p) {
+            const int c = c0 + gt_col(p);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                if (c + e >= k) continue;
+                const float cn = cnorm[c + e];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
-                    const float v = fmaf(-2.f, acc[i][j], cn);
-                    const uint64_t key = make_key(f2ord(v), (uint32_t)c);
+                    float lo, hi;
+                    unpack2(acc[i][p], lo, hi);
+                    const float v = fmaf(-2.f, e ? hi : lo, cn);
+                    const uint64_t key = make_key(f2ord(v), (uint32_t)(c + e));
                     best[i] = key < best[i] ? key : best[i];
                 }
             }
@@ -405,13 +411,19 @@ int kmeans_l2_device(const float *X, int64_t n, int d, int dp, int64_t k, int64_
     int64_t *dcnt = dstat.as<int64_t>() + 1;
     GN_CUDA_TRY(cudaMemsetAsync(labels, 0, (size_t)n * sizeof(int32_t), st));
     std::vector<int64_t> hstat((size_t)k + 1);
+    GN_CUDA_TRY(cudaFuncSetAttribute(kmeans_assign_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(GemmTileSmem<2>)));
     int64_t it = 0;
     for (; it < max_iter; ++it) {
         row_norms_kernel<<<(unsigned)ceil_div(k, 8), 256, 0, st>>>(C, k, dp, cnorm);
         GN_CUDA_TRY(cudaMemsetAsync(dstat.p, 0, hstat.size() * sizeof(int64_t), st));
         GN_CUDA_TRY(cudaMemsetAsync(dsum.p, 0, (size_t)k * dp * sizeof(double), st));
-        kmeans_assign_kernel<<<(unsigned)ceil_div(n, GT_BM), GT_THREADS, 0, st>>>(X, n, dp, C, cnorm, (int)k, labels,
-                                                                                  dchg);
+        if (k <= GT_BN)
+            kmeans_assign_kernel<1><<<(unsigned)ceil_div(n, GT_BM), GT_THREADS, sizeof(GemmTileSmem<1>), st>>>(
+                X, n, dp, C, cnorm, (int)k, labels, dchg);
+        else
+            kmeans_assign_kernel<2><<<(unsigned)ceil_div(n, GT_BM), GT_THREADS, sizeof(GemmTileSmem<2>), st>>>(
+                X, n, dp, C, cnorm, (int)k, labels, dchg);
         kmeans_accumulate_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, st>>>(X, n, d, dp, labels, dchg,
                                                                           dsum.as<double>(), dcnt);
         kmeans_finalize_kernel<<<(unsigned)ceil_div(k * dp, 256), 256, 0, st>>>(dsum.as<double>(), dcnt, (int)k, d, dp,

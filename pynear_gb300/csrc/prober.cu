@@ -393,11 +393,11 @@ int prober_apply(gn_index *pr, gn_index *ivf, const float *dQ, int64_t nq, float
     ProberState &P = *pst(pr);
     IvfL2State &V = *ivf->ivfl2;
     IvfScratch &T = V.s;
-    int nsplit = 0;
-    GN_TRY(ivfl2_coarse_run(ivf, dQ, nq, PB_C, true, &nsplit, st));  // T.cpart: nsplit sorted lists per query
+    GN_TRY(T.ckeys.ensure((size_t)nq * PB_C * 8));
+    GN_TRY(ivfl2_coarse_sorted_keys(ivf, dQ, nq, PB_C, T.ckeys.as<uint64_t>(), st));
     const __nv_bfloat16 *w = P.wbf.as<__nv_bfloat16>();
     const float *pf = P.params.as<float>();
-    prober_select_kernel<<<(unsigned)nq, PB_H, 0, st>>>(T.cpart.as<uint64_t>(), nsplit, nq, w + P.oW1, pf + P.ob1,
+    prober_select_kernel<<<(unsigned)nq, PB_H, 0, st>>>(T.ckeys.as<uint64_t>(), 1, nq, w + P.oW1, pf + P.ob1,
                                                        w + P.oW2, pf + P.ob2, w + P.oW3, pf + P.ob3, logit_tau,
                                                        probes, nprobed);
     GN_CUDA_TRY(cudaGetLastError());

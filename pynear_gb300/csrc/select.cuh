@@ -95,15 +95,15 @@ __device__ __forceinline__ uint64_t warp_select(const uint64_t (&v)[R], int m, i
 }
 
 // One round of warp_best: the S best of the `kept` keys in sel and the `take` keys
-// at p (at most 32 R together) into sel.
-template <int R>
-__device__ __forceinline__ int warp_best_round(const uint64_t *p, int take, int kept, int S, uint64_t *sel) {
+// get(0) .. (at most 32 R together) into sel.
+template <int R, typename Get>
+__device__ __forceinline__ int warp_best_round(Get &&get, int take, int kept, int S, uint64_t *sel) {
     const int lane = threadIdx.x & 31;
     uint64_t v[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         const int x = i * 32 + lane;
-        v[i] = x < kept ? sel[x] : x - kept < take ? p[x - kept] : KEY_EMPTY;
+        v[i] = x < kept ? sel[x] : x - kept < take ? get(x - kept) : KEY_EMPTY;
     }
     const uint64_t thr = warp_select<R>(v, kept + take, S);
     __syncwarp();
@@ -119,18 +119,83 @@ __device__ __forceinline__ int warp_best_round(const uint64_t *p, int take, int 
     return kept;
 }
 
-// The S best of m keys at p into sel[0 .. min(S, m)), any order, by one warp;
-// returns their number.  S <= 256.
+// The S best of m keys get(0) .. get(m - 1) into sel[0 .. min(S, m)), any order, by
+// one warp; returns their number.  S <= 256.
 constexpr int SEL_R = 16;  // keys per lane held in registers at a time
-__device__ __forceinline__ int warp_best(const uint64_t *p, int m, int S, uint64_t *sel) {
-    if (m <= 128) return warp_best_round<4>(p, m, 0, S, sel);
+template <typename Get>
+__device__ __forceinline__ int warp_best_of(Get &&get, int m, int S, uint64_t *sel) {
+    if (m <= 128) return warp_best_round<4>(get, m, 0, S, sel);
     int kept = 0;
     for (int i0 = 0; i0 < m;) {  // earlier rounds' best join each round's keys
         const int take = min(m - i0, SEL_R * 32 - kept);
-        kept = warp_best_round<SEL_R>(p + i0, take, kept, S, sel);
+        kept = warp_best_round<SEL_R>([&](int i) { return get(i0 + i); }, take, kept, S, sel);
         i0 += take;
     }
     return kept;
+}
+__device__ __forceinline__ int warp_best(const uint64_t *p, int m, int S, uint64_t *sel) {
+    return warp_best_of([&](int i) { return p[i]; }, m, S, sel);
+}
+
+// ── unordered candidate buffers ───────────────────────────────────────────
+// A list keeps its candidates without order in a buffer of LIST_CAP_S (k <= 64) or
+// LIST_CAP_L (k <= 256) keys; one that holds more than `most` is cut to its k best.
+constexpr int LIST_CAP_S = 128, LIST_CAP_L = 512;
+__host__ __device__ inline int list_cap(int k) { return k <= 64 ? LIST_CAP_S : LIST_CAP_L; }
+// a late cut leaves the threshold loose, an early one is paid more often (and
+// appending adds up to 32 keys before the next check)
+__host__ __device__ inline int list_most(int k) {
+    return k > 64 ? LIST_CAP_L - 32 : 2 * k + 24 < LIST_CAP_S - 32 ? 2 * k + 24 : LIST_CAP_S - 32;
+}
+
+// Cut a buffer of m keys (k < m <= 32 R) down to its k best, in place; returns
+// the k-th best key's distance bits.  (A call, not inlined: it runs a few times
+// per list and would crowd the scan's registers and instruction cache.)
+template <int R>
+__device__ __noinline__ uint32_t list_cut(uint64_t *buf, int m, int k) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    uint64_t v[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) v[i] = i * 32 + lane < m ? buf[i * 32 + lane] : KEY_EMPTY;
+    const uint64_t thr = warp_select<R>(v, m, k);
+    __syncwarp();
+    int kept = 0;
+    uint32_t far = 0u;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        const bool in = v[i] <= thr && v[i] != KEY_EMPTY;
+        const unsigned b = __ballot_sync(0xffffffffu, in);
+        if (in) {
+            buf[kept + __popc(b & ((1u << lane) - 1))] = v[i];
+            far = max(far, key_dist(v[i]));
+        }
+        kept += __popc(b);
+    }
+    __syncwarp();
+    return __reduce_max_sync(0xffffffffu, far);
+}
+__device__ __forceinline__ uint32_t list_cut_k(uint64_t *buf, int m, int k) {
+    return k <= 64 ? list_cut<LIST_CAP_S / 32>(buf, m, k) : list_cut<LIST_CAP_L / 32>(buf, m, k);
+}
+
+// Add the lanes' (bits, index) keys with bits below the threshold state.y to a
+// list of state.x keys, cutting it once it holds more than `most`.  ASCENDING:
+// indices come in ascending order, so after a cut only smaller bits displace the
+// k-th; otherwise equal bits may too, by a lower index.
+template <bool ASCENDING>
+__device__ __forceinline__ uint2 list_add(uint64_t *buf, uint2 state, uint32_t bits, bool in, uint32_t index, int k,
+                                          int most) {
+    in = in && bits < state.y;
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    const int lane = threadIdx.x & 31;
+    if (in) buf[state.x + __popc(m & ((1u << lane) - 1))] = make_key(bits, index);
+    state.x += __popc(m);
+    if ((int)state.x > most) {
+        state.y = list_cut_k(buf, state.x, k) + (ASCENDING ? 0u : 1u);
+        state.x = k;
+    }
+    return state;
 }
 
 }  // namespace gn

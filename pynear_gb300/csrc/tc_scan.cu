@@ -29,7 +29,7 @@
 // What makes passing scores rare is the bound that every unit starts from.
 // With a warp's 32 lanes being 32 queries, a block of 32 x 32 scores is only
 // cheap when none of 1,024 passes.  So a pilot launch of the same pipeline first
-// scores every 8th tile or so and keeps, per query, only the minima of groups
+// scores every 8th row or so and keeps, per query, only the minima of groups
 // of rows (32 per unit, one per column of a block: no insertion, no branch).
 // The S-th smallest minimum over at least S groups is a score that at least S
 // rows reach, hence an upper bound of the query's S-th best score, and close
@@ -73,6 +73,7 @@ constexpr int TC_COLS = TC_N / (TC_NEPI / 4);  // columns of a tile per epilogue
 constexpr int TC_THREADS = 64 + 32 * TC_NEPI;
 constexpr int TC_MAX_STAGES = 6;
 constexpr int TC_NR = 4;                // tiles of row norms (and scales) in flight
+constexpr int64_t TC_PILOT_MIN = 32768; // rows from which a pilot runs
 constexpr int64_t TC_QBLOCK = 65536;    // queries scanned at a time (bounds the scratch)
 constexpr int TC_CAP = 128;             // entries of a buffer (S <= 64, and a block adds up to 32)
 
@@ -131,8 +132,7 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 }
 
 // MODE: operand form.  PILOT: group minima of the sampled tiles instead of lists.
-// QT: query tiles per unit.  Tile i of the launch is database tile i * tstride;
-// unit u is (chunk u / nqp of the tiles, queries 128 QT (u % nqp) ..): chunk-major,
+// QT: query tiles per unit.  Unit u is (chunk u / nqp of the tiles, queries 128 QT (u % nqp) ..): chunk-major,
 // so that the CTAs running together scan the same chunk and L2 serves it.
 template <int MODE, bool PILOT, int QT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                                         (int)(q0 + qt * TC_M), afull);
                 }
                 for (int64_t t = t0; t < t1 && ok; ++t, ++tile_it) {
-                    const int n0 = (int)(t * a.tstride * TC_N);
+                    const int n0 = (int)(t * TC_N);
                     for (int kb = 0; kb < nk; ++kb, ++it) {
                         if (!mbar_wait(empty + sl, ph, verr)) { ok = false; break; }
                         uint8_t *sb = ring + (size_t)sl * stage_bytes;
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             for (int j = 0; j < (PILOT ? 32 : 1); ++j) g[j] = inf;
 
             for (int64_t t = t0; t < t1 && ok; ++t, ++tile_it) {
-                const int64_t n0 = t * a.tstride * TC_N + quarter * TC_COLS;
+                const int64_t n0 = t * TC_N + quarter * TC_COLS;
                 const bool tail = MODE == TC_SIGN && n0 + TC_COLS > a.n;
                 const int ns = tile_it % TC_NR;
                 // the tile's row norms (NaN past the last row: such scores never pass)
@@ -533,10 +533,11 @@ __global__ void tc_bound_kernel(const float *__restrict__ gmin, int m, int64_t n
 
 // ── host: tensor maps, plan and launch ────────────────────────────────────
 // K-major operand rows of K elements (BF16, or FP8 stored as bytes), boxes of
-// 128 bytes of K by box_rows rows, 128-byte swizzle.
-static int make_tmap_rows(CUtensorMap *map, const void *base, int64_t rows, int64_t K, int box_rows, bool f8) {
+// 128 bytes of K by box_rows rows, 128-byte swizzle; stride: every stride-th row.
+static int make_tmap_rows(CUtensorMap *map, const void *base, int64_t rows, int64_t K, int box_rows, bool f8,
+                          int stride = 1) {
     return tmap_encode_2d(map, f8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base,
-                          (uint64_t)K, (uint64_t)rows, (uint64_t)K * (f8 ? 1 : 2), f8 ? TC_BK8 : TC_BK,
+                          (uint64_t)K, (uint64_t)rows, (uint64_t)K * (f8 ? 1 : 2) * stride, f8 ? TC_BK8 : TC_BK,
                           (uint32_t)box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
@@ -559,6 +560,27 @@ static int64_t tc_chunks(int64_t nqp, int64_t nt, int64_t lo, int64_t hi, int64_
     return best;
 }
 
+// Rows, not whole tiles, are sampled: where near rows stand together in the
+// database, tiles would miss most queries' neighbourhoods.
+int tc_pilot_stride(int64_t n) {
+    return n < TC_PILOT_MIN ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(8, n / 16384));
+}
+
+// Every stride-th of n values, whole tiles of them (NaN past the last).
+__global__ void tc_stride_kernel(const float *__restrict__ x, int64_t n, int stride, int64_t m,
+                                 float *__restrict__ out) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < m) out[i] = i * stride < n ? x[i * stride] : __int_as_float(0x7fc00000);
+}
+
+int tc_pilot_values(const float *x, int64_t n, DBuf &out, cudaStream_t st) {
+    const int stride = tc_pilot_stride(n);
+    const int64_t m = round_up(ceil_div(n, stride), TC_N);
+    GN_TRY(out.ensure((size_t)m * 4));
+    tc_stride_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, st>>>(x, n, stride, m, out.as<float>());
+    return GN_OK;
+}
+
 static int tc_slices(int mode, int K) { return K / (mode == TC_BF16 ? TC_BK : TC_BK8); }
 
 TcPlan tc_plan(int mode, int K, int64_t nq, int64_t n, int S) {
@@ -569,12 +591,11 @@ TcPlan tc_plan(int mode, int K, int64_t nq, int64_t n, int S) {
     // about five units per SM at most: shorter ones sort more lists at their ends
     // than they save in the last wave
     p.nchunks = (int)tc_chunks(nqp, nt, 1, std::min<int64_t>(64, std::max<int64_t>(1, ceil_div(5 * sms, nqp))), 2);
-    // pilot: every 8th tile (more where that would be under 16k rows), full tiles
-    // only; below 32k rows the lists' own first fill costs less than the launches
-    const int64_t full = n / TC_N;
-    if (n >= 32768) {
-        p.pilot_stride = (int)std::max<int64_t>(1, std::min<int64_t>(8, full / 64));
-        p.pilot_tiles = full / p.pilot_stride;
+    // pilot: every 8th row (more where that would be under 16k rows), whole tiles
+    // of them; below 32k rows the lists' own first fill costs less than the launches
+    if (n >= TC_PILOT_MIN) {
+        p.pilot_stride = tc_pilot_stride(n);
+        p.pilot_tiles = n / p.pilot_stride / TC_N;
         // 128 groups of minima per chunk
         p.pilot_chunks = (int)tc_chunks(nqp1, p.pilot_tiles, 1, std::max<int64_t>(1, ceil_div(4 * sms, nqp1)), 2);
     }
@@ -588,7 +609,7 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
     if (a.K <= 0 || a.K % kblk) return fail(GN_ERR_INVALID, "tensor-core scan: K must be whole 128-byte slices");
     if (a.S < 1 || a.S > 64) return fail(GN_ERR_UNSUPPORTED, "tensor-core scan: 1 to 64 results per query");
     if (a.mode == TC_FP8 && (!a.ascale || !a.bscale)) return fail(GN_ERR_INVALID, "FP8 shortlist: no row scales");
-    CUtensorMap ma, mb;
+    CUtensorMap ma, mb, mp;
     GN_TRY(make_tmap_rows(&ma, a.A, a.a_rows, a.K, TC_M, f8));
     GN_TRY(make_tmap_rows(&mb, a.B, a.b_rows, a.K, TC_N, f8));
     const int sms = dev_info().num_sms;
@@ -596,13 +617,10 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
     GN_TRY(sc.cand.ensure((size_t)sms * TC_NEPI * 2 * 32 * TC_CAP * sizeof(uint2)));
     TcScanArgs s;
     s.nq = a.nq;
-    s.n = a.n;
     s.kblk = kblk;
     s.S = a.S;
     s.nbits = a.nbits;
-    s.bnorm = a.bnorm;
     s.ascale = a.ascale;
-    s.bscale = a.bscale;
     s.part = a.part;
     s.qcount = a.qcount;
     s.slot_keys = p.slot_keys;
@@ -610,7 +628,7 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
     s.cand = sc.cand.as<uint2>();
     s.gmin = nullptr;
     s.err = a.err;
-    auto run = [&](auto kern, const TcGeom &g) -> int {
+    auto run = [&](auto kern, const TcGeom &g, const CUtensorMap &mb) -> int {
         s.nk = g.nk;
         s.stages = g.stages;
         s.resident = g.resident;
@@ -623,14 +641,17 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
     GN_CUDA_TRY(cudaMemsetAsync(a.qcount, 0, (size_t)a.nq * 4, st));
     if (p.pilot_chunks) {
         const TcGeom gp = tc_geom(a.K / kblk, true);
+        GN_TRY(make_tmap_rows(&mp, a.B, a.n / p.pilot_stride, a.K, TC_N, f8, p.pilot_stride));
         GN_TRY(sc.gmin.ensure((size_t)a.nq * p.pilot_chunks * TC_N / 2 * 4));
         s.gmin = sc.gmin.as<float>();
         s.nchunks = p.pilot_chunks;
         s.ntiles = p.pilot_tiles;
-        s.tstride = p.pilot_stride;
-        GN_TRY(a.mode == TC_BF16  ? run(tc_topk_kernel<TC_BF16, true, 1>, gp)
-               : a.mode == TC_FP8 ? run(tc_topk_kernel<TC_FP8, true, 1>, gp)
-                                  : run(tc_topk_kernel<TC_SIGN, true, 1>, gp));
+        s.n = p.pilot_tiles * TC_N;
+        s.bnorm = a.pnorm;
+        s.bscale = a.pscale;
+        GN_TRY(a.mode == TC_BF16  ? run(tc_topk_kernel<TC_BF16, true, 1>, gp, mp)
+               : a.mode == TC_FP8 ? run(tc_topk_kernel<TC_FP8, true, 1>, gp, mp)
+                                  : run(tc_topk_kernel<TC_SIGN, true, 1>, gp, mp));
         tc_bound_kernel<<<(unsigned)ceil_div(a.nq, 8), 256, 0, st>>>(s.gmin, (TC_NEPI / 4) * p.pilot_chunks, a.nq,
                                                                     a.S, s.qbound);
     } else {
@@ -638,14 +659,16 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
     }
     s.nchunks = p.nchunks;
     s.ntiles = ceil_div(a.n, TC_N);
-    s.tstride = 1;
+    s.n = a.n;
+    s.bnorm = a.bnorm;
+    s.bscale = a.bscale;
     if (g.qt == 2)
-        return a.mode == TC_BF16  ? run(tc_topk_kernel<TC_BF16, false, 2>, g)
-               : a.mode == TC_FP8 ? run(tc_topk_kernel<TC_FP8, false, 2>, g)
-                                  : run(tc_topk_kernel<TC_SIGN, false, 2>, g);
-    return a.mode == TC_BF16  ? run(tc_topk_kernel<TC_BF16, false, 1>, g)
-           : a.mode == TC_FP8 ? run(tc_topk_kernel<TC_FP8, false, 1>, g)
-                              : run(tc_topk_kernel<TC_SIGN, false, 1>, g);
+        return a.mode == TC_BF16  ? run(tc_topk_kernel<TC_BF16, false, 2>, g, mb)
+               : a.mode == TC_FP8 ? run(tc_topk_kernel<TC_FP8, false, 2>, g, mb)
+                                  : run(tc_topk_kernel<TC_SIGN, false, 2>, g, mb);
+    return a.mode == TC_BF16  ? run(tc_topk_kernel<TC_BF16, false, 1>, g, mb)
+           : a.mode == TC_FP8 ? run(tc_topk_kernel<TC_FP8, false, 1>, g, mb)
+                              : run(tc_topk_kernel<TC_SIGN, false, 1>, g, mb);
 }
 
 // ── conversion and norms ──────────────────────────────────────────────────
@@ -822,7 +845,7 @@ void ham_tc_reset(gn_index *ix) {
 // than half a millisecond on the POPC scan, stay there.
 bool ham_tc_wanted(const gn_index *ix, int64_t nq, int64_t k) {
     const int64_t words = ceil_div(ix->dim, 4);
-    return k <= 64 && ix->dim <= 512 && ix->n >= 32768 && nq >= 128 && nq * ix->n >= 2000000000ll / words;
+    return k <= 64 && ix->dim <= 512 && ix->n >= TC_PILOT_MIN && nq >= 128 && nq * ix->n >= 2000000000ll / words;
 }
 
 // Returns GN_ERR_UNSUPPORTED where the expanded rows do not fit (the caller
@@ -893,6 +916,7 @@ struct TcFlatState {
     int fp8 = 0;  // 0: BF16 operands; 1: FP8 E4M3 with per-row scales
     int64_t n = 0;
     DBuf x32, x16, xnorm, xscale;  // fp32 rows (dp), low-precision rows (K), |x|^2, FP8 row scales
+    DBuf pnorm, pscale;            // norms and scales of the pilot's rows
     DBuf q32, q16, qscale, part, qcount, err, out_idx, out_dist;
     TcScratch scr;
 };
@@ -907,6 +931,7 @@ static int tcflat_lowp(TcFlatState &S, cudaStream_t st) {
     if (S.fp8) {
         GN_TRY(S.xscale.ensure((size_t)round_up(S.n, TC_N) * 4));  // whole tiles are read
         to_e4m3_rows(S.x32.as<float>(), S.n, S.d, S.dp, S.x16.p, S.xscale.as<float>(), S.K, st);
+        GN_TRY(tc_pilot_values(S.xscale.as<float>(), S.n, S.pscale, st));
     } else {
         S.xscale.release();
         to_bf16_rows(S.x32.as<float>(), S.n, S.d, S.dp, S.x16.p, S.K, st);
@@ -956,6 +981,7 @@ int gn_tcflat_set(gn_index *ix, const float *data, int64_t n, int64_t d) {
     GN_TRY(S.xnorm.ensure(np * 4));
     GN_CUDA_TRY(cudaMemsetAsync(S.xnorm.as<float>() + n, 0xff, (np - (size_t)n) * 4, st));
     row_norms(S.x32.as<float>(), n, S.dp, S.xnorm.as<float>(), st);
+    GN_TRY(tc_pilot_values(S.xnorm.as<float>(), n, S.pnorm, st));
     GN_TRY(tcflat_lowp(S, st));
     GN_TRY(S.err.ensure(4));
     GN_CUDA_TRY(cudaMemsetAsync(S.err.p, 0, 4, st));
@@ -1003,12 +1029,14 @@ static int tcflat_search_locked(gn_index *ix, const float *d_queries, int64_t nq
         a.b_rows = std::max<int64_t>(S.n, TC_N);
         a.K = S.K;
         a.bnorm = S.xnorm.as<float>();
+        a.pnorm = S.pnorm.as<float>();
         a.part = S.part.as<uint64_t>();
         a.qcount = S.qcount.as<int>();
         a.err = S.err.as<int>();
         a.S = S.S;
         a.ascale = S.fp8 ? S.qscale.as<float>() : nullptr;
         a.bscale = S.fp8 ? S.xscale.as<float>() : nullptr;
+        a.pscale = S.fp8 ? S.pscale.as<float>() : nullptr;
         timing_begin(st, "tc_topk_kernel");
         GN_TRY(tc_topk_launch(a, plan, S.scr, st));
         timing_end(st);

@@ -31,6 +31,7 @@ struct TcLaunch {
     int nbits = 0;                 // TC_SIGN: bits per row
     const float *bnorm = nullptr;  // |B row|^2, FP32, whole 256-row tiles, NaN past n (not TC_SIGN)
     const float *ascale = nullptr, *bscale = nullptr;  // TC_FP8 (bscale: whole tiles)
+    const float *pnorm = nullptr, *pscale = nullptr;   // the same of the pilot's rows (tc_pilot_values)
     uint64_t *part = nullptr;      // per query slot_keys keys: its candidate list ...
     int *qcount = nullptr;         // ... and its length (the S best keys are among them)
     int *err = nullptr;            // device error word (0 = ok)
@@ -53,7 +54,7 @@ struct TcScratch {
 // Kernel arguments.
 struct TcScanArgs {
     int64_t nq, n, ntiles;
-    int nk, kblk, stages, resident, nchunks, tstride, S, nbits;
+    int nk, kblk, stages, resident, nchunks, S, nbits;
     const float *bnorm, *ascale, *bscale;
     int64_t slot_keys;
     uint64_t *part;
@@ -64,6 +65,8 @@ struct TcScanArgs {
     int *err;
 };
 
+int tc_pilot_stride(int64_t n);
+int tc_pilot_values(const float *x, int64_t n, DBuf &out, cudaStream_t st);
 TcPlan tc_plan(int mode, int K, int64_t nq, int64_t n, int S);
 int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream_t st);
 // Exact Hamming k-NN of a flat Hamming index on the tensor cores: whether a

@@ -268,7 +268,7 @@ int gn_flat_set(gn_index *ix, const void *data, int64_t n, int64_t dim) {
     GN_TRY(make_stream(ix));
     ix->n = 0;
     ix->dim = 0;
-    ham_tc_reset(ix);
+    flat_tc_reset(ix);
     if (n == 0) return GN_OK;  // an empty index: searches raise GN_ERR_EMPTY
     const int s4 = row_stride4(ix->metric, dim);
     const int64_t row_bytes = (ix->metric == GN_METRIC_HAMMING) ? dim : dim * 4;
@@ -307,6 +307,12 @@ static int flat_search_dev(gn_index *ix, const void *d_q, int64_t nq, int64_t k,
         GN_TRY(error_word());
         const int rc = ham_tc_search(ix, d_q, nq, (int)k, d_idx, reinterpret_cast<int64_t *>(d_dist), a.err, st);
         if (rc != GN_ERR_UNSUPPORTED) return rc;
+    }
+    if (ix->metric == M_L2 && l2_tc_wanted(ix, nq, k)) {
+        GN_TRY(error_word());
+        const int rc = l2_tc_search(ix, reinterpret_cast<const float *>(d_q), nq, (int)k, d_idx,
+                                    reinterpret_cast<float *>(d_dist), a.err, &a.only_if, st);
+        if (rc != GN_OK && rc != GN_ERR_UNSUPPORTED) return rc;
     }
     if (k <= FLAT_MAX_K_WARP) {
         flat_plan(a);

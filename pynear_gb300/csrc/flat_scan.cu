@@ -164,6 +164,7 @@ struct FsArgs {
     uint64_t *cand;  // per query list_keys candidate keys ...
     int *qcount;     // ... and how many there are
     int *err;
+    const int *only_if;
 };
 
 // One (row, query) pair's accumulators: the packed form of distance.cuh's FAcc.
@@ -263,6 +264,7 @@ __device__ __noinline__ uint2 fs_add(uint64_t *buf, uint2 state, uint32_t v, boo
 template <int METRIC, int QW, int RPT, bool ONE>
 __global__ void __launch_bounds__(FS_THREADS, 3)
     float_scan_kernel(const __grid_constant__ CUtensorMap tm, const FsArgs a) {
+    if (a.only_if && *a.only_if == 0) return;
     extern __shared__ float4 sqf[];  // [WQ * QW][dp4] negated queries, buffers (k <= 64), the stage ring, barriers
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int slice = blockIdx.x / a.n_groups, group = blockIdx.x % a.n_groups;
@@ -503,9 +505,11 @@ __global__ void __launch_bounds__(FS_THREADS, 3)
 template <int W, int R>
 __global__ void __launch_bounds__(W * 32)
     flat_finish_kernel(const uint64_t *__restrict__ cand, const int *__restrict__ qcount, int64_t list_keys, int k,
-                       int64_t *__restrict__ out_idx, float *__restrict__ out_dist, int64_t *__restrict__ out_cnt) {
+                       int64_t *__restrict__ out_idx, float *__restrict__ out_dist, int64_t *__restrict__ out_cnt,
+                       const int *__restrict__ only_if) {
     __shared__ uint64_t s_sel[(W + 1) * R * 32];
     __shared__ int s_n[W];
+    if (only_if && *only_if == 0) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t q = blockIdx.x;
     const uint64_t *p = cand + q * list_keys;
@@ -831,15 +835,18 @@ static int hamming_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st
 }
 
 int candidates_finish(const uint64_t *cand, const int *qcount, int64_t list_keys, int64_t nq, int k, int64_t *out_idx,
-                      float *out_dist, int64_t *out_cnt, cudaStream_t st) {
+                      float *out_dist, int64_t *out_cnt, const int *only_if, cudaStream_t st) {
     auto finish = [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         if (nq <= dev_info().num_sms && R <= 2)
-            flat_finish_kernel<24, R><<<(unsigned)nq, 768, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist, out_cnt);
+            flat_finish_kernel<24, R><<<(unsigned)nq, 768, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist,
+                                                                  out_cnt, only_if);
         else if (nq <= 4 * dev_info().num_sms)
-            flat_finish_kernel<8, R><<<(unsigned)nq, 256, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist, out_cnt);
+            flat_finish_kernel<8, R><<<(unsigned)nq, 256, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist,
+                                                                  out_cnt, only_if);
         else
-            flat_finish_kernel<1, R><<<(unsigned)nq, 32, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist, out_cnt);
+            flat_finish_kernel<1, R><<<(unsigned)nq, 32, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist,
+                                                                  out_cnt, only_if);
     };
     if (k <= 32) finish(std::integral_constant<int, 1>());
     else if (k <= 64) finish(std::integral_constant<int, 2>());
@@ -880,8 +887,9 @@ static int float_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) 
     f.cand = part + round_up(a.nq * 4, 256) / 8;
     f.gbuf = f.cand + a.nq * a.list_keys;
     f.err = a.err;
+    f.only_if = a.only_if;
     GN_CUDA_TRY(cudaMemsetAsync(f.qcount, 0, (size_t)a.nq * 4, st));
-    timing_begin(st, "float_scan_kernel");
+    if (!a.only_if) timing_begin(st, "float_scan_kernel");
     auto go = [&](auto MC) -> int {
         constexpr int M = decltype(MC)::value;
         auto launch = [&](auto kern) -> int {
@@ -899,9 +907,9 @@ static int float_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) 
     GN_TRY(a.metric == M_L2   ? go(std::integral_constant<int, M_L2>())
            : a.metric == M_L1 ? go(std::integral_constant<int, M_L1>())
                               : go(std::integral_constant<int, M_LINF>()));
-    timing_end(st);
+    if (!a.only_if) timing_end(st);
     return candidates_finish(f.cand, f.qcount, a.list_keys, a.nq, a.k, a.out_idx, reinterpret_cast<float *>(a.out_dist),
-                             nullptr, st);
+                             nullptr, a.only_if, st);
 }
 
 // Launch the k <= 256 path.  part: flat_part_bytes(a) scratch.

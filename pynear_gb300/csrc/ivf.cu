@@ -980,7 +980,8 @@ static int ivfl2_scan_fp32(gn_index *ix, const float *dQ, int64_t nq, int np, in
     if (rc > GT_BN) GN_TRY(scan(std::integral_constant<int, 2>()));
     else GN_TRY(scan(std::integral_constant<int, 1>()));
     timing_end(st);
-    return candidates_finish(T.part.as<uint64_t>(), T.ccount.as<int>(), list_keys, nq, k, d_idx, d_dist, d_cnt, st);
+    return candidates_finish(T.part.as<uint64_t>(), T.ccount.as<int>(), list_keys, nq, k, d_idx, d_dist, d_cnt, nullptr,
+                             st);
 }
 
 // ── binary IVF ────────────────────────────────────────────────────────────

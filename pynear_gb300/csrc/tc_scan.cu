@@ -74,6 +74,7 @@ constexpr int TC_THREADS = 64 + 32 * TC_NEPI;
 constexpr int TC_MAX_STAGES = 6;
 constexpr int TC_NR = 4;                // tiles of row norms (and scales) in flight
 constexpr int64_t TC_PILOT_MIN = 32768; // rows from which a pilot runs
+constexpr int64_t L2TC_QBLOCK = 8192;   // the same of the exact L2 search (longer candidate lists)
 constexpr int64_t TC_QBLOCK = 65536;    // queries scanned at a time (bounds the scratch)
 constexpr int TC_CAP = 128;             // entries of a buffer (S <= 64, and a block adds up to 32)
 
@@ -414,6 +415,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                                 }
                         }
                         unsigned fullm = __ballot_sync(0xffffffffu, cnt[0] > TC_CAP - 32);
+                        if (fullm && a.overflow) *a.overflow = 1;
                         while (fullm) {  // the warp sorts a lane's buffer down to its S best
                             const int l = __ffs(fullm) - 1;
                             fullm &= fullm - 1;
@@ -471,6 +473,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     int n = i == 0 ? cnt[0] : cnt[QT - 1];
                     uint2 *const wbuf = ebuf + (size_t)i * 32 * TC_CAP;
                     unsigned longm = __ballot_sync(0xffffffffu, n > a.S);
+                    if (longm && a.overflow) *a.overflow = 1;
                     while (longm) {  // only a buffer's S best can be among the query's
                         const int l = __ffs(longm) - 1;
                         longm &= longm - 1;
@@ -507,7 +510,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 // A query's bound from the pilot's minima (m groups of 32, warp per query): the
 // S-th smallest of up to 128 groups' minima (groups joined four ways beyond
 // that) is reached by at least S rows.  Fewer than S groups: no bound.
-__global__ void tc_bound_kernel(const float *__restrict__ gmin, int m, int64_t nq, int S,
+// sl.q2 given: the bound is raised so that it holds for exact distances too (see
+// l2_tc_search): B -> B + 2 E + rel (B + |q|^2 + E), E = sl.cross |q| max|x| +
+// sl.norm max|x|^2, and *sl.overflow is set where that is not finite.
+__global__ void tc_bound_kernel(const float *__restrict__ gmin, int m, int64_t nq, int S, TcSlack sl,
                                 uint32_t *__restrict__ qbound) {
     const int lane = threadIdx.x & 31;
     const int64_t q = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -528,7 +534,19 @@ __global__ void tc_bound_kernel(const float *__restrict__ gmin, int m, int64_t n
 #pragma unroll
     for (int r = 0; r < 4; ++r)
         if (r == (S - 1) / 32) key = __shfl_sync(0xffffffffu, v[r], (S - 1) & 31);
-    if (lane == 0) qbound[q] = key == KEY_EMPTY ? 0xffffffffu : key_dist(key);
+    if (lane != 0) return;
+    uint32_t bound = key == KEY_EMPTY ? 0xffffffffu : key_dist(key);
+    if (sl.q2 && bound != 0xffffffffu) {
+        const float b = ord2f(bound), q2 = sl.q2[q], x2 = __uint_as_float(*sl.xmax2);
+        // (1e-35: products that a unit may flush to zero)
+        const float e = __fadd_ru(__fadd_ru(__fmul_ru(sl.cross, __fsqrt_ru(__fmul_ru(q2, x2))), __fmul_ru(sl.norm, x2)),
+                                  1e-35f);
+        const float d = fmaxf(0.f, __fadd_ru(__fadd_ru(b, q2), e));
+        const float raised = __fadd_ru(__fadd_ru(b, __fmul_ru(2.f, e)), __fmul_ru(sl.rel, d));
+        bound = raised < inf ? f2ord(raised) : 0xffffffffu;
+        if (!(raised < inf)) *sl.overflow = 1;  // NaN or infinite: scores say nothing
+    }
+    qbound[q] = bound;
 }
 
 // ── host: tensor maps, plan and launch ────────────────────────────────────
@@ -607,7 +625,7 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
     const bool f8 = a.mode != TC_BF16;
     const int kblk = f8 ? TC_BK8 : TC_BK;
     if (a.K <= 0 || a.K % kblk) return fail(GN_ERR_INVALID, "tensor-core scan: K must be whole 128-byte slices");
-    if (a.S < 1 || a.S > 64) return fail(GN_ERR_UNSUPPORTED, "tensor-core scan: 1 to 64 results per query");
+    if (a.S < 1 || a.S > TC_CAP - 32) return fail(GN_ERR_UNSUPPORTED, "tensor-core scan: too many results per query");
     if (a.mode == TC_FP8 && (!a.ascale || !a.bscale)) return fail(GN_ERR_INVALID, "FP8 shortlist: no row scales");
     CUtensorMap ma, mb, mp;
     GN_TRY(make_tmap_rows(&ma, a.A, a.a_rows, a.K, TC_M, f8));
@@ -628,6 +646,7 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
     s.cand = sc.cand.as<uint2>();
     s.gmin = nullptr;
     s.err = a.err;
+    s.overflow = a.overflow;
     auto run = [&](auto kern, const TcGeom &g, const CUtensorMap &mb) -> int {
         s.nk = g.nk;
         s.stages = g.stages;
@@ -653,7 +672,8 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
                : a.mode == TC_FP8 ? run(tc_topk_kernel<TC_FP8, true, 1>, gp, mp)
                                   : run(tc_topk_kernel<TC_SIGN, true, 1>, gp, mp));
         tc_bound_kernel<<<(unsigned)ceil_div(a.nq, 8), 256, 0, st>>>(s.gmin, (TC_NEPI / 4) * p.pilot_chunks, a.nq,
-                                                                    a.S, s.qbound);
+                                                                    a.bound_rank ? a.bound_rank : a.S, a.slack,
+                                                                    s.qbound);
     } else {
         GN_CUDA_TRY(cudaMemsetAsync(s.qbound, 0xff, (size_t)a.nq * 4, st));
     }
@@ -715,22 +735,15 @@ void to_e4m3_rows(const float *X, int64_t n, int d, int ldx, void *out, float *s
 }
 
 // ── exact re-rank ─────────────────────────────────────────────────────────
-// One warp per query: the S best candidates by score, their L2 distances in the
-// reference's FP32 order (bit-identical to the exact flat scan), the k nearest.
-// Two lanes per candidate row, each with four of the reference's eight
-// accumulators, so a warp's loads take whole 32-byte sectors of 16 rows.
-constexpr int RR_WARPS = 4;
-__global__ void __launch_bounds__(RR_WARPS * 32)
-    tc_rerank_kernel(const uint64_t *__restrict__ part, const int *__restrict__ qcount, int64_t slot_keys, int S,
-                     const float *__restrict__ Q, const float *__restrict__ X, int d, int dp, int64_t nq, int k,
-                     int64_t *__restrict__ out_idx, float *__restrict__ out_dist) {
-    __shared__ uint64_t s_sel[RR_WARPS][64];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t q = (int64_t)blockIdx.x * RR_WARPS + warp;
-    if (q >= nq) return;
-    uint64_t *sel = s_sel[warp];
-    const int m = warp_best(part + q * slot_keys, qcount[q], S, sel);
-    const float4 *q4 = reinterpret_cast<const float4 *>(Q + q * dp);
+// The k nearest (k <= 32) of m candidate keys' rows to query q, by one warp, in
+// the reference's FP32 order (bit-identical to the exact flat scan).  Two lanes
+// per row, each with four of the reference's eight accumulators, so a warp's
+// loads take whole 32-byte sectors of 16 rows.
+__device__ __forceinline__ void l2_rank(const uint64_t *keys, int m, const float *__restrict__ q,
+                                        const float *__restrict__ X, int d, int dp, int k,
+                                        int64_t *__restrict__ out_idx, float *__restrict__ out_dist) {
+    const int lane = threadIdx.x & 31;
+    const float4 *q4 = reinterpret_cast<const float4 *>(q);
     const int half = lane & 1;
     const int nb = d >> 3, rem = d & 7;
     WarpTopK<1> F;
@@ -739,7 +752,7 @@ __global__ void __launch_bounds__(RR_WARPS * 32)
     for (int c0 = 0; c0 < m; c0 += 16) {
         const int c = c0 + (lane >> 1);
         const bool in = c < m;
-        const uint32_t row = in ? key_idx(sel[c]) : key_idx(sel[0]);
+        const uint32_t row = key_idx(keys[in ? c : 0]);
         const float4 *x4 = reinterpret_cast<const float4 *>(X + (int64_t)row * dp);
         float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
 #pragma unroll 8
@@ -772,9 +785,23 @@ __global__ void __launch_bounds__(RR_WARPS * 32)
     if (lane < k) {
         const uint64_t key = F.v[0];
         const bool e = key == KEY_EMPTY;
-        out_idx[q * k + lane] = e ? -1 : (int64_t)key_idx(key);
-        out_dist[q * k + lane] = e ? 0.f : __uint_as_float(key_dist(key));
+        out_idx[lane] = e ? -1 : (int64_t)key_idx(key);
+        out_dist[lane] = e ? 0.f : __uint_as_float(key_dist(key));
     }
+}
+
+// One warp per query: the S best candidates by score, then the k nearest of them.
+constexpr int RR_WARPS = 4;
+__global__ void __launch_bounds__(RR_WARPS * 32)
+    tc_rerank_kernel(const uint64_t *__restrict__ part, const int *__restrict__ qcount, int64_t slot_keys, int S,
+                     const float *__restrict__ Q, const float *__restrict__ X, int d, int dp, int64_t nq, int k,
+                     int64_t *__restrict__ out_idx, float *__restrict__ out_dist) {
+    __shared__ uint64_t s_sel[RR_WARPS][64];
+    const int warp = threadIdx.x >> 5;
+    const int64_t q = (int64_t)blockIdx.x * RR_WARPS + warp;
+    if (q >= nq) return;
+    const int m = warp_best(part + q * slot_keys, qcount[q], S, s_sel[warp]);
+    l2_rank(s_sel[warp], m, Q + q * dp, X, d, dp, k, out_idx + q * k, out_dist + q * k);
 }
 
 // ── exact Hamming k-NN of large batches ───────────────────────────────────
@@ -828,13 +855,6 @@ struct HamTc {
     bool built = false, refused = false;
     int K = 0;
 };
-
-void ham_tc_reset(gn_index *ix) {
-    if (!ix->ext) return;
-    HamTc &H = *reinterpret_cast<HamTc *>(ix->ext);
-    H.built = H.refused = false;
-    H.x8.release();
-}
 
 // Where the tensor cores answer a Hamming search.  Both paths give the same
 // results; the sums of +-1 products are whole numbers of at most 4,096, exact in
@@ -907,6 +927,189 @@ int ham_tc_search(gn_index *ix, const void *d_q, int64_t nq, int k, int64_t *d_i
     }
     GN_CUDA_TRY(cudaGetLastError());
     return GN_OK;
+}
+
+// ── exact L2 k-NN of large batches ────────────────────────────────────────
+// The exact scan's answer (indices, and distances bit for bit) through the
+// tensor cores.  Each FP32 value is split into two BF16 parts, v = hi + lo + r with
+// |lo| <= 2^-9 |v| and |r| <= 2^-18 |v|, and rows are laid out as [hi | lo | hi], the
+// query as [hi | hi | lo], so that one GEMM sums hi hi + hi lo + lo hi.  The
+// score a = |x|^2 - 2 acc then differs from D - |q|^2 (D the squared distance in
+// exact arithmetic) by at most
+//     E = cross |q| max|x| + norm max|x|^2:
+// cross >= 2 (3 2^-18 + u), the products left out and u |q||x| for the FP32 sums
+// of K terms in the tensor core, for which u = 2^-14 per 512 terms is allowed, a
+// thousand roundings of 2^-24 each; norm: the row norms' own FP32 sums.
+//
+// The pilot gives B, a score that k rows reach.  Their D is at most B + |q|^2 +
+// E, and the FP32 distance of any row lies within a relative g = (d / 8 + 16) 2^-23
+// of its D (the eight-accumulator sums, the differences' roundings, the root, and
+// distances that tie after it), so a row among the k nearest has D <= (B + |q|^2 +
+// E)(1 + rel), rel = 4 g, hence a score of at most B + 2 E + rel (B + |q|^2 + E).
+// Every row up to that bound is kept, its distance computed in the reference's
+// order, and the k nearest returned.  If some buffer could not hold its rows (many
+// ties, or values so large against their differences that E spans most rows),
+// a flag is set and the FP32 scan, launched behind it, answers instead (it ends
+// at once when the flag is clear); the index then stays with the FP32 scan until
+// the next set().
+__global__ void split_rows_kernel(const float *__restrict__ X, int64_t n, int d, int ldx, bool query,
+                                  __nv_bfloat16 *__restrict__ out, int K) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n * K) return;
+    const int64_t i = t / K;
+    const int j = (int)(t % K), part = j / d;  // part 3: padding
+    __nv_bfloat16 v = __float2bfloat16_rn(0.f);
+    if (part < 3) {
+        const float x = X[i * ldx + (j - part * d)];
+        const __nv_bfloat16 hi = __float2bfloat16_rn(x);
+        const bool low = part == (query ? 2 : 1);
+        v = low ? __float2bfloat16_rn(__fsub_rn(x, __bfloat162float(hi))) : hi;
+    }
+    out[t] = v;
+}
+
+__global__ void max_value_kernel(const float *__restrict__ x, int64_t n, uint32_t *__restrict__ out) {
+    float m = 0.f;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        m = fmaxf(m, x[i]);
+    const uint32_t w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+    if ((threadIdx.x & 31) == 0) atomicMax(out, w);
+}
+
+// One warp per query: the distances of all its candidates, the k nearest.
+__global__ void __launch_bounds__(RR_WARPS * 32)
+    l2_finish_kernel(const uint64_t *__restrict__ part, const int *__restrict__ qcount, int64_t slot_keys,
+                     const float *__restrict__ Q, const float *__restrict__ X, int d, int dp, int64_t nq, int k,
+                     int64_t *__restrict__ out_idx, float *__restrict__ out_dist, int *flag) {
+    const int64_t q = (int64_t)blockIdx.x * RR_WARPS + (threadIdx.x >> 5);
+    if (q >= nq) return;
+    // fewer candidates than results: rows whose scores are not numbers
+    if ((threadIdx.x & 31) == 0 && qcount[q] < k) *flag = 1;
+    l2_rank(part + q * slot_keys, qcount[q], Q + q * dp, X, d, dp, k, out_idx + q * k, out_dist + q * k);
+}
+
+// Expanded operands and scratch of an L2 index, made by its first large search.
+struct L2Tc {
+    HBuf hflag;  // the flag of an earlier search (copied behind it; freed after the device buffers)
+    DBuf x16, xnorm, pnorm, xmax2, q16, qnorm, part, qcount, flag;
+    TcScratch scr;
+    bool built = false, refused = false;
+    int K = 0;
+};
+
+// Where the tensor cores answer an exact L2 search: measured for 100k x 32, 1,000
+// queries, k 5: 416 us on the FP32 scan, L2TC_MEASURED here, of which 60 us do
+// not depend on the size; the FP32 scan takes about 0.13 ns per element, so
+// batches of less than 1.5 G elements stay there, and small ones, which fill
+// a part of a 128-query tile.
+bool l2_tc_wanted(const gn_index *ix, int64_t nq, int64_t k) {
+    if (k > 32 || ix->n < TC_PILOT_MIN || nq < 64 || ix->dim > 2048) return false;
+    if (ix->ext) {
+        const L2Tc &H = *reinterpret_cast<const L2Tc *>(ix->ext);
+        if (H.refused || (H.hflag.p && *reinterpret_cast<volatile int *>(H.hflag.p))) return false;
+    }
+    return (double)nq * (double)ix->n * (double)ix->dim >= 1.5e9;
+}
+
+// On success *flag is the device word that tells whether the results stand (0) or
+// the caller's FP32 scan has to answer.  GN_ERR_UNSUPPORTED: nothing was
+// launched that the caller needs to know of.
+int l2_tc_search(gn_index *ix, const float *d_q, int64_t nq, int k, int64_t *d_idx, float *d_dist, int *err,
+                 const int **flag, cudaStream_t st) {
+    if (!ix->ext) {
+        ix->ext = new L2Tc();
+        ix->ext_free = [](void *p) { delete reinterpret_cast<L2Tc *>(p); };
+    }
+    L2Tc &H = *reinterpret_cast<L2Tc *>(ix->ext);
+    const int d = (int)ix->dim, dp = ix->stride4 * 4;
+    const int K = (int)round_up(3 * d, TC_BK);
+    const float *x32 = ix->data.as<float>();
+    auto split = [&](const float *x, int64_t n, bool query, DBuf &out) {
+        split_rows_kernel<<<(unsigned)ceil_div(n * K, 256), 256, 0, st>>>(x, n, d, dp, query,
+                                                                         out.as<__nv_bfloat16>(), K);
+    };
+    if (!H.built) {
+        // at most a quarter of the free memory for the split rows
+        size_t free_b = 0, total_b = 0;
+        const size_t want = (size_t)ix->n * K * 2, np = (size_t)round_up(ix->n, TC_N);
+        if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || want > free_b / 4 || H.x16.ensure(want) != GN_OK ||
+            H.xnorm.ensure(np * 4) != GN_OK || H.xmax2.ensure(4) != GN_OK || H.flag.ensure(4) != GN_OK ||
+            H.hflag.ensure(4) != GN_OK) {
+            cudaGetLastError();
+            H.refused = true;  // until the next set()
+            return GN_ERR_UNSUPPORTED;
+        }
+        *reinterpret_cast<volatile int *>(H.hflag.p) = 0;
+        split(x32, ix->n, false, H.x16);
+        GN_CUDA_TRY(cudaMemsetAsync(H.xnorm.as<float>() + ix->n, 0xff, (np - (size_t)ix->n) * 4, st));
+        row_norms(x32, ix->n, dp, H.xnorm.as<float>(), st);
+        GN_TRY(tc_pilot_values(H.xnorm.as<float>(), ix->n, H.pnorm, st));
+        GN_CUDA_TRY(cudaMemsetAsync(H.xmax2.p, 0, 4, st));
+        max_value_kernel<<<256, 256, 0, st>>>(H.xnorm.as<float>(), ix->n, H.xmax2.as<uint32_t>());
+        H.K = K;
+        H.built = true;
+    }
+    GN_CUDA_TRY(cudaMemsetAsync(H.flag.p, 0, 4, st));
+    for (int64_t b0 = 0; b0 < nq; b0 += L2TC_QBLOCK) {
+        const int64_t bq = std::min<int64_t>(L2TC_QBLOCK, nq - b0);
+        const float *bx = d_q + b0 * dp;
+        const TcPlan plan = tc_plan(TC_BF16, K, bq, ix->n, TC_CAP - 32);
+        const int64_t a_rows = std::max<int64_t>(bq, TC_M);
+        if (H.q16.ensure((size_t)a_rows * K * 2) != GN_OK || H.qnorm.ensure((size_t)bq * 4) != GN_OK ||
+            H.part.ensure((size_t)bq * plan.slot_keys * 8) != GN_OK || H.qcount.ensure((size_t)bq * 4) != GN_OK)
+            return GN_ERR_UNSUPPORTED;
+        split(bx, bq, true, H.q16);
+        row_norms(bx, bq, dp, H.qnorm.as<float>(), st);
+        TcLaunch a;
+        a.mode = TC_BF16;
+        a.A = H.q16.p;
+        a.nq = bq;
+        a.a_rows = a_rows;
+        a.B = H.x16.p;
+        a.n = ix->n;
+        a.b_rows = ix->n;
+        a.K = K;
+        a.bnorm = H.xnorm.as<float>();
+        a.pnorm = H.pnorm.as<float>();
+        a.part = H.part.as<uint64_t>();
+        a.qcount = H.qcount.as<int>();
+        a.err = err;
+        a.S = TC_CAP - 32;
+        a.bound_rank = k;
+        a.overflow = H.flag.as<int>();
+        const float g = (float)(d / 8 + 16) * 0x1p-23f;
+        a.slack.q2 = H.qnorm.as<float>();
+        a.slack.xmax2 = H.xmax2.as<uint32_t>();
+        a.slack.overflow = H.flag.as<int>();
+        a.slack.cross = 2.f * (0x1p-16f + 0x1p-14f * (float)ceil_div(K, 512));
+        a.slack.norm = (float)(d / 32 + 16) * 0x1p-23f;
+        a.slack.rel = 4.f * g;
+        timing_begin(st, "tc_topk_kernel");
+        const int rc = tc_topk_launch(a, plan, H.scr, st);
+        timing_end(st);
+        if (rc != GN_OK) return rc == GN_ERR_OOM ? (int)GN_ERR_UNSUPPORTED : rc;
+        l2_finish_kernel<<<(unsigned)ceil_div(bq, RR_WARPS), RR_WARPS * 32, 0, st>>>(
+            H.part.as<uint64_t>(), H.qcount.as<int>(), plan.slot_keys, bx, x32, d, dp, bq, k, d_idx + b0 * k,
+            d_dist + b0 * k, H.flag.as<int>());
+    }
+    GN_CUDA_TRY(cudaMemcpyAsync(H.hflag.p, H.flag.p, 4, cudaMemcpyDeviceToHost, st));
+    *flag = H.flag.as<int>();
+    GN_CUDA_TRY(cudaGetLastError());
+    return GN_OK;
+}
+
+void flat_tc_reset(gn_index *ix) {
+    if (!ix->ext) return;
+    if (ix->metric == M_HAMMING) {
+        HamTc &H = *reinterpret_cast<HamTc *>(ix->ext);
+        H.built = H.refused = false;
+        H.x8.release();
+    } else {
+        L2Tc &H = *reinterpret_cast<L2Tc *>(ix->ext);
+        H.built = H.refused = false;
+        if (H.hflag.p) *reinterpret_cast<volatile int *>(H.hflag.p) = 0;
+        H.x16.release();
+    }
 }
 
 // ── flat tensor-core index (exact L2 via shortlist + re-rank) ─────────────

@@ -47,7 +47,6 @@ struct IvfL2State {
     // +inf past the list's size), and the largest row norm of the index
     DBuf rho;
     float xmax = 0.f;
-    DBuf sel_part, sel_done;     // split selection: partial best-S lists, per-query arrival counters
     DBuf sched;                  // unit counters of the tensor-core scans (coarse, lists)
     DBuf tmin;                   // per (score slot, 32-row quarter): minimum ordered score
     int drill = 0;               // failure drill armed for the next tensor-core list scan (tests)
@@ -59,8 +58,8 @@ struct IvfL2State {
     // 0 = built-in heuristic
     struct TcTune {
         int32_t rc = 0;    // list rows per work unit (256, 1024, 4096)
-        int32_t bmax = 0;  // most blocks one query's selection is split over (1..16)
-        int32_t nt = 0;    // selector threads per block (128, 256)
+        int32_t bmax = 0;  // kept for saved tables, no effect
+        int32_t nt = 0;    // selector threads per query (32, 128, 256)
         int32_t qc = 0;    // queries per list-scan work unit, the MMA's N (32, 64, 128)
     } tune[7];
     // search configuration version (bumped by every setter); CUDA graphs

@@ -19,7 +19,7 @@
 //              is within the query's bound;
 //   5. select  per query: a threshold from the quarter minima, only the
 //              quarters below it are read, the S best keys (S = shortlist) by
-//              radix select, their squared L2 recomputed exactly in FP32 with a
+//              counting, their squared L2 recomputed exactly in FP32 with a
 //              compensated sum, the k nearest returned, ties to the lower
 //              original index.
 // Work units are short (a list holds ~1k rows), so selection is kept out of
@@ -30,9 +30,11 @@
 #include <algorithm>
 #include <vector>
 
+#include "f32x2.cuh"
 #include "ivf.cuh"
 #include "kmeans.cuh"
 #include "prober.cuh"
+#include "select.cuh"
 #include "flat_scan.cuh"
 #include "tc_ivf.cuh"
 #include "tc_scan.cuh"
@@ -148,57 +150,414 @@ __device__ __forceinline__ float l2_warp_total(float s, float c) {
     return __fadd_rn(s, c);
 }
 
-// Exact squared L2 (compensated FP32) of the query row q to rows[0..n) of X
-// (n <= 2), by one warp: lane l takes columns 4l..4l+3 of every 128-column
-// block (coalesced float4 loads, all of a 512-column block issued together).
-__device__ __forceinline__ void l2sq_warp_rows(const float *__restrict__ q, const float *__restrict__ X, int dp,
-                                               int d, const int64_t *rows, int n, float *out, int lane) {
-    float s[2] = {0.f, 0.f}, c[2] = {0.f, 0.f};
-    for (int base = 0; base < d; base += 512) {
-        float4 qa[4], xa[2][4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i0 = base + u * 128 + lane * 4;
-            qa[u] = i0 < d ? *reinterpret_cast<const float4 *>(q + i0) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-            for (int r = 0; r < 2; ++r)
-                xa[r][u] = (r < n && i0 < d) ? __ldg(reinterpret_cast<const float4 *>(X + rows[r] * dp + i0))
-                                             : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int i0 = base + u * 128 + lane * 4;
-            const int valid = min(4, d - i0);
-#pragma unroll
-            for (int r = 0; r < 2; ++r)
-                if (r < n) l2_acc4(qa[u], xa[r][u], valid, s[r], c[r]);
-        }
-    }
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
-        if (r < n) out[r] = l2_warp_total(s[r], c[r]);
+// Exact squared L2 (compensated FP32) of the query row q to the row x by one warp, for
+// distances that l2sq_warp_pair cannot hold: it overflows only where the sum does.
+__device__ __noinline__ float l2sq_warp_row(const float *__restrict__ q, const float *__restrict__ x, int d,
+                                            int lane) {
+    float s = 0.f, c = 0.f;
+#pragma unroll 1
+    for (int i = lane * 4; i < d; i += 128)
+        l2_acc4(*reinterpret_cast<const float4 *>(q + i), __ldg(reinterpret_cast<const float4 *>(x + i)),
+                min(4, d - i), s, c);
+    return l2_warp_total(s, c);
 }
 
-constexpr int SEL_PCH = 256;   // probes staged per pass
-constexpr int SEL_WB = 512;    // candidate keys buffered per warp
-constexpr int SEL_QCAP = 256;  // qualifying quarters listed from the threshold's staged minima
-
-// Ascending bitonic sort of n (power of two, <= 512) keys in shared memory by
-// one warp.
-__device__ __forceinline__ void warp_bitonic_sort(uint64_t *a, int n, int lane) {
-    for (int size = 2; size <= n; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = lane; i < (n >> 1); i += 32) {
-                const int lo = 2 * i - (i & (stride - 1)), hi = lo + stride;
-                const bool asc = (lo & size) == 0;
-                const uint64_t x = a[lo], y = a[hi];
-                if ((x > y) == asc) {
-                    a[lo] = y;
-                    a[hi] = x;
-                }
+// Exact squared L2 (compensated FP32) of the query row q to the rows x[0], x[1] by
+// one warp, the first on lanes 0-15, the second on the others: lane l takes columns
+// 4l..4l+3 of every 128-column block (coalesced float4 loads, all of a 512-column
+// block issued together).  A sum that starts at the largest square of its lane is
+// never below the square it takes next, so r = fl(s + t^2) is at most 2 s, s - r is
+// exact, and fma(t, t, s - r) is the rounding error of r (to 2^-24 of itself): five
+// packed steps for two squares, where the product's and the sum's errors taken
+// separately (l2_acc4, no order assumed) need twelve for each.
+__device__ __forceinline__ float l2sq_warp_pair(const float *__restrict__ q, const float *__restrict__ x0,
+                                                const float *__restrict__ x1, int d, int lane) {
+    const f32x2 minus = dup2(-1.f);
+    float S[2] = {0.f, 0.f}, C[2] = {0.f, 0.f};
+#pragma unroll 1
+    for (int base = 0; base < d; base += 512) {
+        f32x2 t[2][8];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i0 = base + u * 128 + lane * 4;
+            float4 qa = make_float4(0.f, 0.f, 0.f, 0.f), xa[2] = {qa, qa};
+            if (base + u * 128 < d && i0 < d) {
+                qa = __ldg(reinterpret_cast<const float4 *>(q + i0));
+                xa[0] = __ldg(reinterpret_cast<const float4 *>(x0 + i0));
+                xa[1] = __ldg(reinterpret_cast<const float4 *>(x1 + i0));
             }
-            __syncwarp();
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                t[r][2 * u] = fma2(pack2(xa[r].x, xa[r].y), minus, pack2(qa.x, qa.y));
+                t[r][2 * u + 1] = fma2(pack2(xa[r].z, xa[r].w), minus, pack2(qa.z, qa.w));
+            }
         }
+        if ((d & 3) && base + 512 >= d) {  // columns past d count nothing
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int valid = d - (base + u * 128 + lane * 4);
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float lo, hi;
+                        unpack2(t[r][2 * u + h], lo, hi);
+                        t[r][2 * u + h] = pack2(valid > 2 * h ? lo : 0.f, valid > 2 * h + 1 ? hi : 0.f);
+                    }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float m = 0.f;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                float lo, hi;
+                unpack2(t[r][i], lo, hi);
+                m = fmaxf(m, fmaxf(fabsf(lo), fabsf(hi)));
+            }
+            const float start = m * m;
+            f32x2 s = dup2(start), c = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (base + u * 128 < d)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const f32x2 v = t[r][2 * u + h], sum = fma2(v, v, s);
+                        c = add2(c, fma2(v, v, fma2(sum, minus, s)));
+                        s = sum;
+                    }
+            float slo, shi, clo, chi, a, ea, b, eb, e;
+            unpack2(s, slo, shi);
+            unpack2(c, clo, chi);
+            two_sum(slo, shi, a, ea);
+            two_sum(a, -2.f * start, b, eb);
+            two_sum(S[r], b, S[r], e);
+            C[r] = __fadd_rn(C[r], __fadd_rn(__fadd_rn(clo, chi), __fadd_rn(__fadd_rn(ea, eb), e)));
+        }
+    }
+    // the halves of the warp swap rows, then each adds up its own
+    const bool up = lane & 16;
+    float s = up ? S[1] : S[0], c = up ? C[1] : C[0];
+    const float so = __shfl_xor_sync(0xffffffffu, up ? S[0] : S[1], 16),
+                co = __shfl_xor_sync(0xffffffffu, up ? C[0] : C[1], 16);
+    float s2, err;
+    two_sum(s, so, s2, err);
+    s = s2;
+    c = __fadd_rn(c, __fadd_rn(co, err));
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+        const float sx = __shfl_xor_sync(0xffffffffu, s, o), cx = __shfl_xor_sync(0xffffffffu, c, o);
+        two_sum(s, sx, s2, err);
+        s = s2;
+        c = __fadd_rn(c, __fadd_rn(cx, err));
+    }
+    float out = __fadd_rn(s, c);
+    if (__any_sync(0xffffffffu, !(out < INFINITY))) {  // the starts may overflow before the sums do
+        const float a = l2sq_warp_row(q, x0, d, lane), b = l2sq_warp_row(q, x1, d, lane);
+        out = up ? b : a;
+    }
+    return out;
+}
+
+// ── selection and exact re-rank ───────────────────────────────────────────
+constexpr int SEL_P = 64;      // probes whose layout is held at a time (two per lane)
+constexpr int SEL_GROUP = 128; // slots whose minima are held at a time (four per lane)
+constexpr int SEL_BUF = 256;   // candidate keys per warp
+constexpr int SEL_ALL = 512;   // candidate keys of a block's warps brought together
+constexpr int SEL_WARPS = 28;  // warps resident per SM (72 registers a thread)
+
+// Shared memory of one warp of the selection.
+struct SelWarp {
+    uint64_t buf[SEL_BUF];             // candidates (ordered score, row)
+    uint64_t best[64];                 // the S best of them
+    int4 probe[SEL_P];                 // list's first row, rows, first slot (from the query's), slots of the probes before
+    uint16_t list[4 * SEL_GROUP];      // qualifying quarters: probe << 9 | quarter of the group
+    int32_t pre[SEL_P + 1];            // slots of the probes before each
+};
+
+// A bound with at least S of the warp's values (R per lane) at or below it, and at
+// most S / 8 more unless equal values leave no such bound: bit by bit from the
+// highest in which the values differ.
+template <int R>
+__device__ __forceinline__ uint32_t warp_kth(const uint32_t (&v)[R], int S) {
+    uint32_t any = 0u, all = 0xffffffffu;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        any |= v[i];
+        all &= v[i];
+    }
+    any = __reduce_or_sync(0xffffffffu, any);
+    all = __reduce_and_sync(0xffffffffu, all);
+    if (any == all) return all;
+    int bit = 31 - __clz((int)(any ^ all));
+    uint32_t kth = bit == 31 ? 0u : all & ~((2u << bit) - 1u);
+#pragma unroll 1
+    for (; bit >= 0; --bit) {
+        const uint32_t trial = kth | (1u << bit);
+        int c = 0;
+#pragma unroll
+        for (int i = 0; i < R; ++i) c += v[i] < trial;
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (c >= S && c <= S + (S >> 3)) return trial - 1u;
+        if (c < S) kth = trial;
+    }
+    return kth;
+}
+
+// One group of slots of a query, slots g0 .. of the held probes (`all` of them): their
+// quarter minima are read at once; `first` takes the threshold from them; the quarters
+// at or below it are listed, and the listed quarters' scores read sixteen at a time,
+// eight lanes to a quarter, their loads in flight together.  The first group is
+// listed by every warp of the block, which read every NW-th sixteen of the list; a
+// later one belongs to one warp.
+template <int NW>
+__device__ __forceinline__ void sel_group(SelWarp &W, const uint4 *__restrict__ tmin, const float *__restrict__ scores,
+                                          int g0, int all, bool first, int S, int warp, int lane, uint32_t &tau,
+                                          int &wn) {
+    constexpr int U = SEL_GROUP / 32;
+    const unsigned below = (1u << lane) - 1u;
+    uint32_t v[4 * U];
+    int probe[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int f = min(g0 + u * 32 + lane, all - 1);
+        int p = 0;  // pre[p] <= f < pre[p + 1]
+#pragma unroll
+        for (int step = SEL_P / 2; step > 0; step >>= 1)
+            if (W.pre[p + step] <= f) p += step;
+        probe[u] = p;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const int f = g0 + u * 32 + lane;
+        uint4 m = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
+        if (f < all) m = __ldg(tmin + W.probe[probe[u]].z + (f - W.probe[probe[u]].w));
+        v[4 * u] = m.x;
+        v[4 * u + 1] = m.y;
+        v[4 * u + 2] = m.z;
+        v[4 * u + 3] = m.w;
+    }
+    if (first && 4 * min(all - g0, SEL_GROUP) >= S) tau = min(tau, warp_kth<4 * U>(v, S));
+    int n = 0;  // listed
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const bool in = v[4 * u + e] <= tau;
+            const unsigned b = __ballot_sync(0xffffffffu, in);
+            if (in) W.list[n + __popc(b & below)] = (uint16_t)(probe[u] << 9 | (u * 32 + lane) * 4 + e);
+            n += __popc(b);
+        }
+    __syncwarp();
+#pragma unroll 1
+    for (int e0 = first ? 16 * warp : 0; e0 < n; e0 += first ? 16 * NW : 16) {
+        float4 x[4];
+        uint32_t row[4];
+        int rows[4];  // real rows among the lane's four
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const int i = e0 + 4 * u + (lane >> 3);
+            rows[u] = 0;
+            if (i < n) {
+                const int e = W.list[i];
+                const int4 p = W.probe[e >> 9];
+                const int s = g0 + (e >> 2 & (SEL_GROUP - 1)) - p.w, r = s * 128 + (e & 3) * 32 + (lane & 7) * 4;
+                row[u] = (uint32_t)(p.x + r);
+                rows[u] = p.y - r;
+                if (rows[u] > 0)
+                    x[u] = __ldg(reinterpret_cast<const float4 *>(scores + ((size_t)(p.z + s) * 128 + (r & 127))));
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (wn > SEL_BUF - 128) {  // the next four quarters may not fit
+                tau = min(tau, list_cut<SEL_BUF / 32>(W.buf, wn, S));
+                wn = S;
+            }
+            const float xs[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const uint32_t bits = f2ord(xs[c]);
+                const bool in = rows[u] > c && bits <= tau;
+                const unsigned b = __ballot_sync(0xffffffffu, in);
+                if (in) W.buf[wn + __popc(b & below)] = make_key(bits, row[u] + c);
+                wn += __popc(b);
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// Selection of one query by a block of NW warps.  The list scan leaves, per
+// (query, list) pair, the scores of the list's rows in 128-row slots and the
+// minimum score of every 32-row quarter of every slot.  Keys are (score, row),
+// so ties go to the lower row.
+//   threshold  tau = the S-th smallest quarter minimum of the query's first 128
+//              slots, counted out of registers by every warp for itself: S
+//              distinct rows score <= tau, so tau bounds the query's S-th best
+//              score; capped by the query's bound from the probe stage, above
+//              which the scan stored no quarter;
+//   sweep      only the quarters with a minimum <= tau are read (a few dozen of
+//              the query's hundreds); scores <= tau become keys in the warp's
+//              buffer, cut to its best S when it fills, which lowers tau;
+//   select     the S smallest keys of all the warps' buffers, by counting;
+//   re-rank    two rows per warp at a time: exact squared L2 in FP32
+//              (compensated sum); warp 0 returns the k nearest, ties to the
+//              lower original index.
+// Nothing but the hand-over of the candidates and of the distances (NW > 1) waits
+// for another warp.  Measured on 400k x 512 rows, 1,024 lists, 28 probed, S 40: a batch
+// of 4,096 took 203 us with block-wide radix selects, four warps a query (bound by their
+// barriers, and by the twelve steps of each square), 78 us here, where its 336 MB of
+// rows take 50 at the DRAM's measured rate; 16 queries (200k x 256, 16 of 512 lists)
+// 35 us, split over 16 blocks each, 19 here.
+template <int NW>
+__global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW) ivf_tc_select_kernel(
+    const float *__restrict__ scores, const uint4 *__restrict__ tmin4, const uint32_t *__restrict__ qbound,
+    const int32_t *__restrict__ probes, int np, const int64_t *__restrict__ qseg,
+    const int64_t *__restrict__ seg_rel, const int64_t *__restrict__ list_off, int S, const float *__restrict__ Q,
+    const float *__restrict__ X, int d, int dp, const int32_t *__restrict__ ids, int k,
+    int64_t *__restrict__ out_idx, float *__restrict__ out_dist, int64_t *__restrict__ out_cnt) {
+    __shared__ SelWarp s_warp[NW];
+    __shared__ uint64_t s_all[NW > 1 ? SEL_ALL : 1];
+    __shared__ int s_wn[NW];
+    __shared__ float s_d[64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t q = blockIdx.x;
+    SelWarp &W = s_warp[warp];
+    const uint4 *tmin = tmin4 + qseg[q];
+    const float *sc = scores + qseg[q] * 128;
+    uint32_t tau = qbound[q];  // scores <= tau are candidates
+    int wn = 0;                // keys in this warp's buffer
+    int group = 0;
+    for (int p0 = 0; p0 < np; p0 += SEL_P) {
+        // the probes' layout: lane l holds probes l and l + 32
+        int ns[2];
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = h * 32 + lane;
+            const int32_t l = p0 + i < np ? probes[q * np + p0 + i] : -1;
+            int64_t lb = 0, len = 0, sl = 0;
+            if (l >= 0) {
+                lb = list_off[l];
+                len = list_off[l + 1] - lb;
+                sl = seg_rel[q * np + p0 + i];
+            }
+            W.probe[i] = make_int4((int)lb, (int)len, (int)sl, 0);
+            ns[h] = (int)((len + 127) >> 7);
+        }
+        int inc0 = ns[0], inc1 = ns[1];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, inc0, o), b = __shfl_up_sync(0xffffffffu, inc1, o);
+            if (lane >= o) {
+                inc0 += a;
+                inc1 += b;
+            }
+        }
+        inc1 += __shfl_sync(0xffffffffu, inc0, 31);
+        W.pre[lane + 1] = inc0;
+        W.pre[lane + 33] = inc1;
+        W.probe[lane].w = inc0 - ns[0];
+        W.probe[lane + 32].w = inc1 - ns[1];
+        if (lane == 0) W.pre[0] = 0;
+        __syncwarp();
+        const int all = W.pre[SEL_P];
+        for (int g0 = 0; g0 < all; g0 += SEL_GROUP, ++group)
+            if (group == 0 || NW == 1 || group % NW == warp)
+                sel_group<NW>(W, tmin, sc, g0, all, group == 0, S, warp, lane, tau, wn);
+    }
+    __syncwarp();
+    int m;  // candidates re-ranked: best[0 .. m)
+    if (NW == 1) {
+        m = warp_best(W.buf, wn, S, W.best);
+    } else {  // brought together, then every warp selects for itself
+        if (lane == 0) s_wn[warp] = wn;
+        __syncthreads();
+        int total = 0, before = 0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) {
+            if (w == warp) before = total;
+            total += s_wn[w];
+        }
+        if (total <= SEL_ALL) {
+            for (int i = lane; i < wn; i += 32) s_all[before + i] = W.buf[i];
+            __syncthreads();
+            m = warp_best(s_all, total, S, W.best);
+        } else {
+            m = warp_best_of(
+                [&](int i) {
+                    int w = 0;
+                    while (i >= s_wn[w]) i -= s_wn[w++];
+                    return s_warp[w].buf[i];
+                },
+                total, S, W.best);
+        }
+    }
+    __syncwarp();
+    // exact re-rank, two rows per warp at a time.  A warp of a small batch asks for all
+    // its rows first, so that they come in one DRAM round trip; a large batch has
+    // enough other warps to cover that wait.
+    const float *qrow = Q + q * dp;
+    if (NW > 1) {
+        const int lines = (d * 4 + 127) / 128;
+        for (int r = 2 * warp; r < m; r += 2 * NW)
+            for (int i = lane; i < 2 * lines; i += 32) {
+                const int u = i >= lines;
+                if (r + u < m)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(X + (int64_t)key_idx(W.best[r + u]) * dp +
+                                                                  (i - u * lines) * 32));
+            }
+    }
+    uint32_t id[2] = {0u, 0u};
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        if (warp == 0 && h * 32 + lane < m) id[h] = (uint32_t)ids[key_idx(W.best[h * 32 + lane])];
+#pragma unroll 1
+    for (int r = 2 * warp; r < m; r += 2 * NW) {
+        const bool two = r + 1 < m;
+        const float *x0 = X + (int64_t)key_idx(W.best[r]) * dp;
+        const float dist = l2sq_warp_pair(qrow, x0, two ? X + (int64_t)key_idx(W.best[r + 1]) * dp : x0, d, lane);
+        if (lane == 0 || (lane == 16 && two)) s_d[r + (lane >> 4)] = dist;
+    }
+    if (NW > 1) __syncthreads();
+    else __syncwarp();
+    if (warp != 0) return;
+    uint64_t key[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+        key[h] = h * 32 + lane < m ? make_key(__float_as_uint(s_d[h * 32 + lane]), id[h]) : KEY_EMPTY;
+    warp_sort<2>(key);
+    const bool e = key[0] == KEY_EMPTY;
+    if (lane < k) {
+        out_idx[q * k + lane] = e ? -1 : (int64_t)key_idx(key[0]);
+        out_dist[q * k + lane] = e ? 0.f : __uint_as_float(key_dist(key[0]));
+    }
+    const int cnt = __popc(__ballot_sync(0xffffffffu, lane < k && !e));
+    if (lane == 0 && out_cnt) out_cnt[q] = cnt;
+}
+
+// ── tensor-core coarse stage ──────────────────────────────────────────────
+// Units of the centroid scan: every query chunk of 256 against every chunk of
+// 128 centroids; aslot[q] = q * nc so the scores land row-major [nq x nc].
+__global__ void coarse_units_kernel(int64_t nq, int nc, TcUnit *__restrict__ units, int64_t *__restrict__ n_units,
+                                    int64_t *__restrict__ aslot) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t nqc = (nq + TC_QCHUNK - 1) / TC_QCHUNK, ncc = (nc + 127) / 128;
+    if (t == 0) *n_units = nqc * ncc;
+    if (t < nq) aslot[t] = t * nc;
+    if (t >= nqc * ncc) return;
+    const int64_t qc = t / ncc, cc = t % ncc;
+    TcUnit u;
+    u.a0 = qc * TC_QCHUNK;
+    u.na = (int32_t)min((int64_t)TC_QCHUNK, nq - u.a0);
+    u.r0 = cc * 128;
+    u.r1 = min((int64_t)nc, u.r0 + 128);
+    u.rbase = 0;
+    u.xrow = u.r0;
+    u.rch = 0;
+    units[t] = u;
 }
 
 // The S smallest of a key multiset held in shared memory, by the whole block
@@ -275,564 +634,6 @@ __device__ int block_radix_select(const uint64_t *keys, int WB, const int *cnt, 
     }
     __syncthreads();
     return sh[3];
-}
-
-// k-th smallest (1-based) of n unsigned values in shared memory, by the whole
-// block (radix select on 8-bit digits); all ones if n < kth.
-template <int NT>
-__device__ uint32_t block_kth_u32(const uint32_t *v, int n, int kth, int *hist, int *sh) {
-    if (n < kth) return 0xffffffffu;
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    uint32_t prefix = 0, mask = 0;
-    int need = kth;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        for (int i = t; i < 256; i += NT) hist[i] = 0;
-        __syncthreads();
-        for (int i = t; i < n; i += NT) {
-            const uint32_t x = v[i];
-            if ((x & mask) == prefix) atomicAdd(&hist[(x >> shift) & 255], 1);
-        }
-        __syncthreads();
-        if (warp == 0) {
-            int h[8], sum = 0;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                h[e] = hist[lane * 8 + e];
-                sum += h[e];
-            }
-            int inc = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int x = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += x;
-            }
-            int before = inc - sum;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                if (before < need && need <= before + h[e]) {
-                    sh[0] = lane * 8 + e;
-                    sh[1] = before;
-                }
-                before += h[e];
-            }
-        }
-        __syncthreads();
-        prefix |= (uint32_t)sh[0] << shift;
-        mask |= 0xffu << shift;
-        need -= sh[1];
-        __syncthreads();
-    }
-    return prefix;
-}
-
-// Offer each lane's key (want: it is a real row) to the warp's shared-memory
-// buffer W of SEL_WB keys (wn keys held, warp-uniform): keys below the warp
-// threshold are appended; a full buffer is sorted and cut to its best S, its
-// S-th key becoming the new threshold, and the keys that did not fit are
-// offered again.
-__device__ __forceinline__ void sel_buffer_offer(uint64_t key, bool want, uint64_t *W, int &wn, uint64_t &wthr,
-                                                 int S, int lane) {
-    bool w = want && key < wthr;
-    while (true) {
-        const unsigned b2 = __ballot_sync(0xffffffffu, w);
-        if (!b2) break;
-        const int pos = wn + __popc(b2 & ((1u << lane) - 1u));
-        if (w && pos < SEL_WB) {
-            W[pos] = key;
-            w = false;
-        }
-        wn += __popc(b2);
-        if (wn <= SEL_WB) break;
-        __syncwarp();
-        warp_bitonic_sort(W, SEL_WB, lane);
-        wthr = W[S - 1];
-        wn = S;
-        w = w && key < wthr;
-        __syncwarp();
-    }
-}
-
-// Selection of one query by B blocks of NT threads (B = 1 for large batches;
-// small batches split each query's range over up to 16 blocks, whose partial
-// best-S lists the last block to finish merges).  The list scan leaves, per
-// (query, list) pair, the scores of the list's rows in 128-row slots and the
-// minimum score of every 32-row quarter of every slot.  Keys are (score, row),
-// so ties go to the lower row.
-//   threshold  tau = the S-th smallest quarter minimum of the block's slots
-//              (radix select): S distinct rows score <= tau, so tau bounds the
-//              query's S-th best score; tau is capped by the query's bound
-//              from the probe stage, above which the scan stored no quarter;
-//   sweep      the quarters whose minimum is <= tau, listed from the minima
-//              staged for the threshold (typically a few dozen of the query's
-//              hundreds of slots), are read four per warp at a time (one
-//              coalesced 128-byte load each); slots beyond the staged ones are
-//              swept 8 at a time (lane l: quarter l % 4 of slot l / 4);
-//   buffer     scores <= tau become keys in the warp's shared-memory buffer
-//              (512 keys); a full buffer is sorted and cut to its best S;
-//   select     radix select of the S smallest keys of all warps' buffers;
-//   re-rank    two rows per warp at a time: exact squared L2 in FP32
-//              (compensated sum); warp 0 returns the k nearest, ties to the
-//              lower original index.
-template <int NT>
-__global__ void __launch_bounds__(NT, 1024 / NT) ivf_tc_select_kernel(
-    const float *__restrict__ scores, const uint4 *__restrict__ tmin4, const uint32_t *__restrict__ qbound,
-    const int32_t *__restrict__ probes, int np,
-    const int64_t *__restrict__ qseg, const int64_t *__restrict__ seg_rel, const int64_t *__restrict__ list_off,
-    int S, const float *__restrict__ Q, const float *__restrict__ X, int d, int dp, const int32_t *__restrict__ ids,
-    int64_t nq, int k, int B, uint64_t *__restrict__ part, int *__restrict__ done, int64_t *__restrict__ out_idx,
-    float *__restrict__ out_dist, int64_t *__restrict__ out_cnt) {
-    constexpr int NW = NT / 32;
-    __shared__ uint64_t wreg[NW * SEL_WB];
-    __shared__ int64_t p_slot[SEL_PCH], p_lb[SEL_PCH], p_len[SEL_PCH], p_tpre[SEL_PCH + 1];
-    __shared__ int64_t w_sum[NW];
-    __shared__ uint64_t sel[64], s_rk[64];
-    __shared__ int hist[256], sh[4], s_wn[NW];
-    __shared__ int s_last, s_qn;
-    __shared__ int32_t qlist[SEL_QCAP];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int64_t q = blockIdx.x / B;
-    const int bq = (int)(blockIdx.x % B);  // this block's share of the query's slots (B > 1 needs np <= SEL_PCH)
-    uint64_t *W = wreg + warp * SEL_WB;
-    int wn = 0;                 // keys in this warp's buffer (warp-uniform)
-    uint64_t wthr = KEY_EMPTY;  // this warp's threshold (its S-th best key after a cut)
-    uint32_t tau = 0xffffffffu;
-
-    for (int p0 = 0; p0 < np; p0 += SEL_PCH) {
-        int64_t sweep_lo;  // first slot of this pass the sweep reads minima for
-        const int pc = min(SEL_PCH, np - p0);
-        // per-probe metadata and the prefix sum of the slot counts
-        int64_t nslot = 0;
-        if (t < pc) {
-            const int64_t pair = q * np + p0 + t;
-            const int32_t l = probes[pair];
-            p_lb[t] = 0;
-            p_len[t] = 0;
-            p_slot[t] = 0;
-            if (l >= 0) {
-                p_lb[t] = list_off[l];
-                p_len[t] = list_off[l + 1] - p_lb[t];
-                p_slot[t] = qseg[q] + seg_rel[pair];
-                nslot = (p_len[t] + 127) >> 7;
-            }
-        }
-        int64_t inc = nslot;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int64_t v = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += v;
-        }
-        if (lane == 31) w_sum[warp] = inc;
-        __syncthreads();
-        int64_t before = 0;
-        for (int w = 0; w < warp; ++w) before += w_sum[w];
-        if (t < pc) p_tpre[t + 1] = before + inc;
-        if (t == 0) p_tpre[0] = 0;
-        __syncthreads();
-        const int64_t all = p_tpre[pc];
-        // parts actually used: at least 2S slots each, so that every part's
-        // threshold comes from enough slot minima (idle parts publish nothing)
-        const int bu = (int)max((int64_t)1, min((int64_t)B, all / (2 * S)));
-        const int64_t lo = bq < bu ? all * bq / bu : all, hi = bq < bu ? all * (bq + 1) / bu : all;
-        sweep_lo = lo;
-        if (p0 == 0) {
-            // threshold from the quarter minima of the block's first slots (any
-            // S of them are S distinct rows' scores, so they bound it)
-            uint32_t *tm = reinterpret_cast<uint32_t *>(wreg);
-            const int ns = (int)min(hi - lo, (int64_t)NW * SEL_WB / 2);
-            int p = 0;
-            for (int i = t; i < ns; i += NT) {
-                const int64_t f = lo + i;
-                while (p_tpre[p + 1] <= f) ++p;
-                const uint4 m = __ldg(tmin4 + p_slot[p] + (f - p_tpre[p]));
-                tm[4 * i] = m.x;
-                tm[4 * i + 1] = m.y;
-                tm[4 * i + 2] = m.z;
-                tm[4 * i + 3] = m.w;
-            }
-            __syncthreads();
-            // and never above the query's bound: quarters above it were not stored
-            tau = min(block_kth_u32<NT>(tm, 4 * ns, S, hist, sh), qbound[q]);
-            wthr = tau == 0xffffffffu ? KEY_EMPTY : make_key(tau, 0xffffffffu);
-            // the qualifying quarters among the staged minima, listed (any order)
-            if (t == 0) s_qn = 0;
-            __syncthreads();
-            for (int i = t; i < 4 * ns; i += NT)
-                if (tm[i] <= tau) {
-                    const int pos = atomicAdd(&s_qn, 1);
-                    if (pos < SEL_QCAP) qlist[pos] = i;
-                }
-            __syncthreads();
-            // all of them listed: they are read straight from the list, four
-            // quarters per warp at a time with their loads in flight together;
-            // the sweep below covers the slots past the staged ones
-            if (s_qn <= SEL_QCAP) {
-                const int nl = s_qn;
-                for (int e0 = warp * 4; e0 < nl; e0 += NW * 4) {
-                    const int nb = min(4, nl - e0);
-                    uint64_t key[4];
-                    bool want[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int idx = u < nb ? qlist[e0 + u] : 0;
-                        const int64_t f = lo + (idx >> 2);
-                        int a = 0, b = pc;  // probe pp: p_tpre[pp] <= f < p_tpre[pp + 1]
-                        while (b - a > 1) {
-                            const int mid = (a + b) >> 1;
-                            if (p_tpre[mid] <= f) a = mid;
-                            else b = mid;
-                        }
-                        const int64_t slot = f - p_tpre[a];
-                        const int i = (idx & 3) * 32 + lane;  // row within the slot
-                        const int64_t r0 = slot * 128;
-                        const bool ok = u < nb && r0 + i < p_len[a];
-                        const uint32_t v = ok ? f2ord(__ldg(scores + (p_slot[a] + slot) * 128 + i)) : 0xffffffffu;
-                        key[u] = make_key(v, (uint32_t)(p_lb[a] + r0 + i));
-                        want[u] = ok;
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) sel_buffer_offer(key[u], want[u], W, wn, wthr, S, lane);
-                }
-                sweep_lo = lo + ns;
-            }
-            __syncthreads();  // the list and the staged minima are done with before the buffers fill
-        }
-        int p = 0;  // probe of this lane's slot (monotone over the sweep)
-        // warp w takes 8 slots at a time: lane l looks at quarter l % 4 of slot g0 + l / 4
-        for (int64_t g0 = sweep_lo + (int64_t)warp * 8; g0 < hi; g0 += (int64_t)NW * 8) {
-            const int64_t f = g0 + (lane >> 2);
-            const int qu = lane & 3;
-            bool qual = false;
-            if (f < hi) {
-                while (p_tpre[p + 1] <= f) ++p;
-                qual = __ldg(reinterpret_cast<const uint32_t *>(tmin4 + p_slot[p] + (f - p_tpre[p])) + qu) <= tau;
-            }
-            unsigned bal = __ballot_sync(0xffffffffu, qual);
-            while (bal) {
-                // up to four qualifying quarters at a time, their loads in flight together
-                int src[4], nb = 0;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    src[u] = bal ? __ffs(bal) - 1 : -1;
-                    if (bal) {
-                        bal &= bal - 1;
-                        ++nb;
-                    }
-                }
-                uint32_t v[4];
-                uint64_t key[4];
-                bool want[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    const int sl = src[u] < 0 ? 0 : src[u];
-                    const int pp = __shfl_sync(0xffffffffu, p, sl);
-                    const int64_t slot = g0 + (sl >> 2) - p_tpre[pp];
-                    const int i = (sl & 3) * 32 + lane;  // row within the slot
-                    const int64_t r0 = slot * 128;
-                    const bool ok = u < nb && r0 + i < p_len[pp];
-                    v[u] = ok ? f2ord(__ldg(scores + (p_slot[pp] + slot) * 128 + i)) : 0xffffffffu;
-                    key[u] = make_key(v[u], (uint32_t)(p_lb[pp] + r0 + i));
-                    want[u] = ok;
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) sel_buffer_offer(key[u], want[u], W, wn, wthr, S, lane);
-            }
-        }
-        __syncthreads();
-    }
-    if (lane == 0) s_wn[warp] = wn;
-    __syncthreads();
-    int m = block_radix_select<NT>(wreg, SEL_WB, s_wn, S, sel, hist, sh);
-    if (B > 1) {
-        // publish this block's best S; the last block of the query merges all
-        uint64_t *mine = part + ((size_t)q * B + bq) * S;
-        for (int i = t; i < S; i += NT) mine[i] = i < m ? sel[i] : KEY_EMPTY;
-        __threadfence();
-        __syncthreads();
-        if (t == 0) s_last = atomicAdd(done + q, 1) == B - 1;
-        __syncthreads();
-        if (!s_last) return;
-        __threadfence();
-        // block b's list goes to region b mod 8 (at offset (b / 8) * S)
-        const uint64_t *all_q = part + (size_t)q * B * S;
-        for (int i = t; i < B * S; i += NT) {
-            const int b = i / S;
-            wreg[(b % NW) * SEL_WB + (b / NW) * S + i % S] = __ldcg(all_q + i);
-        }
-        if (t < NW) s_wn[t] = ((B - t + NW - 1) / NW) * S;
-        if (t == 0) done[q] = 0;  // ready for the next batch
-        __syncthreads();
-        m = block_radix_select<NT>(wreg, SEL_WB, s_wn, S, sel, hist, sh);
-    }
-
-    // exact re-rank of the candidates, two rows per warp at a time; first every
-    // thread prefetches a share of all candidate rows' 128-byte lines into L2,
-    // so that the warps' row loads do not each wait a full DRAM round trip
-    const float *qrow = Q + q * dp;
-    {
-        const int lines = (d * 4 + 127) / 128, nc = min(m, S);
-        for (int i = t; i < nc * lines; i += NT) {
-            const uint64_t c = sel[i / lines];
-            if (c != KEY_EMPTY)
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(X + (int64_t)key_idx(c) * dp + (i % lines) * 32));
-        }
-    }
-    for (int r = 2 * warp; r < S; r += 2 * NW) {
-        int64_t rows[2];
-        int n = 0;
-        for (int u = 0; u < 2; ++u) {
-            const uint64_t c = (r + u < S && r + u < m) ? sel[r + u] : KEY_EMPTY;
-            rows[u] = c != KEY_EMPTY ? (int64_t)key_idx(c) : -1;
-        }
-        n = rows[0] < 0 ? 0 : (rows[1] < 0 ? 1 : 2);
-        if (rows[0] < 0 && rows[1] >= 0) {  // keep the valid row first
-            rows[0] = rows[1];
-            rows[1] = -1;
-            n = 1;
-        }
-        float dd[2];
-        if (n) l2sq_warp_rows(qrow, X, dp, d, rows, n, dd, lane);
-        if (lane == 0)
-            for (int u = 0; u < 2 && r + u < S; ++u) s_rk[r + u] = KEY_EMPTY;
-        __syncwarp();
-        if (lane == 0)
-            for (int u = 0; u < n; ++u) s_rk[r + u] = make_key(__float_as_uint(dd[u]), (uint32_t)ids[rows[u]]);
-    }
-    __syncthreads();
-    if (warp != 0) return;
-    WarpTopK<1> F;
-    F.init();
-    uint64_t fthr = KEY_EMPTY;
-    for (int r0 = 0; r0 < S; r0 += 32) {
-        const uint64_t key = (r0 + lane < S) ? s_rk[r0 + lane] : KEY_EMPTY;
-        F.offer(key, fthr, k);
-    }
-    const uint64_t key = F.v[0];
-    const bool e = key == KEY_EMPTY;
-    if (lane < k) {
-        out_idx[q * k + lane] = e ? -1 : (int64_t)key_idx(key);
-        out_dist[q * k + lane] = e ? 0.f : __uint_as_float(key_dist(key));
-    }
-    const int cnt = __popc(__ballot_sync(0xffffffffu, lane < k && !e));
-    if (lane == 0 && out_cnt) out_cnt[q] = cnt;
-}
-
-// Selection of one query per warp (no block barriers; an autotuner option): the
-// same keys (score, row), the same S smallest, the same exact re-rank and
-// output as ivf_tc_select_kernel.
-//   threshold  tau = the S-th smallest quarter minimum of the query's first 64
-//              slots (a bitwise select over the warp's 256 values): S distinct
-//              rows score <= tau; capped by the query's bound;
-//   sweep      the block kernel's warp loop over all the query's slots: 8
-//              slots a step, only quarters whose minimum is <= tau are read,
-//              their scores <= the warp threshold buffered as keys;
-//   select     bitonic sort of the buffer (a full buffer is cut to its best S
-//              on the way), the first S keys;
-//   re-rank    two rows at a time (rows prefetched into L2 first), then the k
-//              nearest, ties to the lower original index.
-// Needs np <= 64 probes.
-constexpr int SELW_WARPS = 4;
-
-__global__ void __launch_bounds__(32 * SELW_WARPS) ivf_tc_select_warp_kernel(
-    const float *__restrict__ scores, const uint4 *__restrict__ tmin4, const uint32_t *__restrict__ qbound,
-    const int32_t *__restrict__ probes, int np,
-    const int64_t *__restrict__ qseg, const int64_t *__restrict__ seg_rel, const int64_t *__restrict__ list_off,
-    int S, const float *__restrict__ Q, const float *__restrict__ X, int d, int dp, const int32_t *__restrict__ ids,
-    int64_t nq, int k, int64_t *__restrict__ out_idx, float *__restrict__ out_dist, int64_t *__restrict__ out_cnt) {
-    __shared__ uint64_t wreg[SELW_WARPS * SEL_WB];
-    __shared__ int64_t w_pre[SELW_WARPS][65], w_lb[SELW_WARPS][64], w_len[SELW_WARPS][64], w_sb[SELW_WARPS][64];
-    __shared__ uint64_t w_rk[SELW_WARPS][64];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t q = (int64_t)blockIdx.x * SELW_WARPS + warp;
-    if (q >= nq) return;  // the whole warp; no block barrier below
-    uint64_t *W = wreg + warp * SEL_WB;
-    int64_t *pre = w_pre[warp], *plb = w_lb[warp], *plen = w_len[warp], *psb = w_sb[warp];
-    // probes: lane l holds probes l and l + 32; the slot counts' prefix sum in probe order
-    int64_t ns[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int p = h * 32 + lane;
-        ns[h] = 0;
-        plb[p] = 0;
-        plen[p] = 0;
-        psb[p] = 0;
-        const int32_t l = p < np ? probes[q * np + p] : -1;
-        if (l >= 0) {
-            plb[p] = list_off[l];
-            plen[p] = list_off[l + 1] - plb[p];
-            psb[p] = qseg[q] + seg_rel[q * np + p];
-            ns[h] = (plen[p] + 127) >> 7;
-        }
-    }
-    int64_t inc0 = ns[0], inc1 = ns[1];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int64_t a = __shfl_up_sync(0xffffffffu, inc0, o), b = __shfl_up_sync(0xffffffffu, inc1, o);
-        if (lane >= o) {
-            inc0 += a;
-            inc1 += b;
-        }
-    }
-    const int64_t tot0 = __shfl_sync(0xffffffffu, inc0, 31);
-    inc1 += tot0;
-    pre[lane + 1] = inc0;
-    pre[lane + 33] = inc1;
-    if (lane == 0) pre[0] = 0;
-    __syncwarp();
-    const int64_t all = pre[64];
-    // threshold from the quarter minima of the first (up to) 64 slots
-    uint32_t mv[8];
-    const int64_t nfirst = min(all, (int64_t)64);
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int64_t f = h * 32 + lane;
-        uint4 m4 = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);
-        if (f < nfirst) {
-            int lo = 0, hi = 64;  // the probe whose slots hold f: pre[p] <= f < pre[p + 1]
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (pre[mid] <= f) lo = mid;
-                else hi = mid;
-            }
-            m4 = __ldg(tmin4 + psb[lo] + (f - pre[lo]));
-        }
-        mv[4 * h] = m4.x;
-        mv[4 * h + 1] = m4.y;
-        mv[4 * h + 2] = m4.z;
-        mv[4 * h + 3] = m4.w;
-    }
-    uint32_t tau = 0xffffffffu;
-    if (4 * nfirst >= S) {
-        tau = 0;
-        for (int b = 31; b >= 0; --b) {
-            const uint32_t t = tau | ((1u << b) - 1u);
-            int cnt = 0;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) cnt += __popc(__ballot_sync(0xffffffffu, mv[u] <= t));
-            if (cnt < S) tau |= 1u << b;
-        }
-    }
-    tau = min(tau, qbound[q]);  // quarters above the query's bound were not stored
-    uint64_t wthr = tau == 0xffffffffu ? KEY_EMPTY : make_key(tau, 0xffffffffu);
-    int wn = 0;
-    int p = 0;  // probe of this lane's slot (monotone over the sweep)
-    for (int64_t g0 = 0; g0 < all; g0 += 8) {
-        const int64_t f = g0 + (lane >> 2);
-        const int qu = lane & 3;
-        bool qual = false;
-        if (f < all) {
-            while (pre[p + 1] <= f) ++p;
-            qual = __ldg(reinterpret_cast<const uint32_t *>(tmin4 + psb[p] + (f - pre[p])) + qu) <= tau;
-        }
-        unsigned bal = __ballot_sync(0xffffffffu, qual);
-        while (bal) {
-            // up to four qualifying quarters at a time, their loads in flight together
-            int src[4], nb = 0;
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                src[u] = bal ? __ffs(bal) - 1 : -1;
-                if (bal) {
-                    bal &= bal - 1;
-                    ++nb;
-                }
-            }
-            uint64_t key[4];
-            bool want[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int sl = src[u] < 0 ? 0 : src[u];
-                const int pp = __shfl_sync(0xffffffffu, p, sl);
-                const int64_t slot = g0 + (sl >> 2) - pre[pp];
-                const int i = (sl & 3) * 32 + lane;  // row within the slot
-                const int64_t r0 = slot * 128;
-                const bool ok = u < nb && r0 + i < plen[pp];
-                const uint32_t v = ok ? f2ord(__ldg(scores + (psb[pp] + slot) * 128 + i)) : 0xffffffffu;
-                key[u] = make_key(v, (uint32_t)(plb[pp] + r0 + i));
-                want[u] = ok;
-            }
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                bool w = want[u] && key[u] < wthr;
-                while (true) {
-                    const unsigned b2 = __ballot_sync(0xffffffffu, w);
-                    if (!b2) break;
-                    const int pos = wn + __popc(b2 & ((1u << lane) - 1u));
-                    if (w && pos < SEL_WB) {
-                        W[pos] = key[u];
-                        w = false;
-                    }
-                    wn += __popc(b2);
-                    if (wn <= SEL_WB) break;
-                    // full: keep the best S; keys that did not fit are offered again
-                    __syncwarp();
-                    warp_bitonic_sort(W, SEL_WB, lane);
-                    wthr = W[S - 1];
-                    wn = S;
-                    w = w && key[u] < wthr;
-                    __syncwarp();
-                }
-            }
-        }
-    }
-    // the S best of the buffer: sort it (padded to a power of two)
-    int P = 32;
-    while (P < wn) P <<= 1;
-    for (int i = wn + lane; i < P; i += 32) W[i] = KEY_EMPTY;
-    __syncwarp();
-    warp_bitonic_sort(W, P, lane);
-    const int m = min(S, wn);
-    // exact re-rank; every candidate row prefetched into L2 first
-    const float *qrow = Q + q * dp;
-    {
-        const int lines = (d * 4 + 127) / 128;
-        for (int i = lane; i < m * lines; i += 32)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(X + (int64_t)key_idx(W[i / lines]) * dp + (i % lines) * 32));
-    }
-    for (int r = 0; r < m; r += 2) {
-        int64_t rows[2] = {(int64_t)key_idx(W[r]), r + 1 < m ? (int64_t)key_idx(W[r + 1]) : -1};
-        const int n = r + 1 < m ? 2 : 1;
-        float dd[2];
-        l2sq_warp_rows(qrow, X, dp, d, rows, n, dd, lane);
-        if (lane == 0)
-            for (int u = 0; u < n; ++u) w_rk[warp][r + u] = make_key(__float_as_uint(dd[u]), (uint32_t)ids[rows[u]]);
-    }
-    __syncwarp();
-    WarpTopK<1> F;
-    F.init();
-    uint64_t fthr = KEY_EMPTY;
-    for (int r0 = 0; r0 < S; r0 += 32) {
-        const uint64_t key = (r0 + lane < m) ? w_rk[warp][r0 + lane] : KEY_EMPTY;
-        F.offer(key, fthr, k);
-    }
-    const uint64_t key = F.v[0];
-    const bool e = key == KEY_EMPTY;
-    if (lane < k) {
-        out_idx[q * k + lane] = e ? -1 : (int64_t)key_idx(key);
-        out_dist[q * k + lane] = e ? 0.f : __uint_as_float(key_dist(key));
-    }
-    const int cnt = __popc(__ballot_sync(0xffffffffu, lane < k && !e));
-    if (lane == 0 && out_cnt) out_cnt[q] = cnt;
-}
-
-// ── tensor-core coarse stage ──────────────────────────────────────────────
-// Units of the centroid scan: every query chunk of 256 against every chunk of
-// 128 centroids; aslot[q] = q * nc so the scores land row-major [nq x nc].
-__global__ void coarse_units_kernel(int64_t nq, int nc, TcUnit *__restrict__ units, int64_t *__restrict__ n_units,
-                                    int64_t *__restrict__ aslot) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t nqc = (nq + TC_QCHUNK - 1) / TC_QCHUNK, ncc = (nc + 127) / 128;
-    if (t == 0) *n_units = nqc * ncc;
-    if (t < nq) aslot[t] = t * nc;
-    if (t >= nqc * ncc) return;
-    const int64_t qc = t / ncc, cc = t % ncc;
-    TcUnit u;
-    u.a0 = qc * TC_QCHUNK;
-    u.na = (int32_t)min((int64_t)TC_QCHUNK, nq - u.a0);
-    u.r0 = cc * 128;
-    u.r1 = min((int64_t)nc, u.r0 + 128);
-    u.rbase = 0;
-    u.xrow = u.r0;
-    u.rch = 0;
-    units[t] = u;
 }
 
 constexpr int PROBE_MAX_D = 2048;  // query row staged in shared memory
@@ -1522,50 +1323,22 @@ int ivfl2_search_tc(gn_index *ix, const float *dQ, int64_t nq, int k, int64_t *d
     timing_begin(st, "tc_ivf_kernel");
     GN_TRY(tc_ivf_launch(a, st));
     timing_end(st);
-    // selector: a warp per query when the autotuner chose it (nt = 32; it
-    // measured slower than the block selectors on the 1M x 512 mixture, whose
-    // queries probe ~300 slots each: one warp sweeps them one dependent load
-    // after another), else blocks of nt threads per query
-    const int nsm = dev_info().num_sms;
-    if (np <= 64 && tn.nt == 32) {
-        ivf_tc_select_warp_kernel<<<(unsigned)ceil_div(nq, SELW_WARPS), 32 * SELW_WARPS, 0, st>>>(
+    // selection: as many warps per query as fit the GPU at once, 8 at most (the tuned
+    // nt threads, if set)
+    int nw = 8;
+    while (nw > 1 && nq * nw > (int64_t)dev_info().num_sms * SEL_WARPS) nw /= 2;
+    if (tn.nt) nw = tn.nt / 32;
+    auto sel = [&](auto NWC) {
+        constexpr int NW = decltype(NWC)::value;
+        ivf_tc_select_kernel<NW><<<(unsigned)nq, 32 * NW, 0, st>>>(
             S.scores.as<float>(), S.tmin.as<uint4>(), T.qbound.as<uint32_t>(), T.probes.as<int32_t>(), np,
             T.qslot.as<int64_t>(), T.slot_rel.as<int64_t>(), S.list_off.as<int64_t>(), S.shortlist, dQ,
-            S.vecs.as<float>(), S.d, S.dp, S.ids.as<int32_t>(), nq, k, d_idx, d_dist, d_cnt);
-        GN_CUDA_TRY(cudaGetLastError());
-        return GN_OK;
-    }
-    // B blocks per query: split small batches so that they still fill the GPU
-    int B = 1;
-    const int bmax = tn.bmax ? tn.bmax : 16;
-    if (np <= SEL_PCH)
-        while (B < bmax && nq * B * 2 <= (int64_t)nsm * 4) B *= 2;
-    if (B > 1) {
-        // nq * B <= 4 * SMs here: one size for every small batch
-        GN_TRY(S.sel_part.ensure((size_t)std::max<int64_t>(nq * B, (int64_t)nsm * 4) * S.shortlist * 8));
-        const size_t cap0 = S.sel_done.cap;
-        GN_TRY(S.sel_done.ensure((size_t)std::max<int64_t>(nq, 1024) * 4));
-        if (S.sel_done.cap != cap0) GN_CUDA_TRY(cudaMemsetAsync(S.sel_done.p, 0, S.sel_done.cap, st));
-    }
-    const unsigned blocks = (unsigned)(nq * B);
-    // small batches: 8 warps per query part; large: 4 warps, more queries in flight
-    auto sel = [&](auto NTC) -> int {
-        constexpr int NT = decltype(NTC)::value;
-        static bool carve = false;  // shared memory over L1: the scores are streamed once
-        if (!carve) {
-            GN_CUDA_TRY(cudaFuncSetAttribute(ivf_tc_select_kernel<NT>,
-                                             cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-            carve = true;
-        }
-        ivf_tc_select_kernel<NT><<<blocks, NT, 0, st>>>(
-            S.scores.as<float>(), S.tmin.as<uint4>(), T.qbound.as<uint32_t>(), T.probes.as<int32_t>(), np,
-            T.qslot.as<int64_t>(), T.slot_rel.as<int64_t>(),
-            S.list_off.as<int64_t>(), S.shortlist, dQ, S.vecs.as<float>(), S.d, S.dp, S.ids.as<int32_t>(), nq, k, B,
-            S.sel_part.as<uint64_t>(), S.sel_done.as<int>(), d_idx, d_dist, d_cnt);
-        return GN_OK;
+            S.vecs.as<float>(), S.d, S.dp, S.ids.as<int32_t>(), k, d_idx, d_dist, d_cnt);
     };
-    if (tn.nt == 128 || (tn.nt != 256 && nq * B >= (int64_t)nsm * 8)) GN_TRY(sel(std::integral_constant<int, 128>()));
-    else GN_TRY(sel(std::integral_constant<int, 256>()));
+    if (nw == 8) sel(std::integral_constant<int, 8>());
+    else if (nw == 4) sel(std::integral_constant<int, 4>());
+    else if (nw == 2) sel(std::integral_constant<int, 2>());
+    else sel(std::integral_constant<int, 1>());
     GN_CUDA_TRY(cudaGetLastError());
     return GN_OK;
 }

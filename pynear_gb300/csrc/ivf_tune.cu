@@ -1,19 +1,19 @@
 // ivf_tune.cu — autotuner of the tensor-core IVF engine's launch choices.
 //
-// The tensor-core engine has four launch choices whose best values depend on
+// The tensor-core engine has three launch choices whose best values depend on
 // the batch size, the list-length distribution, the probe width and the GPU:
 //   rc    list rows per work unit of the list scan (256, 1024, 4096): short
 //         units spread a small batch's few lists over all SMs, long ones cut
 //         per-unit overhead;
-//   bmax  most blocks one query's selection is split over (1, 4, 16): splitting
-//         shortens a small batch's critical path, at the price of a merge;
-//   nt    selector threads per query (32, 128, 256): 32 is one warp per query
-//         (no block barriers, for large batches), 128 and 256 a block of that
-//         many threads per query (part);
+//   nt    selector threads per query (32, 128, 256): one warp for batches that
+//         fill the GPU, more for small ones;
 //   qc    queries per list-scan work unit, the MMA's N side (32, 64, 128): the
 //         tile shape; smaller units spread a mid-size batch's lists over more
 //         SMs at the price of more reads of each list's rows.
-// The first three are timed jointly with qc = 128, then qc with the best of them.
+// The first two are timed jointly with qc = 128, then qc with the best of them.  A
+// fourth column of the table, once the most blocks that one query's selection was
+// split over (1 .. 16), is kept for the tables saved with it and has no effect: the
+// selection is no longer split.
 // gn_ivfl2_autotune times every combination on the caller's sample queries,
 // for each batch-size bucket the sample covers ([1,4) [4,16) ... [4096,..)),
 // with CUDA events on the index's stream, and keeps the fastest per bucket in
@@ -27,7 +27,6 @@
 namespace gn {
 
 static const int TUNE_RC[] = {256, 1024, 4096};
-static const int TUNE_BMAX[] = {1, 4, 16};
 static const int TUNE_NT[] = {32, 128, 256};  // 32: one warp per query
 static const int TUNE_QC[] = {32, 64};  // besides the built-in 128
 constexpr int TUNE_COLS = 4;
@@ -65,7 +64,6 @@ extern "C" int gn_ivfl2_autotune(gn_index *ix, const float *queries, int64_t nq,
             cudaEventDestroy(b);
         }
     } ev{e0, e1};
-    const int nsm = dev_info().num_sms;
     for (int b = 0; b < 7; ++b) {
         const int64_t lo = b == 0 ? 1 : ((int64_t)1 << (2 * b));
         const int64_t nb = std::min<int64_t>(TUNE_NQ[b], nmax);
@@ -73,29 +71,25 @@ extern "C" int gn_ivfl2_autotune(gn_index *ix, const float *queries, int64_t nq,
         float best = 0.f;
         IvfL2State::TcTune best_t;
         for (int rc : TUNE_RC)
-            for (int bm : TUNE_BMAX)
-                for (int nt : TUNE_NT) {
-                    // a split the batch never uses would time the same launch again (the
-                    // warp-per-query selector never splits)
-                    if (bm > 1 && (nb * 2 > (int64_t)nsm * 4 || nt == 32)) continue;
-                    S.tune[b].rc = rc;
-                    S.tune[b].bmax = bm;
-                    S.tune[b].nt = nt;
-                    GN_TRY(ivfl2_search_core(ix, dq.as<float>(), nb, (int)k, di.as<int64_t>(), dd.as<float>(),
-                                             dc.as<int64_t>(), st));  // warm-up (sizes the scratch)
-                    GN_CUDA_TRY(cudaEventRecord(e0, st));
-                    for (int r = 0; r < reps; ++r)
-                        GN_TRY(ivfl2_search_core(ix, dq.as<float>(), nb, (int)k, di.as<int64_t>(),
-                                                 dd.as<float>(), dc.as<int64_t>(), st));
-                    GN_CUDA_TRY(cudaEventRecord(e1, st));
-                    GN_CUDA_TRY(cudaEventSynchronize(e1));
-                    float ms = 0.f;
-                    GN_CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
-                    if (best_t.rc == 0 || ms < best) {
-                        best = ms;
-                        best_t = S.tune[b];
-                    }
+            for (int nt : TUNE_NT) {
+                S.tune[b].rc = rc;
+                S.tune[b].bmax = 1;
+                S.tune[b].nt = nt;
+                GN_TRY(ivfl2_search_core(ix, dq.as<float>(), nb, (int)k, di.as<int64_t>(), dd.as<float>(),
+                                         dc.as<int64_t>(), st));  // warm-up (sizes the scratch)
+                GN_CUDA_TRY(cudaEventRecord(e0, st));
+                for (int r = 0; r < reps; ++r)
+                    GN_TRY(ivfl2_search_core(ix, dq.as<float>(), nb, (int)k, di.as<int64_t>(),
+                                             dd.as<float>(), dc.as<int64_t>(), st));
+                GN_CUDA_TRY(cudaEventRecord(e1, st));
+                GN_CUDA_TRY(cudaEventSynchronize(e1));
+                float ms = 0.f;
+                GN_CUDA_TRY(cudaEventElapsedTime(&ms, e0, e1));
+                if (best_t.rc == 0 || ms < best) {
+                    best = ms;
+                    best_t = S.tune[b];
                 }
+            }
         // the tile shape, with the other choices fixed at their best (timed above
         // with the built-in 128 queries per unit)
         for (int qc : TUNE_QC) {

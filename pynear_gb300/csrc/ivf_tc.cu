@@ -83,8 +83,12 @@ __device__ void tc_units_body(int64_t i, const int64_t *__restrict__ item_off, i
 }
 
 // One launch for both: blocks [0, qb_blocks) fill Qb — row pos = the BF16 row
-// of the query of the pair bucket[pos], warp per row, with the pair's slot
-// base and its query's score bound — the rest build the work units.
+// of the query of the pair bucket[pos], with the pair's slot base and its
+// query's score bound — the rest build the work units.  A warp moves QB_ROWS rows
+// together: their loads (pair, then its query's row) are in flight at once, where
+// one row a warp waited out each in turn (114,688 rows of 1 KB: 42 us,
+// 27 here).
+constexpr int QB_ROWS = 4;
 __global__ void qb_units_kernel(const uint4 *__restrict__ q16, int K8, int np, const int64_t *__restrict__ bucket,
                                 const int64_t *__restrict__ boff, int nc, const int64_t *__restrict__ qslot,
                                 const int64_t *__restrict__ slot_rel, uint4 *__restrict__ qb,
@@ -95,14 +99,29 @@ __global__ void qb_units_kernel(const uint4 *__restrict__ q16, int K8, int np, c
                                 TcUnit *__restrict__ units, int64_t *__restrict__ n_units) {
     if (blockIdx.x < qb_blocks) {
         const int lane = threadIdx.x & 31;
-        const int64_t pos = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-        if (pos >= max_pairs || pos >= boff[nc]) return;
-        const int64_t pair = bucket[pos];
-        const int64_t q = pair / np;
-        for (int j = lane; j < K8; j += 32) qb[pos * K8 + j] = q16[q * K8 + j];
-        if (lane == 0) {
-            aslot[pos] = qslot[q] + slot_rel[pair];
-            abound[pos] = qbound[q];
+        const int64_t pos0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * QB_ROWS;
+        const int64_t left = min(max_pairs, boff[nc]) - pos0;
+        if (left <= 0) return;
+        const int n = (int)min((int64_t)QB_ROWS, left);
+        int64_t q = 0;
+        if (lane < n) {
+            const int64_t pair = bucket[pos0 + lane];
+            q = pair / np;
+            aslot[pos0 + lane] = qslot[q] + slot_rel[pair];
+            abound[pos0 + lane] = qbound[q];
+        }
+        const uint4 *src[QB_ROWS];
+#pragma unroll
+        for (int r = 0; r < QB_ROWS; ++r) src[r] = q16 + __shfl_sync(0xffffffffu, q, r) * K8;
+        uint4 *dst = qb + pos0 * K8;
+#pragma unroll 2
+        for (int j = lane; j < K8; j += 32) {
+            uint4 v[QB_ROWS];
+#pragma unroll
+            for (int r = 0; r < QB_ROWS; ++r) v[r] = __ldg(src[r] + j);
+#pragma unroll
+            for (int r = 0; r < QB_ROWS; ++r)
+                if (r < n) dst[(int64_t)r * K8 + j] = v[r];
         }
         return;
     }
@@ -276,10 +295,10 @@ struct SelWarp {
 };
 
 // A bound with at least S of the warp's values (R per lane) at or below it, and at
-// most S / 8 more unless equal values leave no such bound: bit by bit from the
+// most `more` others unless equal values leave no such bound: bit by bit from the
 // highest in which the values differ.
 template <int R>
-__device__ __forceinline__ uint32_t warp_kth(const uint32_t (&v)[R], int S) {
+__device__ __forceinline__ uint32_t warp_kth(const uint32_t (&v)[R], int S, int more) {
     uint32_t any = 0u, all = 0xffffffffu;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
@@ -298,7 +317,7 @@ __device__ __forceinline__ uint32_t warp_kth(const uint32_t (&v)[R], int S) {
 #pragma unroll
         for (int i = 0; i < R; ++i) c += v[i] < trial;
         c = __reduce_add_sync(0xffffffffu, c);
-        if (c >= S && c <= S + (S >> 3)) return trial - 1u;
+        if (c >= S && c <= S + more) return trial - 1u;
         if (c < S) kth = trial;
     }
     return kth;
@@ -337,7 +356,7 @@ __device__ __forceinline__ void sel_group(SelWarp &W, const uint4 *__restrict__ 
         v[4 * u + 2] = m.z;
         v[4 * u + 3] = m.w;
     }
-    if (first && 4 * min(all - g0, SEL_GROUP) >= S) tau = min(tau, warp_kth<4 * U>(v, S));
+    if (first && 4 * min(all - g0, SEL_GROUP) >= S) tau = min(tau, warp_kth<4 * U>(v, S, S / 8));
     int n = 0;  // listed
     __syncwarp();
 #pragma unroll
@@ -538,6 +557,20 @@ __global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW) ivf_tc_select_kernel(
     if (lane == 0 && out_cnt) out_cnt[q] = cnt;
 }
 
+// Warps per query (8, 4, 2 or 1) of the kernels that give a query a block: the most
+// that fit the GPU at once, SEL_WARPS per SM, so that a small batch has its query's work
+// split and a large one has no more warps than can be resident.
+template <typename Launch>
+static void warps_per_query(int64_t nq, int fixed, Launch &&launch) {
+    int nw = 8;
+    while (nw > 1 && nq * nw > (int64_t)dev_info().num_sms * SEL_WARPS) nw /= 2;
+    if (fixed) nw = fixed;
+    if (nw == 8) launch(std::integral_constant<int, 8>());
+    else if (nw == 4) launch(std::integral_constant<int, 4>());
+    else if (nw == 2) launch(std::integral_constant<int, 2>());
+    else launch(std::integral_constant<int, 1>());
+}
+
 // ── tensor-core coarse stage ──────────────────────────────────────────────
 // Units of the centroid scan: every query chunk of 256 against every chunk of
 // 128 centroids; aslot[q] = q * nc so the scores land row-major [nq x nc].
@@ -560,83 +593,7 @@ __global__ void coarse_units_kernel(int64_t nq, int nc, TcUnit *__restrict__ uni
     units[t] = u;
 }
 
-// The S smallest of a key multiset held in shared memory, by the whole block
-// (radix select on 8-bit digits from the top, stopping as soon as the
-// boundary digit is taken whole).  The keys are keys[w * WB + i], i < cnt[w],
-// one region per warp (warp w reads region w).  The S smallest (all, if
-// fewer) go to out[], in no particular order; returns how many.  Keys are
-// unique, so exactly min(S, total) are selected.
-template <int NT>
-__device__ int block_radix_select(const uint64_t *keys, int WB, const int *cnt, int S, uint64_t *out, int *hist,
-                                  int *sh) {
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint64_t *mine = keys + (size_t)warp * WB;
-    const int nmine = cnt[warp];
-    uint64_t prefix = 0, mask = 0;
-    int need = S;
-    bool all = false;  // keys matching the prefix are all taken
-    for (int shift = 56; shift >= 0; shift -= 8) {
-        for (int i = t; i < 256; i += NT) hist[i] = 0;
-        __syncthreads();
-        for (int i = lane; i < nmine; i += 32) {
-            const uint64_t k = mine[i];
-            if ((k & mask) == prefix) atomicAdd(&hist[(k >> shift) & 255], 1);
-        }
-        __syncthreads();
-        if (warp == 0) {
-            int h[8], sum = 0;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                h[e] = hist[lane * 8 + e];
-                sum += h[e];
-            }
-            int inc = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += v;
-            }
-            int before = inc - sum;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                if (before < need && need <= before + h[e]) {
-                    sh[0] = lane * 8 + e;
-                    sh[1] = before;
-                }
-                before += h[e];
-            }
-            if (lane == 31) sh[2] = inc;  // keys matching the prefix
-        }
-        __syncthreads();
-        if (shift == 56 && sh[2] <= S) {  // no more keys than S: take them all
-            all = true;
-            break;
-        }
-        const int dg = sh[0];
-        need -= sh[1];
-        prefix |= (uint64_t)dg << shift;
-        mask |= (uint64_t)0xff << shift;
-        const bool whole = hist[dg] == need;
-        __syncthreads();
-        if (whole) {
-            all = true;
-            break;
-        }
-    }
-    // take every key below the prefix and the keys equal to it (all of them,
-    // or the single key left after all eight digits)
-    if (t == 0) sh[3] = 0;
-    __syncthreads();
-    for (int i = lane; i < nmine; i += 32) {
-        const uint64_t k = mine[i];
-        const uint64_t km = k & mask;
-        if (km < prefix || (km == prefix && (all || need > 0))) out[atomicAdd(&sh[3], 1)] = k;
-    }
-    __syncthreads();
-    return sh[3];
-}
-
-constexpr int PROBE_MAX_D = 2048;  // query row staged in shared memory
+constexpr int PROBE_MAX_D = 2048;
 
 // The query's score bound for the list scan, from b = this thread's probed
 // candidate list's distance bound (+inf for threads without one): with D the
@@ -647,8 +604,7 @@ constexpr int PROBE_MAX_D = 2048;  // query row staged in shared memory
 // (both operands rounded to 8 significant bits; 2^-9 of sum |q_i x_i| allowed
 // for the tensor core's accumulation, far above FP32's), so the bound adds
 // 0.03 |q| xmax + 2^-12 (xmax + |q|)^2 and rounds every other term outwards.
-// Block-wide (all threads call it); thread 0 writes the ordered bound, or all
-// ones when there is none.
+// All ones when there is none.
 __device__ __forceinline__ uint32_t probe_bound_key(float D, float qn, float xmax) {
     const float qa = sqrtf(qn);
     const float B = D * (1.f + 1.f / 1024.f) - qn * (1.f - 1.f / 1024.f) + 0.03f * qa * xmax +
@@ -656,147 +612,188 @@ __device__ __forceinline__ uint32_t probe_bound_key(float D, float qn, float xma
     return (B < INFINITY && B == B) ? f2ord(B) : 0xffffffffu;
 }
 
-__device__ __forceinline__ void write_probe_bound(float b, const float *sqr, int d, float xmax,
-                                                  uint32_t *__restrict__ qbound, int64_t q, float *red) {
-    const int j = threadIdx.x, lane = j & 31, warp = j >> 5;
+// |q|^2 by one warp
+__device__ __forceinline__ float warp_sqnorm(const float *__restrict__ q, int d, int lane) {
+    float s = 0.f;
+    for (int t = lane; t < d; t += 32) s = fmaf(q[t], q[t], s);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) b = fminf(b, __shfl_xor_sync(0xffffffffu, b, o));
-    if (warp == 2) {
-        float s = 0.f;
-        for (int t = lane; t < d; t += 32) s = fmaf(sqr[t], sqr[t], s);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) red[2] = s;
-    }
-    if (lane == 0 && warp < 2) red[warp] = b;
-    __syncthreads();
-    if (j == 0) qbound[q] = probe_bound_key(fminf(red[0], red[1]), red[2], xmax);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
 }
 
-// Per query (block of 256 threads): the 64 best centroids by BF16 score, their
+// The PROBER_CAND smallest keys (score, centroid) of a query's nc >= PROBER_CAND scores
+// into best, by one warp: a threshold out of 32 R group minima held in registers
+// (every 32 R-th score a group), then the best of the scores at or below it.
+template <int R>
+__device__ __forceinline__ void probe_candidates(const float *__restrict__ sq, int nc, uint64_t *buf, uint64_t *best,
+                                                 int lane) {
+    constexpr int NC = PROBER_CAND;
+    uint32_t v[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        v[i] = 0xffffffffu;
+        if (i * 32 < nc && i * 32 + lane < nc) v[i] = f2ord(__ldg(sq + i * 32 + lane));
+    }
+#pragma unroll 1
+    for (int g = 32 * R; g < nc; g += 32 * R)
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+            if (g + i * 32 + lane < nc) v[i] = min(v[i], f2ord(__ldg(sq + g + i * 32 + lane)));
+    uint32_t tau = warp_kth<R>(v, NC, NC / 2);
+    int wn = 0;
+#pragma unroll 1
+    for (int g = 0; g < nc; g += 32 * R)
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const int c = g + i * 32 + lane;
+            if (g + i * 32 >= nc) break;
+            const uint32_t bits = nc <= 32 * R ? v[i] : c < nc ? f2ord(__ldg(sq + c)) : 0xffffffffu;
+            const bool in = c < nc && bits <= tau;
+            const unsigned b = __ballot_sync(0xffffffffu, in);
+            if (b == 0) continue;
+            if (in) buf[wn + __popc(b & ((1u << lane) - 1u))] = make_key(bits, (uint32_t)c);
+            wn += __popc(b);
+            if (wn > SEL_BUF - 32) {
+                tau = min(tau, list_cut<SEL_BUF / 32>(buf, wn, NC));
+                wn = NC;
+            }
+        }
+    __syncwarp();
+    const int ntop = warp_best(buf, wn, NC, best);
+    for (int i = ntop + lane; i < NC; i += 32) best[i] = KEY_EMPTY;
+    __syncwarp();
+}
+
+// Per query (block of NW warps): the 64 best centroids by BF16 score, their
 // exact squared distances (FP32), sorted nearest first; then either the first
 // np of them (fixed probing) or the learned prober's choice (MLP fused here).
-template <bool MLP>
-__global__ void __launch_bounds__(256) coarse_probe_kernel(const float *__restrict__ scores, int nc, int ncp2,
-                                                           const float *__restrict__ Q, int d, int dp,
-                                                           const float *__restrict__ C, int64_t nq, int np,
-                                                           ProberWeights w, float logit_tau,
-                                                           int32_t *__restrict__ probes,
-                                                           int32_t *__restrict__ nprobed,
-                                                           const float *__restrict__ rho, int shortlist, float xmax,
-                                                           uint32_t *__restrict__ qbound, float *__restrict__ h1_out,
-                                                           int32_t *__restrict__ cand_out,
-                                                           float *__restrict__ cb_out, float *__restrict__ qn_out) {
+// The candidates are the 64 smallest keys (BF16 score, centroid): every warp
+// counts for itself, so that no barrier stands between the scores and the
+// distances; these are split over the warps, four candidates at a time.  Measured with
+// 1,024 centroids of 512 dimensions: 88 us for 4,096 queries with a block-wide radix
+// select, 49 here (their 537 MB of centroid rows come from L2).
+template <bool MLP, int NW>
+__global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW)
+    coarse_probe_kernel(const float *__restrict__ scores, int nc, const float *__restrict__ Q, int d, int dp,
+                        const float *__restrict__ C, int np, ProberWeights w, float logit_tau,
+                        int32_t *__restrict__ probes, int32_t *__restrict__ nprobed,
+                        const float *__restrict__ rho, int shortlist, float xmax,
+                        uint32_t *__restrict__ qbound, float *__restrict__ h1_out, int32_t *__restrict__ cand_out,
+                        float *__restrict__ cb_out, float *__restrict__ qn_out) {
     constexpr int NC = PROBER_CAND, H = PROBER_HIDDEN;
     static_assert(H == 256 && NC == 64, "warp-per-row MLP layout: 32 lanes x 8 weights, 8 warps x 8 candidates");
-    __shared__ int32_t sc[NC];
-    __shared__ float sd[NC], sf[NC], sz[NC], sb[NC], sred[4];
-    __shared__ __align__(16) float sh1[H], sh2[H];
-    __shared__ int s_cnt0;
-    __shared__ __align__(16) float sqr[PROBE_MAX_D];
-    __shared__ int hist[256], rsh[4], rcnt[8];
-    __shared__ uint64_t top[NC];
-    extern __shared__ uint64_t skeys[];  // next_pow2(nc) keys, 8 regions of next_pow2(nc) / 8
+    static_assert(!MLP || NW == 8, "one thread per hidden unit");
+    __shared__ uint64_t buf[NW][SEL_BUF], best[NW][NC];
+    __shared__ float sd[NC];
     const int64_t q = blockIdx.x;
     const int j = threadIdx.x, lane = j & 31, warp = j >> 5;
-    const float *sq = scores + q * nc;
-    for (int t = j; t < d; t += 256) sqr[t] = Q[q * dp + t];
-    // the 64 smallest keys (BF16 score, centroid) are the candidates: radix
-    // select over the 8 warps' regions
-    const int wb = ncp2 >> 3;
-    for (int c = j; c < nc; c += 256) skeys[c] = make_key(f2ord(sq[c]), (uint32_t)c);
-    if (j < 8) rcnt[j] = max(0, min(wb, nc - j * wb));
-    __syncthreads();
-    const int ntop = block_radix_select<256>(skeys, wb, rcnt, NC, top, hist, rsh);
-    if (j < NC) sc[j] = j < ntop ? (int32_t)key_idx(top[j]) : -1;
-    __syncthreads();
-    {   // exact squared distances: one warp per candidate (eight per warp), so
-        // that each load instruction reads 512 contiguous bytes of a centroid row
-        const float4 *qr = reinterpret_cast<const float4 *>(sqr);
+    const float *sq = scores + q * nc, *qrow = Q + q * dp;
+    if (nc <= 512) probe_candidates<16>(sq, nc, buf[warp], best[warp], lane);
+    else probe_candidates<32>(sq, nc, buf[warp], best[warp], lane);
+    {   // exact squared distances, four candidates together: each load instruction
+        // reads 512 contiguous bytes of a centroid row
+        const float4 *qr = reinterpret_cast<const float4 *>(qrow);
         const int n4 = d >> 2;
+#pragma unroll 1
+        for (int i0 = 4 * warp; i0 < NC; i0 += 4 * NW) {
+            const float *cr[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint64_t key = best[warp][i0 + u];
+                cr[u] = C + (int64_t)(key == KEY_EMPTY ? 0 : key_idx(key)) * dp;
+            }
+            float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 2
-        for (int i = warp; i < NC; i += 8) {
-            const int c = sc[i];  // warp-uniform
-            float s0 = 0.f, s1 = 0.f;
-            if (c >= 0) {
-                const float4 *cr = reinterpret_cast<const float4 *>(C + (int64_t)c * dp);
-                for (int t = lane; t < n4; t += 32) {
-                    const float4 a = __ldg(cr + t), b = qr[t];
-                    const float e0 = b.x - a.x, e1 = b.y - a.y, e2 = b.z - a.z, e3 = b.w - a.w;
-                    s0 = fmaf(e0, e0, s0);
-                    s1 = fmaf(e1, e1, s1);
-                    s0 = fmaf(e2, e2, s0);
-                    s1 = fmaf(e3, e3, s1);
-                }
-                for (int t = (n4 << 2) + lane; t < d; t += 32) {  // d % 4 tail
-                    const float e = sqr[t] - C[(int64_t)c * dp + t];
-                    s0 = fmaf(e, e, s0);
+            for (int t = lane; t < n4; t += 32) {
+                const float4 b = __ldg(qr + t);
+                float4 a[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) a[u] = __ldg(reinterpret_cast<const float4 *>(cr[u]) + t);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float e0 = b.x - a[u].x, e1 = b.y - a[u].y, e2 = b.z - a[u].z, e3 = b.w - a[u].w;
+                    s0[u] = fmaf(e0, e0, s0[u]);
+                    s1[u] = fmaf(e1, e1, s1[u]);
+                    s0[u] = fmaf(e2, e2, s0[u]);
+                    s1[u] = fmaf(e3, e3, s1[u]);
                 }
             }
-            float sum = s0 + s1;
+            for (int t = (n4 << 2) + lane; t < d; t += 32)  // d % 4 tail
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-            if (lane == 0) sd[i] = sum;
+                for (int u = 0; u < 4; ++u) {
+                    const float e = qrow[t] - cr[u][t];
+                    s0[u] = fmaf(e, e, s0[u]);
+                }
+            // the four sums over the lanes: lanes 0, 8, 16, 24 end with candidates 0, 2, 1, 3's
+            const bool h16 = lane & 16, h8 = lane & 8;
+            float x = s0[0] + s1[0], y = s0[1] + s1[1];
+            float p = (h16 ? y : x) + __shfl_xor_sync(0xffffffffu, h16 ? x : y, 16);
+            x = s0[2] + s1[2];
+            y = s0[3] + s1[3];
+            const float p2 = (h16 ? y : x) + __shfl_xor_sync(0xffffffffu, h16 ? x : y, 16);
+            p = (h8 ? p2 : p) + __shfl_xor_sync(0xffffffffu, h8 ? p : p2, 8);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+            if ((lane & 7) == 0) sd[i0 + (h8 ? 2 : 0) + (h16 ? 1 : 0)] = p;
         }
     }
-    __syncthreads();
+    __shared__ float s_qn;
+    if (warp == NW - 1 && !MLP && qbound) {
+        const float qn = warp_sqnorm(qrow, d, lane);
+        if (lane == 0) s_qn = qn;
+    }
+    if (NW > 1) __syncthreads();
+    else __syncwarp();
+    __shared__ int32_t sc[MLP ? NC : 1];
+    __shared__ float sf[MLP ? NC : 1], sb[MLP ? NC : 1];
     if (warp == 0) {
-        // sort the 64 (exact distance, centroid) keys in registers: lane l
-        // holds positions l and l + 32 (bitonic network, shuffles only)
-        uint64_t r2[2];
+        uint64_t key[2];  // sorted: lane l holds positions l and l + 32
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int i = h * 32 + lane;
-            r2[h] = sc[i] >= 0 ? make_key(__float_as_uint(sd[i]), (uint32_t)sc[i]) : KEY_EMPTY;
+            const uint64_t c = best[0][i];
+            key[h] = c == KEY_EMPTY ? KEY_EMPTY : make_key(__float_as_uint(sd[i]), key_idx(c));
         }
+        warp_sort<2>(key);
+        const float d1 = __shfl_sync(0xffffffffu, __uint_as_float(key_dist(key[0])), 0);
+        float near = INFINITY;
 #pragma unroll
-        for (int size = 2; size <= NC; size <<= 1)
-#pragma unroll
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                if (stride == 32) {
-                    const uint64_t a = r2[0], b = r2[1];
-                    r2[0] = a < b ? a : b;
-                    r2[1] = a < b ? b : a;
-                } else {
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const int i = h * 32 + lane;
-                        const uint64_t y = __shfl_xor_sync(0xffffffffu, r2[h], stride);
-                        const bool lower = (i & stride) == 0, asc = (i & size) == 0;
-                        const bool take_min = lower == asc;
-                        r2[h] = take_min ? (r2[h] < y ? r2[h] : y) : (r2[h] < y ? y : r2[h]);
-                    }
+        for (int h = 0; h < 2; ++h) {
+            const int i = h * 32 + lane;
+            const bool e = key[h] == KEY_EMPTY;
+            const int32_t c = e ? -1 : (int32_t)key_idx(key[h]);
+            // bound on the squared distance of the query's shortlist-th nearest row if
+            // this list is probed: its `shortlist` rows nearest the centroid lie within
+            // rho of it, hence within |q - c| + rho of the query
+            float b = INFINITY;
+            if (qbound && !e) {
+                const float r = rho[(size_t)c * IVF_RHO + shortlist - 1];
+                if (r < INFINITY) {
+                    const float t = sqrtf(__uint_as_float(key_dist(key[h])) * (1.f + 1.f / 1024.f)) + r;
+                    b = t * t;
                 }
             }
-        skeys[lane] = r2[0];
-        skeys[lane + 32] = r2[1];
-    }
-    __syncthreads();
-    if (j < NC) {
-        const uint64_t k = skeys[j];
-        const bool e = k == KEY_EMPTY;
-        const float d1 = __uint_as_float(key_dist(skeys[0]));
-        sc[j] = e ? -1 : (int32_t)key_idx(k);
-        sf[j] = e ? 0.f : fmaxf(0.f, 1.f - (__uint_as_float(key_dist(k)) - d1) / fmaxf(d1, 1e-12f));
-        // bound on the squared distance of the query's shortlist-th nearest row if
-        // this list is probed: its `shortlist` rows nearest the centroid lie within
-        // rho of it, hence within |q - c| + rho of the query
-        float b = INFINITY;
-        if (qbound && !e) {
-            const float r = rho[(size_t)key_idx(k) * IVF_RHO + shortlist - 1];
-            if (r < INFINITY) {
-                const float t = sqrtf(__uint_as_float(key_dist(k)) * (1.f + 1.f / 1024.f)) + r;
-                b = t * t;
+            if (MLP) {
+                sc[i] = c;
+                sf[i] = e ? 0.f
+                          : fmaxf(0.f, 1.f - (__uint_as_float(key_dist(key[h])) - d1) / fmaxf(d1, 1e-12f));
+                sb[i] = b;
+            } else if (i < np) {
+                probes[q * np + i] = c;
+                near = fminf(near, b);
             }
         }
-        sb[j] = b;
+        if (!MLP && qbound) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) near = fminf(near, __shfl_xor_sync(0xffffffffu, near, o));
+            if (lane == 0) qbound[q] = probe_bound_key(near, s_qn, xmax);
+        }
     }
+    if (!MLP) return;
+    __shared__ float sz[MLP ? NC : 1], sred[4];
+    __shared__ __align__(16) float sh1[MLP ? H : 4], sh2[MLP ? H : 4];
+    __shared__ int s_cnt0;
     __syncthreads();
-    if (!MLP) {
-        if (j < np) probes[q * np + j] = sc[j];
-        if (qbound) write_probe_bound(j < np ? sb[j] : INFINITY, sqr, d, xmax, qbound, q, sred);
-        return;
-    }
     const __nv_bfloat16 *W1 = reinterpret_cast<const __nv_bfloat16 *>(w.W1);
     const __nv_bfloat16 *W2 = reinterpret_cast<const __nv_bfloat16 *>(w.W2);
     const __nv_bfloat16 *W3 = reinterpret_cast<const __nv_bfloat16 *>(w.W3);
@@ -819,10 +816,7 @@ __global__ void __launch_bounds__(256) coarse_probe_kernel(const float *__restri
             cb_out[q * NC + j] = sb[j];
         }
         if (warp == 2) {
-            float qs = 0.f;
-            for (int t = lane; t < d; t += 32) qs = fmaf(sqr[t], sqr[t], qs);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) qs += __shfl_xor_sync(0xffffffffu, qs, o);
+            const float qs = warp_sqnorm(qrow, d, lane);
             if (lane == 0) qn_out[q] = qs;
         }
         return;
@@ -920,7 +914,18 @@ __global__ void __launch_bounds__(256) coarse_probe_kernel(const float *__restri
             if (lane == 0 && nprobed) nprobed[q] = total;
         }
     }
-    if (qbound) write_probe_bound(keep ? sb[i] : INFINITY, sqr, d, xmax, qbound, q, sred);
+    if (qbound) {
+        float b = keep ? sb[i] : INFINITY;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) b = fminf(b, __shfl_xor_sync(0xffffffffu, b, o));
+        if (lane == 0 && warp < 2) sred[warp] = b;
+        if (warp == 2) {
+            const float qs = warp_sqnorm(qrow, d, lane);
+            if (lane == 0) sred[2] = qs;
+        }
+        __syncthreads();
+        if (j == 0) qbound[q] = probe_bound_key(fminf(sred[0], sred[1]), sred[2], xmax);
+    }
 }
 
 // Layers 2 and 3 of the prober and the probe choice for MLP_QB queries per
@@ -1097,12 +1102,6 @@ static int ivfl2_probes_tc(gn_index *ix, const float *dQ, int64_t nq, int *np_ou
     a.next_unit = S.sched.as<unsigned long long>() + 0;
     a.grid = (int)std::min<int64_t>(dev_info().num_sms, units);
     GN_TRY(tc_ivf_launch(a, st));
-    const int ncp2 = (int)next_pow2(S.nc);
-    const size_t ksm = (size_t)ncp2 * 8;
-    if (ksm > 48 * 1024) {
-        GN_CUDA_TRY(cudaFuncSetAttribute(coarse_probe_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ksm));
-        GN_CUDA_TRY(cudaFuncSetAttribute(coarse_probe_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ksm));
-    }
     ProberWeights w;
     float *h1 = nullptr, *cbnd = nullptr, *qnv = nullptr;
     int32_t *cand = nullptr;
@@ -1119,22 +1118,22 @@ static int ivfl2_probes_tc(gn_index *ix, const float *dQ, int64_t nq, int *np_ou
             cbnd = T.mcb.as<float>();
             qnv = T.mqn.as<float>();
         }
-        coarse_probe_kernel<true><<<(unsigned)nq, 256, ksm, st>>>(S.cscores.as<float>(), S.nc, ncp2, dQ, S.d, S.dp,
-                                                               S.cent.as<float>(), nq, np, w, S.prober_tau,
-                                                               T.probes.as<int32_t>(), T.nprobed.as<int32_t>(),
-                                                               S.rho.as<float>(), S.shortlist, S.xmax,
-                                                               T.qbound.as<uint32_t>(), h1, cand, cbnd, qnv);
+        coarse_probe_kernel<true, 8><<<(unsigned)nq, 256, 0, st>>>(
+            S.cscores.as<float>(), S.nc, dQ, S.d, S.dp, S.cent.as<float>(), np, w, S.prober_tau,
+            T.probes.as<int32_t>(), T.nprobed.as<int32_t>(), S.rho.as<float>(), S.shortlist, S.xmax,
+            T.qbound.as<uint32_t>(), h1, cand, cbnd, qnv);
         if (h1)
             mlp_probe_kernel<<<(unsigned)ceil_div(nq, MLP_QB), 256, 0, st>>>(
                 h1, cand, cbnd, qnv, nq, w, S.prober_tau, S.xmax, T.probes.as<int32_t>(), T.nprobed.as<int32_t>(),
                 T.qbound.as<uint32_t>());
     } else {
-        coarse_probe_kernel<false><<<(unsigned)nq, 256, ksm, st>>>(S.cscores.as<float>(), S.nc, ncp2, dQ, S.d, S.dp,
-                                                                S.cent.as<float>(), nq, np, w, 0.f,
-                                                                T.probes.as<int32_t>(), nullptr,
-                                                                S.rho.as<float>(), S.shortlist, S.xmax,
-                                                                T.qbound.as<uint32_t>(), nullptr, nullptr, nullptr,
-                                                                nullptr);
+        warps_per_query(nq, 0, [&](auto NWC) {
+            constexpr int NW = decltype(NWC)::value;
+            coarse_probe_kernel<false, NW><<<(unsigned)nq, 32 * NW, 0, st>>>(
+                S.cscores.as<float>(), S.nc, dQ, S.d, S.dp, S.cent.as<float>(), np, w, 0.f, T.probes.as<int32_t>(),
+                nullptr, S.rho.as<float>(), S.shortlist, S.xmax, T.qbound.as<uint32_t>(), nullptr, nullptr, nullptr,
+                nullptr);
+        });
     }
     GN_CUDA_TRY(cudaGetLastError());
     return GN_OK;
@@ -1283,7 +1282,7 @@ int ivfl2_search_tc(gn_index *ix, const float *dQ, int64_t nq, int k, int64_t *d
     const int64_t max_units = (ceil_div(npairs, qch) + S.nc) * (ceil_div(maxlen, 256) + 1);
     GN_TRY(S.units.ensure((size_t)max_units * sizeof(TcUnit)));
     GN_TRY(S.nunits.ensure(8));
-    const unsigned qb_blocks = (unsigned)ceil_div(npairs, 8);
+    const unsigned qb_blocks = (unsigned)ceil_div(npairs, 8 * QB_ROWS);
     qb_units_kernel<<<qb_blocks + (unsigned)ceil_div(max_units, 256), 256, 0, st>>>(
         S.q16.as<uint4>(), S.K / 8, np, T.bucket.as<int64_t>(), T.boff.as<int64_t>(), S.nc, T.qslot.as<int64_t>(),
         T.slot_rel.as<int64_t>(), S.qb.as<uint4>(), S.aslot.as<int64_t>(), T.qbound.as<uint32_t>(),
@@ -1323,22 +1322,14 @@ int ivfl2_search_tc(gn_index *ix, const float *dQ, int64_t nq, int k, int64_t *d
     timing_begin(st, "tc_ivf_kernel");
     GN_TRY(tc_ivf_launch(a, st));
     timing_end(st);
-    // selection: as many warps per query as fit the GPU at once, 8 at most (the tuned
-    // nt threads, if set)
-    int nw = 8;
-    while (nw > 1 && nq * nw > (int64_t)dev_info().num_sms * SEL_WARPS) nw /= 2;
-    if (tn.nt) nw = tn.nt / 32;
-    auto sel = [&](auto NWC) {
+    // selection (the tuned nt threads per query, if set)
+    warps_per_query(nq, tn.nt / 32, [&](auto NWC) {
         constexpr int NW = decltype(NWC)::value;
         ivf_tc_select_kernel<NW><<<(unsigned)nq, 32 * NW, 0, st>>>(
             S.scores.as<float>(), S.tmin.as<uint4>(), T.qbound.as<uint32_t>(), T.probes.as<int32_t>(), np,
             T.qslot.as<int64_t>(), T.slot_rel.as<int64_t>(), S.list_off.as<int64_t>(), S.shortlist, dQ,
             S.vecs.as<float>(), S.d, S.dp, S.ids.as<int32_t>(), k, d_idx, d_dist, d_cnt);
-    };
-    if (nw == 8) sel(std::integral_constant<int, 8>());
-    else if (nw == 4) sel(std::integral_constant<int, 4>());
-    else if (nw == 2) sel(std::integral_constant<int, 2>());
-    else sel(std::integral_constant<int, 1>());
+    });
     GN_CUDA_TRY(cudaGetLastError());
     return GN_OK;
 }

@@ -85,7 +85,8 @@ __device__ __forceinline__ bool kpp_last_block(unsigned *done) {
 }
 
 // ── float seeding ─────────────────────────────────────────────────────────
-// One launch per k-means++ draw: every block lowers its chunk's min_sq by the
+// One launch per k-means++ draw, for rows past the SMs' shared memory (see
+// kpp_seed_kernel for the others): every block lowers its chunk's min_sq by the
 // distances to the newest centroid (row ci - 1 of C) and sums the chunk in
 // double; the last block to finish draws centroid ci and copies its row.
 //
@@ -274,6 +275,352 @@ __global__ void __launch_bounds__(KPP_NT) kpp_kernel(const float *__restrict__ X
     for (int j = t; j < dp; j += KPP_NT) C[ci * dp + j] = X[ch * dp + j];
 }
 
+// ── seeding in one launch ─────────────────────────────────────────────────
+// All the draws of a k-means++ whose rows fit the SMs' shared memory: one
+// cooperative launch, a block per SM, which keeps its rows and their distances
+// there, so that a draw reads nothing but the newest centroid's row.  Between the
+// blocks two words travel per draw: every block's sum, which all of them read to
+// find the block that holds the point, and that block's row number.  Each word
+// carries its draw's tag and is polled directly (no counter, no fence: nothing
+// else is handed over), in a slot per parity: a block writes draw e + 2's sum only
+// after every block has written e + 1's, hence read e's.
+// What bounds a draw is the chain of these two round trips and the scans between
+// them, so the sums are 64-bit integers (an FP64 addition's latency is about 140
+// clocks here) of 16 or 32 rows each, left by the warps that made the distances.
+// Measured: 15 us a draw for 100k x 64 rows as one launch each (9.4 us for 200k x 32
+// bytes), 5.0 us here (3.9 us).
+constexpr int SEED_NT = 1024;
+constexpr int SEED_SPAN = 8;                   // block sums per lane: at most 32 * SEED_SPAN blocks
+constexpr unsigned SEED_SPINS = 1u << 22;      // polls before a wait gives up (seconds)
+constexpr size_t SEED_SMEM_MAX = 222 * 1024;   // dynamic shared memory of a block
+constexpr int SEED_TAG = 40;                   // row words: draw << SEED_TAG | row
+constexpr unsigned long long SEED_AGAIN = 1ull << 39;  // row word: the serial rule decides
+
+__device__ __forceinline__ unsigned long long seed_load(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void seed_store(unsigned long long *p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+// Poll the row word of draw ci; false (and *err set) when the limit runs out.
+__device__ __forceinline__ bool seed_wait(const unsigned long long *p, int ci, unsigned long long *word, int *err,
+                                          unsigned limit = SEED_SPINS) {
+    for (unsigned i = 0; i < limit; ++i) {
+        *word = seed_load(p);
+        if (*word >> SEED_TAG == (unsigned)ci) return true;
+    }
+    *reinterpret_cast<volatile int *>(err) = 1;
+    return false;
+}
+// All G blocks' words (value << 2 | ci & 3) of draw ci, by one warp: polled together
+// (five loads of a warp in flight, where one word after another took a round trip
+// each), then handed over through shared memory: lane l gets values l * span .. in v.
+__device__ __forceinline__ bool seed_gather(const unsigned long long *words, int G, int ci,
+                                            unsigned long long *s_words, unsigned long long (&v)[SEED_SPAN],
+                                            int *err) {
+    const int lane = threadIdx.x & 31, span = (G + 31) / 32;
+    const unsigned long long tag = ci & 3;
+    bool ok = false;
+#pragma unroll
+    for (int i = 0; i < SEED_SPAN; ++i) v[i] = ~tag;  // not yet there
+    // all blocks polling the same ten lines delay the words' own way there: 8.6 us a
+    // draw without this pause, 5.0 with it (100 to 600 ns made no difference)
+    __nanosleep(300);
+    for (unsigned tries = 0; !ok && tries < SEED_SPINS; ++tries) {
+#pragma unroll
+        for (int i = 0; i < SEED_SPAN; ++i)
+            if (i < span && i * 32 + lane < G && (v[i] & 3) != tag) v[i] = seed_load(words + i * 32 + lane);
+        ok = true;
+#pragma unroll
+        for (int i = 0; i < SEED_SPAN; ++i)
+            if (i < span && i * 32 + lane < G) ok = ok && (v[i] & 3) == tag;
+        ok = __all_sync(0xffffffffu, ok);
+    }
+    if (!ok) *reinterpret_cast<volatile int *>(err) = 1;
+#pragma unroll
+    for (int i = 0; i < SEED_SPAN; ++i)
+        if (i < span && i * 32 + lane < G) s_words[i * 32 + lane] = v[i] >> 2;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < SEED_SPAN; ++i) v[i] = i < span && lane * span + i < G ? s_words[lane * span + i] : 0ull;
+    __syncwarp();
+    return ok;
+}
+// Inclusive scan over a warp.
+__device__ __forceinline__ unsigned long long seed_scan(unsigned long long v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += y;
+    }
+    return v;
+}
+// One draw, by one warp of every block: s_group holds the sums of the block's rows,
+// GROUP at a time, value(i) is row i's.  aim(total, &target, &band, &word) says what is
+// looked for, the first row whose running sum reaches target, and how far from both
+// running sums the target has to be (or returns false, with the row word of a draw
+// that needs no search).  Returns the row word, 0 if a wait gave up.
+template <int GROUP, typename Value, typename Aim>
+__device__ __forceinline__ unsigned long long seed_draw(unsigned long long *sums, unsigned long long *row_word, int ci,
+                                                        const unsigned long long *s_group, int rows, int64_t b0,
+                                                        unsigned long long *s_words, Value &&value, Aim &&aim,
+                                                        int *err) {
+    const int lane = threadIdx.x & 31, G = gridDim.x;
+    const int groups = (rows + GROUP - 1) / GROUP, per = (groups + 31) / 32;
+    const int g0 = min(groups, lane * per), g1 = min(groups, g0 + per);
+    unsigned long long own = 0;
+    for (int g = g0; g < g1; ++g) own += s_group[g];
+    const unsigned long long end = seed_scan(own, lane);  // sum of the block's rows up to this lane's last
+    if (lane == 31) seed_store(sums + blockIdx.x, end << 2 | (unsigned)(ci & 3));
+    unsigned long long ps[SEED_SPAN], mine = 0;
+    bool ok = seed_gather(sums, G, ci, s_words, ps, err);
+#pragma unroll
+    for (int i = 0; i < SEED_SPAN; ++i) mine += ps[i];
+    const unsigned long long incl = seed_scan(mine, lane), total = __shfl_sync(0xffffffffu, incl, 31);
+    unsigned long long target, band, w = 0;
+    if (aim(total, target, band, w)) {
+        const int span = (G + 31) / 32;
+        unsigned long long cum = incl - mine, base = 0;
+        int b = G;  // the block that holds the point
+#pragma unroll
+        for (int i = 0; i < SEED_SPAN; ++i) {
+            if (i < span && b == G && cum + ps[i] >= target && lane * span + i < G) {
+                b = lane * span + i;
+                base = cum;
+            }
+            cum += ps[i];
+        }
+        const unsigned has = __ballot_sync(0xffffffffu, b < G);
+        const int src = has ? __ffs(has) - 1 : 0;
+        b = __shfl_sync(0xffffffffu, b, src);
+        base = __shfl_sync(0xffffffffu, base, src);
+        if ((int)blockIdx.x == (b < G ? b : 0)) {
+            // the lane whose groups reach the target, its group, then the row
+            unsigned long long row = SEED_AGAIN;
+            const unsigned runs = __ballot_sync(0xffffffffu, base + end >= target);
+            if (b < G && runs) {
+                const int l = __ffs(runs) - 1;
+                unsigned long long before = base + __shfl_sync(0xffffffffu, end - own, l);
+                int g = l * per;
+                while (g + 1 < groups && before + s_group[g] < target) before += s_group[g++];
+                const int i = g * GROUP + lane;
+                const bool real = lane < GROUP && i < rows;
+                const unsigned long long v = real ? value(i) : 0ull, at = before + seed_scan(v, lane);
+                const unsigned hit = __ballot_sync(0xffffffffu, real && at >= target);
+                const int f = hit ? __ffs(hit) - 1 : 0;
+                const unsigned long long at_f = __shfl_sync(0xffffffffu, at, f),
+                                         before_f = __shfl_sync(0xffffffffu, at - v, f);
+                if (hit && at_f - target >= band && target - before_f > band)
+                    row = (unsigned long long)(b0 + g * GROUP + f);
+            }
+            w = (unsigned long long)ci << SEED_TAG | row;
+            if (lane == 0) seed_store(row_word, w);
+        } else if (lane == 0) {
+            ok = ok && seed_wait(row_word, ci, &w, err);
+        }
+    }
+    return __all_sync(0xffffffffu, ok) ? w : 0ull;
+}
+
+// A distance as a multiple of 2^e, rounded down.
+__device__ __forceinline__ unsigned long long seed_fixed(float m, int e) {
+    const unsigned bits = __float_as_uint(m), x = bits >> 23;
+    const unsigned long long mant = (bits & 0x7fffffu) | (x ? 0x800000u : 0u);
+    const int shift = (x ? (int)x - 150 : -149) - e;
+    return shift >= 0 ? mant << min(shift, 63) : mant >> min(-shift, 63);
+}
+
+// The float draws: kpp_kernel's arithmetic and rule.  The sums are exact multiples of
+// 2^e, e chosen before each draw so that they stay below 2^62 (from the largest first
+// distance, then from the draw before: distances only fall), so they are n 2^e at most
+// below the exact ones; the target is u * total to one such step.  The reference's
+// double sums lie within 2 n 2^-53 total of the exact ones, and where these bounds
+// leave a doubt the serial rule decides (rare): the blocks write their distances out to
+// min_sq and arrive at *done, and thread 0 of block 0 repeats the reference's loop.
+// u: the draws' uniforms; words, zeroed: [2][grid] sums, [2] rows, [2] rows of the
+// serial rule, [grid] largest first distances.
+__global__ void __launch_bounds__(SEED_NT, 1) kpp_seed_kernel(const float *__restrict__ X, int64_t n, int d, int dp,
+                                                              float *C, int k, const float *__restrict__ u,
+                                                              float *min_sq, int chunk, unsigned long long *words,
+                                                              unsigned *done, int *err) {
+    extern __shared__ __align__(16) float seed_smem[];
+    __shared__ unsigned long long s_word, s_words[32 * SEED_SPAN];
+    __shared__ int s_e;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, G = gridDim.x;
+    const int64_t b0 = min(n, (int64_t)blockIdx.x * chunk);
+    const int rows = (int)(min(n, b0 + chunk) - b0);
+    const int stride = dp + 8;  // 32 bytes past a multiple of 64: four rows' 32 bytes in different banks
+    float *const s_c = seed_smem, *const s_m = s_c + dp;
+    unsigned long long *const s_group = reinterpret_cast<unsigned long long *>(s_m + ((chunk + 15) & ~15));
+    float *const s_x = reinterpret_cast<float *>(s_group + (chunk + 31) / 32 * 2);
+    const int dp4 = dp >> 2;
+    for (int i = t; i < rows * dp4; i += SEED_NT)
+        *reinterpret_cast<float4 *>(s_x + (i / dp4) * stride + (i % dp4) * 4) =
+            __ldg(reinterpret_cast<const float4 *>(X + b0 * dp) + i);
+    for (int i = t; i < rows; i += SEED_NT) s_m[i] = 3.402823466e+38f;
+    for (int j = t; j < dp; j += SEED_NT) s_c[j] = C[j];
+    __syncthreads();
+    const int half = t & 1, nb = d >> 3, rem = d & 7;
+    const float4 *c4 = reinterpret_cast<const float4 *>(s_c);
+    int e = 0;
+    unsigned again = 0;
+    // the sum of the 16 distances of a warp's even lanes (0 on the odd ones): three
+    // 21-bit parts, so that 32 lanes' sums fit a word
+    const auto group_sum = [&](int g, float m) {
+        const unsigned long long f = seed_fixed(m, e);
+        const unsigned a = __reduce_add_sync(0xffffffffu, (unsigned)(f & 0x1fffffu));
+        const unsigned b = __reduce_add_sync(0xffffffffu, (unsigned)(f >> 21 & 0x1fffffu));
+        const unsigned c = __reduce_add_sync(0xffffffffu, (unsigned)(f >> 42));
+        if (lane == 0) s_group[g] = ((unsigned long long)c << 42) + ((unsigned long long)b << 21) + a;
+    };
+    for (int ci = 1; ci < k; ++ci) {
+        for (int g = warp; g * 16 < rows; g += SEED_NT / 32) {  // 16 rows a warp, two lanes a row
+            const int i = g * 16 + (lane >> 1);
+            const bool in = i < rows;
+            const float4 *x4 = reinterpret_cast<const float4 *>(s_x + (in ? i : 0) * stride);
+            float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll 4
+            for (int c = 0; c < nb; ++c) {
+                const float4 x = x4[2 * c + half], q = c4[2 * c + half];
+                const float t0 = __fsub_rn(q.x, x.x), t1 = __fsub_rn(q.y, x.y);
+                const float t2 = __fsub_rn(q.z, x.z), t3 = __fsub_rn(q.w, x.w);
+                a0 = __fmaf_rn(t0, t0, a0);
+                a1 = __fmaf_rn(t1, t1, a1);
+                a2 = __fmaf_rn(t2, t2, a2);
+                a3 = __fmaf_rn(t3, t3, a3);
+            }
+            float s0 = __fadd_rn(a0, __shfl_xor_sync(0xffffffffu, a0, 1));
+            float s1 = __fadd_rn(a1, __shfl_xor_sync(0xffffffffu, a1, 1));
+            float s2 = __fadd_rn(a2, __shfl_xor_sync(0xffffffffu, a2, 1));
+            float s3 = __fadd_rn(a3, __shfl_xor_sync(0xffffffffu, a3, 1));
+            for (int w = 0; 4 * w < rem; ++w) {
+                const float4 x = x4[2 * nb + w], q = c4[2 * nb + w];
+                const float t0 = __fsub_rn(q.x, x.x), t1 = __fsub_rn(q.y, x.y);
+                const float t2 = __fsub_rn(q.z, x.z), t3 = __fsub_rn(q.w, x.w);
+                s0 = __fmaf_rn(t0, t0, s0);
+                s1 = __fmaf_rn(t1, t1, s1);
+                s2 = __fmaf_rn(t2, t2, s2);
+                s3 = __fmaf_rn(t3, t3, s3);
+            }
+            float m = 0.f;
+            if (half == 0 && in) {
+                const float rt = __fsqrt_rn(__fadd_rn(__fadd_rn(s0, s1), __fadd_rn(s2, s3)));
+                const float v = __fmul_rn(rt, rt);
+                m = s_m[i];
+                if (v < m) s_m[i] = m = v;
+            }
+            if (ci > 1) group_sum(g, m);
+        }
+        if (ci == 1) {
+            // the first draw's e, from the largest distance of all blocks
+            __syncthreads();
+            if (t < 32) {
+                unsigned top = 0;  // floats >= 0 order as their bits
+                for (int i = t; i < rows; i += 32) top = max(top, __float_as_uint(s_m[i]));
+                top = __reduce_max_sync(0xffffffffu, top);
+                unsigned long long *const maxs = words + 2 * (size_t)G + 4, v[SEED_SPAN];
+                if (t == 0) seed_store(maxs + blockIdx.x, (unsigned long long)top << 2 | 1u);
+                const bool ok = seed_gather(maxs, G, 1, s_words, v, err);
+#pragma unroll
+                for (int i = 0; i < SEED_SPAN; ++i) top = max(top, (unsigned)v[i]);
+                top = __reduce_max_sync(0xffffffffu, top);
+                // top < 2^(x - 126), so n of them stay below 2^(x - 126 + bits of n)
+                if (t == 0) {
+                    s_e = max((int)(top >> 23) - 126 + (64 - __clzll(n)) - 61, -149);
+                    s_word = ok;
+                }
+            }
+            __syncthreads();
+            if (s_word == 0) return;
+            e = s_e;
+            for (int g = warp; g * 16 < rows; g += SEED_NT / 32) {
+                const int i = g * 16 + (lane >> 1);
+                group_sum(g, half == 0 && i < rows ? s_m[i] : 0.f);
+            }
+        }
+        __syncthreads();
+        if (t < 32) {
+            int next_e = e;
+            const unsigned bits = __float_as_uint(u[ci - 1]), x = bits >> 23;
+            const unsigned long long w = seed_draw<16>(
+                words + (size_t)(ci & 1) * G, words + 2 * (size_t)G + (ci & 1), ci, s_group, rows, b0, s_words,
+                [&](int i) { return seed_fixed(s_m[i], e); },
+                [&](unsigned long long total, unsigned long long &target, unsigned long long &band,
+                    unsigned long long &) {
+                    // u in 2^-64ths; u = 1 (rounded up by the generator's library): the total
+                    const unsigned long long mant = (bits & 0x7fffffu) | 0x800000u;
+                    const int shift = (int)x - 86;
+                    const unsigned long long u64 = shift >= 0 ? mant << min(shift, 40) : mant >> min(-shift, 63);
+                    target = x >= 127 ? total : __umul64hi(total, u64);
+                    // 2 x 2 n 2^-53 total, and four rows' worth of the roundings to 2^e
+                    band = __umul64hi(total, (unsigned long long)n << 13) + 4ull * (unsigned long long)n + 4ull;
+                    // the next draw's total is below this one's and n more
+                    next_e = max(e - max(__clzll((long long)(total + (unsigned long long)n)) - 3, 0), -149);
+                    return true;
+                },
+                err);
+            if (lane == 0) {
+                s_word = w;
+                s_e = next_e;
+            }
+        }
+        __syncthreads();
+        unsigned long long w = s_word;
+        if (w == 0) return;  // a wait gave up (in every block, in the end)
+        e = s_e;
+        if (w & SEED_AGAIN) {
+            ++again;
+            for (int i = t; i < rows; i += SEED_NT) min_sq[b0 + i] = s_m[i];
+            __threadfence();
+            __syncthreads();
+            unsigned long long *const serial = words + 2 * (size_t)G + 2 + (ci & 1);
+            if (t == 0) {
+                atomicAdd(done, 1u);
+                bool ok = true;
+                if (blockIdx.x == 0) {
+                    unsigned polls = 0;
+                    while (*reinterpret_cast<volatile unsigned *>(done) < again * (unsigned)G && ok)
+                        ok = ++polls < SEED_SPINS;
+                    __threadfence();
+                    if (ok) {
+                        double tot = 0.0;
+                        for (int64_t i = 0; i < n; ++i) tot += (double)__ldcg(min_sq + i);
+                        const double rr = (double)u[ci - 1] * tot;
+                        double c = 0.0;
+                        int64_t ch = n - 1;
+                        for (int64_t i = 0; i < n; ++i) {
+                            c += (double)__ldcg(min_sq + i);
+                            if (c >= rr) {
+                                ch = i;
+                                break;
+                            }
+                        }
+                        w = (unsigned long long)ci << SEED_TAG | (unsigned long long)ch;
+                        seed_store(serial, w);
+                    } else {
+                        *reinterpret_cast<volatile int *>(err) = 1;
+                    }
+                } else {
+                    ok = seed_wait(serial, ci, &w, err, SEED_SPINS * 16u);
+                }
+                s_word = ok ? w : 0;
+            }
+            __syncthreads();
+            w = s_word;
+            if (w == 0) return;
+        }
+        const float *row = X + (int64_t)(w & (SEED_AGAIN - 1)) * dp;
+        for (int j = t; j < dp; j += SEED_NT) {
+            const float v = __ldg(row + j);
+            s_c[j] = v;
+            if (blockIdx.x == 0) C[(int64_t)ci * dp + j] = v;
+        }
+        __syncthreads();
+    }
+}
+
 // ── row norms ─────────────────────────────────────────────────────────────
 __global__ void row_norms_kernel(const float *__restrict__ X, int64_t n, int dp, float *__restrict__ out) {
     const int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -388,7 +735,8 @@ int kmeans_l2_device(const float *X, int64_t n, int d, int dp, int64_t k, int64_
     // k-means++ seeding, all on the device: the reference's draws (the first
     // point, then one uniform per further centroid) do not depend on the data,
     // so they are taken from the mt19937 stream up front in the reference's
-    // order; each further centroid is one kpp_kernel launch
+    // order; each further centroid is one kpp_kernel launch, or all of them one
+    // kpp_seed_kernel launch where the rows fit the SMs' shared memory
     GN_CUDA_TRY(cudaMemcpyAsync(C, X + pick_point(rng) * dp, row_bytes, cudaMemcpyDeviceToDevice, st));
     DBuf dmin, dpart, ddone;
     GN_TRY(dmin.ensure((size_t)n * sizeof(float)));
@@ -397,9 +745,38 @@ int kmeans_l2_device(const float *X, int64_t n, int d, int dp, int64_t k, int64_
     GN_TRY(dpart.ensure((size_t)P * sizeof(double)));
     GN_TRY(ddone.ensure(sizeof(unsigned)));
     GN_CUDA_TRY(cudaMemsetAsync(ddone.p, 0, sizeof(unsigned), st));
-    for (int64_t ci = 1; ci < k; ++ci)
-        kpp_kernel<<<(unsigned)P, KPP_NT, 0, st>>>(X, n, d, dp, C, ci, unif01(rng), dmin.as<float>(), chunk, P,
-                                                   dpart.as<double>(), ddone.as<unsigned>());
+    std::vector<float> us((size_t)std::max<int64_t>(k - 1, 0));
+    for (float &v : us) v = unif01(rng);
+    const int G = dev_info().num_sms;
+    const int64_t seed_chunk = ceil_div(n, G);
+    const size_t seed_smem = ((size_t)dp + round_up(seed_chunk, 16) + (size_t)seed_chunk * (dp + 8)) * 4 +
+                             (size_t)ceil_div(seed_chunk, 32) * 16;
+    DBuf dus, dwords;  // dwords: the blocks' words, then the arrivals and the error word
+    const bool seeded = k > 1 && k < (1 << 23) && G <= 32 * SEED_SPAN && seed_smem <= SEED_SMEM_MAX;
+    if (seeded) {
+        const size_t words = 3 * (size_t)G + 4;
+        GN_TRY(dus.ensure(us.size() * sizeof(float)));
+        GN_TRY(dwords.ensure((words + 1) * 8));
+        GN_CUDA_TRY(cudaMemcpyAsync(dus.p, us.data(), us.size() * sizeof(float), cudaMemcpyHostToDevice, st));
+        GN_CUDA_TRY(cudaMemsetAsync(dwords.p, 0, (words + 1) * 8, st));
+        GN_CUDA_TRY(cudaFuncSetAttribute(kpp_seed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)SEED_SMEM_MAX));
+        unsigned long long *dw = dwords.as<unsigned long long>();
+        unsigned *arrived = reinterpret_cast<unsigned *>(dw + words);
+        int *derr = reinterpret_cast<int *>(dw + words) + 1, ki = (int)k, chunk_i = (int)seed_chunk;
+        const float *du = dus.as<float>();
+        float *dm = dmin.as<float>();
+        void *args[] = {&X, &n, &d, &dp, &C, &ki, &du, &dm, &chunk_i, &dw, &arrived, &derr};
+        GN_CUDA_TRY(cudaLaunchCooperativeKernel((void *)kpp_seed_kernel, dim3(G), dim3(SEED_NT), args, seed_smem, st));
+        int herr = 0;
+        GN_CUDA_TRY(cudaMemcpyAsync(&herr, derr, 4, cudaMemcpyDeviceToHost, st));
+        GN_CUDA_TRY(cudaStreamSynchronize(st));
+        if (herr) return fail(GN_ERR_TIMEOUT, "kmeans: a wait of the seeding ran out");
+    } else {
+        for (int64_t ci = 1; ci < k; ++ci)
+            kpp_kernel<<<(unsigned)P, KPP_NT, 0, st>>>(X, n, d, dp, C, ci, us[(size_t)ci - 1], dmin.as<float>(), chunk,
+                                                       P, dpart.as<double>(), ddone.as<unsigned>());
+    }
     GN_CUDA_TRY(cudaGetLastError());
 
     // Lloyd iterations; one host synchronisation each (the change count and the
@@ -568,6 +945,66 @@ __global__ void __launch_bounds__(KPP_NT) bin_kpp_kernel(const uint4 *__restrict
     }
 }
 
+// The binary draws in one launch (see kpp_seed_kernel): bin_kpp_kernel's draws, which
+// every block makes for itself from the generator's outputs, since it reads all the
+// sums.  words: [2][grid] sums, then [2] rows, zeroed; *cursor: outputs used.
+__global__ void __launch_bounds__(SEED_NT, 1) bin_seed_kernel(const uint4 *__restrict__ X, int64_t n, int w4, uint4 *C,
+                                                              int k, int chunk, unsigned long long *words,
+                                                              const uint32_t *__restrict__ raw, int nraw, int *cursor,
+                                                              int *err) {
+    extern __shared__ __align__(16) uint4 bseed_smem[];
+    __shared__ unsigned long long s_word, s_words[32 * SEED_SPAN];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5, G = gridDim.x;
+    const int64_t b0 = min(n, (int64_t)blockIdx.x * chunk);
+    const int rows = (int)(min(n, b0 + chunk) - b0);
+    const int stride = w4 | 1;  // odd: neighbouring rows in different banks
+    uint4 *const s_c = bseed_smem, *const s_x = s_c + w4;
+    unsigned long long *const s_group = reinterpret_cast<unsigned long long *>(s_x + (size_t)chunk * stride);
+    uint32_t *const s_m = reinterpret_cast<uint32_t *>(s_group + (chunk + 31) / 32);
+    for (int i = t; i < rows * w4; i += SEED_NT) s_x[(i / w4) * stride + i % w4] = ldg_nc_u4(X + b0 * w4 + i);
+    for (int i = t; i < rows; i += SEED_NT) s_m[i] = 0xffffffffu;
+    for (int j = t; j < w4; j += SEED_NT) s_c[j] = C[j];
+    __syncthreads();
+    int cur = 0;
+    for (int ci = 1; ci < k; ++ci) {
+        for (int g = warp; g * 32 < rows; g += SEED_NT / 32) {
+            const int i = g * 32 + lane;
+            uint32_t m = 0;
+            if (i < rows) s_m[i] = m = min(s_m[i], (uint32_t)hdist(s_c, s_x + i * stride, w4));
+            m = __reduce_add_sync(0xffffffffu, m);
+            if (lane == 0) s_group[g] = m;
+        }
+        __syncthreads();
+        if (t < 32) {
+            const unsigned long long w = seed_draw<32>(
+                words + (size_t)(ci & 1) * G, words + 2 * (size_t)G + (ci & 1), ci, s_group, rows, b0, s_words,
+                [&](int i) { return (unsigned long long)s_m[i]; },
+                [&](unsigned long long total, unsigned long long &target, unsigned long long &band,
+                    unsigned long long &word) {
+                    // every row equals a centroid: the first draw stands
+                    word = (unsigned long long)ci << SEED_TAG | bin_draw(raw, nraw, &cur, (uint32_t)n);
+                    if (total == 0) return false;
+                    target = 1ull + bin_draw(raw, nraw, &cur, (uint32_t)total);  // the running sum passes the draw
+                    band = 0;
+                    return true;
+                },
+                err);
+            if (lane == 0) s_word = w;
+        }
+        __syncthreads();
+        const unsigned long long w = s_word;
+        if (w == 0) return;  // a wait gave up (in every block, in the end)
+        const uint4 *row = X + (int64_t)(w & (SEED_AGAIN - 1)) * w4;
+        for (int j = t; j < w4; j += SEED_NT) {
+            const uint4 v = ldg_nc_u4(row + j);
+            s_c[j] = v;
+            if (blockIdx.x == 0) C[(int64_t)ci * w4 + j] = v;
+        }
+        __syncthreads();
+    }
+    if (blockIdx.x == 0 && t == 0) *cursor = cur;
+}
+
 // The pick for an r that the host drew.
 __global__ void __launch_bounds__(KPP_NT) bin_pick_kernel(const uint4 *__restrict__ X, int64_t n, int w4, uint4 *C,
                                                           int64_t ci, const int32_t *min_d, int64_t chunk, int P,
@@ -671,7 +1108,7 @@ int kmeans_bin_device(const uint8_t *X, int64_t n, int nbytes, int w4, int32_t k
     const int P = (int)ceil_div(n, chunk);
     GN_TRY(dmin.ensure((size_t)n * 4));
     GN_TRY(dsums.ensure((size_t)P * 8));
-    GN_TRY(daux.ensure(24));  // [0] total (int64), [2] arrival counter, [3] stream cursor
+    GN_TRY(daux.ensure(24));  // [0] total (int64), [2] arrival counter, [3] stream cursor, [4] error word
     GN_CUDA_TRY(cudaMemsetAsync(daux.p, 0, 24, st));
     int64_t *dtotal = daux.as<int64_t>();
     unsigned *ddone = daux.as<unsigned>() + 2;
@@ -693,15 +1130,35 @@ int kmeans_bin_device(const uint8_t *X, int64_t n, int nbytes, int w4, int32_t k
         for (uint32_t &v : raw) v = (uint32_t)ahead();
         GN_TRY(draw.ensure(raw.size() * 4));
         GN_CUDA_TRY(cudaMemcpyAsync(draw.p, raw.data(), raw.size() * 4, cudaMemcpyHostToDevice, st));
-        for (int32_t ci = 1; ci < k; ++ci)
-            bin_kpp_kernel<<<(unsigned)P, KPP_NT, 0, st>>>(X4, n, w4, C4, ci, dmin.as<int32_t>(), chunk, P,
-                                                           dsums.as<int64_t>(), ddone, draw.as<uint32_t>(),
-                                                           (int)raw.size(), dcur, dtotal);
-        int used = 0;
-        GN_CUDA_TRY(cudaMemcpyAsync(&used, dcur, 4, cudaMemcpyDeviceToHost, st));
+        const int G = dev_info().num_sms;
+        const int64_t seed_chunk = ceil_div(n, G);
+        const size_t seed_smem =
+            ((size_t)w4 + (size_t)seed_chunk * (w4 | 1)) * 16 + (size_t)ceil_div(seed_chunk, 32) * 8 + (size_t)seed_chunk * 4;
+        DBuf dwords;
+        int used[2] = {0, 0};  // outputs used, error word
+        if (k < (1 << 23) && G <= 32 * SEED_SPAN && seed_smem <= SEED_SMEM_MAX) {
+            const size_t words = 2 * (size_t)G + 2;
+            GN_TRY(dwords.ensure(words * 8));
+            GN_CUDA_TRY(cudaMemsetAsync(dwords.p, 0, words * 8, st));
+            GN_CUDA_TRY(cudaFuncSetAttribute(bin_seed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)SEED_SMEM_MAX));
+            unsigned long long *dw = dwords.as<unsigned long long>();
+            int chunk_i = (int)seed_chunk, nraw = (int)raw.size(), *derr = dcur + 1;
+            const uint32_t *dr = draw.as<uint32_t>();
+            void *args[] = {&X4, &n, &w4, &C4, &k, &chunk_i, &dw, &dr, &nraw, &dcur, &derr};
+            GN_CUDA_TRY(cudaLaunchCooperativeKernel((void *)bin_seed_kernel, dim3(G), dim3(SEED_NT), args, seed_smem,
+                                                    st));
+        } else {
+            for (int32_t ci = 1; ci < k; ++ci)
+                bin_kpp_kernel<<<(unsigned)P, KPP_NT, 0, st>>>(X4, n, w4, C4, ci, dmin.as<int32_t>(), chunk, P,
+                                                               dsums.as<int64_t>(), ddone, draw.as<uint32_t>(),
+                                                               (int)raw.size(), dcur, dtotal);
+        }
+        GN_CUDA_TRY(cudaMemcpyAsync(used, dcur, 8, cudaMemcpyDeviceToHost, st));
         GN_CUDA_TRY(cudaStreamSynchronize(st));
-        on_device = used <= (int)raw.size() - 1;
-        if (on_device) rng.discard((unsigned long long)used);
+        if (used[1]) return fail(GN_ERR_TIMEOUT, "kmeans: a wait of the seeding ran out");
+        on_device = used[0] <= (int)raw.size() - 1;
+        if (on_device) rng.discard((unsigned long long)used[0]);
     }
     if (!on_device)
         for (int32_t ci = 1; ci < k; ++ci) {

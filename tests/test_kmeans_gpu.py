@@ -33,3 +33,16 @@ def test_binary_build_equals_the_oracle(gn, oracle, n, nbytes, nlist, iters, dis
     cent, labels = ix.export()
     oc, ol = oracle.ivfbin_build(db, nlist, iters)
     assert np.array_equal(cent, oc) and np.array_equal(labels, ol)
+
+
+@pytest.mark.parametrize("n,d,k,distinct", [(300, 3, 9, 5), (2000, 16, 40, 7), (152 * 33 + 1, 8, 12, 3), (5000, 64, 300, None)])
+def test_float_seeds_where_the_serial_sum_decides(gn, oracle, n, d, k, distinct):
+    """Fewer distinct rows than centroids: the later draws' distances are all zero,
+    and a draw of the first ones may fall on a boundary between equal rows."""
+    rng = np.random.default_rng(n + k)
+    data = rng.standard_normal((distinct or n, d)).astype(np.float32)
+    if distinct:
+        data = data[rng.integers(0, distinct, n)]
+    _, cent = gn.kmeans_l2(data, k, 0, 42)
+    _, ocent, _ = oracle.kmeans_l2(data, k, 0, 42)
+    assert np.array_equal(cent.view(np.uint32), ocent.view(np.uint32))

@@ -108,18 +108,53 @@ static bool host_pinned(const void *p) {
 
 void begin_blocking(gn_index *ix) {
     ix->pending.clear();
-    ix->pending_bytes = 0;
+    ix->small_bytes = ix->stage_bytes = 0;
+    ix->status = nullptr;
+    ix->status_set = false;
+}
+
+// Room for `bytes` in the small pinned block's out part, null if there is none.
+static int small_out(gn_index *ix, size_t bytes, char **p) {
+    *p = nullptr;
+    const size_t span = (bytes + 255) & ~(size_t)255;
+    if (ix->small_bytes + span > SMALL_BYTES) return GN_OK;
+    GN_TRY(ix->small.ensure(256 + 2 * SMALL_BYTES));
+    *p = static_cast<char *>(ix->small.p) + 256 + SMALL_BYTES + ix->small_bytes;
+    ix->small_bytes += span;
+    return GN_OK;
+}
+
+int place_result(gn_index *ix, DBuf &buf, void *dst, size_t bytes, void **out) {
+    char *p = nullptr;
+    if (bytes > 0 && bytes <= SMALL_BYTES && !host_pinned(dst)) GN_TRY(small_out(ix, bytes, &p));
+    if (p) {
+        ix->status = static_cast<int *>(ix->small.p);
+        *ix->status = 0;
+        ix->pending.push_back({dst, p, bytes});
+        *out = p;
+        return GN_OK;
+    }
+    GN_TRY(buf.ensure(bytes));
+    *out = buf.p;
+    return GN_OK;
 }
 
 int stage_queries(gn_index *ix, const void *src, size_t bytes, cudaStream_t st, const void **out) {
     *out = src;
     if (bytes == 0 || bytes > STAGE_BYTES || host_pinned(src)) return GN_OK;
-    GN_TRY(ix->stage_in.ensure(STAGE_BYTES));  // one fixed size: never reallocated under a queued copy
     // a search that ended early (an error) may have left a copy from it queued
     if (ix->stage_in_busy) GN_CUDA_TRY(cudaStreamSynchronize(st));
-    std::memcpy(ix->stage_in.p, src, bytes);
+    void *p;
+    if (bytes <= SMALL_BYTES) {  // (fixed sizes: never reallocated under a queued copy)
+        GN_TRY(ix->small.ensure(256 + 2 * SMALL_BYTES));
+        p = static_cast<char *>(ix->small.p) + 256;
+    } else {
+        GN_TRY(ix->stage_in.ensure(STAGE_BYTES));
+        p = ix->stage_in.p;
+    }
+    std::memcpy(p, src, bytes);
     ix->stage_in_busy = true;
-    *out = ix->stage_in.p;
+    *out = p;
     return GN_OK;
 }
 
@@ -132,14 +167,22 @@ int upload_queries(gn_index *ix, DBuf &dst, const void *src, int64_t n, int64_t 
 
 int download_result(gn_index *ix, void *dst, const void *dsrc, size_t bytes, cudaStream_t st) {
     if (bytes == 0) return GN_OK;
-    const size_t off = ix->pending_bytes, span = (bytes + 255) & ~(size_t)255;
-    if (off + span <= STAGE_BYTES && !host_pinned(dst)) {
-        GN_TRY(ix->stage_out.ensure(STAGE_BYTES));
-        GN_CUDA_TRY(cudaMemcpyAsync(static_cast<char *>(ix->stage_out.p) + off, dsrc, bytes, cudaMemcpyDeviceToHost,
-                                    st));
-        ix->pending.push_back({dst, off, bytes});
-        ix->pending_bytes = off + span;
-        return GN_OK;
+    const char *small = static_cast<const char *>(ix->small.p), *src = static_cast<const char *>(dsrc);
+    if (small && src >= small && src < small + 256 + 2 * SMALL_BYTES) return GN_OK;
+    if (!host_pinned(dst)) {
+        char *p = nullptr;
+        const size_t span = (bytes + 255) & ~(size_t)255;
+        if (bytes <= SMALL_BYTES) GN_TRY(small_out(ix, bytes, &p));
+        if (!p && ix->stage_bytes + span <= STAGE_BYTES) {
+            GN_TRY(ix->stage_out.ensure(STAGE_BYTES));
+            p = static_cast<char *>(ix->stage_out.p) + ix->stage_bytes;
+            ix->stage_bytes += span;
+        }
+        if (p) {
+            GN_CUDA_TRY(cudaMemcpyAsync(p, dsrc, bytes, cudaMemcpyDeviceToHost, st));
+            ix->pending.push_back({dst, p, bytes});
+            return GN_OK;
+        }
     }
     GN_CUDA_TRY(cudaMemcpyAsync(dst, dsrc, bytes, cudaMemcpyDeviceToHost, st));
     return GN_OK;
@@ -148,19 +191,18 @@ int download_result(gn_index *ix, void *dst, const void *dsrc, size_t bytes, cud
 int finish_blocking(gn_index *ix, int *d_err, cudaStream_t st, const char *what) {
     int *h = nullptr;
     if (d_err) {
-        GN_TRY(ix->hstatus.ensure(sizeof(int)));
-        h = static_cast<int *>(ix->hstatus.p);
-        *h = 0;  // no copy into it is pending: every blocking search ends synchronised
-        GN_CUDA_TRY(cudaMemcpyAsync(h, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        GN_TRY(ix->small.ensure(256 + 2 * SMALL_BYTES));
+        h = static_cast<int *>(ix->small.p);
+        if (!ix->status_set) {
+            *h = 0;  // no copy into it is pending: every blocking search ends synchronised
+            GN_CUDA_TRY(cudaMemcpyAsync(h, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        }
     }
     const cudaError_t se = cudaStreamSynchronize(st);
     if (ix->stage_in_busy) ix->stage_in_busy = false;
-    if (!ix->pending.empty()) {  // (the entry points that stage hold the index's lock throughout)
-        if (se == cudaSuccess)
-            for (const auto &pd : ix->pending)
-                std::memcpy(pd.dst, static_cast<const char *>(ix->stage_out.p) + pd.off, pd.bytes);
-        begin_blocking(ix);
-    }
+    if (se == cudaSuccess)  // (the entry points that stage hold the index's lock throughout)
+        for (const auto &pd : ix->pending) std::memcpy(pd.dst, pd.src, pd.bytes);
+    begin_blocking(ix);
     GN_CUDA_TRY(se);
     if (h && *h) {
         GN_CUDA_TRY(cudaMemsetAsync(d_err, 0, sizeof(int), st));
@@ -280,9 +322,10 @@ int gn_flat_set(gn_index *ix, const void *data, int64_t n, int64_t dim) {
     return GN_OK;
 }
 
-// Shared search body.  queries/out are device pointers here.
+// Shared search body.  queries/out are device pointers here; status: where a float
+// scan's last kernel writes the error word (pinned, may be null).
 static int flat_search_dev(gn_index *ix, const void *d_q, int64_t nq, int64_t k, int64_t *d_idx, void *d_dist,
-                           cudaStream_t st) {
+                           int *status, cudaStream_t st) {
     FlatScanArgs a;
     a.metric = ix->metric;
     a.db = ix->data.p;
@@ -318,7 +361,11 @@ static int flat_search_dev(gn_index *ix, const void *d_q, int64_t nq, int64_t k,
         flat_plan(a);
         if (!flat_smem_ok(a)) return fail(GN_ERR_UNSUPPORTED, "dimension too large for the exact flat scan");
         GN_TRY(ix->part.ensure(flat_part_bytes(a)));
-        if (a.metric != M_HAMMING) GN_TRY(error_word());
+        if (a.metric != M_HAMMING) {
+            GN_TRY(error_word());
+            a.status = status;
+            ix->status_set = status != nullptr;
+        }
         GN_TRY(flat_launch(a, ix->part.as<uint64_t>(), st));
     } else {
         // materialise keys for chunks of queries (<= 512 MB of keys per chunk)
@@ -352,12 +399,14 @@ int gn_flat_search_knn(gn_index *ix, const void *queries, int64_t nq, int64_t k,
     begin_blocking(ix);
     const int64_t row_bytes = (ix->metric == GN_METRIC_HAMMING) ? ix->dim : ix->dim * 4;
     GN_TRY(upload_queries(ix, ix->q, queries, nq, row_bytes, ix->stride4, st));
-    GN_TRY(ix->out_idx.ensure((size_t)nq * k * 8));
-    GN_TRY(ix->out_dist.ensure((size_t)nq * k * 8));
-    GN_TRY(flat_search_dev(ix, ix->q.p, nq, k, ix->out_idx.as<int64_t>(), ix->out_dist.p, st));
+    const size_t idx_bytes = (size_t)nq * k * 8;
     const size_t dist_bytes = (size_t)nq * k * (ix->metric == GN_METRIC_HAMMING ? 8 : 4);
-    GN_TRY(download_result(ix, out_idx, ix->out_idx.p, (size_t)nq * k * 8, st));
-    GN_TRY(download_result(ix, out_dist, ix->out_dist.p, dist_bytes, st));
+    void *d_idx = nullptr, *d_dist = nullptr;
+    GN_TRY(place_result(ix, ix->out_idx, out_idx, idx_bytes, &d_idx));
+    GN_TRY(place_result(ix, ix->out_dist, out_dist, dist_bytes, &d_dist));
+    GN_TRY(flat_search_dev(ix, ix->q.p, nq, k, static_cast<int64_t *>(d_idx), d_dist, ix->status, st));
+    GN_TRY(download_result(ix, out_idx, d_idx, idx_bytes, st));
+    GN_TRY(download_result(ix, out_dist, d_dist, dist_bytes, st));
     // a float scan's pipeline wait that ran out (reported once, then cleared)
     return finish_blocking(ix, ix->err.p ? ix->err.as<int>() : nullptr, st,
                            "flat scan: a pipeline wait timed out; results are invalid");
@@ -372,7 +421,7 @@ int gn_flat_search_knn_device(gn_index *ix, const void *d_queries, int64_t nq, i
     GN_TRY(flat_check(ix, nq, k));
     std::lock_guard<std::mutex> lk(ix->mu);
     // device queries must already use the index's padded row layout
-    return flat_search_dev(ix, d_queries, nq, k, d_idx, d_dist, (cudaStream_t)stream);
+    return flat_search_dev(ix, d_queries, nq, k, d_idx, d_dist, nullptr, (cudaStream_t)stream);
 }
 
 }  // extern "C"

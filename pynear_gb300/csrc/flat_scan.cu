@@ -506,9 +506,10 @@ template <int W, int R>
 __global__ void __launch_bounds__(W * 32)
     flat_finish_kernel(const uint64_t *__restrict__ cand, const int *__restrict__ qcount, int64_t list_keys, int k,
                        int64_t *__restrict__ out_idx, float *__restrict__ out_dist, int64_t *__restrict__ out_cnt,
-                       const int *__restrict__ only_if) {
+                       const int *__restrict__ only_if, const int *err, int *status) {
     __shared__ uint64_t s_sel[(W + 1) * R * 32];
     __shared__ int s_n[W];
+    if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = *err;
     if (only_if && *only_if == 0) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t q = blockIdx.x;
@@ -835,18 +836,19 @@ static int hamming_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st
 }
 
 int candidates_finish(const uint64_t *cand, const int *qcount, int64_t list_keys, int64_t nq, int k, int64_t *out_idx,
-                      float *out_dist, int64_t *out_cnt, const int *only_if, cudaStream_t st) {
+                      float *out_dist, int64_t *out_cnt, const int *only_if, cudaStream_t st, const int *err,
+                      int *status) {
     auto finish = [&](auto RC) {
         constexpr int R = decltype(RC)::value;
         if (nq <= dev_info().num_sms && R <= 2)
             flat_finish_kernel<24, R><<<(unsigned)nq, 768, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist,
-                                                                  out_cnt, only_if);
+                                                                  out_cnt, only_if, err, status);
         else if (nq <= 4 * dev_info().num_sms)
             flat_finish_kernel<8, R><<<(unsigned)nq, 256, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist,
-                                                                  out_cnt, only_if);
+                                                                  out_cnt, only_if, err, status);
         else
             flat_finish_kernel<1, R><<<(unsigned)nq, 32, 0, st>>>(cand, qcount, list_keys, k, out_idx, out_dist,
-                                                                  out_cnt, only_if);
+                                                                  out_cnt, only_if, err, status);
     };
     if (k <= 32) finish(std::integral_constant<int, 1>());
     else if (k <= 64) finish(std::integral_constant<int, 2>());
@@ -909,7 +911,7 @@ static int float_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) 
                               : go(std::integral_constant<int, M_LINF>()));
     if (!a.only_if) timing_end(st);
     return candidates_finish(f.cand, f.qcount, a.list_keys, a.nq, a.k, a.out_idx, reinterpret_cast<float *>(a.out_dist),
-                             nullptr, a.only_if, st);
+                             nullptr, a.only_if, st, a.err, a.status);
 }
 
 // Launch the k <= 256 path.  part: flat_part_bytes(a) scratch.

@@ -17,6 +17,7 @@ struct FlatScanArgs {
     int64_t *out_idx = nullptr;  // nq*k
     void *out_dist = nullptr;    // nq*k float32 or int64
     int *err = nullptr;          // float metrics: device error word of the scan's bounded waits
+    int *status = nullptr;  // float metrics: pinned word that the last kernel copies the error word to (may be null)
     const int *only_if = nullptr;  // float metrics: device word; 0 = the results are there already, do nothing
     // filled by flat_plan
     int warps = 4, n_slices = 1, n_groups = 1;
@@ -32,9 +33,10 @@ int flat_smem_ok(const FlatScanArgs &a);
 int flat_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st);
 // The k nearest (k <= 256) of each query's qcount[q] candidate (distance, index)
 // keys at cand + q * list_keys, nearest first, with their number where out_cnt is given.
-// only_if: see FlatScanArgs.
+// only_if, err, status: see FlatScanArgs.
 int candidates_finish(const uint64_t *cand, const int *qcount, int64_t list_keys, int64_t nq, int k, int64_t *out_idx,
-                      float *out_dist, int64_t *out_cnt, const int *only_if, cudaStream_t st);
+                      float *out_dist, int64_t *out_cnt, const int *only_if, cudaStream_t st,
+                      const int *err = nullptr, int *status = nullptr);
 int flat_preload_hamming();
 int64_t next_pow2(int64_t v);
 void flat_large_k_launch(const FlatScanArgs &a, int64_t q_begin, int64_t qc, uint64_t *keys, uint64_t *sorted,

@@ -62,17 +62,21 @@ struct gn_index {
     // per-call scratch (reused across calls)
     gn::DBuf q, part, out_idx, out_dist, keys, sorted;
     gn::DBuf err;         // float flat scans: error word of their bounded pipeline waits
-    gn::HBuf hstatus;     // pinned: a blocking search's error word, copied behind its results
-    // pinned staging of a blocking search's small pageable copies (queries in,
-    // results out); staged results reach the caller's buffers after the sync
+    // pinned staging of a blocking search's pageable copies (queries in, results out),
+    // which reach the caller's buffers after the sync: one small block, in one
+    // allocation, for what most calls move, and larger ones where needed
+    gn::HBuf small;  // [256: error word][SMALL_BYTES in][SMALL_BYTES out]
     gn::HBuf stage_in, stage_out;
     struct Pending {
         void *dst;
-        size_t off, bytes;
+        const void *src;
+        size_t bytes;
     };
     std::vector<Pending> pending;
-    size_t pending_bytes = 0;
-    bool stage_in_busy = false;  // a copy from stage_in may still be queued
+    size_t small_bytes = 0, stage_bytes = 0;  // of small's out part and of stage_out in use
+    bool stage_in_busy = false;  // a copy from the staged queries may still be queued
+    int *status = nullptr;       // small's error word, while a search's last kernel can write it there itself
+    bool status_set = false;     // ... and has been launched so
     // kind-specific state
     gn::IvfL2State *ivfl2 = nullptr;
     gn::IvfBinState *ivfbin = nullptr;
@@ -94,7 +98,7 @@ int make_stream(gn_index *ix);
 // Blocking searches (the host-buffer entry points), in this order:
 // begin_blocking, then upload_queries / download_result for the caller's
 // buffers, then finish_blocking.  Pageable buffers of up to STAGE_BYTES go
-// through the index's pinned stage_in / stage_out, so that each copy is one
+// through the index's pinned staging, so that each copy is one
 // asynchronous DMA instead of the CUDA driver's staged pageable copy (about
 // 19 us of a 76 us one-query call measured); pinned or larger buffers are
 // copied directly.
@@ -104,12 +108,20 @@ void begin_blocking(gn_index *ix);
 int upload_queries(gn_index *ix, DBuf &dst, const void *src, int64_t n, int64_t row_bytes, int stride4,
                    cudaStream_t st);
 // Host staging of query rows for a copy the caller issues: returns src, or
-// the pinned stage_in holding a copy of its `bytes`.
+// pinned memory holding a copy of its `bytes`.
 int stage_queries(gn_index *ix, const void *src, size_t bytes, cudaStream_t st, const void **out);
-// Device -> host copy of `bytes` of results into the caller's dst.
+// Where a search's kernels put `bytes` of results for the caller's dst: the pinned
+// block itself for a small pageable dst (device-accessible; results are written once,
+// by a search's last kernel, and never read back on the device), else buf.  A
+// one-query call spent 9 of 48 us in the two results' and the error word's copies.
+int place_result(gn_index *ix, DBuf &buf, void *dst, size_t bytes, void **out);
+constexpr size_t SMALL_BYTES = (size_t)64 << 10;
+// Device -> host copy of `bytes` of results into the caller's dst (none for results
+// that place_result put into the pinned block).
 int download_result(gn_index *ix, void *dst, const void *dsrc, size_t bytes, cudaStream_t st);
 // End of a blocking search on stream st: the device error word d_err (may be
-// null) is copied into the index's pinned status word behind the results'
+// null) is copied into the index's pinned error word (unless the last kernel
+// wrote it there, status_set) behind the results'
 // copies, the stream is synchronised once, staged results are copied to the
 // caller's buffers, and a pipeline wait that ran out is reported as
 // GN_ERR_TIMEOUT with message `what` (the word is cleared).

@@ -1241,6 +1241,7 @@ int gn_ivfl2_search_knn_device(gn_index *ix, const float *d_queries, int64_t nq,
     if (ix->ivfl2->nc == 0) return fail(GN_ERR_EMPTY, "Index is empty — call set() first");
     if (k <= 0) return fail(GN_ERR_INVALID, "k must be positive");
     std::lock_guard<std::mutex> lk(ix->mu);
+    ix->status = nullptr;  // of a blocking search that ended early
     IvfL2State &S = *ix->ivfl2;
     if (S.graphs && nq > 0 && nq <= S.graphs->max_batch && k == S.graphs->k && !timing_on())
         return ivfl2_search_graph(ix, d_queries, false, nq, (int)k, d_idx, d_dist, d_cnt, false, (cudaStream_t)stream);
@@ -1272,14 +1273,15 @@ int gn_ivfl2_search_knn(gn_index *ix, const float *queries, int64_t nq, int64_t 
     }
     cudaStream_t st = ix->stream;
     GN_TRY(upload_queries(ix, S.s.q, queries, nq, S.d * 4, S.dp / 4, st));
-    GN_TRY(ix->out_idx.ensure((size_t)nq * k * 8));
-    GN_TRY(ix->out_dist.ensure((size_t)nq * k * 4));
-    GN_TRY(ix->part.ensure((size_t)nq * 8));
-    GN_TRY(ivfl2_search_core(ix, S.s.q.as<float>(), nq, (int)k, ix->out_idx.as<int64_t>(), ix->out_dist.as<float>(),
-                            ix->part.as<int64_t>(), st));
-    GN_TRY(download_result(ix, out_idx, ix->out_idx.p, (size_t)nq * k * 8, st));
-    GN_TRY(download_result(ix, out_dist, ix->out_dist.p, (size_t)nq * k * 4, st));
-    GN_TRY(download_result(ix, out_cnt, ix->part.p, (size_t)nq * 8, st));
+    void *d_idx = nullptr, *d_dist = nullptr, *d_cnt = nullptr;
+    GN_TRY(place_result(ix, ix->out_idx, out_idx, (size_t)nq * k * 8, &d_idx));
+    GN_TRY(place_result(ix, ix->out_dist, out_dist, (size_t)nq * k * 4, &d_dist));
+    GN_TRY(place_result(ix, ix->part, out_cnt, (size_t)nq * 8, &d_cnt));
+    GN_TRY(ivfl2_search_core(ix, S.s.q.as<float>(), nq, (int)k, static_cast<int64_t *>(d_idx),
+                             static_cast<float *>(d_dist), static_cast<int64_t *>(d_cnt), st));
+    GN_TRY(download_result(ix, out_idx, d_idx, (size_t)nq * k * 8, st));
+    GN_TRY(download_result(ix, out_dist, d_dist, (size_t)nq * k * 4, st));
+    GN_TRY(download_result(ix, out_cnt, d_cnt, (size_t)nq * 8, st));
     GN_CUDA_TRY(cudaGetLastError());
     return ivfl2_finish(ix, st);
 }
@@ -1404,14 +1406,15 @@ int gn_ivfbin_search_knn(gn_index *ix, const uint8_t *queries, int64_t nq, int64
     cudaStream_t st = ix->stream;
     begin_blocking(ix);
     GN_TRY(upload_queries(ix, S.s.q, queries, nq, S.nbytes, S.w4, st));
-    GN_TRY(ix->out_idx.ensure((size_t)nq * k * 8));
-    GN_TRY(ix->out_dist.ensure((size_t)nq * k * 8));
-    GN_TRY(ix->part.ensure((size_t)nq * 8));
-    GN_TRY(ivfbin_search_dev(ix, S.s.q.as<uint8_t>(), nq, (int)k, ix->out_idx.as<int64_t>(),
-                             ix->out_dist.as<int64_t>(), ix->part.as<int64_t>(), st));
-    GN_TRY(download_result(ix, out_idx, ix->out_idx.p, (size_t)nq * k * 8, st));
-    GN_TRY(download_result(ix, out_dist, ix->out_dist.p, (size_t)nq * k * 8, st));
-    GN_TRY(download_result(ix, out_cnt, ix->part.p, (size_t)nq * 8, st));
+    void *d_idx = nullptr, *d_dist = nullptr, *d_cnt = nullptr;
+    GN_TRY(place_result(ix, ix->out_idx, out_idx, (size_t)nq * k * 8, &d_idx));
+    GN_TRY(place_result(ix, ix->out_dist, out_dist, (size_t)nq * k * 8, &d_dist));
+    GN_TRY(place_result(ix, ix->part, out_cnt, (size_t)nq * 8, &d_cnt));
+    GN_TRY(ivfbin_search_dev(ix, S.s.q.as<uint8_t>(), nq, (int)k, static_cast<int64_t *>(d_idx),
+                             static_cast<int64_t *>(d_dist), static_cast<int64_t *>(d_cnt), st));
+    GN_TRY(download_result(ix, out_idx, d_idx, (size_t)nq * k * 8, st));
+    GN_TRY(download_result(ix, out_dist, d_dist, (size_t)nq * k * 8, st));
+    GN_TRY(download_result(ix, out_cnt, d_cnt, (size_t)nq * 8, st));
     GN_TRY(finish_blocking(ix, nullptr, st, ""));
     GN_CUDA_TRY(cudaGetLastError());
     return GN_OK;

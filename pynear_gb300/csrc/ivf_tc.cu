@@ -436,8 +436,10 @@ __global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW) ivf_tc_select_kernel(
     const int32_t *__restrict__ probes, int np, const int64_t *__restrict__ qseg,
     const int64_t *__restrict__ seg_rel, const int64_t *__restrict__ list_off, int S, const float *__restrict__ Q,
     const float *__restrict__ X, int d, int dp, const int32_t *__restrict__ ids, int k,
-    int64_t *__restrict__ out_idx, float *__restrict__ out_dist, int64_t *__restrict__ out_cnt) {
+    int64_t *__restrict__ out_idx, float *__restrict__ out_dist, int64_t *__restrict__ out_cnt, const int *err,
+    int *status) {
     __shared__ SelWarp s_warp[NW];
+    if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = *err;
     __shared__ uint64_t s_all[NW > 1 ? SEL_ALL : 1];
     __shared__ int s_wn[NW];
     __shared__ float s_d[64];
@@ -1328,8 +1330,10 @@ int ivfl2_search_tc(gn_index *ix, const float *dQ, int64_t nq, int k, int64_t *d
         ivf_tc_select_kernel<NW><<<(unsigned)nq, 32 * NW, 0, st>>>(
             S.scores.as<float>(), S.tmin.as<uint4>(), T.qbound.as<uint32_t>(), T.probes.as<int32_t>(), np,
             T.qslot.as<int64_t>(), T.slot_rel.as<int64_t>(), S.list_off.as<int64_t>(), S.shortlist, dQ,
-            S.vecs.as<float>(), S.d, S.dp, S.ids.as<int32_t>(), k, d_idx, d_dist, d_cnt);
+            S.vecs.as<float>(), S.d, S.dp, S.ids.as<int32_t>(), k, d_idx, d_dist, d_cnt, S.err.as<int>(),
+            ix->status);
     });
+    ix->status_set = ix->status != nullptr;
     GN_CUDA_TRY(cudaGetLastError());
     return GN_OK;
 }

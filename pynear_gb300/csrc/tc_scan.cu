@@ -1270,11 +1270,13 @@ int gn_tcflat_search_knn(gn_index *ix, const float *queries, int64_t nq, int64_t
     std::lock_guard<std::mutex> lk(ix->mu);
     begin_blocking(ix);
     GN_TRY(upload_queries(ix, S.q32, queries, nq, S.d * 4, S.dp / 4, st));
-    GN_TRY(S.out_idx.ensure((size_t)nq * k * 8));
-    GN_TRY(S.out_dist.ensure((size_t)nq * k * 4));
-    GN_TRY(tcflat_search_locked(ix, S.q32.as<float>(), nq, k, S.out_idx.as<int64_t>(), S.out_dist.as<float>(), st));
-    GN_TRY(download_result(ix, out_idx, S.out_idx.p, (size_t)nq * k * 8, st));
-    GN_TRY(download_result(ix, out_dist, S.out_dist.p, (size_t)nq * k * 4, st));
+    void *d_idx = nullptr, *d_dist = nullptr;
+    GN_TRY(place_result(ix, S.out_idx, out_idx, (size_t)nq * k * 8, &d_idx));
+    GN_TRY(place_result(ix, S.out_dist, out_dist, (size_t)nq * k * 4, &d_dist));
+    GN_TRY(tcflat_search_locked(ix, S.q32.as<float>(), nq, k, static_cast<int64_t *>(d_idx),
+                                static_cast<float *>(d_dist), st));
+    GN_TRY(download_result(ix, out_idx, d_idx, (size_t)nq * k * 8, st));
+    GN_TRY(download_result(ix, out_dist, d_dist, (size_t)nq * k * 4, st));
     return finish_blocking(ix, S.err.as<int>(), st, "tensor-core scan: a pipeline wait timed out");
 }
 

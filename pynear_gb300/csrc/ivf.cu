@@ -508,7 +508,8 @@ __global__ void __launch_bounds__(GT_THREADS, 2) ivf_scan_kernel(
         }
         f32x2 acc[8][2 * H];
         for (int64_t rb = r0; rb < r1; rb += GT_BN * H) {
-            gt_tile<H>(s, acc, Q, arow, dp, V, rb, r1, dp, dp);
+            gt_tile<H, true>(s, acc, Q, arow, dp, V, rb, r1, dp, dp);
+            if (arow[tm * 8] < 0) continue;  // no query of this warp's (its lists stay empty)
 #pragma unroll
             for (int h = 0; h < H; ++h) {
                 const int64_t row = rb + gt_col(2 * h);

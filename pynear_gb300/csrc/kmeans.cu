@@ -637,6 +637,88 @@ __global__ void row_norms_kernel(const float *__restrict__ X, int64_t n, int dp,
 }
 
 // ── float assignment: tile GEMM + argmin ──────────────────────────────────
+// The first nearest centroid of row x in f2ord's total order, by one warp: for rows with a
+// product that is not finite (a NaN score has a place in that order, but none in
+// AssignBest's compares) or without any score below +inf.
+__device__ __noinline__ int32_t assign_unordered(const float *__restrict__ x, const float *__restrict__ C,
+                                                 const float *__restrict__ cnorm, int k, int dp) {
+    uint64_t best = KEY_EMPTY;
+    for (int c = threadIdx.x & 31; c < k; c += 32) {
+        float dot = 0.f;
+        for (int j = 0; j < dp; ++j) dot = fmaf(x[j], C[(int64_t)c * dp + j], dot);
+        const uint64_t key = make_key(f2ord(fmaf(-2.f, dot, cnorm[c])), (uint32_t)c);
+        best = key < best ? key : best;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t other = __shfl_xor_sync(0xffffffffu, best, o);
+        best = other < best ? other : best;
+    }
+    return (int32_t)key_idx(best);
+}
+
+// The nearest centroid so far of a warp's eight rows, over this lane's columns, which
+// come in ascending order (a key of score and index per product took nine
+// instructions, a compare and two selects take four with the score itself).
+struct AssignBest {
+    float v[8];
+    int c[8];
+    f32x2 sum[8];  // of the products: finite only if all of them are
+    __device__ __forceinline__ void init() {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            v[i] = INFINITY;
+            c[i] = 0;
+            sum[i] = 0ull;
+        }
+    }
+    // cn: |c|^2 of column gt_col(p) + e, +inf past the last
+    template <int H, typename Norm>
+    __device__ __forceinline__ void add(const f32x2 (&acc)[8][2 * H], int c0, Norm &&cn) {
+#pragma unroll
+        for (int p = 0; p < 2 * H; ++p) {
+            const int col = c0 + gt_col(p);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sum[i] = add2(sum[i], acc[i][p]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float norm = cn(col + e);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    float lo, hi;
+                    unpack2(acc[i][p], lo, hi);
+                    const float x = fmaf(-2.f, e ? hi : lo, norm);
+                    const bool less = x < v[i];
+                    v[i] = less ? x : v[i];
+                    c[i] = less ? col + e : c[i];
+                }
+            }
+        }
+    }
+    // the labels of rows p0 .. p0 + 7 (those below p1); adds up the changed ones
+    __device__ __forceinline__ void finish(const float *__restrict__ X, int64_t p0, int64_t p1, int dp,
+                                           const float *__restrict__ C, const float *__restrict__ cnorm, int k,
+                                           int32_t *__restrict__ labels, unsigned long long *__restrict__ n_changed) {
+        const int lane = threadIdx.x & 31;
+        int32_t mine = 0;  // lane i: row i's label
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t o = f2ord(v[i]), top = __reduce_min_sync(0xffffffffu, o);
+            int32_t lab = (int32_t)__reduce_min_sync(0xffffffffu, o == top ? (unsigned)c[i] : 0xffffffffu);
+            float lo, hi;
+            unpack2(sum[i], lo, hi);
+            const bool odd = __any_sync(0xffffffffu, !(fabsf(lo) < INFINITY && fabsf(hi) < INFINITY));
+            if ((odd || top >= f2ord(INFINITY)) && p0 + i < p1)
+                lab = assign_unordered(X + (p0 + i) * dp, C, cnorm, k, dp);
+            if (lane == i) mine = lab;
+        }
+        const bool changed = lane < 8 && p0 + lane < p1 && labels[p0 + lane] != mine;
+        if (changed) labels[p0 + lane] = mine;
+        const unsigned m = __ballot_sync(0xffffffffu, changed);
+        if (lane == 0 && m) atomicAdd(n_changed, (unsigned long long)__popc(m));
+    }
+};
+
 template <int H>
 __global__ void __launch_bounds__(GT_THREADS, 2) kmeans_assign_kernel(const float *__restrict__ X, int64_t n, int dp,
                                                                       const float *__restrict__ C,
@@ -649,52 +731,110 @@ __global__ void __launch_bounds__(GT_THREADS, 2) kmeans_assign_kernel(const floa
     const int64_t p0 = (int64_t)blockIdx.x * GT_BM;
     if (threadIdx.x < GT_BM) arow[threadIdx.x] = (p0 + threadIdx.x < n) ? p0 + threadIdx.x : -1;
     __syncthreads();
-    const int tm = threadIdx.x >> 5, tn = threadIdx.x & 31;
-    uint64_t best[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) best[i] = KEY_EMPTY;
+    AssignBest best;
+    best.init();
     f32x2 acc[8][2 * H];
     for (int c0 = 0; c0 < k; c0 += GT_BN * H) {
         gt_tile<H>(s, acc, X, arow, dp, C, c0, k, dp, dp);
+        best.add<H>(acc, c0, [&](int c) { return c < k ? cnorm[c] : INFINITY; });
+    }
+    best.finish(X, p0 + (threadIdx.x >> 5) * 8, n, dp, C, cnorm, k, labels, n_changed);
+}
+
+// The same for centroids that fit shared memory beside a second block (128 H of them):
+// a block keeps them there over a run of rows and reads nothing but rows, whose next
+// slice is always in flight, also across tiles.  100k x 64 against 256 centroids: 92 us
+// with the centroids read again for every 64 rows, 84 us here (45 us of FP32
+// pipe).
+constexpr size_t ASSIGN_SMEM_MAX = 110 * 1024;
+template <int H>
+static size_t assign_smem(int dp) {
+    return (size_t)dp * (GT_BN * H + 4) * 4 + sizeof(GemmTileSmem<H>::As) + GT_BN * H * 4;
+}
+template <int H>
+__global__ void __launch_bounds__(GT_THREADS, 2)
+    kmeans_assign_resident_kernel(const float *__restrict__ X, int64_t n, int dp, const float *__restrict__ C,
+                                  const float *__restrict__ cnorm, int k, int per_block,
+                                  int32_t *__restrict__ labels, unsigned long long *__restrict__ n_changed) {
+    extern __shared__ __align__(16) uint8_t gt_raw[];
+    constexpr int BP = GT_BN * H + 4;
+    float2(*As)[GT_BK][GT_BM + 2] = reinterpret_cast<float2(*)[GT_BK][GT_BM + 2]>(gt_raw);
+    float *const Bs = reinterpret_cast<float *>(gt_raw + sizeof(GemmTileSmem<H>::As));  // [dp][BP]
+    float *const s_cn = Bs + (size_t)dp * BP;
+    const int t = threadIdx.x, tm = t >> 5, tn = t & 31;
+    const int dp4 = dp >> 2, nk = dp / GT_BK;
+    for (int i = t; i < GT_BN * H * dp4; i += GT_THREADS) {
+        const int c = i / dp4, j = i % dp4;
+        const float4 v = c < k ? __ldg(reinterpret_cast<const float4 *>(C + (int64_t)c * dp) + j)
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
+        Bs[(4 * j + 0) * BP + c] = v.x;
+        Bs[(4 * j + 1) * BP + c] = v.y;
+        Bs[(4 * j + 2) * BP + c] = v.z;
+        Bs[(4 * j + 3) * BP + c] = v.w;
+    }
+    for (int c = t; c < GT_BN * H; c += GT_THREADS) s_cn[c] = c < k ? cnorm[c] : INFINITY;
+    const int64_t p0 = (int64_t)blockIdx.x * per_block, p1 = min(n, p0 + per_block);
+    // this thread's float4 of each slice: row t / 4 of the tile, k 4 (t % 4) ..
+    const int r = t >> 2, k4 = t & 3;
+    float4 ra;
+    auto load = [&](int64_t tile, int kc) {
+        ra = tile + r < p1 ? __ldg(reinterpret_cast<const float4 *>(X + (tile + r) * dp) + kc * (GT_BK / 4) + k4)
+                           : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
+    auto store = [&](int buf) {
+        As[buf][4 * k4 + 0][r] = make_float2(ra.x, ra.x);
+        As[buf][4 * k4 + 1][r] = make_float2(ra.y, ra.y);
+        As[buf][4 * k4 + 2][r] = make_float2(ra.z, ra.z);
+        As[buf][4 * k4 + 3][r] = make_float2(ra.w, ra.w);
+    };
+    if (p0 < p1) {
+        load(p0, 0);
+        store(0);
+    }
+    __syncthreads();
+    int cur = 0;
+    for (int64_t tile = p0; tile < p1; tile += GT_BM) {
+        f32x2 acc[8][2 * H];
 #pragma unroll
-        for (int p = 0; p < 2 * H; ++p) {
-            const int c = c0 + gt_col(p);
+        for (int i = 0; i < 8; ++i)
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                if (c + e >= k) continue;
-                const float cn = cnorm[c + e];
+            for (int p = 0; p < 2 * H; ++p) acc[i][p] = 0ull;
+        const bool work = tile + tm * 8 < p1;  // else this warp has no rows in the last tile
+        for (int kc = 0; kc < nk; ++kc, cur ^= 1) {
+            const bool more = kc + 1 < nk || tile + GT_BM < p1;
+            if (kc + 1 < nk) load(tile, kc + 1);
+            else if (more) load(tile + GT_BM, 0);
+            if (work) {
+                const float *b = Bs + (size_t)kc * GT_BK * BP + tn * 4;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    float lo, hi;
-                    unpack2(acc[i][p], lo, hi);
-                    const float v = fmaf(-2.f, e ? hi : lo, cn);
-                    const uint64_t key = make_key(f2ord(v), (uint32_t)(c + e));
-                    best[i] = key < best[i] ? key : best[i];
+                for (int kk = 0; kk < GT_BK; ++kk) {
+                    f32x2 av[8], bv[2 * H];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(&As[cur][kk][tm * 8 + 2 * i]);
+                        av[2 * i] = x.x;
+                        av[2 * i + 1] = x.y;
+                    }
+#pragma unroll
+                    for (int h = 0; h < H; ++h) {
+                        const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(b + kk * BP + h * GT_BN);
+                        bv[2 * h] = x.x;
+                        bv[2 * h + 1] = x.y;
+                    }
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+#pragma unroll
+                        for (int p = 0; p < 2 * H; ++p) acc[i][p] = fma2(av[i], bv[p], acc[i][p]);
                 }
             }
+            if (more) store(cur ^ 1);
+            __syncthreads();
         }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        uint64_t b = best[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            uint64_t other = __shfl_xor_sync(0xffffffffu, b, o);
-            b = other < b ? other : b;
-        }
-        best[i] = b;
-    }
-    if (tn == 0) {
-        unsigned long long changed = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int64_t p = p0 + tm * 8 + i;
-            if (p < n) {
-                const int32_t lab = (int32_t)key_idx(best[i]);
-                if (labels[p] != lab) { labels[p] = lab; ++changed; }
-            }
-        }
-        if (changed) atomicAdd(n_changed, changed);
+        if (!work) continue;
+        AssignBest best;
+        best.init();
+        best.add<H>(acc, 0, [&](int c) { return s_cn[c]; });
+        best.finish(X, tile + tm * 8, p1, dp, C, cnorm, k, labels, n_changed);
     }
 }
 
@@ -790,17 +930,33 @@ int kmeans_l2_device(const float *X, int64_t n, int d, int dp, int64_t k, int64_
     std::vector<int64_t> hstat((size_t)k + 1);
     GN_CUDA_TRY(cudaFuncSetAttribute(kmeans_assign_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(GemmTileSmem<2>)));
+    GN_CUDA_TRY(cudaFuncSetAttribute(kmeans_assign_resident_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)ASSIGN_SMEM_MAX));
+    GN_CUDA_TRY(cudaFuncSetAttribute(kmeans_assign_resident_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)ASSIGN_SMEM_MAX));
+    // two blocks per SM, each with an equal run of rows (whole warps' eights)
+    const int64_t per_block = std::max<int64_t>(round_up(ceil_div(n, 2 * (int64_t)G), 8), GT_BM);
+    const unsigned blocks = (unsigned)ceil_div(n, per_block), tiles = (unsigned)ceil_div(n, GT_BM);
+    auto assign = [&]() {
+        if (k <= GT_BN && assign_smem<1>(dp) <= ASSIGN_SMEM_MAX && per_block < (1 << 30))
+            kmeans_assign_resident_kernel<1><<<blocks, GT_THREADS, assign_smem<1>(dp), st>>>(
+                X, n, dp, C, cnorm, (int)k, (int)per_block, labels, dchg);
+        else if (k > GT_BN && k <= 2 * GT_BN && assign_smem<2>(dp) <= ASSIGN_SMEM_MAX && per_block < (1 << 30))
+            kmeans_assign_resident_kernel<2><<<blocks, GT_THREADS, assign_smem<2>(dp), st>>>(
+                X, n, dp, C, cnorm, (int)k, (int)per_block, labels, dchg);
+        else if (k <= GT_BN)
+            kmeans_assign_kernel<1><<<tiles, GT_THREADS, sizeof(GemmTileSmem<1>), st>>>(X, n, dp, C, cnorm, (int)k,
+                                                                                        labels, dchg);
+        else
+            kmeans_assign_kernel<2><<<tiles, GT_THREADS, sizeof(GemmTileSmem<2>), st>>>(X, n, dp, C, cnorm, (int)k,
+                                                                                        labels, dchg);
+    };
     int64_t it = 0;
     for (; it < max_iter; ++it) {
         row_norms_kernel<<<(unsigned)ceil_div(k, 8), 256, 0, st>>>(C, k, dp, cnorm);
         GN_CUDA_TRY(cudaMemsetAsync(dstat.p, 0, hstat.size() * sizeof(int64_t), st));
         GN_CUDA_TRY(cudaMemsetAsync(dsum.p, 0, (size_t)k * dp * sizeof(double), st));
-        if (k <= GT_BN)
-            kmeans_assign_kernel<1><<<(unsigned)ceil_div(n, GT_BM), GT_THREADS, sizeof(GemmTileSmem<1>), st>>>(
-                X, n, dp, C, cnorm, (int)k, labels, dchg);
-        else
-            kmeans_assign_kernel<2><<<(unsigned)ceil_div(n, GT_BM), GT_THREADS, sizeof(GemmTileSmem<2>), st>>>(
-                X, n, dp, C, cnorm, (int)k, labels, dchg);
+        assign();
         kmeans_accumulate_kernel<<<(unsigned)ceil_div(n, 8), 256, 0, st>>>(X, n, d, dp, labels, dchg,
                                                                           dsum.as<double>(), dcnt);
         kmeans_finalize_kernel<<<(unsigned)ceil_div(k * dp, 256), 256, 0, st>>>(dsum.as<double>(), dcnt, (int)k, d, dp,

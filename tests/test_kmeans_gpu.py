@@ -46,3 +46,30 @@ def test_float_seeds_where_the_serial_sum_decides(gn, oracle, n, d, k, distinct)
     _, cent = gn.kmeans_l2(data, k, 0, 42)
     _, ocent, _ = oracle.kmeans_l2(data, k, 0, 42)
     assert np.array_equal(cent.view(np.uint32), ocent.view(np.uint32))
+
+
+@pytest.mark.parametrize("n,d,k", [(70, 3, 1), (513, 16, 127), (20_000, 20, 128), (19_457, 33, 129), (4100, 64, 255),
+                                   (40_001, 80, 256), (3000, 100, 256), (3000, 7, 300)])
+def test_labels_are_nearest_centroids(gn, n, d, k):
+    """One assignment, around 128 and 256 centroids and blocks of rows that end inside a
+    tile.  A score's error is at most (d + 3) 2^-24 (2 |x| |c| + |c|^2)."""
+    data = np.random.default_rng(n + k).standard_normal((n, d)).astype(np.float32)
+    _, seeds = gn.kmeans_l2(data, k, 0, 42)
+    labels, _ = gn.kmeans_l2(data, k, 1, 42)
+    x, c = data.astype(np.float64), np.asarray(seeds, np.float64)
+    cn = (c**2).sum(1)
+    score = cn - 2 * x @ c.T
+    err = (d + 3) * 2.0**-24 * (2 * np.sqrt((x**2).sum(1).max() * cn.max()) + cn.max())
+    assert (score[np.arange(n), labels] <= score.min(1) + 2 * err).all()
+
+
+@pytest.mark.parametrize("k", [5, 128, 256])
+def test_labels_where_scores_overflow(gn, k):
+    """Products that overflow (scores of +-inf and NaN): 240 zero columns more take the
+    labels to the other assignment kernel and change no sum."""
+    rng = np.random.default_rng(k)
+    data = (rng.integers(0, 2, (900, 16)) * 2 - 1).astype(np.float32) * np.float32(1e30)
+    data[::3] = rng.standard_normal((300, 16)).astype(np.float32)
+    labels = gn.kmeans_l2(data, k, 1, 42)[0]
+    wide = gn.kmeans_l2(np.pad(data, ((0, 0), (0, 240))), k, 1, 42)[0]
+    assert np.array_equal(labels, wide)

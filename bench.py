@@ -167,6 +167,14 @@ def num_sms() -> int:
     return n.value
 
 
+def last_kernel(lib):
+    """(milliseconds, name) of the last timed kernel."""
+    from pynear_gb300 import _lib
+    t, name = ctypes.c_float(), ctypes.create_string_buffer(64)
+    _lib.check(lib.gn_timing_last(ctypes.byref(t), name, 64))
+    return t.value, name.value.decode()
+
+
 def profile_traffic(kernel: str):
     """DRAM bytes per launch from the committed ncu summary, if present."""
     try:
@@ -551,9 +559,8 @@ def bench_flat_l2(args, dist, clocks_mhz):
         e0.record(stream)
         step()
         e1.record(stream)
-        t = ctypes.c_float()
-        _lib.check(lib.gn_timing_last(ctypes.byref(t), None, 0))
-        kern.append(t.value)
+        t, kernel = last_kernel(lib)
+        kern.append(t)
         torch.cuda.synchronize()
         ms.append(e0.elapsed_time(e1))
     lib.gn_timing_enable(0)
@@ -569,14 +576,20 @@ def bench_flat_l2(args, dist, clocks_mhz):
     flops = len(q) * len(db) * 32 * 3  # sub + FMA per element
     kms = statistics.mean(kern)
     mhz = clocks_mhz or 2070.0
-    peak = num_sms() * 128 * 2 * mhz * 1e6  # FP32 FMA lanes x 2 flops
+    if kernel == "tc_topk_kernel":  # candidates from split-BF16 products: 3 x 2 flops per element
+        flops = len(q) * len(db) * 32 * 6
+        roof = {"bound": "tensor", "peak": float(load_peaks()[0].get("bf16_tflops", 1900.0)),
+                "peak_source": "measured (MEASURED_PEAKS.json bf16_tflops, burst)"}
+    else:
+        roof = {"bound": "fp32", "peak": num_sms() * 128 * 2 * mhz * 1e6 / 1e12,  # FP32 FMA lanes x 2 flops
+                "peak_source": f"derived: 128 FP32 FMA/clk/SM x SMs x {mhz:.0f} MHz"}
+    tflops = flops / (kms / 1e3) / 1e12
     return {"value": len(q) * steps * dist.ws / tot, "unit": "queries/s", "ms_per_step": statistics.mean(ms),
             "config": {"n": len(db), "d": 32, "queries_per_step": len(q), "k": 5,
                        "l2": "flushed between steps (256 MB write)"},
             "indices_equal_oracle_100q": bool(np.array_equal(gi, oi)),
-            "roofline": {"bound": "fp32", "kernel": "float_scan_kernel", "achieved": flops / (kms / 1e3) / 1e12,
-                         "peak": peak / 1e12, "unit": "TFLOP/s", "frac": flops / (kms / 1e3) / peak,
-                         "kernel_ms": kms, "peak_source": f"derived: 128 FP32 FMA/clk/SM x SMs x {mhz:.0f} MHz",
+            "roofline": {**roof, "kernel": kernel, "achieved": tflops, "unit": "TFLOP/s", "frac": tflops / roof["peak"],
+                         "kernel_ms": kms,
                          "note": "latency-bound at this size (12.8 MB database, 1,000 queries)"}}
 
 
@@ -586,8 +599,9 @@ def bench_flat_l2_hbm(args, dist, peaks, clocks_mhz):
     than L2 (1,000,000 x 128 float32, 512 MB): with 1 or 8 queries per call
     the scan streams the database once per call and is bound by HBM (reported
     in GB/s of database read against the measured copy bandwidth); with 1,024
-    queries per call it is bound by the FP32 pipe (3 flops per element and
-    query).  Indices checked against the oracle on a subset."""
+    queries per call the candidates come from the tensor cores (split BF16: 6
+    flops per element and query) or, where they don't, from the FP32 pipe (3).
+    Indices checked against the oracle on a subset."""
     import torch
     import pynear_gb300 as gn
     from pynear_gb300 import _lib
@@ -625,9 +639,8 @@ def bench_flat_l2_hbm(args, dist, peaks, clocks_mhz):
         e0.record(stream)
         for _ in range(steps):
             step()
-            t = ctypes.c_float()
-            _lib.check(lib.gn_timing_last(ctypes.byref(t), None, 0))
-            kern.append(t.value)
+            t, kernel = last_kernel(lib)
+            kern.append(t)
         e1.record(stream)
         torch.cuda.synchronize()
         lib.gn_timing_enable(0)
@@ -637,17 +650,22 @@ def bench_flat_l2_hbm(args, dist, peaks, clocks_mhz):
         oi, _ = oracle.knn_float("l2", db, q[:sub], K)
         ok = bool(np.array_equal(d_idx[:sub].cpu().numpy(), oi))
         gbs = db.nbytes / (kms / 1e3) / 1e9
-        flops = 3.0 * nq * db.size
+        flops = (6.0 if kernel == "tc_topk_kernel" else 3.0) * nq * db.size
         entry = {"value": nq / (ms / 1e3), "unit": "queries/s", "ms_per_call": ms, "kernel_ms": kms,
-                 "indices_equal_oracle": ok, "db_read_gbs": gbs, "fp32_tflops": flops / (kms / 1e3) / 1e12}
+                 "indices_equal_oracle": ok, "db_read_gbs": gbs, "tflops": flops / (kms / 1e3) / 1e12}
         if nq <= 8:
             entry["roofline"] = {"bound": "hbm", "kernel": "float_scan_kernel", "achieved": gbs, "peak": hbm_peak,
                                  "unit": "GB/s", "frac": gbs / hbm_peak,
                                  "traffic": profile_traffic(f"float_scan_kernel_q{nq}"),
                                  "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)",
                                  "algorithmic_per_launch": {"bytes": int(db.nbytes)}}
+        elif kernel == "tc_topk_kernel":
+            peak = float(peaks.get("bf16_tflops", 1900.0))
+            entry["roofline"] = {"bound": "tensor", "kernel": kernel, "achieved": flops / (kms / 1e3) / 1e12,
+                                 "peak": peak, "unit": "TFLOP/s", "frac": flops / (kms / 1e3) / 1e12 / peak,
+                                 "peak_source": "measured (MEASURED_PEAKS.json bf16_tflops, burst)"}
         else:
-            entry["roofline"] = {"bound": "fp32", "kernel": "float_scan_kernel",
+            entry["roofline"] = {"bound": "fp32", "kernel": kernel,
                                  "achieved": flops / (kms / 1e3) / 1e12, "peak": fp32_peak / 1e12, "unit": "TFLOP/s",
                                  "frac": flops / (kms / 1e3) / fp32_peak,
                                  "peak_source": f"derived: 128 FP32 FMA/clk/SM x SMs x {mhz:.0f} MHz"}
@@ -697,15 +715,16 @@ def bench_voronoi(args, dist, clocks_mhz):
         import oracle
         rows = np.linspace(0, h - 1, 8).astype(np.int64)
         oi, _ = oracle.voronoi_raster(seeds, xs, ys[rows])
-        pairs = w * h * ns
-        # per pixel-seed pair: subtract, multiply, add, compare = 4 FP32-pipe instructions
-        peak_pairs = num_sms() * 128 * mhz * 1e6 / 4
+        # the ids are what a raster has to write; tiles drop the seeds that cannot be nearest,
+        # so the pixel-seed pairs of the brute force are given only for comparison
+        hbm = float(load_peaks()[0].get("hbm_gbs", 6800.0))
+        gbs = w * h * 4 / (ms / 1e3) / 1e9
         out[f"seeds_{ns}"] = {
             "value": w * h * dist.ws / (ms / 1e3), "unit": "pixels/s", "ms_per_raster": ms,
             "ids_equal_oracle_8_rows": bool(np.array_equal(r.ids[rows].cpu().numpy(), oi)),
-            "roofline": {"bound": "fp32 issue", "achieved": pairs / (ms / 1e3) / 1e12, "unit": "T pairs/s",
-                         "peak": peak_pairs / 1e12, "frac": pairs / (ms / 1e3) / peak_pairs,
-                         "peak_source": f"derived: 128 FP32 lanes/clk/SM x SMs x {mhz:.0f} MHz / 4 instr per pair"}}
+            "brute_force_pairs_per_s": w * h * ns / (ms / 1e3),
+            "roofline": {"bound": "hbm", "achieved": gbs, "unit": "GB/s", "peak": hbm, "frac": gbs / hbm,
+                         "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)"}}
     return out
 
 
@@ -831,9 +850,8 @@ def bench_hamming(args, dist, peaks, clocks_mhz):
         e0.record(stream)
         step()
         e1.record(stream)
-        t = ctypes.c_float()
-        _lib.check(lib.gn_timing_last(ctypes.byref(t), None, 0))
-        kern.append(t.value)
+        t, kernel = last_kernel(lib)
+        kern.append(t)
         flush.zero_()  # the 64 MB database fits in L2: flush between steps
         torch.cuda.synchronize()
         ms.append(e0.elapsed_time(e1))
@@ -848,14 +866,19 @@ def bench_hamming(args, dist, peaks, clocks_mhz):
     popc = nq * len(db) * words
     mhz = clocks_mhz or 2070.0
     peak = POPC_PER_CLK_PER_SM * num_sms() * mhz * 1e6
+    if kernel == "tc_topk_kernel":  # +-1 products in FP8: 2 flops per bit
+        tflops, fp8 = 2.0 * nq * len(db) * nbytes * 8 / (kms / 1e3) / 1e12, 2 * float(load_peaks()[0].get("bf16_tflops", 1900.0))
+        roof = {"bound": "tensor", "kernel": kernel, "achieved": tflops, "peak": fp8, "unit": "TFLOP/s",
+                "frac": tflops / fp8, "peak_source": "2 x measured (MEASURED_PEAKS.json bf16_tflops, burst)"}
+    else:
+        roof = {"bound": "int", "kernel": kernel, "achieved": popc / (kms / 1e3) / 1e9, "peak": peak / 1e9,
+                "unit": "Gpopc/s", "frac": popc / (kms / 1e3) / peak,
+                "peak_source": f"derived: {POPC_PER_CLK_PER_SM} POPC/clk/SM x SMs x {mhz:.0f} MHz"}
     return {"value": nq * steps * dist.ws / tot, "unit": "queries/s", "ms_per_step": statistics.mean(ms),
             "config": {"n": len(db), "bits": nbytes * 8, "queries_per_step": nq, "k": K, "flips": 24,
                        "l2": "flushed between steps (256 MB write)"},
-            "roofline": {"bound": "int", "kernel": "hamming_scan_kernel", "achieved": popc / (kms / 1e3) / 1e9,
-                         "peak": peak / 1e9, "unit": "Gpopc/s", "frac": popc / (kms / 1e3) / peak,
-                         "traffic": profile_traffic("hamming_scan_kernel"), "kernel_ms": kms,
-                         "algorithmic_per_launch": {"popc": popc, "int_ops": 3 * popc, "db_bytes": int(db.nbytes)},
-                         "peak_source": f"derived: {POPC_PER_CLK_PER_SM} POPC/clk/SM x SMs x {mhz:.0f} MHz"},
+            "roofline": {**roof, "traffic": profile_traffic(f"{kernel}_hamming"), "kernel_ms": kms,
+                         "algorithmic_per_launch": {"popc": popc, "int_ops": 3 * popc, "db_bytes": int(db.nbytes)}},
             "check": {"planted_row_first": found}, "data": (db, q)}
 
 

@@ -15,7 +15,7 @@ struct IvfScratch {
         cpart, nprobed, qbound,  // qbound: per query, the ordered score bound of the tensor-core list scan
         ckeys,                   // learned probing on the FP32 engine: nearest lists as keys
         ccount, lbuf,            // FP32 scan: candidates per query (part holds them), the CTAs' list buffers
-        mh1, mcand, mcb, mqn;    // batched prober MLP: first-layer outputs, candidates, their bounds, |q|^2
+        mfeat, mcand, mcb, mqn;  // batched prober MLP: candidates' features, candidates, their bounds, |q|^2
 };
 
 // Float IVF (forest.py IVFFlatL2Index semantics, squared L2).

@@ -667,31 +667,36 @@ __device__ __forceinline__ void probe_candidates(const float *__restrict__ sq, i
 }
 
 // Per query (block of NW warps): the 64 best centroids by BF16 score, their
-// exact squared distances (FP32), sorted nearest first; then either the first
-// np of them (fixed probing) or the learned prober's choice (MLP fused here).
-// The candidates are the 64 smallest keys (BF16 score, centroid): every warp
-// counts for itself, so that no barrier stands between the scores and the
-// distances; these are split over the warps, four candidates at a time.  Measured with
+// exact squared distances (FP32), sorted nearest first; then the first np of them
+// (PROBE_FIXED), the learned prober's choice (PROBE_MLP, fused here) or, for
+// mlp_probe_kernel, all of them with their features (PROBE_CANDS).
+// The candidates are the 64 smallest keys (BF16 score, centroid), counted by one
+// warp; the distances are split over the warps, four candidates at a time.  Measured with
 // 1,024 centroids of 512 dimensions: 88 us for 4,096 queries with a block-wide radix
 // select, 49 here (their 537 MB of centroid rows come from L2).
-template <bool MLP, int NW>
+enum { PROBE_FIXED, PROBE_MLP, PROBE_CANDS };
+template <int MODE, int NW>
 __global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW)
     coarse_probe_kernel(const float *__restrict__ scores, int nc, const float *__restrict__ Q, int d, int dp,
                         const float *__restrict__ C, int np, ProberWeights w, float logit_tau,
                         int32_t *__restrict__ probes, int32_t *__restrict__ nprobed,
                         const float *__restrict__ rho, int shortlist, float xmax,
-                        uint32_t *__restrict__ qbound, float *__restrict__ h1_out, int32_t *__restrict__ cand_out,
+                        uint32_t *__restrict__ qbound, float *__restrict__ feat_out, int32_t *__restrict__ cand_out,
                         float *__restrict__ cb_out, float *__restrict__ qn_out) {
     constexpr int NC = PROBER_CAND, H = PROBER_HIDDEN;
+    constexpr bool MLP = MODE == PROBE_MLP;
     static_assert(H == 256 && NC == 64, "warp-per-row MLP layout: 32 lanes x 8 weights, 8 warps x 8 candidates");
     static_assert(!MLP || NW == 8, "one thread per hidden unit");
-    __shared__ uint64_t buf[NW][SEL_BUF], best[NW][NC];
+    __shared__ uint64_t buf[SEL_BUF], best[NC];
     __shared__ float sd[NC];
     const int64_t q = blockIdx.x;
     const int j = threadIdx.x, lane = j & 31, warp = j >> 5;
     const float *sq = scores + q * nc, *qrow = Q + q * dp;
-    if (nc <= 512) probe_candidates<16>(sq, nc, buf[warp], best[warp], lane);
-    else probe_candidates<32>(sq, nc, buf[warp], best[warp], lane);
+    if (warp == 0) {
+        if (nc <= 512) probe_candidates<16>(sq, nc, buf, best, lane);
+        else probe_candidates<32>(sq, nc, buf, best, lane);
+    }
+    if (NW > 1) __syncthreads();
     {   // exact squared distances, four candidates together: each load instruction
         // reads 512 contiguous bytes of a centroid row
         const float4 *qr = reinterpret_cast<const float4 *>(qrow);
@@ -701,7 +706,7 @@ __global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW)
             const float *cr[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const uint64_t key = best[warp][i0 + u];
+                const uint64_t key = best[i0 + u];
                 cr[u] = C + (int64_t)(key == KEY_EMPTY ? 0 : key_idx(key)) * dp;
             }
             float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
@@ -753,7 +758,7 @@ __global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int i = h * 32 + lane;
-            const uint64_t c = best[0][i];
+            const uint64_t c = best[i];
             key[h] = c == KEY_EMPTY ? KEY_EMPTY : make_key(__float_as_uint(sd[i]), key_idx(c));
         }
         warp_sort<2>(key);
@@ -775,17 +780,23 @@ __global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW)
                     b = t * t;
                 }
             }
+            const float f =
+                e ? 0.f : fmaxf(0.f, 1.f - (__uint_as_float(key_dist(key[h])) - d1) / fmaxf(d1, 1e-12f));
             if (MLP) {
                 sc[i] = c;
-                sf[i] = e ? 0.f
-                          : fmaxf(0.f, 1.f - (__uint_as_float(key_dist(key[h])) - d1) / fmaxf(d1, 1e-12f));
+                sf[i] = f;
                 sb[i] = b;
+            } else if (MODE == PROBE_CANDS) {
+                cand_out[q * NC + i] = c;
+                feat_out[q * NC + i] = f;
+                cb_out[q * NC + i] = b;
             } else if (i < np) {
                 probes[q * np + i] = c;
                 near = fminf(near, b);
             }
         }
-        if (!MLP && qbound) {
+        if (MODE == PROBE_CANDS && lane == 0) qn_out[q] = s_qn;
+        if (MODE == PROBE_FIXED && qbound) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) near = fminf(near, __shfl_xor_sync(0xffffffffu, near, o));
             if (lane == 0) qbound[q] = probe_bound_key(near, s_qn, xmax);
@@ -808,21 +819,6 @@ __global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW)
         a = fmaf(sf[i], wv, a);
     }
     sh1[j] = fmaxf(a, 0.f);
-    if (h1_out) {
-        // batched MLP: hand the first layer, the candidates, their bounds and
-        // |q|^2 to mlp_probe_kernel, which runs layers 2 and 3 for 8 queries
-        // per block (W2 read once per 8 queries instead of once per query)
-        h1_out[q * H + j] = sh1[j];
-        if (j < NC) {
-            cand_out[q * NC + j] = sc[j];
-            cb_out[q * NC + j] = sb[j];
-        }
-        if (warp == 2) {
-            const float qs = warp_sqnorm(qrow, d, lane);
-            if (lane == 0) qn_out[q] = qs;
-        }
-        return;
-    }
     __syncthreads();
     // layer 2: warp w computes outputs 32w .. 32w + 31, one W2 row (512 bytes,
     // lane l its 16 bytes) per load instruction, four rows in flight; lane l
@@ -930,8 +926,10 @@ __global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW)
     }
 }
 
-// Layers 2 and 3 of the prober and the probe choice for MLP_QB queries per
-// block (large batches; the first layer ran in coarse_probe_kernel):
+// The prober and its probe choice for MLP_QB queries per block (large batches, from
+// coarse_probe_kernel<PROBE_CANDS>'s candidates and features):
+//   layer 1  thread j = hidden unit j: the candidates' rows of W1, gathered,
+//            query by query, 32 loads in flight;
 //   layer 2  thread j = hidden unit j for the block's queries, its W2 row
 //            read once (16-byte loads), the queries' first-layer outputs from
 //            shared memory;
@@ -945,7 +943,7 @@ __global__ void __launch_bounds__(32 * NW, SEL_WARPS / NW)
 // product within a lane) matches the fused kernel's up to summation order.
 constexpr int MLP_QB = 8;
 constexpr int64_t MLP_BATCH_MIN = 1024;  // smaller batches keep the MLP fused in coarse_probe_kernel
-__global__ void __launch_bounds__(256) mlp_probe_kernel(const float *__restrict__ H1,
+__global__ void __launch_bounds__(256) mlp_probe_kernel(const float *__restrict__ feat,
                                                         const int32_t *__restrict__ cand,
                                                         const float *__restrict__ cb, const float *__restrict__ qnv,
                                                         int64_t nq, ProberWeights w, float logit_tau, float xmax,
@@ -956,9 +954,28 @@ __global__ void __launch_bounds__(256) mlp_probe_kernel(const float *__restrict_
     const int j = threadIdx.x, lane = j & 31, warp = j >> 5;
     const int64_t q0 = (int64_t)blockIdx.x * MLP_QB;
     const int nqb = (int)min((int64_t)MLP_QB, nq - q0);
-    for (int i = j; i < MLP_QB * H; i += 256) {
-        const int qq = i / H;
-        h1s[qq][i % H] = qq < nqb ? H1[(q0 + qq) * H + i % H] : 0.f;
+    __shared__ int32_t s_c[MLP_QB][NC];
+    __shared__ float s_f[MLP_QB][NC];
+    for (int i = j; i < MLP_QB * NC; i += 256) {
+        const bool in = i / NC < nqb;
+        s_c[i / NC][i % NC] = in ? cand[q0 * NC + i] : -1;
+        s_f[i / NC][i % NC] = in ? feat[q0 * NC + i] : 0.f;
+    }
+    __syncthreads();
+    {   // layer 1
+        const __nv_bfloat16 *W1 = reinterpret_cast<const __nv_bfloat16 *>(w.W1);
+        const float b1 = w.b1[j];
+#pragma unroll 1
+        for (int qq = 0; qq < MLP_QB; ++qq) {
+            float a = b1;
+#pragma unroll 32
+            for (int i = 0; i < NC; ++i) {
+                const int c = s_c[qq][i];
+                const float wv = c >= 0 ? __bfloat162float(W1[(size_t)c * H + j]) : 0.f;
+                a = fmaf(s_f[qq][i], wv, a);
+            }
+            h1s[qq][j] = fmaxf(a, 0.f);
+        }
     }
     __syncthreads();
     {   // layer 2
@@ -1105,33 +1122,40 @@ static int ivfl2_probes_tc(gn_index *ix, const float *dQ, int64_t nq, int *np_ou
     a.grid = (int)std::min<int64_t>(dev_info().num_sms, units);
     GN_TRY(tc_ivf_launch(a, st));
     ProberWeights w;
-    float *h1 = nullptr, *cbnd = nullptr, *qnv = nullptr;
+    float *feat = nullptr, *cbnd = nullptr, *qnv = nullptr;
     int32_t *cand = nullptr;
     if (mlp) {
         GN_TRY(prober_weights(S.prober, &w));
         GN_TRY(T.nprobed.ensure((size_t)nq * 4));
         if (nq >= MLP_BATCH_MIN) {  // layers 2 and 3 batched over 8 queries per block
-            GN_TRY(T.mh1.ensure((size_t)nq * PROBER_HIDDEN * 4));
+            GN_TRY(T.mfeat.ensure((size_t)nq * PROBER_CAND * 4));
             GN_TRY(T.mcand.ensure((size_t)nq * PROBER_CAND * 4));
             GN_TRY(T.mcb.ensure((size_t)nq * PROBER_CAND * 4));
             GN_TRY(T.mqn.ensure((size_t)nq * 4));
-            h1 = T.mh1.as<float>();
+            feat = T.mfeat.as<float>();
             cand = T.mcand.as<int32_t>();
             cbnd = T.mcb.as<float>();
             qnv = T.mqn.as<float>();
         }
-        coarse_probe_kernel<true, 8><<<(unsigned)nq, 256, 0, st>>>(
-            S.cscores.as<float>(), S.nc, dQ, S.d, S.dp, S.cent.as<float>(), np, w, S.prober_tau,
-            T.probes.as<int32_t>(), T.nprobed.as<int32_t>(), S.rho.as<float>(), S.shortlist, S.xmax,
-            T.qbound.as<uint32_t>(), h1, cand, cbnd, qnv);
-        if (h1)
+        auto probe = [&](auto MODEC, auto NWC) {
+            constexpr int MODE = decltype(MODEC)::value, NW = decltype(NWC)::value;
+            coarse_probe_kernel<MODE, NW><<<(unsigned)nq, 32 * NW, 0, st>>>(
+                S.cscores.as<float>(), S.nc, dQ, S.d, S.dp, S.cent.as<float>(), np, w, S.prober_tau,
+                T.probes.as<int32_t>(), T.nprobed.as<int32_t>(), S.rho.as<float>(), S.shortlist, S.xmax,
+                T.qbound.as<uint32_t>(), feat, cand, cbnd, qnv);
+        };
+        if (feat) {
+            warps_per_query(nq, 0, [&](auto NWC) { probe(std::integral_constant<int, PROBE_CANDS>(), NWC); });
             mlp_probe_kernel<<<(unsigned)ceil_div(nq, MLP_QB), 256, 0, st>>>(
-                h1, cand, cbnd, qnv, nq, w, S.prober_tau, S.xmax, T.probes.as<int32_t>(), T.nprobed.as<int32_t>(),
-                T.qbound.as<uint32_t>());
+                feat, cand, cbnd, qnv, nq, w, S.prober_tau, S.xmax, T.probes.as<int32_t>(),
+                T.nprobed.as<int32_t>(), T.qbound.as<uint32_t>());
+        } else {
+            probe(std::integral_constant<int, PROBE_MLP>(), std::integral_constant<int, 8>());
+        }
     } else {
         warps_per_query(nq, 0, [&](auto NWC) {
             constexpr int NW = decltype(NWC)::value;
-            coarse_probe_kernel<false, NW><<<(unsigned)nq, 32 * NW, 0, st>>>(
+            coarse_probe_kernel<PROBE_FIXED, NW><<<(unsigned)nq, 32 * NW, 0, st>>>(
                 S.cscores.as<float>(), S.nc, dQ, S.d, S.dp, S.cent.as<float>(), np, w, 0.f, T.probes.as<int32_t>(),
                 nullptr, S.rho.as<float>(), S.shortlist, S.xmax, T.qbound.as<uint32_t>(), nullptr, nullptr, nullptr,
                 nullptr);

@@ -1186,7 +1186,14 @@ __global__ void bin_assign_kernel(const uint4 *__restrict__ X, int64_t n, int w4
             const uint4 x0 = x[0], x1 = x[1], x2 = x[2], x3 = x[3];
             for (int c = 0; c < k; ++c) {
                 const uint4 *cc = sc + c * 4;
-                const uint32_t dd = popc4(x0, cc[0]) + popc4(x1, cc[1]) + popc4(x2, cc[2]) + popc4(x3, cc[3]);
+                const uint32_t dd = popc8(x0, cc[0], x1, cc[1]) + popc8(x2, cc[2], x3, cc[3]);
+                if (dd < best) { best = dd; bc = c; }
+            }
+        } else if (w4 == 2) {
+            const uint4 x0 = x[0], x1 = x[1];
+#pragma unroll 4
+            for (int c = 0; c < k; ++c) {
+                const uint32_t dd = popc8(x0, sc[2 * c], x1, sc[2 * c + 1]);
                 if (dd < best) { best = dd; bc = c; }
             }
         } else {

@@ -360,12 +360,17 @@ static int flat_search_dev(gn_index *ix, const void *d_q, int64_t nq, int64_t k,
     if (k <= FLAT_MAX_K_WARP) {
         flat_plan(a);
         if (!flat_smem_ok(a)) return fail(GN_ERR_UNSUPPORTED, "dimension too large for the exact flat scan");
-        GN_TRY(ix->part.ensure(flat_part_bytes(a)));
-        if (a.metric != M_HAMMING) {
-            GN_TRY(error_word());
-            a.status = status;
-            ix->status_set = status != nullptr;
+        if (a.metric == M_HAMMING) {
+            ham_plan(a);
+            GN_TRY(ix->part.ensure(ham_part_bytes(a)));
+            GN_TRY(ham_launch(a, ix->part.as<uint64_t>(), st));
+            GN_CUDA_TRY(cudaGetLastError());
+            return GN_OK;
         }
+        GN_TRY(ix->part.ensure(flat_part_bytes(a)));
+        GN_TRY(error_word());
+        a.status = status;
+        ix->status_set = status != nullptr;
         GN_TRY(flat_launch(a, ix->part.as<uint64_t>(), st));
     } else {
         // materialise keys for chunks of queries (<= 512 MB of keys per chunk)

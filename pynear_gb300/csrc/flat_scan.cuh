@@ -31,6 +31,10 @@ void flat_plan(FlatScanArgs &a);
 size_t flat_part_bytes(const FlatScanArgs &a);
 int flat_smem_ok(const FlatScanArgs &a);
 int flat_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st);
+// Hamming with scratch of any size (flat_plan and flat_launch: a caller's, in slices).
+void ham_plan(FlatScanArgs &a);
+size_t ham_part_bytes(const FlatScanArgs &a);
+int ham_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st);
 // The k nearest (k <= 256) of each query's qcount[q] candidate (distance, index)
 // keys at cand + q * list_keys, nearest first, with their number where out_cnt is given.
 // only_if, err, status: see FlatScanArgs.

@@ -73,7 +73,8 @@ constexpr int TC_COLS = TC_N / (TC_NEPI / 4);  // columns of a tile per epilogue
 constexpr int TC_THREADS = 64 + 32 * TC_NEPI;
 constexpr int TC_MAX_STAGES = 6;
 constexpr int TC_NR = 4;                // tiles of row norms (and scales) in flight
-constexpr int64_t TC_PILOT_MIN = 32768; // rows from which a pilot runs
+constexpr int64_t TC_PILOT_MIN = 256;   // rows from which a pilot runs
+constexpr int64_t TC_EXACT_MIN = 4096;  // ... and from which exact Hamming and L2 searches come here
 constexpr int64_t L2TC_QBLOCK = 8192;   // the same of the exact L2 search (longer candidate lists)
 constexpr int64_t TC_QBLOCK = 65536;    // queries scanned at a time (bounds the scratch)
 constexpr int TC_CAP = 128;             // entries of a buffer (S <= 64, and a block adds up to 32)
@@ -581,7 +582,7 @@ static int64_t tc_chunks(int64_t nqp, int64_t nt, int64_t lo, int64_t hi, int64_
 // Rows, not whole tiles, are sampled: where near rows stand together in the
 // database, tiles would miss most queries' neighbourhoods.
 int tc_pilot_stride(int64_t n) {
-    return n < TC_PILOT_MIN ? 1 : (int)std::max<int64_t>(1, std::min<int64_t>(8, n / 16384));
+    return (int)std::max<int64_t>(1, std::min<int64_t>(8, n / 16384));
 }
 
 // Every stride-th of n values, whole tiles of them (NaN past the last).
@@ -610,7 +611,9 @@ TcPlan tc_plan(int mode, int K, int64_t nq, int64_t n, int S) {
     // than they save in the last wave
     p.nchunks = (int)tc_chunks(nqp, nt, 1, std::min<int64_t>(64, std::max<int64_t>(1, ceil_div(5 * sms, nqp))), 2);
     // pilot: every 8th row (more where that would be under 16k rows), whole tiles
-    // of them; below 32k rows the lists' own first fill costs less than the launches
+    // of them.  It pays for small databases as well, where the units' buffers would
+    // fill with most rows they see: 24,813 x 126 rows, 2,956 queries, S 40: 1289 us per
+    // search without it, below 300 with it.
     if (n >= TC_PILOT_MIN) {
         p.pilot_stride = tc_pilot_stride(n);
         p.pilot_tiles = n / p.pilot_stride / TC_N;
@@ -861,11 +864,16 @@ struct HamTc {
 // any accumulator.  Measured per 1e10 pairs of 512 bits: 36.5 ms on the POPC
 // scan, 4.1 ms here; the expanded rows cost 8 bytes per packed byte, the
 // batch is padded to whole tiles of 128 queries and the pilot, the selection
-// and the launches take some 60 us, so batches below 128 queries, or of less
-// than half a millisecond on the POPC scan, stay there.
+// and the launches take some 60 to 100 us.  So batches below 128 queries stay on
+// the POPC scan, and those of less than half a millisecond there (2 G words; or,
+// where the expanded rows are small enough for the first search to make them in
+// passing, a quarter: a pair costs the POPC scan as much as 32 words do, its
+// selection included: 31,361 x 160 bits, 3,585 queries, k 3: 460 us there).
 bool ham_tc_wanted(const gn_index *ix, int64_t nq, int64_t k) {
     const int64_t words = ceil_div(ix->dim, 4);
-    return k <= 64 && ix->dim <= 512 && ix->n >= TC_PILOT_MIN && nq >= 128 && nq * ix->n >= 2000000000ll / words;
+    const bool small = ix->n * round_up(ix->dim * 8, TC_BK8) <= (int64_t)128 << 20;
+    const int64_t weight = small ? std::max<int64_t>(words, 32) : words;
+    return k <= 64 && ix->dim <= 512 && ix->n >= TC_EXACT_MIN && nq >= 128 && nq * ix->n >= 2000000000ll / weight;
 }
 
 // Returns GN_ERR_UNSUPPORTED where the expanded rows do not fit (the caller
@@ -1003,7 +1011,7 @@ struct L2Tc {
 // batches of less than 1.5 G elements stay there, and small ones, which fill
 // a part of a 128-query tile.
 bool l2_tc_wanted(const gn_index *ix, int64_t nq, int64_t k) {
-    if (k > 32 || ix->n < TC_PILOT_MIN || nq < 64 || ix->dim > 2048) return false;
+    if (k > 32 || ix->n < TC_EXACT_MIN || nq < 64 || ix->dim > 2048) return false;
     if (ix->ext) {
         const L2Tc &H = *reinterpret_cast<const L2Tc *>(ix->ext);
         if (H.refused || (H.hflag.p && *reinterpret_cast<volatile int *>(H.hflag.p))) return false;

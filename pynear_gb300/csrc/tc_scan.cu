@@ -867,12 +867,12 @@ struct HamTc {
 // and the launches take some 60 to 100 us.  So batches below 128 queries stay on
 // the POPC scan, and those of less than half a millisecond there (2 G words; or,
 // where the expanded rows are small enough for the first search to make them in
-// passing, a quarter: a pair costs the POPC scan as much as 32 words do, its
-// selection included: 31,361 x 160 bits, 3,585 queries, k 3: 460 us there).
+// passing, half of that or 62 M pairs, which cost the POPC scan's selection as much:
+// 31,361 x 160 bits, 3,585 queries, k 3: 410 us a search there, 189 here).
 bool ham_tc_wanted(const gn_index *ix, int64_t nq, int64_t k) {
     const int64_t words = ceil_div(ix->dim, 4);
     const bool small = ix->n * round_up(ix->dim * 8, TC_BK8) <= (int64_t)128 << 20;
-    const int64_t weight = small ? std::max<int64_t>(words, 32) : words;
+    const int64_t weight = small ? std::max<int64_t>(2 * words, 32) : words;
     return k <= 64 && ix->dim <= 512 && ix->n >= TC_EXACT_MIN && nq >= 128 && nq * ix->n >= 2000000000ll / weight;
 }
 

@@ -440,10 +440,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     __syncwarp();
                     if (lane == 0) mbar_arrive(accempty + b);
                     block(acc, 1);
-                    if (MODE != TC_SIGN && qt == nqt - 1) {
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(nempty + ns);
-                    }
+                    if (MODE != TC_SIGN && qt == nqt - 1) mbar_release_warp(nempty + ns);
                     if (QT == 2 && nqt == 2) {  // the other query tile's turn
                         const float tf = thr[0], tq = qc[0];
                         const int ti = cnt[0];

@@ -461,8 +461,7 @@ __global__ void __launch_bounds__(FS_THREADS, 3)
             kc = 0;
             y0 += a.rows;
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(empty + slot);
+        mbar_release_warp(empty + slot);
         if (++slot == FS_STAGES) {
             slot = 0;
             ph ^= 1;

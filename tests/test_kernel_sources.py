@@ -1,0 +1,34 @@
+"""Rules that the kernels' pipelines keep and that no run can show reliably, checked in
+the sources."""
+import os
+import re
+
+REPO = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(REPO, "pynear_gb300", "csrc")
+
+
+def _source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        text = f.read()
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def _body(text, kernel):
+    """The definition of a kernel, from its name to its closing brace."""
+    at = re.search(r"\b%s\(const __grid_constant__" % kernel, text).start()
+    i = text.index("{", at)
+    depth = 0
+    for j in range(i, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[j], 0)
+        if depth == 0:
+            return text[i:j + 1]
+    raise AssertionError(kernel)
+
+
+def test_slots_read_by_ordinary_loads_are_released_behind_a_proxy_fence():
+    """A slot that copies refill and that a warp reads with ordinary loads: the release
+    has to order those loads before the copies' writes (mbar_release_warp)."""
+    scan = _body(_source("flat_scan.cu"), "float_scan_kernel")
+    assert "mbar_release_warp(empty + slot)" in scan and "mbar_arrive(" not in scan
+    topk = _body(_source("tc_scan.cu"), "tc_topk_kernel")
+    assert "mbar_release_warp(nempty + ns)" in topk and "mbar_arrive(nempty" not in topk

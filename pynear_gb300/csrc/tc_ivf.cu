@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(TI_THREADS, 1)
         bool ok = true;
         for (uint32_t ui = 0; ok; ++ui) {
             const int r = ui % TI_UR;
-            if (!mbar_wait(ufull + r, (ui / TI_UR) & 1, verr, wait_limit)) break;
+            if (!mbar_wait_warp(ufull + r, (ui / TI_UR) & 1, verr, wait_limit)) break;
             const int64_t u = uring[r];
             const TcUnit un = uunit[r];
             __syncwarp();
@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(TI_THREADS, 1)
                 const bool rok = row < un.r1;
                 const float xn = xn_next;
                 if (t + 2 < ntile) xn_next = xload(t + 2);
-                if (!mbar_wait(accfull + b, tph, verr, wait_limit)) { ok = false; break; }
+                if (!mbar_wait_warp(accfull + b, tph, verr, wait_limit)) { ok = false; break; }
                 tc_fence_after();
 #pragma unroll 1
                 for (int cc = 0; grp + 2 * cc < nchunk; ++cc) {

@@ -354,9 +354,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 #pragma unroll 1
                 for (int qt = 0; qt < nqt; ++qt, ++vt) {
                     const int b = vt & 1;
-                    if (!mbar_wait(accfull + b, (vt >> 1) & 1, verr)) { ok = false; break; }
+                    if (!mbar_wait_warp(accfull + b, (vt >> 1) & 1, verr)) { ok = false; break; }
                     tc_fence_after();
-                    if (MODE != TC_SIGN && qt == 0 && !mbar_wait(nfull + ns, (tile_it / TC_NR) & 1, verr)) {
+                    if (MODE != TC_SIGN && qt == 0 && !mbar_wait_warp(nfull + ns, (tile_it / TC_NR) & 1, verr)) {
                         ok = false;
                         break;
                     }

@@ -32,3 +32,33 @@ def test_slots_read_by_ordinary_loads_are_released_behind_a_proxy_fence():
     assert "mbar_release_warp(empty + slot)" in scan and "mbar_arrive(" not in scan
     topk = _body(_source("tc_scan.cu"), "tc_topk_kernel")
     assert "mbar_release_warp(nempty + ns)" in topk and "mbar_arrive(nempty" not in topk
+
+
+def _waits_outside_one_thread(body):
+    """mbar_wait calls in code that a whole warp runs and whose results may differ
+    between its lanes."""
+    found, scopes, i = [], [], 0
+    head = ""  # text since the last brace or semicolon: what a block opens with
+    for m in re.finditer(r"[{};]|\bmbar_wait\(", body):
+        head += body[i:m.start()]
+        i = m.end()
+        if m.group() == "{":
+            scopes.append(head)
+            head = ""
+        elif m.group() == "}":
+            scopes.pop()
+            head = ""
+        elif m.group() == ";":
+            head = ""
+        else:
+            one = any(re.search(r"if \(.*(lane|threadIdx\.x) == 0\b", s) for s in scopes)
+            if not one and "__all_sync(0xffffffffu" not in head:
+                found.append(head.strip() + " mbar_wait")
+            head += m.group()
+    return found
+
+
+def test_waits_of_a_warp_have_one_answer():
+    for name, kernel in (("flat_scan.cu", "float_scan_kernel"), ("tc_scan.cu", "tc_topk_kernel"),
+                         ("tc_ivf.cu", "tc_ivf_kernel")):
+        assert not _waits_outside_one_thread(_body(_source(name), kernel)), kernel

@@ -197,24 +197,25 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     if (warp == 0) {
         // ── TMA producer ──
         if (lane == 0) {
-            uint32_t it = 0, un = 0, tile_it = 0;
+            uint32_t it = 0, aloads = 0, nloads = 0;  // copies issued: slices, units' queries, tiles' norms
             int sl = 0;
             uint32_t ph = 1;  // parity of the ring pass before this one: slots start free
             bool ok = true;
-            for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x, ++un) {
+            for (int64_t u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
                 int64_t q0, t0, t1;
                 int na;
                 unit(u, q0, na, t0, t1);
                 const int nqt = QT == 2 && na > TC_M ? 2 : 1;
                 if (res) {  // the unit's queries, once the previous unit's MMAs have read theirs
-                    if (!mbar_wait(aempty, (un & 1) ^ 1, verr)) { ok = false; break; }
+                    if (!mbar_wait(aempty, (aloads & 1) ^ 1, verr)) { ok = false; break; }
                     mbar_expect_tx(afull, (uint32_t)(nqt * nk) * TC_ASLICE);
                     for (int qt = 0; qt < nqt; ++qt)
                         for (int kb = 0; kb < nk; ++kb)
                             tma_load_2d(sA + (size_t)(qt * nk + kb) * TC_ASLICE, &tmA, kb * a.kblk,
                                         (int)(q0 + qt * TC_M), afull);
+                    ++aloads;
                 }
-                for (int64_t t = t0; t < t1 && ok; ++t, ++tile_it) {
+                for (int64_t t = t0; t < t1 && ok; ++t) {
                     const int n0 = (int)(t * TC_N);
                     for (int kb = 0; kb < nk; ++kb, ++it) {
                         if (!mbar_wait(empty + sl, ph, verr)) { ok = false; break; }
@@ -228,11 +229,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                         }
                     }
                     if (MODE != TC_SIGN && ok) {
-                        const int ns = tile_it % TC_NR;
-                        if (!mbar_wait(nempty + ns, ((tile_it / TC_NR) & 1) ^ 1, verr)) { ok = false; break; }
+                        const int ns = nloads % TC_NR;
+                        if (!mbar_wait(nempty + ns, ((nloads / TC_NR) & 1) ^ 1, verr)) { ok = false; break; }
                         mbar_expect_tx(nfull + ns, TC_N * 4 * (MODE == TC_FP8 ? 2 : 1));
                         bulk_load(snorm + ns * TC_N, a.bnorm + n0, TC_N * 4, nfull + ns);
                         if (MODE == TC_FP8) bulk_load(sscale + ns * TC_N, a.bscale + n0, TC_N * 4, nfull + ns);
+                        ++nloads;
                     }
                 }
             }
@@ -243,10 +245,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     }
                 };
                 for (uint32_t x = it > (uint32_t)ST ? it - ST : 0; x < it; ++x) settle(full + x % ST, (x / ST) & 1);
-                if (MODE != TC_SIGN)
-                    for (uint32_t x = tile_it > TC_NR ? tile_it - TC_NR : 0; x < tile_it; ++x)
-                        settle(nfull + x % TC_NR, (x / TC_NR) & 1);
-                if (res) settle(afull, un & 1);
+                for (uint32_t x = nloads > TC_NR ? nloads - TC_NR : 0; x < nloads; ++x)
+                    settle(nfull + x % TC_NR, (x / TC_NR) & 1);
+                if (aloads) settle(afull, (aloads - 1) & 1);
             }
         }
     } else if (warp == 1) {

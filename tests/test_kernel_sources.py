@@ -62,3 +62,18 @@ def test_waits_of_a_warp_have_one_answer():
     for name, kernel in (("flat_scan.cu", "float_scan_kernel"), ("tc_scan.cu", "tc_topk_kernel"),
                          ("tc_ivf.cu", "tc_ivf_kernel")):
         assert not _waits_outside_one_thread(_body(_source(name), kernel)), kernel
+
+
+def test_an_early_end_waits_for_the_copies_that_were_issued():
+    """The producer of a tensor-core scan whose wait ran out: what it waits for before
+    the block ends is counted at the copies (a unit's or a tile's own count has moved on
+    by then, and the other parity of a barrier is no wait at all)."""
+    body = _body(_source("tc_scan.cu"), "tc_topk_kernel")
+    at = body.index("auto settle")
+    ends = re.findall(r"settle\(([^;]*)\);", body[at:])
+    assert len(ends) == 3 and "(aloads - 1) & 1" in ends[2]
+    issue = body[:at]
+    assert re.search(r"&tmA[^;]*afull\);\s*\+\+aloads;", issue)
+    assert re.search(r"bulk_load\(sscale[^;]*;\s*\+\+nloads;", issue)
+    assert issue.count("++aloads") == 1 and issue.count("++nloads") == 1
+    assert "nloads" in ends[1] or "x < nloads" in body[at:]

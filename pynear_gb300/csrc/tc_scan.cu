@@ -938,14 +938,15 @@ int ham_tc_search(gn_index *ix, const void *d_q, int64_t nq, int k, int64_t *d_i
 // ── exact L2 k-NN of large batches ────────────────────────────────────────
 // The exact scan's answer (indices, and distances bit for bit) through the
 // tensor cores.  Each FP32 value is split into two BF16 parts, v = hi + lo + r with
-// |lo| <= 2^-9 |v| and |r| <= 2^-18 |v|, and rows are laid out as [hi | lo | hi], the
-// query as [hi | hi | lo], so that one GEMM sums hi hi + hi lo + lo hi.  The
-// score a = |x|^2 - 2 acc then differs from D - |q|^2 (D the squared distance in
-// exact arithmetic) by at most
+// |lo| <= L |v| and |r| <= L^2 |v|, L = 2^-8 (BF16 keeps eight significant bits), and
+// rows are laid out as [hi | lo | hi], the query as [hi | hi | lo], so that one GEMM
+// sums hi hi + hi lo + lo hi.  Left out are lo lo, r times a row's value and a query's
+// hi + lo times r: (3 + L^2) L^2 |q||x| at most.  The score a = |x|^2 - 2 acc then differs
+// from D - |q|^2 (D the squared distance in exact arithmetic) by at most
 //     E = cross |q| max|x| + norm max|x|^2:
-// cross >= 2 (3 2^-18 + u), the products left out and u |q||x| for the FP32 sums
-// of K terms in the tensor core, for which u = 2^-14 per 512 terms is allowed, a
-// thousand roundings of 2^-24 each; norm: the row norms' own FP32 sums.
+// cross = 2 (SPLIT_LEFT + u), u |q||x| for the FP32 sums of K terms in the tensor
+// core, for which u = 2^-14 per 512 terms is allowed, a thousand roundings of 2^-24
+// each; norm: the row norms' own FP32 sums.
 //
 // The pilot gives B, a score that k rows reach.  Their D is at most B + |q|^2 +
 // E, and the FP32 distance of any row lies within a relative g = (d / 8 + 16) 2^-23
@@ -958,6 +959,8 @@ int ham_tc_search(gn_index *ix, const void *d_q, int64_t nq, int k, int64_t *d_i
 // a flag is set and the FP32 scan, launched behind it, answers instead (it ends
 // at once when the flag is clear); the index then stays with the FP32 scan until
 // the next set().
+constexpr float SPLIT_LO = 0x1p-8f;                              // L
+constexpr float SPLIT_LEFT = 3.01f * SPLIT_LO * SPLIT_LO;        // the products left out, of |q||x|
 __global__ void split_rows_kernel(const float *__restrict__ X, int64_t n, int d, int ldx, bool query,
                                   __nv_bfloat16 *__restrict__ out, int K) {
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1087,7 +1090,7 @@ int l2_tc_search(gn_index *ix, const float *d_q, int64_t nq, int k, int64_t *d_i
         a.slack.q2 = H.qnorm.as<float>();
         a.slack.xmax2 = H.xmax2.as<uint32_t>();
         a.slack.overflow = H.flag.as<int>();
-        a.slack.cross = 2.f * (0x1p-16f + 0x1p-14f * (float)ceil_div(K, 512));
+        a.slack.cross = 2.f * (SPLIT_LEFT + 0x1p-14f * (float)ceil_div(K, 512));
         a.slack.norm = (float)(d / 32 + 16) * 0x1p-23f;
         a.slack.rel = 4.f * g;
         timing_begin(st, "tc_topk_kernel");

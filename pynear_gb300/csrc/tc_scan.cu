@@ -957,8 +957,9 @@ int ham_tc_search(gn_index *ix, const void *d_q, int64_t nq, int k, int64_t *d_i
 // order, and the k nearest returned.  If some buffer could not hold its rows (many
 // ties, or values so large against their differences that E spans most rows),
 // a flag is set and the FP32 scan, launched behind it, answers instead (it ends
-// at once when the flag is clear); the index then stays with the FP32 scan until
-// the next set().
+// at once when the flag is clear).  One such search says little (a query that is not
+// a number is enough), several in a row that the rows are not for this path: see
+// l2_tc_given_up.
 constexpr float SPLIT_LO = 0x1p-8f;                              // L
 constexpr float SPLIT_LEFT = 3.01f * SPLIT_LO * SPLIT_LO;        // the products left out, of |q||x|
 __global__ void split_rows_kernel(const float *__restrict__ X, int64_t n, int d, int ldx, bool query,
@@ -999,12 +1000,29 @@ __global__ void __launch_bounds__(RR_WARPS * 32)
 
 // Expanded operands and scratch of an L2 index, made by its first large search.
 struct L2Tc {
-    HBuf hflag;  // the flag of an earlier search (copied behind it; freed after the device buffers)
+    HBuf hflag;  // the flag of the last search done, -1 once it is counted (freed after the device buffers)
     DBuf x16, xnorm, pnorm, xmax2, q16, qnorm, part, qcount, flag;
     TcScratch scr;
     bool built = false, refused = false;
     int K = 0;
+    int overflows = 0, passed_by = 0;  // searches in a row that set the flag, and searches since then
 };
+
+// The FP32 scan alone answers where it had to answer L2TC_OVERFLOWS searches in a row,
+// but for every L2TC_RETRY-th search: a batch of odd queries is forgotten again, and
+// rows that never fit cost a 32nd of the tensor-core scan's time at most.
+constexpr int L2TC_OVERFLOWS = 4, L2TC_RETRY = 32;
+static bool l2_tc_given_up(L2Tc &H) {
+    if (!H.hflag.p) return false;
+    volatile int *word = reinterpret_cast<volatile int *>(H.hflag.p);
+    const int flag = *word;  // (a copy that lands in between is not counted)
+    if (flag >= 0) {
+        H.overflows = flag ? H.overflows + 1 : 0;
+        *word = -1;
+    }
+    if (H.overflows < L2TC_OVERFLOWS) return false;
+    return ++H.passed_by % L2TC_RETRY != 0;
+}
 
 // Where the tensor cores answer an exact L2 search: measured for 100k x 32, 1,000
 // queries, k 5: 416 us on the FP32 scan, 148 us the whole call here, of which 60 us do
@@ -1013,11 +1031,10 @@ struct L2Tc {
 // a part of a 128-query tile.
 bool l2_tc_wanted(const gn_index *ix, int64_t nq, int64_t k) {
     if (k > 32 || ix->n < TC_EXACT_MIN || nq < 64 || ix->dim > 2048) return false;
-    if (ix->ext) {
-        const L2Tc &H = *reinterpret_cast<const L2Tc *>(ix->ext);
-        if (H.refused || (H.hflag.p && *reinterpret_cast<volatile int *>(H.hflag.p))) return false;
-    }
-    return (double)nq * (double)ix->n * (double)ix->dim >= 1.5e9;
+    if ((double)nq * (double)ix->n * (double)ix->dim < 1.5e9) return false;
+    if (!ix->ext) return true;
+    L2Tc &H = *reinterpret_cast<L2Tc *>(ix->ext);
+    return !H.refused && !l2_tc_given_up(H);
 }
 
 // On success *flag is the device word that tells whether the results stand (0) or
@@ -1048,7 +1065,7 @@ int l2_tc_search(gn_index *ix, const float *d_q, int64_t nq, int k, int64_t *d_i
             H.refused = true;  // until the next set()
             return GN_ERR_UNSUPPORTED;
         }
-        *reinterpret_cast<volatile int *>(H.hflag.p) = 0;
+        *reinterpret_cast<volatile int *>(H.hflag.p) = -1;
         split(x32, ix->n, false, H.x16);
         GN_CUDA_TRY(cudaMemsetAsync(H.xnorm.as<float>() + ix->n, 0xff, (np - (size_t)ix->n) * 4, st));
         row_norms(x32, ix->n, dp, H.xnorm.as<float>(), st);
@@ -1116,8 +1133,9 @@ void flat_tc_reset(gn_index *ix) {
     } else {
         L2Tc &H = *reinterpret_cast<L2Tc *>(ix->ext);
         H.built = H.refused = false;
-        if (H.hflag.p) *reinterpret_cast<volatile int *>(H.hflag.p) = 0;
-        H.x16.release();
+        H.overflows = H.passed_by = 0;
+        H.x16.release();  // (waits for the searches queued, and with them for their flags' copies)
+        if (H.hflag.p) *reinterpret_cast<volatile int *>(H.hflag.p) = -1;
     }
 }
 

@@ -1006,7 +1006,15 @@ struct L2Tc {
     bool built = false, refused = false;
     int K = 0;
     int overflows = 0, passed_by = 0;  // searches in a row that set the flag, and searches since then
+    double seen = 0.0;                 // what searches had to gain from split rows, in elements of the FP32 scan
 };
+static L2Tc &l2_tc_state(gn_index *ix) {
+    if (!ix->ext) {
+        ix->ext = new L2Tc();
+        ix->ext_free = [](void *p) { delete reinterpret_cast<L2Tc *>(p); };
+    }
+    return *reinterpret_cast<L2Tc *>(ix->ext);
+}
 
 // The FP32 scan alone answers where it had to answer L2TC_OVERFLOWS searches in a row,
 // but for every L2TC_RETRY-th search: a batch of odd queries is forgotten again, and
@@ -1029,12 +1037,25 @@ static bool l2_tc_given_up(L2Tc &H) {
 // not depend on the size; the FP32 scan takes about 0.13 ns per element, so
 // batches of less than 1.5 G elements stay there, and small ones, which fill
 // a part of a 128-query tile.
-bool l2_tc_wanted(const gn_index *ix, int64_t nq, int64_t k) {
+// The split rows are made once the searches of these rows have had about as much to
+// gain from them as they cost.  A search gains the FP32 scan's time less some 0.8 G
+// elements' worth; making the rows takes about 27 elements' time a byte (0.4 TB/s, most of
+// it the allocation) and, with the scratch of an index's first search, 1.6 G elements' (0.8 G
+// later).  First searches after set(), in us, always here / on the FP32 scan / with
+// this rule: 20,000 x 64 rows, 1,200 queries 577 / 413 / 413; 200,000 x 128, 64 queries
+// 741 / 318 / 318 (later searches 215 and 253); 100,000 x 32, 1,000 queries 552 / 612 / 552.
+bool l2_tc_wanted(gn_index *ix, int64_t nq, int64_t k) {
     if (k > 32 || ix->n < TC_EXACT_MIN || nq < 64 || ix->dim > 2048) return false;
-    if ((double)nq * (double)ix->n * (double)ix->dim < 1.5e9) return false;
-    if (!ix->ext) return true;
-    L2Tc &H = *reinterpret_cast<L2Tc *>(ix->ext);
-    return !H.refused && !l2_tc_given_up(H);
+    const double work = (double)nq * (double)ix->n * (double)ix->dim;
+    if (work < 1.5e9) return false;
+    L2Tc &H = l2_tc_state(ix);
+    if (H.refused) return false;
+    if (!H.built) {
+        const double bytes = (double)ix->n * (double)round_up(3 * ix->dim, TC_BK) * 2.0;
+        H.seen += work - 0.8e9;
+        return H.seen >= (H.part.p ? 0.8e9 : 1.6e9) + 27.0 * bytes;
+    }
+    return !l2_tc_given_up(H);
 }
 
 // On success *flag is the device word that tells whether the results stand (0) or
@@ -1042,11 +1063,7 @@ bool l2_tc_wanted(const gn_index *ix, int64_t nq, int64_t k) {
 // launched that the caller needs to know of.
 int l2_tc_search(gn_index *ix, const float *d_q, int64_t nq, int k, int64_t *d_idx, float *d_dist, int *err,
                  const int **flag, cudaStream_t st) {
-    if (!ix->ext) {
-        ix->ext = new L2Tc();
-        ix->ext_free = [](void *p) { delete reinterpret_cast<L2Tc *>(p); };
-    }
-    L2Tc &H = *reinterpret_cast<L2Tc *>(ix->ext);
+    L2Tc &H = l2_tc_state(ix);
     const int d = (int)ix->dim, dp = ix->stride4 * 4;
     const int K = (int)round_up(3 * d, TC_BK);
     const float *x32 = ix->data.as<float>();
@@ -1134,6 +1151,7 @@ void flat_tc_reset(gn_index *ix) {
         L2Tc &H = *reinterpret_cast<L2Tc *>(ix->ext);
         H.built = H.refused = false;
         H.overflows = H.passed_by = 0;
+        H.seen = 0.0;
         H.x16.release();  // (waits for the searches queued, and with them for their flags' copies)
         if (H.hflag.p) *reinterpret_cast<volatile int *>(H.hflag.p) = -1;
     }

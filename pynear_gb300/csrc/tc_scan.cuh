@@ -89,7 +89,7 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
 bool ham_tc_wanted(const gn_index *ix, int64_t nq, int64_t k);
 int ham_tc_search(gn_index *ix, const void *d_q, int64_t nq, int k, int64_t *d_idx, int64_t *d_dist, int *err,
                   cudaStream_t st);
-bool l2_tc_wanted(const gn_index *ix, int64_t nq, int64_t k);
+bool l2_tc_wanted(gn_index *ix, int64_t nq, int64_t k);
 int l2_tc_search(gn_index *ix, const float *d_q, int64_t nq, int k, int64_t *d_idx, float *d_dist, int *err,
                  const int **flag, cudaStream_t st);
 void flat_tc_reset(gn_index *ix);

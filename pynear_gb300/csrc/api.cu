@@ -346,12 +346,24 @@ static int flat_search_dev(gn_index *ix, const void *d_q, int64_t nq, int64_t k,
         a.err = ix->err.as<int>();
         return GN_OK;
     };
-    if (ix->metric == M_HAMMING && ham_tc_wanted(ix, nq, k)) {
+    // A search that is being captured reads nothing but the rows: the graph may be replayed
+    // after a set() of as many rows, which ends what the tensor cores keep of the old ones.
+    auto captured = [&]() {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &capture) == cudaSuccess) return capture != cudaStreamCaptureStatusNone;
+        cudaGetLastError();
+        return true;
+    };
+    if (ix->metric == M_HAMMING && ham_tc_wanted(ix, nq, k) && !captured()) {
         GN_TRY(error_word());
         const int rc = ham_tc_search(ix, d_q, nq, (int)k, d_idx, reinterpret_cast<int64_t *>(d_dist), a.err, st);
+        if (rc == GN_OK) {  // the scratch of the same search captured, which cannot allocate (if there is room)
+            ham_plan(a);
+            ix->part.ensure(ham_part_bytes(a));
+        }
         if (rc != GN_ERR_UNSUPPORTED) return rc;
     }
-    if (ix->metric == M_L2 && l2_tc_wanted(ix, nq, k)) {
+    if (ix->metric == M_L2 && l2_tc_wanted(ix, nq, k) && !captured()) {
         GN_TRY(error_word());
         const int rc = l2_tc_search(ix, reinterpret_cast<const float *>(d_q), nq, (int)k, d_idx,
                                     reinterpret_cast<float *>(d_dist), a.err, &a.only_if, st);

@@ -590,9 +590,11 @@ __global__ void tc_stride_kernel(const float *__restrict__ x, int64_t n, int str
     if (i < m) out[i] = i * stride < n ? x[i * stride] : __int_as_float(0x7fc00000);
 }
 
+static size_t tc_pilot_count(int64_t n) { return (size_t)round_up(ceil_div(n, tc_pilot_stride(n)), TC_N); }
+
 int tc_pilot_values(const float *x, int64_t n, DBuf &out, cudaStream_t st) {
     const int stride = tc_pilot_stride(n);
-    const int64_t m = round_up(ceil_div(n, stride), TC_N);
+    const int64_t m = (int64_t)tc_pilot_count(n);
     GN_TRY(out.ensure((size_t)m * 4));
     tc_stride_kernel<<<(unsigned)ceil_div(m, 256), 256, 0, st>>>(x, n, stride, m, out.as<float>());
     return GN_OK;
@@ -1076,7 +1078,7 @@ int l2_tc_search(gn_index *ix, const float *d_q, int64_t nq, int k, int64_t *d_i
         size_t free_b = 0, total_b = 0;
         const size_t want = (size_t)ix->n * K * 2, np = (size_t)round_up(ix->n, TC_N);
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || want > free_b / 4 || H.x16.ensure(want) != GN_OK ||
-            H.xnorm.ensure(np * 4) != GN_OK || H.xmax2.ensure(4) != GN_OK || H.flag.ensure(4) != GN_OK ||
+            H.xnorm.ensure(np * 4) != GN_OK || H.pnorm.ensure(tc_pilot_count(ix->n) * 4) != GN_OK || H.xmax2.ensure(4) != GN_OK || H.flag.ensure(4) != GN_OK ||
             H.hflag.ensure(4) != GN_OK) {
             cudaGetLastError();
             H.refused = true;  // until the next set()

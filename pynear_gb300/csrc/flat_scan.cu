@@ -121,7 +121,7 @@ constexpr int FS_STAGES = 3;
 constexpr int FS_STAGE = 16384; // bytes of a stage at most
 constexpr int FS_THREADS = 128, FS_WARPS = 4;
 
-// Launch shape (FlatScanArgs::fs).
+// Launch shape of a batch.
 struct FsGeom {
     int qw, rpt, wq, wr;  // queries per warp, rows per lane, warps across queries and rows
     int nbx, bw;          // boxes per row, floats per box row: 32 (swizzled) or the row width (narrow rows)

@@ -1,10 +1,10 @@
 // ivf_tc.cu — tensor-core engine of the float IVF index.
 //
 //   0. probes  coarse_probe_kernel: BF16 centroid scores (tc_ivf_kernel over
-//              the centroids), radix select of the 64 best, exact FP32
+//              the centroids), the 64 best by counting, exact FP32
 //              distances, then the first n_probe or the learned prober's
-//              choice (its MLP fused here; from 1,024 queries its layers 2
-//              and 3 run in mlp_probe_kernel over 8 queries per block), and
+//              choice (its MLP fused here; from 1,024 queries the whole of it
+//              runs in mlp_probe_kernel over 8 queries per block), and
 //              each query's score bound for the scan;
 //   1. plan    the same bucketing and work plan as the FP32 scan (ivf.cu),
 //              score segments in 128-row slots;
@@ -78,7 +78,6 @@ __device__ void tc_units_body(int64_t i, const int64_t *__restrict__ item_off, i
     u.r1 = min(le, u.r0 + rc);
     u.rbase = lb;
     u.xrow = xoff[l] + (u.r0 - lb);  // rc is a multiple of 128: stays tile-aligned
-    u.rch = (int32_t)rch;
     units[i] = u;
 }
 
@@ -591,7 +590,6 @@ __global__ void coarse_units_kernel(int64_t nq, int nc, TcUnit *__restrict__ uni
     u.r1 = min((int64_t)nc, u.r0 + 128);
     u.rbase = 0;
     u.xrow = u.r0;
-    u.rch = 0;
     units[t] = u;
 }
 
@@ -1127,7 +1125,7 @@ static int ivfl2_probes_tc(gn_index *ix, const float *dQ, int64_t nq, int *np_ou
     if (mlp) {
         GN_TRY(prober_weights(S.prober, &w));
         GN_TRY(T.nprobed.ensure((size_t)nq * 4));
-        if (nq >= MLP_BATCH_MIN) {  // layers 2 and 3 batched over 8 queries per block
+        if (nq >= MLP_BATCH_MIN) {  // the MLP batched over 8 queries per block
             GN_TRY(T.mfeat.ensure((size_t)nq * PROBER_CAND * 4));
             GN_TRY(T.mcand.ensure((size_t)nq * PROBER_CAND * 4));
             GN_TRY(T.mcb.ensure((size_t)nq * PROBER_CAND * 4));

@@ -26,7 +26,6 @@
 #include "index.cuh"
 #include "ivf.cuh"
 #include "prober.cuh"
-#include "topk.cuh"
 
 namespace gn {
 
@@ -232,11 +231,10 @@ __global__ void prober_labels_kernel(const int32_t *__restrict__ cand, const int
     lab[t] = y;
 }
 
-// ── inference, fused with the merge of the coarse top-64 ──────────────────
-// block per query, 256 threads.  part: nsplit sorted partial lists of PB_C
-// coarse keys per query.  Writes probes[q][0..PB_C): selected list ids in
-// distance order, then -1.
-__global__ void __launch_bounds__(PB_H) prober_select_kernel(const uint64_t *__restrict__ part, int nsplit, int64_t nq,
+// ── inference ─────────────────────────────────────────────────────────────
+// block per query, 256 threads.  keys: PB_C coarse keys per query, nearest
+// first.  Writes probes[q][0..PB_C): selected list ids in distance order, then -1.
+__global__ void __launch_bounds__(PB_H) prober_select_kernel(const uint64_t *__restrict__ keys, int64_t nq,
                                                               const __nv_bfloat16 *__restrict__ W1,
                                                               const float *__restrict__ b1,
                                                               const __nv_bfloat16 *__restrict__ W2,
@@ -250,16 +248,11 @@ __global__ void __launch_bounds__(PB_H) prober_select_kernel(const uint64_t *__r
     const int64_t q = blockIdx.x;
     const int j = threadIdx.x, lane = j & 31, warp = j >> 5;
     if (warp == 0) {
-        WarpTopK<PB_C / 32> L;
-        L.init();
-        uint64_t thr = KEY_EMPTY;
-        for (int sp = 0; sp < nsplit; ++sp)
-            for (int i0 = 0; i0 < PB_C; i0 += 32)
-                L.offer(part[((size_t)q * nsplit + sp) * PB_C + i0 + lane], thr, PB_C);
-        const float d1 = __uint_as_float(key_dist(L.at(0)));
+        const uint64_t *mine = keys + (size_t)q * PB_C;
+        const float d1 = __uint_as_float(key_dist(mine[0]));
 #pragma unroll
         for (int r = 0; r < PB_C / 32; ++r) {
-            const uint64_t k = L.v[r];
+            const uint64_t k = mine[r * 32 + lane];
             const bool e = k == KEY_EMPTY;
             sc[r * 32 + lane] = e ? -1 : (int32_t)key_idx(k);
             sf[r * 32 + lane] = e ? 0.f : gap_feature(__uint_as_float(key_dist(k)), d1);
@@ -397,7 +390,7 @@ int prober_apply(gn_index *pr, gn_index *ivf, const float *dQ, int64_t nq, float
     GN_TRY(ivfl2_coarse_sorted_keys(ivf, dQ, nq, PB_C, T.ckeys.as<uint64_t>(), st));
     const __nv_bfloat16 *w = P.wbf.as<__nv_bfloat16>();
     const float *pf = P.params.as<float>();
-    prober_select_kernel<<<(unsigned)nq, PB_H, 0, st>>>(T.ckeys.as<uint64_t>(), 1, nq, w + P.oW1, pf + P.ob1,
+    prober_select_kernel<<<(unsigned)nq, PB_H, 0, st>>>(T.ckeys.as<uint64_t>(), nq, w + P.oW1, pf + P.ob1,
                                                        w + P.oW2, pf + P.ob2, w + P.oW3, pf + P.ob3, logit_tau,
                                                        probes, nprobed);
     GN_CUDA_TRY(cudaGetLastError());

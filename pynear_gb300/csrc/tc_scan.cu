@@ -75,8 +75,8 @@ constexpr int TC_MAX_STAGES = 6;
 constexpr int TC_NR = 4;                // tiles of row norms (and scales) in flight
 constexpr int64_t TC_PILOT_MIN = 256;   // rows from which a pilot runs
 constexpr int64_t TC_EXACT_MIN = 4096;  // ... and from which exact Hamming and L2 searches come here
-constexpr int64_t L2TC_QBLOCK = 8192;   // the same of the exact L2 search (longer candidate lists)
-constexpr int64_t TC_QBLOCK = 65536;    // queries scanned at a time (bounds the scratch)
+constexpr int64_t TC_QBLOCK = 65536;    // queries scanned at a time (bounds the scratch) ...
+constexpr int64_t L2TC_QBLOCK = 8192;   // ... and by the exact L2 search, whose candidate lists are longer
 constexpr int TC_CAP = 128;             // entries of a buffer (S <= 64, and a block adds up to 32)
 
 // Shared memory: [queries, resident: qt x nk slices][ring][norms, scales of TC_NR tiles][barriers].
@@ -856,7 +856,6 @@ struct HamTc {
     DBuf x8, q8, part, qcount;
     TcScratch scr;
     bool built = false, refused = false;
-    int K = 0;
 };
 
 // Where the tensor cores answer a Hamming search.  Both paths give the same
@@ -902,7 +901,6 @@ int ham_tc_search(gn_index *ix, const void *d_q, int64_t nq, int k, int64_t *d_i
             return GN_ERR_UNSUPPORTED;
         }
         expand(ix->data.p, ix->n, H.x8);
-        H.K = K;
         H.built = true;
     }
     for (int64_t b0 = 0; b0 < nq; b0 += TC_QBLOCK) {
@@ -1000,13 +998,12 @@ __global__ void __launch_bounds__(RR_WARPS * 32)
     l2_rank(part + q * slot_keys, qcount[q], Q + q * dp, X, d, dp, k, out_idx + q * k, out_dist + q * k);
 }
 
-// Expanded operands and scratch of an L2 index, made by its first large search.
+// Split operands and scratch of an L2 index, made by its large searches.
 struct L2Tc {
     HBuf hflag;  // the flag of the last search done, -1 once it is counted (freed after the device buffers)
     DBuf x16, xnorm, pnorm, xmax2, q16, qnorm, part, qcount, flag;
     TcScratch scr;
     bool built = false, refused = false;
-    int K = 0;
     int overflows = 0, passed_by = 0;  // searches in a row that set the flag, and searches since then
     double seen = 0.0;                 // what searches had to gain from split rows, in elements of the FP32 scan
 };
@@ -1091,7 +1088,6 @@ int l2_tc_search(gn_index *ix, const float *d_q, int64_t nq, int k, int64_t *d_i
         GN_TRY(tc_pilot_values(H.xnorm.as<float>(), ix->n, H.pnorm, st));
         GN_CUDA_TRY(cudaMemsetAsync(H.xmax2.p, 0, 4, st));
         max_value_kernel<<<256, 256, 0, st>>>(H.xnorm.as<float>(), ix->n, H.xmax2.as<uint32_t>());
-        H.K = K;
         H.built = true;
     }
     GN_CUDA_TRY(cudaMemsetAsync(H.flag.p, 0, 4, st));

@@ -5,16 +5,15 @@
 
 namespace gn {
 
-// One work unit: A rows [a0, a0 + na) against B rows [r0, r1).  Query row
-// a0 + i writes its S best keys to partial slot arow_slot[a0 + i] + rch.
+// One work unit of the IVF scans (tc_ivf.cu): query rows [a0, a0 + na) against rows
+// [r0, r1), whose scores go to the query rows' score segments.
 struct TcUnit {
     int64_t a0;
     int64_t r0;
     int64_t r1;
-    int64_t rbase;  // store mode: first B row of the list the unit belongs to
+    int64_t rbase;  // first row of the list the unit belongs to
     int64_t xrow;   // IVF list scan, tiled row layout: the padded row of r0 (a multiple of 128)
     int32_t na;
-    int32_t rch;
 };
 
 // Operand form of a scan: BF16 rows, FP8 E4M3 rows with one FP32 scale each, or

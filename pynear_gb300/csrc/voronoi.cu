@@ -54,6 +54,100 @@ __device__ __forceinline__ void vr_bounds(float2 s, float x0, float x1, float y0
     ub = __fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy));
 }
 
+// Four neighbouring pixels of a row and the nearest seed so far of each.
+struct VrQuad {
+    f32x2 px01, px23;
+    float py, bs[4], br[4];
+    int bi[4];
+    __device__ __forceinline__ void start(const float (&px)[4], float y) {
+        px01 = pack2(px[0], px[1]);
+        px23 = pack2(px[2], px[3]);
+        py = y;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+            bs[p] = INFINITY;
+            br[p] = INFINITY;
+            bi[p] = 0;
+        }
+    }
+    // offer seed `idx` with squared sum s to pixel p (seed order is kept)
+    __device__ __forceinline__ void offer(int p, float s, int idx) {
+        if (s < bs[p]) {
+            const float r = __fsqrt_rn(s);
+            if (r < br[p]) {  // strictly nearer: equal distances keep the lower index
+                bs[p] = s;
+                br[p] = r;
+                bi[p] = idx;
+            }
+        }
+    }
+    // the four pixels' squared sums
+    __device__ __forceinline__ void sums(float2 s, float (&o)[4]) const {
+        const float dy = __fsub_rn(py, s.y);
+        const f32x2 dy2 = dup2(__fmul_rn(dy, dy)), nx = dup2(-s.x);
+        const f32x2 d01 = add2(px01, nx), d23 = add2(px23, nx);
+        float d0, d1, d2, d3;
+        unpack2(d01, d0, d1);
+        unpack2(d23, d2, d3);
+        // scalar products: a packed product and sum came out fused (one rounding
+        // instead of the two of the reference's arithmetic)
+        unpack2(add2(pack2(__fmul_rn(d0, d0), __fmul_rn(d1, d1)), dy2), o[0], o[1]);
+        unpack2(add2(pack2(__fmul_rn(d2, d2), __fmul_rn(d3, d3)), dy2), o[2], o[3]);
+    }
+    __device__ __forceinline__ void seed(float2 s, int idx) {
+        float o[4];
+        sums(s, o);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) offer(p, o[p], idx);
+    }
+    // the outputs of pixels pc .. pc + 3 (those below w) of row pr
+    __device__ __forceinline__ void store(int pr, int pc, int w, int32_t *__restrict__ ids, float *__restrict__ dist,
+                                          const uchar4 *__restrict__ palette, int npal,
+                                          uchar4 *__restrict__ rgba) const {
+        const int64_t off = (int64_t)pr * w + pc;
+        const int here = w - pc;
+        uchar4 col[4];
+        if (rgba) {
+#pragma unroll
+            for (int p = 0; p < 4; ++p) col[p] = palette[bi[p] < npal ? bi[p] : bi[p] % npal];
+        }
+        // whole 16-byte stores where the row starts allow them
+        const bool vec = here >= 4 && (w & 3) == 0;
+        if (ids) {
+            if (vec && ((uintptr_t)ids & 15) == 0) {
+                *reinterpret_cast<int4 *>(ids + off) = make_int4(bi[0], bi[1], bi[2], bi[3]);
+            } else {
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+                    if (p < here) ids[off + p] = bi[p];
+            }
+        }
+        if (dist) {
+            if (vec && ((uintptr_t)dist & 15) == 0) {
+                *reinterpret_cast<float4 *>(dist + off) = make_float4(br[0], br[1], br[2], br[3]);
+            } else {
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+                    if (p < here) dist[off + p] = br[p];
+            }
+        }
+        if (rgba) {
+            if (vec && ((uintptr_t)rgba & 15) == 0) {
+                uint4 v;
+                v.x = *reinterpret_cast<unsigned *>(&col[0]);
+                v.y = *reinterpret_cast<unsigned *>(&col[1]);
+                v.z = *reinterpret_cast<unsigned *>(&col[2]);
+                v.w = *reinterpret_cast<unsigned *>(&col[3]);
+                *reinterpret_cast<uint4 *>(rgba + off) = v;
+            } else {
+#pragma unroll
+                for (int p = 0; p < 4; ++p)
+                    if (p < here) rgba[off + p] = col[p];
+            }
+        }
+    }
+};
+
 // Block tile: TX x TY warp tiles.
 template <int TX, int TY>
 __global__ void __launch_bounds__(VR_NT) voronoi_kernel(const float2 *__restrict__ seeds, int ns,
@@ -177,63 +271,28 @@ __global__ void __launch_bounds__(VR_NT) voronoi_kernel(const float2 *__restrict
             }
             wu = __fsqrt_rn(__uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(wu))));
 
-            float bs[4], br[4];
-            int bi[4];
-#pragma unroll
-            for (int p = 0; p < 4; ++p) {
-                bs[p] = INF;
-                br[p] = INF;
-                bi[p] = 0;
-            }
-            const f32x2 px01 = pack2(px[0], px[1]), px23 = pack2(px[2], px[3]);
-            // offer seed `idx` with squared sum s to pixel p (seed order is kept)
-            auto offer = [&](int p, float s, int idx) {
-                if (s < bs[p]) {
-                    const float r = __fsqrt_rn(s);
-                    if (r < br[p]) {  // strictly nearer: equal distances keep the lower index
-                        bs[p] = s;
-                        br[p] = r;
-                        bi[p] = idx;
-                    }
-                }
-            };
-            auto sums = [&](float2 s, float (&o)[4]) {  // the four pixels' squared sums
-                const float dy = __fsub_rn(py, s.y);
-                const f32x2 dy2 = dup2(__fmul_rn(dy, dy)), nx = dup2(-s.x);
-                const f32x2 d01 = add2(px01, nx), d23 = add2(px23, nx);
-                float d0, d1, d2, d3;
-                unpack2(d01, d0, d1);
-                unpack2(d23, d2, d3);
-                // scalar products: a packed product and sum came out fused (one rounding
-                // instead of the two of the reference's arithmetic)
-                unpack2(add2(pack2(__fmul_rn(d0, d0), __fmul_rn(d1, d1)), dy2), o[0], o[1]);
-                unpack2(add2(pack2(__fmul_rn(d2, d2), __fmul_rn(d3, d3)), dy2), o[2], o[3]);
-            };
+            VrQuad px4;
+            px4.start(px, py);
             float2 *lxy = wxy[warp];
             int *lid = wid[warp];
             auto evaluate = [&](int cnt) {
                 int j = 0;
                 for (; j + 4 <= cnt; j += 4) {
                     float s0[4], s1[4], s2[4], s3[4];
-                    sums(lxy[j], s0);
-                    sums(lxy[j + 1], s1);
-                    sums(lxy[j + 2], s2);
-                    sums(lxy[j + 3], s3);
+                    px4.sums(lxy[j], s0);
+                    px4.sums(lxy[j + 1], s1);
+                    px4.sums(lxy[j + 2], s2);
+                    px4.sums(lxy[j + 3], s3);
 #pragma unroll
                     for (int p = 0; p < 4; ++p)
-                        if (fminf(fminf(s0[p], s1[p]), fminf(s2[p], s3[p])) < bs[p]) {
-                            offer(p, s0[p], lid[j]);
-                            offer(p, s1[p], lid[j + 1]);
-                            offer(p, s2[p], lid[j + 2]);
-                            offer(p, s3[p], lid[j + 3]);
+                        if (fminf(fminf(s0[p], s1[p]), fminf(s2[p], s3[p])) < px4.bs[p]) {
+                            px4.offer(p, s0[p], lid[j]);
+                            px4.offer(p, s1[p], lid[j + 1]);
+                            px4.offer(p, s2[p], lid[j + 2]);
+                            px4.offer(p, s3[p], lid[j + 3]);
                         }
                 }
-                for (; j < cnt; ++j) {
-                    float s0[4];
-                    sums(lxy[j], s0);
-#pragma unroll
-                    for (int p = 0; p < 4; ++p) offer(p, s0[p], lid[j]);
-                }
+                for (; j < cnt; ++j) px4.seed(lxy[j], lid[j]);
             };
             int cnt = 0;
             for (int j0 = 0; j0 < nsrc; j0 += 32) {
@@ -263,48 +322,28 @@ __global__ void __launch_bounds__(VR_NT) voronoi_kernel(const float2 *__restrict
             evaluate(cnt);
             __syncwarp();
 
-            if (pr >= h) continue;
-            const int64_t off = (int64_t)pr * w + pc;
-            uchar4 col[4];
-            if (rgba) {
-#pragma unroll
-                for (int p = 0; p < 4; ++p) col[p] = palette[bi[p] < npal ? bi[p] : bi[p] % npal];
-            }
-            // whole 16-byte stores where the row starts allow them
-            const bool vec = pc + 4 <= w && (w & 3) == 0;
-            if (ids) {
-                if (vec && ((uintptr_t)ids & 15) == 0) {
-                    *reinterpret_cast<int4 *>(ids + off) = make_int4(bi[0], bi[1], bi[2], bi[3]);
-                } else {
-#pragma unroll
-                    for (int p = 0; p < 4; ++p)
-                        if (pc + p < w) ids[off + p] = bi[p];
-                }
-            }
-            if (dist) {
-                if (vec && ((uintptr_t)dist & 15) == 0) {
-                    *reinterpret_cast<float4 *>(dist + off) = make_float4(br[0], br[1], br[2], br[3]);
-                } else {
-#pragma unroll
-                    for (int p = 0; p < 4; ++p)
-                        if (pc + p < w) dist[off + p] = br[p];
-                }
-            }
-            if (rgba) {
-                if (vec && ((uintptr_t)rgba & 15) == 0) {
-                    uint4 v;
-                    v.x = *reinterpret_cast<unsigned *>(&col[0]);
-                    v.y = *reinterpret_cast<unsigned *>(&col[1]);
-                    v.z = *reinterpret_cast<unsigned *>(&col[2]);
-                    v.w = *reinterpret_cast<unsigned *>(&col[3]);
-                    *reinterpret_cast<uint4 *>(rgba + off) = v;
-                } else {
-#pragma unroll
-                    for (int p = 0; p < 4; ++p)
-                        if (pc + p < w) rgba[off + p] = col[p];
-                }
-            }
+            if (pr < h) px4.store(pr, pc, w, ids, dist, palette, npal, rgba);
         }
+    }
+}
+
+// Few seeds: every seed for every pixel, a warp to 128 pixels of a row.
+constexpr int VR_FROWS = 8;
+__global__ void __launch_bounds__(32 * VR_FROWS)
+    voronoi_few_kernel(const float2 *__restrict__ seeds, int ns, const float *__restrict__ xs,
+                       const float *__restrict__ ys, int w, int h, int32_t *__restrict__ ids,
+                       float *__restrict__ dist, const uchar4 *__restrict__ palette, int npal,
+                       uchar4 *__restrict__ rgba) {
+    const int64_t pc = (int64_t)blockIdx.x * 128 + (threadIdx.x & 31) * 4;
+    if (pc >= w) return;
+    float px[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) px[p] = xs[min(pc + p, (int64_t)w - 1)];
+    for (int64_t pr = (int64_t)blockIdx.y * VR_FROWS + (threadIdx.x >> 5); pr < h; pr += (int64_t)gridDim.y * VR_FROWS) {
+        VrQuad px4;
+        px4.start(px, ys[pr]);
+        for (int j = 0; j < ns; ++j) px4.seed(__ldg(seeds + j), j);
+        px4.store((int)pr, (int)pc, w, ids, dist, palette, npal, rgba);
     }
 }
 
@@ -334,6 +373,21 @@ static int voronoi_launch(const float *seeds, int64_t ns, const float *xs, const
                                      (int)tiles_y, ids, dist, reinterpret_cast<const uchar4 *>(palette), (int)npal,
                                      reinterpret_cast<uchar4 *>(rgba));
     };
+    // Few seeds are cheaper without the tiles' bounds, the more so where there are few
+    // pixels for a block's bounds to serve.  In us, tiles / all seeds: 1377 x 466 with 1, 8
+    // and 16 seeds 9.1 / 3.6, 9.1 / 5.5, 9.1 / 7.3; 1920 x 1080 15.3 / 6.5, 15.5 / 11.3,
+    // 15.5 / 15.9; 3840 x 2160 37 / 20, 38 / 37, 38 / 54; 7680 x 4320 with 1, 4 and 8 seeds 129 /
+    // 77, 130 / 105, 130 / 141; 256 x 256 with 8 and 16 4.0 / 3.6, 4.6 / 5.4.
+    const int64_t pixels = w * h;
+    const int few = pixels < (1 << 18) ? 9 : pixels < (1 << 22) ? 16 : pixels < (1 << 24) ? 8 : 6;
+    if (ns <= few) {
+        const dim3 grid((unsigned)ceil_div(w, 128), (unsigned)std::min<int64_t>(ceil_div(h, VR_FROWS), 65535));
+        voronoi_few_kernel<<<grid, 32 * VR_FROWS, 0, st>>>(
+            reinterpret_cast<const float2 *>(seeds), (int)ns, xs, ys, (int)w, (int)h, ids, dist,
+            reinterpret_cast<const uchar4 *>(palette), (int)npal, reinterpret_cast<uchar4 *>(rgba));
+        GN_CUDA_TRY(cudaGetLastError());
+        return GN_OK;
+    }
     // large tiles share one pass over the seeds among 64 warp tiles; small ones
     // where large ones would not give every SM two blocks
     if (ceil_div(w, 8 * VR_SW) * ceil_div(h, 8 * VR_SH) >= 2 * dev_info().num_sms)

@@ -73,8 +73,7 @@ constexpr int TC_COLS = TC_N / (TC_NEPI / 4);  // columns of a tile per epilogue
 constexpr int TC_THREADS = 64 + 32 * TC_NEPI;
 constexpr int TC_MAX_STAGES = 6;
 constexpr int TC_NR = 4;                // tiles of row norms (and scales) in flight
-constexpr int64_t TC_PILOT_MIN = 256;   // rows from which a pilot runs
-constexpr int64_t TC_EXACT_MIN = 4096;  // ... and from which exact Hamming and L2 searches come here
+constexpr int64_t TC_EXACT_MIN = 4096;  // rows from which exact Hamming and L2 searches come here
 constexpr int64_t TC_QBLOCK = 65536;    // queries scanned at a time (bounds the scratch) ...
 constexpr int64_t L2TC_QBLOCK = 8192;   // ... and by the exact L2 search, whose candidate lists are longer
 constexpr int TC_CAP = 128;             // entries of a buffer (S <= 64, and a block adds up to 32)
@@ -471,9 +470,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     const int row = i * TC_M + quad * 32 + lane;
                     int n = i == 0 ? cnt[0] : cnt[QT - 1];
                     uint2 *const wbuf = ebuf + (size_t)i * 32 * TC_CAP;
-                    unsigned longm = __ballot_sync(0xffffffffu, n > a.S);
+                    unsigned longm = __ballot_sync(0xffffffffu, n > a.keep);
                     if (longm && a.overflow) *a.overflow = 1;
-                    while (longm) {  // only a buffer's S best can be among the query's
+                    while (longm) {  // only a buffer's S best can be among the query's, and more have no room
                         const int l = __ffs(longm) - 1;
                         longm &= longm - 1;
                         const uint64_t last = tc_compact<TC_CAP / 32>(wbuf + (size_t)l * TC_CAP,
@@ -613,14 +612,19 @@ TcPlan tc_plan(int mode, int K, int64_t nq, int64_t n, int S) {
     // pilot: every 8th row (more where that would be under 16k rows), whole tiles
     // of them.  It pays for small databases as well, where the units' buffers would
     // fill with most rows they see: 24,813 x 126 rows, 2,956 queries, S 40: 1289 us per
-    // search without it, below 300 with it.
-    if (n >= TC_PILOT_MIN) {
+    // search without it, below 300 with it; 255 x 64 rows, 5,000 queries, S 32: 388 and 152.
+    // (Of at most 48 rows too many pass all the same.)
+    if (n > std::max(S, 48)) {
         p.pilot_stride = tc_pilot_stride(n);
-        p.pilot_tiles = n / p.pilot_stride / TC_N;
+        p.pilot_tiles = std::max<int64_t>(1, n / p.pilot_stride / TC_N);
         // 128 groups of minima per chunk
         p.pilot_chunks = (int)tc_chunks(nqp1, p.pilot_tiles, 1, std::max<int64_t>(1, ceil_div(4 * sms, nqp1)), 2);
     }
-    p.slot_keys = (int64_t)p.nchunks * (TC_NEPI / 4) * S;
+    // A unit hands over its S best of each buffer, or, from a single tile, all of its columns:
+    // many of few rows pass, and sorting a warp's 32 buffers one after another costs more
+    // than their keys (82 x 50 rows, 3,618 queries, S 48: 380 us with it, 244 without)
+    p.keep = nt == 1 ? std::max(S, TC_COLS) : S;
+    p.slot_keys = (int64_t)p.nchunks * (TC_NEPI / 4) * p.keep;
     return p;
 }
 
@@ -640,6 +644,7 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
     s.nq = a.nq;
     s.kblk = kblk;
     s.S = a.S;
+    s.keep = p.keep;
     s.nbits = a.nbits;
     s.ascale = a.ascale;
     s.part = a.part;
@@ -663,7 +668,7 @@ int tc_topk_launch(const TcLaunch &a, const TcPlan &p, TcScratch &sc, cudaStream
     GN_CUDA_TRY(cudaMemsetAsync(a.qcount, 0, (size_t)a.nq * 4, st));
     if (p.pilot_chunks) {
         const TcGeom gp = tc_geom(a.K / kblk, true);
-        GN_TRY(make_tmap_rows(&mp, a.B, a.n / p.pilot_stride, a.K, TC_N, f8, p.pilot_stride));
+        GN_TRY(make_tmap_rows(&mp, a.B, std::max<int64_t>(a.n / p.pilot_stride, TC_N), a.K, TC_N, f8, p.pilot_stride));
         GN_TRY(sc.gmin.ensure((size_t)a.nq * p.pilot_chunks * TC_N / 2 * 4));
         s.gmin = sc.gmin.as<float>();
         s.nchunks = p.pilot_chunks;

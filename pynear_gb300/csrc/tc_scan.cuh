@@ -52,6 +52,7 @@ struct TcLaunch {
 // Launch shape for nq queries over n rows.
 struct TcPlan {
     int nchunks = 1;                                       // database chunks
+    int keep = 0;                                          // entries of a buffer that a unit hands over at most
     int64_t slot_keys = 0;                                 // room of a query's candidate list
     int pilot_chunks = 0, pilot_stride = 1;                // 0: no pilot
     int64_t pilot_tiles = 0;
@@ -65,7 +66,7 @@ struct TcScratch {
 // Kernel arguments.
 struct TcScanArgs {
     int64_t nq, n, ntiles;
-    int nk, kblk, stages, resident, nchunks, S, nbits;
+    int nk, kblk, stages, resident, nchunks, S, keep, nbits;
     const float *bnorm, *ascale, *bscale;
     int64_t slot_keys;
     uint64_t *part;

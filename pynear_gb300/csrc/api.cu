@@ -382,13 +382,17 @@ static int flat_search_dev(gn_index *ix, const void *d_q, int64_t nq, int64_t k,
         GN_TRY(error_word());
         a.status = status;
         ix->status_set = status != nullptr;
-        const int64_t blocks = k > 64 ? ceil_div(nq, FLAT_QBLOCK) : 1, step = round_up(ceil_div(nq, blocks), 16);
+        const int64_t blocks = k > 64 ? ceil_div(nq, FLAT_QBLOCK) : 1;
+        int64_t step = round_up(ceil_div(nq, blocks), 16);
+        if (a.wave_queries && !a.only_if) step = a.wave_queries;
         for (int64_t q0 = 0; q0 < nq; q0 += step) {
-            a.nq = std::min(step, nq - q0);
-            a.q = static_cast<const char *>(d_q) + (size_t)q0 * ix->stride4 * 16;
-            a.out_idx = d_idx + q0 * k;
-            a.out_dist = static_cast<float *>(d_dist) + q0 * k;
-            flat_plan(a);
+            if (step < nq) {
+                a.nq = std::min(step, nq - q0);
+                a.q = static_cast<const char *>(d_q) + (size_t)q0 * ix->stride4 * 16;
+                a.out_idx = d_idx + q0 * k;
+                a.out_dist = static_cast<float *>(d_dist) + q0 * k;
+                flat_plan(a);
+            }
             GN_TRY(ix->part.ensure(flat_part_bytes(a)));
             GN_TRY(flat_launch(a, ix->part.as<uint64_t>(), st));
         }

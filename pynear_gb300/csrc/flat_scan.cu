@@ -130,7 +130,7 @@ struct FsGeom {
     size_t smem;
 };
 
-static FsGeom fs_geom(int64_t nq, int k, int dp4) {
+static FsGeom fs_geom(int64_t n, int64_t nq, int k, int dp4) {
     FsGeom g;
     g.cap = list_cap(k);  // k <= 64: in shared memory, else in global
     g.most = list_most(k);
@@ -142,9 +142,12 @@ static FsGeom fs_geom(int64_t nq, int k, int dp4) {
     auto qbytes = [&]() { return (size_t)g.wq * g.qw * dp4 * 16; };
     while (qbytes() > 100 * 1024 && g.wq > 1) g.wq >>= 1;
     while (qbytes() > 130 * 1024 && g.qw > 1) g.qw >>= 1;
-    g.rpt = g.wq > 1 ? 2 : 1;  // (several warps across the queries: four queries each)
+    // (several warps across the queries: four queries each; up to 32 rows fill one per lane)
+    g.rpt = g.wq > 1 && n > 32 ? 2 : 1;
     g.wr = FS_WARPS / g.wq;
-    const int unit = 32 * g.rpt * g.wr;  // rows the four warps take at a time
+    // rows the four warps take at a time, no more than there are: a stage of fewer rows
+    // has room for more boxes of each
+    const int unit = (int)std::min<int64_t>(32 * g.rpt * g.wr, round_up(std::max<int64_t>(n, 1), 32 * g.rpt));
     g.nbx = (dp4 * 4 + FS_BOX - 1) / FS_BOX;
     g.bw = dp4 * 4 < FS_BOX ? dp4 * 4 : FS_BOX;
     g.cb = std::min(g.nbx, std::max(1, FS_STAGE / (unit * 128)));
@@ -878,6 +881,45 @@ static int64_t fullest_slices(int64_t n_groups, int64_t slots, int64_t hi) {
     return slices;
 }
 
+// Slices of `stages` stages of `rows` rows for the float scan with k <= 64, at most hi: the
+// fewest whose time is within 3 % of the least.  In rows, a unit takes its own and what
+// starting its lists anew costs (about 5,000 coordinates' work).  Units that fit the GPU
+// together take 0.63, 0.82 or all of a full wave's time, with one, two or three of them per
+// SM; more of them go as slots become free, with a third of a wave left over at the end.
+// Scan alone in us, by slices: 2,318 x 32 rows, 8,145 queries 1: 150, 2: 149, 4: 165, 8: 190;
+// 20,000 x 8, 7,500 queries 1: 439, 2: 411, 4: 444, 8: 529; 6,592 x 12, 725 queries 3: 49, 7: 36,
+// 9: 34, 13: 46.
+struct SlicePlan {
+    int64_t slices;
+    double time;
+};
+static SlicePlan cheapest_slices(int64_t stages, int rows, int d, int64_t n_groups, int64_t slots) {
+    const int64_t hi = std::min<int64_t>(stages, std::max<int64_t>(1, ceil_div(2 * slots, n_groups)));
+    const int64_t sms = dev_info().num_sms;
+    const double occ = (double)slots / (double)sms, anew = 5000.0 / std::max(d, 4);
+    auto time = [&](int64_t t) {  // of slices of t stages
+        const int64_t units = n_groups * ceil_div(stages, t);
+        const double waves = units <= slots
+                                 ? 0.45 + 0.55 * (double)ceil_div(units, sms) / occ
+                                 : std::min((double)ceil_div(units, slots), (double)units / (double)slots + 0.35);
+        return waves * ((double)(t * rows) + anew);
+    };
+    // the stages of a slice fall as the slices grow: every value once
+    double least = 0.0;
+    for (int64_t s = 1; s <= hi;) {
+        const int64_t t = ceil_div(stages, s);
+        const double c = time(t);
+        if (s == 1 || c < least) least = c;
+        if (t == 1) break;
+        s = ceil_div(stages, t - 1);
+    }
+    for (int64_t s = 1;;) {
+        const int64_t t = ceil_div(stages, s);
+        if (time(t) <= 1.03 * least) return {ceil_div(stages, t), time(t)};
+        s = ceil_div(stages, t - 1);
+    }
+}
+
 void flat_plan(FlatScanArgs &a) {
     const DevInfo &di = dev_info();
     if (a.metric == M_HAMMING) {
@@ -894,15 +936,30 @@ void flat_plan(FlatScanArgs &a) {
         a.n_groups = (int)n_groups;
         return;
     }
-    const FsGeom g = fs_geom(a.nq, a.k, a.stride4);
+    const FsGeom g = fs_geom(a.n, a.nq, a.k, a.stride4);
     const int64_t n_groups = ceil_div(a.nq, (int64_t)g.wq * g.qw);
-    // units of equal cost: the slice count (up to about two waves of resident
-    // CTAs) whose last wave is fullest, the fewest slices on a tie: every slice
-    // starts its lists empty
+    // up to about two waves of resident CTAs; k > 64: the slice count whose last wave is
+    // fullest, the fewest slices on a tie, since every slice starts its lists empty
     const int64_t slots = (int64_t)std::max(1, fs_occupancy(g)) * di.num_sms;
     const int64_t max_slices = std::max<int64_t>(1, ceil_div(a.n, g.rows));
-    const int64_t hi = std::min<int64_t>(max_slices, std::max<int64_t>(1, ceil_div(2 * slots, n_groups)));
-    int64_t slices = fullest_slices(n_groups, slots, hi);
+    int64_t slices;
+    a.wave_queries = 0;
+    if (a.k <= 64) {
+        const SlicePlan p = cheapest_slices(max_slices, g.rows, a.d, n_groups, slots);
+        slices = p.slices;
+        // a batch of more than a wave and less than two: the whole wave first, the rest in
+        // slices of its own, where that is worth the launches (about 8 us, 6,700 coordinates a
+        // unit).  3,000 x 32 rows, 9,000 queries: 326 us a search in one piece, 306 so; 5,000 x
+        // 32, 7,400: 420 and 362.
+        if (n_groups > slots && n_groups < 2 * slots &&
+            cheapest_slices(max_slices, g.rows, a.d, slots, slots).time +
+                    cheapest_slices(max_slices, g.rows, a.d, n_groups - slots, slots).time + 6700.0 / a.d <
+                0.95 * p.time)
+            a.wave_queries = slots * g.wq * g.qw;
+    } else {
+        slices = fullest_slices(n_groups, slots,
+                                std::min<int64_t>(max_slices, std::max<int64_t>(1, ceil_div(2 * slots, n_groups))));
+    }
     if (n_groups * max_slices <= slots) slices = max_slices;  // one stage each
     a.slice_rows = round_up(ceil_div(a.n, slices), g.rows);
     a.n_slices = (int)ceil_div(a.n, a.slice_rows);
@@ -932,7 +989,7 @@ int flat_smem_ok(const FlatScanArgs &a) {
     const size_t stage = nbx <= 2 ? (size_t)nbx * 128 * std::min(a.stride4 * 4, FS_BOX) * 4
                                   : (size_t)std::min(nbx, 8) * 32 * FS_BOX * 4;
     return per_warp * warps + 1024 + 3 * stage + 24 <= (size_t)dev_info().max_smem_optin &&
-           fs_geom(a.nq, a.k, a.stride4).smem <= (size_t)dev_info().max_smem_optin;
+           fs_geom(a.n, a.nq, a.k, a.stride4).smem <= (size_t)dev_info().max_smem_optin;
 }
 
 static int hamming_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) {
@@ -995,7 +1052,7 @@ int candidates_finish(const uint64_t *cand, const int *qcount, int64_t list_keys
 
 static int float_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) {
     if (!a.err) return fail(GN_ERR_INVALID, "float scan: no error word");
-    const FsGeom g = fs_geom(a.nq, a.k, a.stride4);
+    const FsGeom g = fs_geom(a.n, a.nq, a.k, a.stride4);
     // the rows as a TMA tensor: n rows x dp floats, boxes of 32 floats x the stage's rows, 128-byte swizzle
     CUtensorMap tm;
     GN_TRY(tmap_encode_2d(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, a.db, (uint64_t)a.stride4 * 4, (uint64_t)a.n,

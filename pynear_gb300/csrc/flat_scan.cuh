@@ -23,6 +23,7 @@ struct FlatScanArgs {
     int warps = 4, n_slices = 1, n_groups = 1;
     int64_t slice_rows = 0;
     int64_t units = 0, list_keys = 0, gbuf_keys = 0;  // float scan: CTAs, candidates per query, buffer keys
+    int64_t wave_queries = 0;  // float scan: queries better scanned on their own before the others (0: none)
 };
 
 constexpr int FLAT_MAX_K_WARP = 256;

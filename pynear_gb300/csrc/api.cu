@@ -322,6 +322,14 @@ int gn_flat_set(gn_index *ix, const void *data, int64_t n, int64_t dim) {
     return GN_OK;
 }
 
+// The plan and the scratch of a Hamming scan.
+static int ham_reserve(gn_index *ix, FlatScanArgs &a) {
+    flat_plan(a);
+    if (ham_ordered(a)) return ix->part.ensure(flat_part_bytes(a));
+    ham_plan(a);
+    return ix->part.ensure(ham_part_bytes(a));
+}
+
 // Shared search body.  queries/out are device pointers here; status: where a float
 // scan's last kernel writes the error word (pinned, may be null).
 static int flat_search_dev(gn_index *ix, const void *d_q, int64_t nq, int64_t k, int64_t *d_idx, void *d_dist,
@@ -357,10 +365,8 @@ static int flat_search_dev(gn_index *ix, const void *d_q, int64_t nq, int64_t k,
     if (ix->metric == M_HAMMING && ham_tc_wanted(ix, nq, k) && !captured()) {
         GN_TRY(error_word());
         const int rc = ham_tc_search(ix, d_q, nq, (int)k, d_idx, reinterpret_cast<int64_t *>(d_dist), a.err, st);
-        if (rc == GN_OK) {  // the scratch of the same search captured, which cannot allocate (if there is room)
-            ham_plan(a);
-            ix->part.ensure(ham_part_bytes(a));
-        }
+        // the scratch of the same search captured, which cannot allocate (if there is room)
+        if (rc == GN_OK) ham_reserve(ix, a);
         if (rc != GN_ERR_UNSUPPORTED) return rc;
     }
     if (ix->metric == M_L2 && l2_tc_wanted(ix, nq, k) && !captured()) {
@@ -373,9 +379,9 @@ static int flat_search_dev(gn_index *ix, const void *d_q, int64_t nq, int64_t k,
         flat_plan(a);
         if (!flat_smem_ok(a)) return fail(GN_ERR_UNSUPPORTED, "dimension too large for the exact flat scan");
         if (a.metric == M_HAMMING) {
-            ham_plan(a);
-            GN_TRY(ix->part.ensure(ham_part_bytes(a)));
-            GN_TRY(ham_launch(a, ix->part.as<uint64_t>(), st));
+            GN_TRY(ham_reserve(ix, a));
+            GN_TRY(ham_ordered(a) ? flat_launch(a, ix->part.as<uint64_t>(), st)
+                                  : ham_launch(a, ix->part.as<uint64_t>(), st));
             GN_CUDA_TRY(cudaGetLastError());
             return GN_OK;
         }

@@ -1172,6 +1172,27 @@ int ham_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) {
     return GN_OK;
 }
 
+// Hamming searches that keep ordered lists (flat_plan, flat_launch) rather than appended
+// candidates (ham_plan, ham_launch).  Whole searches in us, ordered / appended:
+//   k > 64 with many pairs to count: two queries a warp, all that the larger buffers leave
+//   room for, count slower than eight, the more so where rows are long, while the lists cost
+//   the same whatever the rows.  100k x 115 bytes, k 65: 1,000 queries 3357 / 1619, 5,000
+//   7393 / 8683, 14,000 15112 / 21181; k 100: 4268 / 1617, 9005 / 8705, 17105 / 21198; 500k x 64, 5,000
+//   queries, k 65: 13423 / 14312; k 200 there: 43550 / 14584;
+//   a handful of rows, or a few hundred for thousands of queries: little to leave out, and a
+//   launch less.  120 x 64, 18,000 queries, k 4: 133 / 158; 5 x 64, 2,000: 49 / 61 (k 20 over 120
+//   rows, 18,000 queries: 163 / 165);
+//   rows of so few bits that most distances are tied: 15,000 x 1, 90 queries, k 4: 64 / 77.
+bool ham_ordered(const FlatScanArgs &a) {
+    if (a.k > 64) {
+        const double work = (double)a.nq * (double)a.n * (double)(4 * a.stride4);
+        return work >= (a.stride4 > 4 ? 1.2e10 : 3.5e10) * (a.k / 65.0) * (a.k > 128 ? 3.0 : 1.0);
+    }
+    if (a.k > 8) return false;
+    const bool tied = a.d <= 2 && a.n >= (int64_t)2 << (8 * a.d);
+    return a.n <= 16 || (a.n <= 512 && a.nq >= 6000) || (tied && a.nq >= 24);
+}
+
 // Launch the k <= 256 path.  part: flat_part_bytes(a) scratch.
 int flat_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st) {
     return a.metric == M_HAMMING ? hamming_launch(a, part, st) : float_launch(a, part, st);

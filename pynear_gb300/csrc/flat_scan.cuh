@@ -37,7 +37,9 @@ void flat_plan(FlatScanArgs &a);
 size_t flat_part_bytes(const FlatScanArgs &a);
 int flat_smem_ok(const FlatScanArgs &a);
 int flat_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st);
-// Hamming with scratch of any size (flat_plan and flat_launch: a caller's, in slices).
+// Hamming with appended candidates, and the searches that keep ordered lists instead
+// (flat_plan and flat_launch, as do searches in a caller's scratch).
+bool ham_ordered(const FlatScanArgs &a);
 void ham_plan(FlatScanArgs &a);
 size_t ham_part_bytes(const FlatScanArgs &a);
 int ham_launch(const FlatScanArgs &a, uint64_t *part, cudaStream_t st);

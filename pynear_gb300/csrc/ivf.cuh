@@ -14,7 +14,6 @@ struct IvfScratch {
     DBuf q, qn, probes, probes64, pdist, bcnt, boff, bucket, fill, slot_rel, qcount, qslot, item_off, counter, part,
         cpart, nprobed, qbound,  // qbound: per query, the ordered score bound of the tensor-core list scan
         ckeys,                   // learned probing on the FP32 engine: nearest lists as keys
-        ccount, lbuf,            // FP32 scan: candidates per query (part holds them), the CTAs' list buffers
         mfeat, mcand, mcb, mqn;  // batched prober MLP: candidates' features, candidates, their bounds, |q|^2
 };
 

@@ -85,6 +85,36 @@ __device__ __forceinline__ bool kpp_last_block(unsigned *done) {
 }
 
 // ── float seeding ─────────────────────────────────────────────────────────
+// The reference's serial draw (KMeans.hpp:45-70), by one thread: the first row whose
+// running sum in double reaches u times the sum of all.  A chain of additions as long as
+// the rows; the values are loaded 16 ahead, or each would wait for its load too (344,491
+// rows: 46 ms, 25 so).
+__device__ __noinline__ int64_t kpp_serial(const float *min_sq, int64_t n, float u) {
+    constexpr int AHEAD = 16;
+    auto load = [&](int64_t i0, float (&v)[AHEAD]) {
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) v[i] = i0 + i < n ? __ldcg(min_sq + i0 + i) : 0.f;
+    };
+    float v[AHEAD];
+    double total = 0.0, sum = 0.0;
+    for (int64_t i0 = 0; i0 < n; i0 += AHEAD) {
+        load(i0, v);
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) total += (double)v[i];
+    }
+    const double target = (double)u * total;
+    for (int64_t i0 = 0; i0 < n; i0 += AHEAD) {
+        load(i0, v);
+        double at[AHEAD];
+#pragma unroll
+        for (int i = 0; i < AHEAD; ++i) at[i] = sum = sum + (double)v[i];
+        if (sum < target) continue;  // (the values are not negative: nor are the sums before)
+        for (int i = 0; i < AHEAD && i0 + i < n; ++i)
+            if (at[i] >= target) return i0 + i;
+    }
+    return n - 1;
+}
+
 // One launch per k-means++ draw, for rows past the SMs' shared memory (see
 // kpp_seed_kernel for the others): every block lowers its chunk's min_sq by the
 // distances to the newest centroid (row ci - 1 of C) and sums the chunk in
@@ -255,21 +285,7 @@ __global__ void __launch_bounds__(KPP_NT) kpp_kernel(const float *__restrict__ X
         s_amb = 1;  // r beyond every partial sum: the serial rule decides
     }
     __syncthreads();
-    if (s_amb && t == 0) {
-        double tot = 0.0;
-        for (int64_t i = 0; i < n; ++i) tot += (double)__ldcg(min_sq + i);
-        const double rr = (double)u * tot;
-        double c = 0.0;
-        int64_t ch = n - 1;
-        for (int64_t i = 0; i < n; ++i) {
-            c += (double)__ldcg(min_sq + i);
-            if (c >= rr) {
-                ch = i;
-                break;
-            }
-        }
-        s_chosen = (unsigned long long)ch;
-    }
+    if (s_amb && t == 0) s_chosen = (unsigned long long)kpp_serial(min_sq, n, u);
     __syncthreads();
     const int64_t ch = (int64_t)s_chosen;
     for (int j = t; j < dp; j += KPP_NT) C[ci * dp + j] = X[ch * dp + j];
@@ -585,19 +601,7 @@ __global__ void __launch_bounds__(SEED_NT, 1) kpp_seed_kernel(const float *__res
                         ok = ++polls < SEED_SPINS;
                     __threadfence();
                     if (ok) {
-                        double tot = 0.0;
-                        for (int64_t i = 0; i < n; ++i) tot += (double)__ldcg(min_sq + i);
-                        const double rr = (double)u[ci - 1] * tot;
-                        double c = 0.0;
-                        int64_t ch = n - 1;
-                        for (int64_t i = 0; i < n; ++i) {
-                            c += (double)__ldcg(min_sq + i);
-                            if (c >= rr) {
-                                ch = i;
-                                break;
-                            }
-                        }
-                        w = (unsigned long long)ci << SEED_TAG | (unsigned long long)ch;
+                        w = (unsigned long long)ci << SEED_TAG | (unsigned long long)kpp_serial(min_sq, n, u[ci - 1]);
                         seed_store(serial, w);
                     } else {
                         *reinterpret_cast<volatile int *>(err) = 1;
@@ -879,12 +883,14 @@ int kmeans_l2_device(const float *X, int64_t n, int d, int dp, int64_t k, int64_
     // kpp_seed_kernel launch where the rows fit the SMs' shared memory
     GN_CUDA_TRY(cudaMemcpyAsync(C, X + pick_point(rng) * dp, row_bytes, cudaMemcpyDeviceToDevice, st));
     DBuf dmin, dpart, ddone;
-    GN_TRY(dmin.ensure((size_t)n * sizeof(float)));
     const int64_t chunk = round_up(ceil_div(n, KPP_NT * KPP_SPAN), KPP_ROWS);
     const int P = (int)ceil_div(n, chunk);
-    GN_TRY(dpart.ensure((size_t)P * sizeof(double)));
-    GN_TRY(ddone.ensure(sizeof(unsigned)));
-    GN_CUDA_TRY(cudaMemsetAsync(ddone.p, 0, sizeof(unsigned), st));
+    if (k > 1) {
+        GN_TRY(dmin.ensure((size_t)n * sizeof(float)));
+        GN_TRY(dpart.ensure((size_t)P * sizeof(double)));
+        GN_TRY(ddone.ensure(sizeof(unsigned)));
+        GN_CUDA_TRY(cudaMemsetAsync(ddone.p, 0, sizeof(unsigned), st));
+    }
     std::vector<float> us((size_t)std::max<int64_t>(k - 1, 0));
     for (float &v : us) v = unif01(rng);
     const int G = dev_info().num_sms;

@@ -245,13 +245,14 @@ __global__ void __launch_bounds__(VR_NT) voronoi_kernel(const float2 *__restrict
         const int nsrc = listed ? m : ns;
 
         for (int wt = warp; wt < TX * TY; wt += VR_WARPS) {
-            const int wc = c0 + (wt % TX) * VR_SW, wr = r0 + (wt / TX) * VR_SH;
-            if (wc >= w || wr >= h) continue;
-            const int pc = wc + (lane & 3) * 4, pr = wr + (lane >> 2);
-            const float py = ys[min(pr, h - 1)];
+            const int oc = (wt % TX) * VR_SW, orow = (wt / TX) * VR_SH;
+            if (oc >= nc || orow >= nr) continue;
+            // (unsigned: the last tile's pixels may lie past the largest int)
+            const unsigned pc = (unsigned)(c0 + oc) + (lane & 3) * 4, pr = (unsigned)(r0 + orow) + (lane >> 2);
+            const float py = ys[min(pr, (unsigned)h - 1)];
             float px[4];
 #pragma unroll
-            for (int p = 0; p < 4; ++p) px[p] = xs[min(pc + p, w - 1)];
+            for (int p = 0; p < 4; ++p) px[p] = xs[min(pc + p, (unsigned)w - 1)];
             float a0 = fminf(fminf(px[0], px[1]), fminf(px[2], px[3])), b0 = py;
             float a1 = fmaxf(fmaxf(px[0], px[1]), fmaxf(px[2], px[3])), b1 = py;
 #pragma unroll
@@ -322,7 +323,8 @@ __global__ void __launch_bounds__(VR_NT) voronoi_kernel(const float2 *__restrict
             evaluate(cnt);
             __syncwarp();
 
-            if (pr < h) px4.store(pr, pc, w, ids, dist, palette, npal, rgba);
+            if (pr < (unsigned)h && pc < (unsigned)w)
+                px4.store((int)pr, (int)pc, w, ids, dist, palette, npal, rgba);
         }
     }
 }

@@ -79,10 +79,22 @@ int gn_flat_set(gn_index *ix, const void *data, int64_t n, int64_t dim);
  * Host-buffer searches (this one, gn_ivfl2_search_knn, gn_ivfbin_search_knn,
  * gn_tcflat_search_knn) block until the results are in the caller's buffers;
  * they accept pageable or page-locked memory (pageable buffers of up to 1 MB
- * are staged through the index's own page-locked buffers). */
+ * are staged through the index's own page-locked buffers).
+ * Large searches (Hamming: k <= 64, rows of at most 512 bytes, 128 queries or more; L2:
+ * k <= 32, 64 queries or more) take their candidates from the tensor cores, with the same
+ * results, and make a second copy of the rows for it: 8 bytes per packed byte
+ * (Hamming), 6 bytes per coordinate (L2).  It is made by the first of them or, where
+ * that one would not gain what the copy costs, by a later one; only where it takes no
+ * more than a quarter of the device memory free then; and it is kept until the next
+ * gn_flat_set.  With it the index keeps the scratch of its largest search: 160 MB of
+ * candidate buffers, the batch in that form, and its candidate lists (a few hundred MB
+ * for the largest batches). */
 int gn_flat_search_knn(gn_index *ix, const void *queries, int64_t nq, int64_t k, int64_t *out_idx, void *out_dist);
 /* 1-NN shortcut (VPTree::search1NN, pynear/include/VPTree.hpp:169-191) */
 int gn_flat_search_1nn(gn_index *ix, const void *queries, int64_t nq, int64_t *out_idx, void *out_dist);
+/* A search on a stream that is being captured reads only the rows themselves (no
+ * tensor cores), so that the graph stays valid for later sets of as many rows, and
+ * cannot allocate: make the same search once before the capture. */
 int gn_flat_search_knn_device(gn_index *ix, const void *d_queries, int64_t nq, int64_t k, int64_t *d_idx,
                               void *d_dist, void *stream);
 int gn_index_size(gn_index *ix, int64_t *n, int64_t *dim);

@@ -5,12 +5,13 @@
 // numbered slice-major so that the CTAs resident at the same time read the same
 // slice and share it through L2.
 //
-// Hamming: hamming_append_kernel for an index's searches; hamming_scan_kernel, whose
-// partial lists fit a caller's fixed scratch, for gn_hamming_knn_noalloc: each warp
-// owns QW queries, lane l scores row base+l against all of them (query words come
-// from shared memory as broadcasts), then offers the keys to the warp's register
-// top-k lists; each (query, slice) writes its sorted k keys to a partial buffer, and
-// flat_merge_kernel (flat_merge_split_kernel for small batches) reduces the slices.
+// Hamming: hamming_append_kernel for most of an index's searches.  hamming_scan_kernel
+// for those of ham_ordered, and for gn_hamming_knn_noalloc, whose partial lists have to
+// fit a fixed scratch: each warp owns QW queries, lane l scores row base+l against all
+// of them (query words come from shared memory as broadcasts), then offers the keys to
+// the warp's register top-k lists; each (query, slice) writes its sorted k keys to a
+// partial buffer, and flat_merge_kernel (flat_merge_split_kernel for small batches)
+// reduces the slices.
 // Float: see float_scan_kernel.  Large batches of either go to the tensor cores
 // instead (tc_scan.cu).
 //

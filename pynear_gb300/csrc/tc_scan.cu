@@ -12,7 +12,8 @@
 //   warp 0     TMA producer: the unit's queries once (where their K fits shared
 //              memory: "resident"), then 256-row, 128-byte K slices of the
 //              database into a ring (otherwise a query slice rides along), and
-//              the rows' norms into a ring of their own;
+//              the rows' norms into a ring of their own (whose slots the epilogue
+//              gives back behind a fence: mbar_release_warp);
 //   warp 1     allocates 512 TMEM columns, one thread issues tcgen05.mma
 //              (M=128, N=256) into one of two 256-column accumulators, query
 //              tile by query tile for each database tile;
@@ -29,7 +30,8 @@
 // What makes passing scores rare is the bound that every unit starts from.
 // With a warp's 32 lanes being 32 queries, a block of 32 x 32 scores is only
 // cheap when none of 1,024 passes.  So a pilot launch of the same pipeline first
-// scores every 8th row or so and keeps, per query, only the minima of groups
+// scores every 8th row or so (all rows of a small database; none where the buffers
+// hold them all) and keeps, per query, only the minima of groups
 // of rows (32 per unit, one per column of a block: no insertion, no branch).
 // The S-th smallest minimum over at least S groups is a score that at least S
 // rows reach, hence an upper bound of the query's S-th best score, and close
@@ -1084,8 +1086,8 @@ int l2_tc_search(gn_index *ix, const float *d_q, int64_t nq, int k, int64_t *d_i
         size_t free_b = 0, total_b = 0;
         const size_t want = (size_t)ix->n * K * 2, np = (size_t)round_up(ix->n, TC_N);
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || want > free_b / 4 || H.x16.ensure(want) != GN_OK ||
-            H.xnorm.ensure(np * 4) != GN_OK || H.pnorm.ensure(tc_pilot_count(ix->n) * 4) != GN_OK || H.xmax2.ensure(4) != GN_OK || H.flag.ensure(4) != GN_OK ||
-            H.hflag.ensure(4) != GN_OK) {
+            H.xnorm.ensure(np * 4) != GN_OK || H.pnorm.ensure(tc_pilot_count(ix->n) * 4) != GN_OK ||
+            H.xmax2.ensure(4) != GN_OK || H.flag.ensure(4) != GN_OK || H.hflag.ensure(4) != GN_OK) {
             cudaGetLastError();
             H.refused = true;  // until the next set()
             return GN_ERR_UNSUPPORTED;

@@ -25,6 +25,9 @@
 // whatever is left out, NaN seeds never win, and an infinite pixel coordinate
 // makes min ub infinite, which keeps every seed.
 //
+// A handful of seeds is not worth the bounds: voronoi_few_kernel evaluates all of
+// them for four neighbouring pixels a thread.
+//
 // Block list: up to VR_CAP surviving seeds in shared memory; where more
 // survive (seeds crowded together), the warps read all seeds instead.  A warp
 // collects its own survivors VR_WCAP at a time and evaluates four seeds for
